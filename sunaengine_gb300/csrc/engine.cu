@@ -425,7 +425,7 @@ struct World {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
     void* ptrs[] = {b.state, b.stacc, b.predSlot, b.sceneOf, b.keys, b.inv, b.bond, b.bondCand, b.skey,
-                    b.sslot, b.cellStart, b.PL, b.PL2, b.RX, b.NQ, b.POS, b.SCN, b.DP, b.HEAT, b.CORR, b.NBR,
+                    b.sslot, b.cellStart, recBuf, b.RX, b.NQ, b.POS, b.SCN, b.DP, b.HEAT, b.CORR, b.NBR,
                     b.NBRL, b.NBRN, (void*)b.tiles, b.TR, b.OVF, b.CB,
                     (void*)b.luts, (void*)b.WG, (void*)b.CA, (void*)b.mats, (void*)b.rcp,
                     b.scenes, b.world, b.acc, b.accLast, b.chain, b.dbg, b.err, b.work, tmpK, tmpV, hist,
@@ -493,8 +493,8 @@ struct World {
     b.bondCand = dalloc<uint32_t>(C * BOND_CAP, err);
     b.skey = dalloc<uint32_t>(C, err);
     b.sslot = dalloc<uint32_t>(C, err);
-    b.PL = dalloc<int4>(C, err);
-    b.PL2 = dalloc<int4>(C, err);
+    recBuf = b.PL = dalloc<int4>(2 * C, err);
+    b.PL2 = b.PL + C;
     b.RX = dalloc<int4>(C, err);
     b.NQ = dalloc<int4>(C, err);
     b.POS = dalloc<int2>(C, err);
@@ -1011,17 +1011,9 @@ struct World {
       return;
     }
     const int g = grid_occ((const void*)k_colour<DBG, L>, (uint64_t)hw.nAct * L / 4 + 256);
-    for (int c = 0; c < 4; ++c) {
-      const int4* src = (c & 1) ? b.PL2 : b.PL;
-      int4* dst = (c & 1) ? b.PL : b.PL2;
-      cudaEventRecord(evFork, st);
-      cudaStreamWaitEvent(st2, evFork, 0);
-      k_colour_copy<<<2 * numSMs, 256, 0, st2>>>(b, c, src, dst);
-      cudaEventRecord(evJoin, st2);
-      k_colour<DBG, L><<<g, 256, 0, st>>>(b, c, src, dst, 0);
-      cudaStreamWaitEvent(st, evJoin, 0);
-    }
+    for (int c = 0; c < 4; ++c) k_colour<DBG, L><<<g, 256, 0, st>>>(b, c);
   }
+  int4* recBuf = nullptr;  // both record buffers (b.PL, b.PL2)
   // One cooperative launch of every solver iteration (k_iters_persistent):
   // the grid is exactly the resident capacity, which the cooperative launch
   // guarantees to run at once (its grid barriers need every CTA resident).
@@ -1104,6 +1096,10 @@ struct World {
     radix::sort_pairs(b.keys, hw.slotEnd, bits, b.skey, b.sslot, tmpK, tmpV, hist, st);
     Lc += (uint64_t)radix::LAUNCHES_PER_PASS * ((bits + radix::RBITS - 1) / radix::RBITS);
     mark();
+    // each iteration of the colour-major sweep leaves the current records in
+    // the other buffer: an odd count starts in PL2, so every one ends in PL
+    // (b is passed to each launch by value)
+    if (!staged && (iters & 1u)) swap_records(b);
     // the cell ranges (from the sorted keys) and the gather (from the sorted
     // slots) share no word: the ranges run on the side branch
     cudaEventRecord(evFork, st);
@@ -1127,6 +1123,7 @@ struct World {
     const bool persist = persistent && !staged && nB == 0 && pev == nullptr;
     if (persist) {
       SN_LANES(lc.c, (launch_persistent<DBG, L_>()));
+      if (iters & 1u) swap_records(b);
       Lc += 1;
     }
     for (uint32_t it = 0; it < (persist ? 0u : iters); ++it) {
@@ -1134,8 +1131,9 @@ struct World {
       SN_LANES(lc.a, (launch_solveA<DBG, L_>(last)));
       mark();
       SN_LANES(lc.c, (launch_colours<DBG, L_>()));
+      if (!staged) swap_records(b);
       mark();
-      Lc += staged ? 5 : 9;
+      Lc += 5;
       if (hasFriction) {
         SN_LANES(lc.c, (launch_friction<DBG, L_>()));
         k_apply_fric<DBG><<<ga, 256, 0, st>>>(b);

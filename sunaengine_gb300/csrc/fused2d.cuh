@@ -1,0 +1,416 @@
+// The whole 2D substep of a small world as one cooperative launch.
+//
+// A world of a few thousand particles spends its substep between kernels: 51
+// dependent launches of 1-3 us of work each took 167 us at 4,096 particles.
+// Here one CTA per SM runs every phase of sim2d.cuh, the phases separated by
+// grid barriers, and what a phase hands to itself in the next one stays on the
+// SM:
+//
+//   * each CTA owns an equal share of every colour class (its particles are
+//     contiguous in sorted space, colour by colour), and keeps their neighbour
+//     lists, records and wall bounds in shared memory through all iterations,
+//     with the kernel tables: what is left on a phase's critical path is one
+//     load of the neighbours' records;
+//   * the grid is a counting sort over the cells: the cell counts fit every
+//     CTA, so each scans them by itself (no phase of its own, and the cell
+//     ranges the list build needs are in shared memory). Arrival order inside
+//     a cell is whatever the count's atomics gave; each particle then ranks
+//     itself among its cell's slots, which puts the cell into ascending slot
+//     order, the canonical order the radix sort of the large path gives;
+//   * the last CTA to finish folds the chain.
+//
+// The sums are those of the per-phase kernels (the same device functions), so
+// the results are equal word by word. Every wait is bounded (grid_wait).
+#pragma once
+#include "rigid.cuh"
+
+namespace sn {
+namespace d2 {
+
+constexpr int FU_T = 1024;
+constexpr uint32_t FU_ROW = 52;  // words per list row: 8 lanes of 4 rows, or 4 of 8, fall on different banks
+constexpr uint32_t FU_OWN_BYTES = 16 + 8 + 4 + 4 + 4 * FU_ROW;
+
+struct FusedPar {
+  uint32_t iters, friction, bonds, seal, chain;
+  uint32_t slots;    // slots that can be active: [0, slots)
+  uint32_t xWords;   // shared words for the cell ranges, then the CA table
+  uint32_t ownCap;   // particles a CTA can own
+  uint32_t* count;   // [K] cell counts, zero between launches
+  uint32_t* tmp;     // slots by cell in arrival order
+  uint32_t* bar;     // [2] barrier arrivals and finished CTAs, zero between launches
+};
+
+// Grid barrier of a cooperative launch: `target` counts the arrivals every CTA
+// waits for (monotonic over the launch). A CTA that waits longer than
+// BARRIER_WAIT_CYCLES raises ERR_BARRIER; false sends the whole CTA out.
+__device__ __forceinline__ bool grid_wait(uint32_t* bar, uint32_t* err, uint32_t& target) {
+  __syncthreads();
+  int bad = 0;
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    const long long t0 = clock64();
+    for (;;) {
+      uint32_t v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if ((int32_t)(v - target) >= 0) break;
+      if (clock64() - t0 > BARRIER_WAIT_CYCLES) {
+        atomicOr(err, ERR_BARRIER);
+        bad = 1;
+        break;
+      }
+    }
+  }
+  return __syncthreads_or(bad) == 0;
+}
+
+// Neighbour access of an owned particle: its list row and the kernel tables in
+// shared memory, records in the current buffer (or, in a colour pass, split as
+// NbrSplit does).
+struct NbrOwned {
+  const int4* g;
+  const uint32_t* rows;
+  const int2* swg;
+  const int2* sca;
+  uint32_t cut, off;
+  __device__ __forceinline__ uint32_t entry(uint32_t row, uint32_t k) const { return rows[row * FU_ROW + k]; }
+  __device__ __forceinline__ int4 rec(uint32_t e) const {
+    const uint32_t q = e & ~NBR_BOUNDARY;
+    return g[(int32_t)(q < cut ? q + off : q)];
+  }
+  __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e & ~NBR_BOUNDARY); }
+  __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBR_BOUNDARY) != 0u; }
+  __device__ __forceinline__ int2 wg(const Bufs&, int id) const { return swg[id]; }
+  __device__ __forceinline__ int2 ca(const Bufs&, int id) const { return sca[id]; }
+};
+
+// Exclusive prefix of x[0, n) in place by the whole CTA, the total in x[n];
+// returns the largest element (to every thread).
+__device__ __forceinline__ uint32_t cta_scan(uint32_t* x, uint32_t n, uint32_t* ws) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t per = (n + FU_T - 1) / FU_T, lo = min(tid * per, n), hi = min(lo + per, n);
+  uint32_t sum = 0, most = 0;
+  for (uint32_t k = lo; k < hi; ++k) {
+    sum += x[k];
+    most = max(most, x[k]);
+  }
+  uint32_t inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += v;
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 31) ws[warp] = inc;
+  if (lane == 0) ws[32 + warp] = most;
+  __syncthreads();
+  uint32_t run = inc - sum;
+  for (uint32_t w = 0; w < warp; ++w) run += ws[w];
+  for (uint32_t k = lo; k < hi; ++k) {
+    const uint32_t v = x[k];
+    x[k] = run;
+    run += v;
+  }
+  if (tid == FU_T - 1) x[n] = run;
+  most = __reduce_max_sync(0xffffffffu, ws[32 + lane]);
+  __syncthreads();
+  return most;
+}
+
+// L lanes share a particle's list in the sweeps over every owned particle, LC
+// in the colour passes (a quarter of the particles each).
+template <int L, int LC>
+__global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
+  extern __shared__ int4 dyn[];
+  int4* rec = dyn;                                              // [ownCap] records
+  int2* wall = reinterpret_cast<int2*>(rec + P.ownCap);         // [ownCap] domain - WALL
+  int2* swg = wall + P.ownCap;                                  // [TN]
+  uint32_t* X = reinterpret_cast<uint32_t*>(swg + TN);          // [xWords]
+  uint32_t* pOf = X + P.xWords;                                 // [ownCap] sorted index
+  uint32_t* word = pOf + P.ownCap;                              // [ownCap] NBRN words
+  uint32_t* rows = word + P.ownCap;                             // [ownCap][FU_ROW]
+  __shared__ uint32_t ws[64];
+  __shared__ int4 smat1[MAT_MAX], smat2[MAT_MAX];
+  __shared__ int2 scol[MAT_MAX];  // {eps, dpMax}
+  __shared__ uint32_t dsacc[8], dsscene, lastCta;
+  const Flags<false> f{b.dbg};
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, G = gridDim.x, cta = blockIdx.x;
+  const uint32_t K = b.world->K;
+  uint32_t target = 0;
+
+  // ---- predict and cell counts: one slot per thread, warps dealt round the CTAs
+  if (cta == 0 && tid < 8 && tid != 4) b.work[tid] = 0u;
+  const uint32_t slot = ((tid >> 5) * G + cta) * 32u + lane;
+  bool on = false;
+  uint32_t sc = 0, key = 0, arrival = 0, info = 0;
+  int2 pos = make_int2(0, 0), pred = pos;
+  int32_t temp = 0;
+  if (slot < P.slots) {
+    sc = b.sceneOf[slot];
+    const ScenePar& S = b.scenes[sc];
+    const uint32_t i = slot - S.slotBase;
+    on = S.active && i < S.n;
+    if (on) {
+      if (i == 0) b.scenes[sc].formNow = form_now(S);
+      const int4* w4 = reinterpret_cast<const int4*>(b.state + (size_t)slot * 8);
+      const int4 a = w4[0], c = w4[1];
+      pos = make_int2(a.x, a.y);
+      temp = c.z;
+      info = info_of((uint32_t)c.x, (uint32_t)c.y, i >= S.nFluid);
+      pred = predict_pos(b, S, slot, i, a, c, f);
+      const int2 cc = cell_coord(S, pred);
+      key = key_of(S, cc.x, cc.y);
+      arrival = atomicAdd(P.count + key, 1u);
+    }
+  }
+  for (uint32_t k = tid; k < (uint32_t)TN; k += FU_T) swg[k] = __ldg(b.WG + k);
+  post1_mats(b, smat1);
+  post2_mats(b, smat2);
+  if (tid < (uint32_t)MAT_MAX) scol[tid] = make_int2(matw(b, tid, M_eps), matw(b, tid, M_dpMax));
+  if (!grid_wait(P.bar, b.err, target)) return;
+
+  // ---- cell ranges (every CTA its own copy), slots to their cells
+  for (uint32_t k = tid; k < K; k += FU_T) X[k] = __ldcg(P.count + k);
+  __syncthreads();
+  const bool crowded = cta_scan(X, K, ws) > CELL_BIG;
+  for (uint32_t k = cta * FU_T + tid; k <= K; k += G * FU_T) b.cellStart[k] = X[k];
+  if (on) P.tmp[X[key] + arrival] = slot;
+  if (!grid_wait(P.bar, b.err, target)) return;
+
+  // ---- canonical order inside the cell, working set into sorted space
+  for (uint32_t k = cta * FU_T + tid; k < K; k += G * FU_T) P.count[k] = 0u;
+  if (on) {
+    const uint32_t lo = X[key], hi = X[key + 1];
+    uint32_t p = lo;
+    for (uint32_t q = lo; q < hi; ++q) p += P.tmp[q] < slot ? 1u : 0u;
+    const int4 r = make_int4(pred.x, pred.y, 0, (int32_t)info);
+    b.PL[p] = r;
+    if (info & INFO_BOUNDARY) b.PL2[p] = r;
+    b.RX[p] = make_int4(0, 0, temp, 0);
+    b.POS[p] = pos;
+    b.SCN[p] = sc;
+    b.inv[slot] = p;
+    b.sslot[p] = slot;
+    gather_flags(b, b.scenes[sc], info);
+    // containStress has work: a held fluid particle
+    raise_work(b, 6, !(info & INFO_BOUNDARY) && (info & INFO_PINNED));
+  }
+  if (!grid_wait(P.bar, b.err, target)) return;
+
+  // ---- the owned share of each colour class
+  uint32_t own[5], first[4], lo4[4];
+  own[0] = 0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    lo4[c] = X[b.world->colourBase[c]];
+    const uint32_t n = X[b.world->colourBase[c + 1]] - lo4[c], per = (n + G - 1) / G;
+    const uint32_t s0 = min(cta * per, n), e0 = min(s0 + per, n);
+    first[c] = lo4[c] + s0;
+    own[c + 1] = own[c] + (e0 - s0);
+  }
+  for (uint32_t i = tid; i < own[4]; i += FU_T) {
+    const uint32_t p = i < own[1]   ? first[0] + i
+                       : i < own[2] ? first[1] + (i - own[1])
+                       : i < own[3] ? first[2] + (i - own[2])
+                                    : first[3] + (i - own[3]);
+    pOf[i] = p;
+    rec[i] = b.PL[p];
+    const ScenePar& S = b.scenes[b.SCN[p]];
+    wall[i] = make_int2(S.domW - WALL, S.domH - WALL);
+  }
+  // pred boxes of crowded cells (k_cellbox), one warp per cell
+  if (crowded) {
+    for (uint32_t k = (tid >> 5) * G + cta; k < K; k += G * (FU_T / 32)) {
+      const uint32_t lo = X[k], hi = X[k + 1];
+      if (hi - lo <= CELL_BIG) continue;
+      int4 box = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
+      for (uint32_t q = lo + lane; q < hi; q += 32) {
+        const int2 pq = ld_pred(b.PL, q);
+        box = make_int4(min(box.x, pq.x), min(box.y, pq.y), max(box.z, pq.x), max(box.w, pq.y));
+      }
+      box.x = __reduce_min_sync(0xffffffffu, box.x);
+      box.y = __reduce_min_sync(0xffffffffu, box.y);
+      box.z = __reduce_max_sync(0xffffffffu, box.z);
+      box.w = __reduce_max_sync(0xffffffffu, box.w);
+      if (lane == 0) b.CB[k] = box;
+    }
+    if (!grid_wait(P.bar, b.err, target)) return;
+  }
+  __syncthreads();
+
+  // ---- neighbour lists
+  const uint32_t sub = tid & (L - 1);
+  const bool cutLists = *(volatile uint32_t*)(b.work + 1) == 0u;
+  for (uint32_t i = tid / L;; i += FU_T / L) {
+    if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;  // warp-uniform exit
+    const bool valid = i < own[4];
+    const uint32_t r = valid ? i : 0u, p = pOf[r];
+    const uint32_t w = nbr_lanes<false, L, false>(
+        b, X, cutLists, valid, p, rec[r],
+        [&](uint32_t at, uint32_t q, uint32_t iq, uint32_t) { rows[r * FU_ROW + at] = q | (iq & INFO_BOUNDARY); }, f);
+    if (valid && sub == 0) {
+      word[r] = w;
+      b.NBRN[p] = w;
+    }
+  }
+  __syncthreads();
+  int2* sca = reinterpret_cast<int2*>(X);  // the cell ranges are not read again
+  for (uint32_t k = tid; k < (uint32_t)TN; k += FU_T) sca[k] = __ldg(b.CA + k);
+
+  // ---- solver iterations
+  const int32_t W0 = swg[0].x;  // the tables' first entry: luts[0]
+  const bool fric = P.friction && *(volatile uint32_t*)b.work != 0u;
+  for (uint32_t it = 0; it < P.iters; ++it) {
+    const bool last = it + 1 == P.iters;
+    NbrOwned nb{b.PL, rows, swg, sca, 0u, (uint32_t)(b.PL2 - b.PL)};
+    for (uint32_t i = tid / L;; i += FU_T / L) {
+      if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+      const bool valid = i < own[4];
+      const uint32_t r = valid ? i : 0u;
+      const int4 me = rec[r];
+      const bool act = valid && !((uint32_t)me.w & INFO_BOUNDARY);
+      const uint32_t cnt = act ? (word[r] & NBRN_COUNT) : 0u;
+      int32_t rho = 0, S = 0, sgx = 0, sgy = 0;
+      solveA_sums<false, L>(b, nb, r, cnt, sub, xy(me), f, rho, S, sgx, sgy);
+      if (!act || sub != 0) continue;
+      int32_t rinv;
+      const int32_t lam =
+          solveA_lambda(b, scol[(uint32_t)me.w & INFO_MAT].x, W0, rho, S, sgx, sgy, last, rinv, f);
+      const uint32_t p = pOf[r];
+      rec[r].z = lam;
+      b.PL[p].z = lam;
+      b.RX[p].x = rho;
+      if (last) b.RX[p].y = rinv;
+    }
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      if (!grid_wait(P.bar, b.err, target)) return;
+      nb.cut = c == 0 ? lo4[0] : c == 1 ? lo4[1] : c == 2 ? lo4[2] : lo4[3];
+      const uint32_t i0 = c == 0 ? own[0] : c == 1 ? own[1] : c == 2 ? own[2] : own[3];
+      const uint32_t i1 = c == 0 ? own[1] : c == 1 ? own[2] : c == 2 ? own[3] : own[4];
+      const uint32_t subC = tid & (LC - 1);
+      for (uint32_t i = i0 + tid / LC;; i += FU_T / LC) {
+        if (__shfl_sync(0xffffffffu, i, 0) >= i1) break;
+        const bool valid = i < i1;
+        const uint32_t r = valid ? i : i0;
+        int4 me = rec[r];
+        const uint32_t inf = (uint32_t)me.w;
+        const bool act = valid && !(inf & INFO_BOUNDARY);
+        const uint32_t cnt = act ? (word[r] & NBRN_COUNT) : 0u;
+        const int2 dp = solveB_dp<false, LC, false>(b, nb, r, cnt, subC, xy(me), me.z, f);
+        if (!act || subC != 0) continue;
+        if (!(inf & INFO_PINNED)) {
+          const int2 pr = apply_dp_in(scol[inf & INFO_MAT].y, wall[r], xy(me), dp, f);
+          me.x = pr.x;
+          me.y = pr.y;
+          rec[r] = me;
+        }
+        b.PL2[pOf[r]] = me;
+      }
+    }
+    swap_records(b);
+    if (!grid_wait(P.bar, b.err, target)) return;
+    if (fric) {
+      const NbrOwned nf{b.PL, rows, swg, sca, 0u, 0u};
+      for (uint32_t i = tid / L;; i += FU_T / L) {
+        if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+        const bool valid = i < own[4];
+        const uint32_t r = valid ? i : 0u;
+        friction_particle<false, L>(b, nf, valid, pOf[r], r, sub, f);
+      }
+      if (!grid_wait(P.bar, b.err, target)) return;
+      for (uint32_t i = tid; i < own[4]; i += FU_T) {
+        int4 me = rec[i];
+        const uint32_t inf = (uint32_t)me.w, m = inf & INFO_MAT;
+        if ((inf & (INFO_BOUNDARY | INFO_PINNED)) || !friction_row(b, m)) continue;
+        const uint32_t p = pOf[i];
+        const int2 pr = apply_dp_in(scol[m].y, wall[i], xy(me), b.DP[p], f);
+        me.x = pr.x;
+        me.y = pr.y;
+        rec[i] = me;
+        b.PL[p] = me;
+      }
+      if (!grid_wait(P.bar, b.err, target)) return;
+    }
+  }
+
+  // ---- containment, then the post sweeps
+  const NbrOwned nb{b.PL, rows, swg, sca, 0u, 0u};
+  if (P.seal && !cutLists) {
+    for (uint32_t i = tid; i < own[4]; i += FU_T) contain_particle(b, nb, pOf[i], i, f);
+    if (!grid_wait(P.bar, b.err, target)) return;
+  }
+  for (uint32_t i = tid / L;; i += FU_T / L) {
+    if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+    const bool valid = i < own[4];
+    const uint32_t r = valid ? i : 0u;
+    post1_particle<false, L>(b, nb, smat1, valid, pOf[r], r, sub, f);
+  }
+  if (!grid_wait(P.bar, b.err, target)) return;
+  for (uint32_t i = tid / L;; i += FU_T / L) {
+    if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+    const bool valid = i < own[4];
+    const uint32_t r = valid ? i : 0u, p = pOf[r];
+    bool act;
+    const int2 a2 = post2_sums<false, L>(b, nb, smat2, valid, p, r, sub, act, f);
+    if (act && sub == 0) {
+      const uint32_t sl = b.sslot[p];
+      const ScenePar& S = b.scenes[b.SCN[p]];
+      post2_finish(b, S, p, sl, sl - S.slotBase, a2, !P.bonds, b.state + (size_t)sl * 8, f);
+    }
+  }
+  if (P.seal && *(volatile uint32_t*)(b.work + 6) != 0u) {
+    if (!grid_wait(P.bar, b.err, target)) return;
+    for (uint32_t i = tid / L;; i += FU_T / L) {
+      if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+      const bool valid = i < own[4];
+      const uint32_t r = valid ? i : 0u;
+      contain_stress_slot<false, L>(b, nb, valid, b.sslot[pOf[r]], r, sub, f);
+    }
+  }
+  if (P.bonds && *(volatile uint32_t*)(b.work + 5) != 0u) {
+    if (!grid_wait(P.bar, b.err, target)) return;
+    for (uint32_t i = tid; i < own[4]; i += FU_T) form1_particle(b, nb, pOf[i], i, f);
+    if (!grid_wait(P.bar, b.err, target)) return;
+    const bool live = *(volatile uint32_t*)(b.work + 4) != 0u;
+    for (uint32_t i = tid; i < own[4]; i += FU_T) {
+      const uint32_t sl = b.sslot[pOf[i]];
+      const ScenePar& S = b.scenes[b.SCN[pOf[i]]];
+      if (sl - S.slotBase < S.nFluid && S.formNow) form2_slot(b, S, sl, sl - S.slotBase, live);
+    }
+  }
+
+  // ---- digest and chain
+  __syncthreads();
+  if (P.chain) {
+    digest_block_begin(dsacc, &dsscene);
+    const bool live = P.bonds && *(volatile uint32_t*)(b.work + 4) != 0u;
+    for (uint32_t i0 = 0; i0 < own[4]; i0 += FU_T) {
+      const bool valid = i0 + tid < own[4];
+      uint32_t s = 0, h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (valid) {
+        const uint32_t p = pOf[i0 + tid], sl = b.sslot[p];
+        s = b.SCN[p];
+        const uint32_t idx = sl - b.scenes[s].slotBase;
+        const bool fluid = !((uint32_t)rec[i0 + tid].w & INFO_BOUNDARY);
+        particle_digest(b.state + (size_t)sl * 8, idx, live && fluid ? b.bond + (size_t)sl * BOND_CAP : nullptr, h);
+      }
+      digest_add_block(b.acc, dsacc, &dsscene, valid, s, h);
+    }
+    digest_block_end(b.acc, dsacc, &dsscene);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    lastCta = atomicAdd(P.bar + 1, 1u) == G - 1 ? 1u : 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!lastCta) return;
+  for (uint32_t s = tid; s < b.world->numScenes; s += FU_T) fold_scene(b, s, P.chain != 0u);
+  if (tid < 2) P.bar[tid] = 0u;
+}
+
+}  // namespace d2
+}  // namespace sn

@@ -391,7 +391,6 @@ __global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal)
     const uint32_t p = b.inv[slot];
     const int2 pr = rg_at(qx, qy, c, s, b.rest[slot], f);
     *reinterpret_cast<int2*>(b.PL + p) = pr;
-    *reinterpret_cast<int2*>(b.PL2 + p) = pr;
   }
 }
 

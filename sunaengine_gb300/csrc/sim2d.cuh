@@ -11,9 +11,8 @@
 //   k_nbr           neighbour lists, reference traversal order and MAXNBR cut
 //   ITERS x { k_solveA; k_colour x 4; [k_friction; k_apply_fric] }
 //                   density/lambda, then colour-classed Gauss-Seidel position
-//                   correction; solveB and applyDp are fused per colour over a
-//                   double-buffered pred (see k_colour), each pass's copy of
-//                   the other colours (k_colour_copy) on a side branch beside it
+//                   correction; solveB and applyDp are fused per colour over
+//                   two record buffers (see NbrSplit)
 //   k_contain       containment of intruders (when a seal particle is live)
 //   k_post1         finalize + xsph + normals + conduct in one neighbour sweep
 //   k_post2         surfaceTension + thermal + formation flag clear + state hash
@@ -124,8 +123,8 @@ struct Bufs {
   uint32_t* sslot;      // [cap]
   uint32_t* cellStart;  // [K + 1]
   // sorted space
-  int4* PL;             // {pred.x, pred.y, lam, info}  (buffer A)
-  int4* PL2;            // buffer B of the colour sweep (same layout)
+  int4* PL;             // {pred.x, pred.y, lam, info}: the current records
+  int4* PL2;            // the other buffer of the colour sweep (one allocation with PL)
   int4* RX;             // {rho, rinv, temp, 0}
   int4* NQ;             // {nrm.x, nrm.y, rho, 0}
   int2* POS;
@@ -353,7 +352,29 @@ __device__ __forceinline__ int2 jet_accel(const ScenePar& S, int2 p, const Flags
   return a;
 }
 
-// predict (src/sim.wgsl:958-1000) + the grid key of every slot.
+// predict (src/sim.wgsl:958-1000) of one particle: slot `slot`, scene index i,
+// state words a, c.
+template <bool DBG>
+__device__ __forceinline__ int2 predict_pos(const Bufs& b, const ScenePar& S, uint32_t slot, uint32_t i, int4 a,
+                                            int4 c, const Flags<DBG>& f) {
+  const int2 pos = make_int2(a.x, a.y);
+  if (i >= S.nFluid) return pos;
+  const uint32_t m = (uint32_t)c.x, fl = (uint32_t)c.y;
+  if (matw(b, m, M_phantom) != 0 || (fl & (FLAG_ANCHOR | FLAG_RIGID))) return pos;
+  const int2 st = b.stacc[slot];
+  const int32_t vmax = S.vmax, vmaxN = neg_sat(vmax, f);
+  const int2 jf = jet_accel(S, pos, f);
+  int32_t vx = add_sat(add_sat(a.z, st.x, f), jf.x, f);
+  int32_t vy = add_sat(add_sat(add_sat(a.w, st.y, f), matw(b, m, M_grav), f), jf.y, f);
+  vx = clampi(vx, vmaxN, vmax);
+  vy = clampi(vy, vmaxN, vmax);
+  return wall_clamp(S, make_int2(add_sat(pos.x, vx, f), add_sat(pos.y, vy, f)));
+}
+__device__ __forceinline__ uint32_t form_now(const ScenePar& S) {
+  return ((S.formClock & 3u) == 0u || S.bondDirty) ? 1u : 0u;
+}
+
+// predict + the grid key of every slot.
 template <bool DBG>
 __global__ void __launch_bounds__(256) k_predict_key(Bufs b) {
   Flags<DBG> f{b.dbg};
@@ -370,24 +391,9 @@ __global__ void __launch_bounds__(256) k_predict_key(Bufs b) {
     const ScenePar& S = b.scenes[s];
     uint32_t i = slot - S.slotBase;
     if (!S.active || i >= S.n) { b.keys[slot] = K; continue; }
-    if (i == 0) b.scenes[s].formNow = ((S.formClock & 3u) == 0u || S.bondDirty) ? 1u : 0u;
+    if (i == 0) b.scenes[s].formNow = form_now(S);
     const int4* w4 = reinterpret_cast<const int4*>(b.state + (size_t)slot * 8);
-    int4 a = w4[0], c = w4[1];
-    int2 pos = make_int2(a.x, a.y);
-    int2 pred = pos;
-    if (i < S.nFluid) {
-      uint32_t m = (uint32_t)c.x, fl = (uint32_t)c.y;
-      if (matw(b, m, M_phantom) == 0 && !(fl & (FLAG_ANCHOR | FLAG_RIGID))) {
-        int2 st = b.stacc[slot];
-        int32_t vmax = S.vmax, vmaxN = neg_sat(vmax, f);
-        const int2 jf = jet_accel(S, pos, f);
-        int32_t vx = add_sat(add_sat(a.z, st.x, f), jf.x, f);
-        int32_t vy = add_sat(add_sat(add_sat(a.w, st.y, f), matw(b, m, M_grav), f), jf.y, f);
-        vx = clampi(vx, vmaxN, vmax);
-        vy = clampi(vy, vmaxN, vmax);
-        pred = wall_clamp(S, make_int2(add_sat(pos.x, vx, f), add_sat(pos.y, vy, f)));
-      }
-    }
+    const int2 pred = predict_pos(b, S, slot, i, w4[0], w4[1], f);
     b.predSlot[slot] = pred;
     int2 cc = cell_coord(S, pred);
     b.keys[slot] = key_of(S, cc.x, cc.y);
@@ -397,6 +403,23 @@ __global__ void __launch_bounds__(256) k_predict_key(Bufs b) {
 // cellStart[k] = first sorted position whose key is >= k, for k in [0, K].
 __global__ void __launch_bounds__(256) k_cellstart(Bufs b) {
   cell_starts(b.skey, b.world->slotEnd, b.world->K, b.cellStart);
+}
+
+// The per-substep world flags one particle raises (see Bufs::work): some lanes
+// of the warp may be absent.
+__device__ __forceinline__ void raise_work(const Bufs& b, int k, bool raise) {
+  const unsigned bal = __ballot_sync(__activemask(), raise);
+  if (raise && (threadIdx.x & 31u) == (unsigned)(__ffs(bal) - 1) && *(volatile uint32_t*)(b.work + k) == 0u)
+    atomicOr(b.work + k, 1u);
+}
+__device__ __forceinline__ void gather_flags(const Bufs& b, const ScenePar& S, uint32_t info) {
+  const uint32_t m = info & INFO_MAT;
+  // the particles k_friction or k_apply_fric would touch (a superset of each)
+  raise_work(b, 0, !(info & INFO_BOUNDARY) && (matw(b, m, M_fric) != 0 || matw(b, m, M_bondK) != 0));
+  // a live fluid particle a neighbour-list flag can see (buildNbr's sealSeen / congealSeen)
+  raise_work(b, 1, !(info & (INFO_BOUNDARY | INFO_DEAD)) && (info & (INFO_SEAL | INFO_CONGEAL)));
+  // its scene forms bonds this substep (predict set formNow): k_form1 has work
+  raise_work(b, 5, S.formNow != 0u);
 }
 
 // Move the working set into sorted space.
@@ -412,27 +435,12 @@ __global__ void __launch_bounds__(256) k_gather(Bufs b) {
     int2 pr = b.predSlot[slot];
     int4 rec = make_int4(pr.x, pr.y, 0, (int32_t)info_of((uint32_t)c.x, (uint32_t)c.y, i >= S.nFluid));
     b.PL[p] = rec;
-    b.PL2[p] = rec;
+    if ((uint32_t)rec.w & INFO_BOUNDARY) b.PL2[p] = rec;  // walls never move: the colour passes do not write them
     b.RX[p] = make_int4(0, 0, c.z, 0);
     b.POS[p] = make_int2(a.x, a.y);
     b.SCN[p] = s;
     b.inv[slot] = p;
-    const uint32_t m = (uint32_t)rec.w & INFO_MAT;
-    // the particles k_friction or k_apply_fric would touch (a superset of each)
-    const bool fr = !((uint32_t)rec.w & INFO_BOUNDARY) && (matw(b, m, M_fric) != 0 || matw(b, m, M_bondK) != 0);
-    const unsigned bal = __ballot_sync(__activemask(), fr);
-    if (fr && (threadIdx.x & 31u) == (unsigned)(__ffs(bal) - 1) && *(volatile uint32_t*)b.work == 0u)
-      atomicOr(b.work, 1u);
-    // a live fluid particle a neighbour-list flag can see (buildNbr's sealSeen / congealSeen)
-    const bool fl = !((uint32_t)rec.w & (INFO_BOUNDARY | INFO_DEAD)) && ((uint32_t)rec.w & (INFO_SEAL | INFO_CONGEAL));
-    const unsigned bfl = __ballot_sync(__activemask(), fl);
-    if (fl && (threadIdx.x & 31u) == (unsigned)(__ffs(bfl) - 1) && *(volatile uint32_t*)(b.work + 1) == 0u)
-      atomicOr(b.work + 1, 1u);
-    // its scene forms bonds this substep (k_predict_key set formNow): k_form1 has work
-    const bool fm = S.formNow != 0u;
-    const unsigned bfm = __ballot_sync(__activemask(), fm);
-    if (fm && (threadIdx.x & 31u) == (unsigned)(__ffs(bfm) - 1) && *(volatile uint32_t*)(b.work + 5) == 0u)
-      atomicOr(b.work + 5, 1u);
+    gather_flags(b, S, (uint32_t)rec.w);
   }
 }
 
@@ -452,6 +460,12 @@ __device__ __forceinline__ bool box_reaches(int4 box, int2 pi) {
   if (gx >= REJECT_D || gy >= REJECT_D) return false;
   const int32_t ax = ((int32_t)gx + 8) >> 4, ay = ((int32_t)gy + 8) >> 4;
   return ax * ax + ay * ay < H2S;
+}
+// After an iteration the current records are in the other buffer.
+__host__ __device__ __forceinline__ void swap_records(Bufs& b) {
+  int4* t = b.PL;
+  b.PL = b.PL2;
+  b.PL2 = t;
 }
 struct BoxChunk {
   uint32_t key, lo, hi, pad;
@@ -604,6 +618,82 @@ __global__ void __launch_bounds__(256) k_tiles(Bufs b) {
   }
 }
 
+constexpr uint32_t NO_STAGE = 0x7fffffffu;  // a candidate whose tile is not staged (no such offset: copies hold STAGE_MAX records)
+// The list of one particle by L lanes (a warp calls it together; `valid` false
+// for a lane group with none): p its sorted index, `me` its record. The hits go
+// to out(position, sorted index, info, staged offset); returns the NBRN word.
+template <bool DBG, int L, bool TILED, class OUT>
+__device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cellStart, bool cut, bool valid,
+                                              uint32_t p, int4 me, OUT out, const Flags<DBG>& f) {
+  const uint32_t lane = threadIdx.x & 31u, sub = lane & (L - 1);
+  const uint32_t gmask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << (lane & ~(uint32_t)(L - 1));
+  const uint32_t below = (1u << lane) - 1u;
+  const uint32_t info = (uint32_t)me.w;
+  const bool bnd = (info & INFO_BOUNDARY) != 0;
+  const bool work = valid && !((bnd && !DBG) || (info & INFO_DEAD));
+  const ScenePar& S = b.scenes[work ? b.SCN[p] : 0u];
+  const int2 pi = xy(me);
+  const int2 cc = work ? cell_coord(S, pi) : make_int2(0, 0);
+  const uint32_t skip = work ? far_sides(S, pi, cc) : 0u;
+  uint32_t cnt = 0;
+  bool congeal = false, sealSeen = false;
+  const uint32_t ts = S.tileShift, tx = (uint32_t)cc.x >> ts, ty = (uint32_t)cc.y >> ts;
+  const uint32_t* tr = (TILED && work) ? b.TR + (size_t)tile_of(S, cc.x, cc.y) * TR_STRIDE : b.TR;
+  const bool local = TILED && work && !bnd && tr[TR_BASE + tile_runs(ts)] <= b.world->stageCap;
+  for (int dy = -1; dy <= 1; ++dy) {
+    for (int dx = -1; dx <= 1; ++dx) {
+      const int32_t gy = cc.y + dy, gx = cc.x + dx;
+      uint32_t lo = 0, len = 0, delta = NO_STAGE;
+      const bool far = (dy < 0 && (skip & SKIP_DOWN)) || (dy > 0 && (skip & SKIP_UP)) ||
+                       (dx < 0 && (skip & SKIP_LEFT)) || (dx > 0 && (skip & SKIP_RIGHT));
+      const bool full = cut && cnt >= (uint32_t)MAXNBR;  // uniform over the particle's lanes
+      if (work && !far && !full && gy >= 0 && gy < (int32_t)S.gridH && gx >= 0 && gx < (int32_t)S.gridW) {
+        const uint32_t key = key_of(S, gx, gy);
+        lo = cellStart[key];
+        len = cellStart[key + 1] - lo;
+        if (!DBG && len > CELL_BIG && !box_reaches(b.CB[key], pi)) len = 0;
+        if (TILED && local) {
+          const uint32_t run = halo_run(ts, tx, ty, gx, gy);
+          delta = tr[TR_BASE + run] - tr[run];
+        }
+      }
+      for (uint32_t t = sub;; t += L) {
+        // the warp walks on while any of its particles has candidates left
+        // in this cell and room (or a reason) to keep them
+        const bool more = t < len && !(cut && cnt >= (uint32_t)MAXNBR);
+        if (!__any_sync(0xffffffffu, more)) break;
+        const uint32_t q = lo + t;
+        bool hit = false;
+        uint32_t iq = 0;
+        if (more && q != p) {
+          const int4 o = b.PL[q];
+          iq = (uint32_t)o.w;
+          hit = !(iq & INFO_DEAD) && lut_index(pdelta(pi, xy(o), f), f) >= 0;
+        }
+        uint32_t pos = cnt, nhit = hit ? 1u : 0u;
+        if (L > 1) {
+          const uint32_t bal = __ballot_sync(0xffffffffu, hit) & gmask;
+          pos = cnt + __popc(bal & below);
+          nhit = __popc(bal);
+        }
+        if (hit) {
+          if (!(iq & INFO_BOUNDARY) && (iq & INFO_CONGEAL)) congeal = true;
+          if (!(iq & INFO_BOUNDARY) && (iq & INFO_SEAL)) sealSeen = true;
+          if (pos >= (uint32_t)MAXNBR) f.flag(6);
+          else if (!bnd) out(pos, q, iq, delta);
+        }
+        cnt += nhit;
+      }
+    }
+  }
+  if (L > 1) {
+    congeal = (__ballot_sync(0xffffffffu, congeal) & gmask) != 0u;
+    sealSeen = (__ballot_sync(0xffffffffu, sealSeen) & gmask) != 0u;
+  }
+  return (bnd || !work) ? 0u
+                        : (min(cnt, (uint32_t)MAXNBR) | (congeal ? NBRN_CONGEAL : 0u) | (sealSeen ? NBRN_SEAL : 0u));
+}
+
 // buildNbr (src/sim.wgsl:1190-1254): 3x3 cells, dy outer, dx inner, ascending
 // slot inside a cell; skip self and retired particles; keep pairs inside the
 // kernel range; keep the first MAXNBR in that order (dbg[6] counts the rest).
@@ -693,86 +783,20 @@ __global__ void __launch_bounds__(256, TILED ? 6 : 8) k_nbr(Bufs b) {
   }
   Flags<DBG> f{b.dbg};
   const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
-  const uint32_t lane = threadIdx.x & 31u, sub = lane & (L - 1);
-  const uint32_t gmask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << (lane & ~(uint32_t)(L - 1));
-  const uint32_t below = (1u << lane) - 1u;
   const uint32_t G = gstride() / L;
   for (uint32_t p = gtid() / L;; p += G) {
     if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
     const bool valid = p < nAct;
     const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_DEAD);
-    const uint32_t info = (uint32_t)me.w;
-    const bool bnd = (info & INFO_BOUNDARY) != 0;
-    const bool work = valid && !((bnd && !DBG) || (info & INFO_DEAD));
-    const ScenePar& S = b.scenes[work ? b.SCN[p] : 0u];
-    const int2 pi = xy(me);
-    const int2 cc = work ? cell_coord(S, pi) : make_int2(0, 0);
-    const uint32_t skip = work ? far_sides(S, pi, cc) : 0u;
-    uint32_t cnt = 0;
-    bool congeal = false, sealSeen = false;
-    uint32_t* out = b.NBR + p;
-    const uint32_t ts = S.tileShift, tx = (uint32_t)cc.x >> ts, ty = (uint32_t)cc.y >> ts;
-    const uint32_t* tr = (TILED && work) ? b.TR + (size_t)tile_of(S, cc.x, cc.y) * TR_STRIDE : b.TR;
-    const bool local = TILED && work && !bnd && tr[TR_BASE + tile_runs(ts)] <= b.world->stageCap;
-    for (int dy = -1; dy <= 1; ++dy) {
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int32_t gy = cc.y + dy, gx = cc.x + dx;
-        uint32_t lo = 0, len = 0, delta = 0;
-        const bool far = (dy < 0 && (skip & SKIP_DOWN)) || (dy > 0 && (skip & SKIP_UP)) ||
-                         (dx < 0 && (skip & SKIP_LEFT)) || (dx > 0 && (skip & SKIP_RIGHT));
-        const bool full = cut && cnt >= (uint32_t)MAXNBR;  // uniform over the particle's lanes
-        if (work && !far && !full && gy >= 0 && gy < (int32_t)S.gridH && gx >= 0 && gx < (int32_t)S.gridW) {
-          const uint32_t key = key_of(S, gx, gy);
-          lo = b.cellStart[key];
-          len = b.cellStart[key + 1] - lo;
-          if (!DBG && len > CELL_BIG && !box_reaches(b.CB[key], pi)) len = 0;
-          if (TILED && local) {
-            const uint32_t run = halo_run(ts, tx, ty, gx, gy);
-            delta = tr[TR_BASE + run] - tr[run];
-          }
-        }
-        for (uint32_t t = sub;; t += L) {
-          // the warp walks on while any of its particles has candidates left
-          // in this cell and room (or a reason) to keep them
-          const bool more = t < len && !(cut && cnt >= (uint32_t)MAXNBR);
-          if (!__any_sync(0xffffffffu, more)) break;
-          const uint32_t q = lo + t;
-          bool hit = false;
-          uint32_t iq = 0;
-          if (more && q != p) {
-            const int4 o = b.PL[q];
-            iq = (uint32_t)o.w;
-            hit = !(iq & INFO_DEAD) && lut_index(pdelta(pi, xy(o), f), f) >= 0;
-          }
-          uint32_t pos = cnt, nhit = hit ? 1u : 0u;
-          if (L > 1) {
-            const uint32_t bal = __ballot_sync(0xffffffffu, hit) & gmask;
-            pos = cnt + __popc(bal & below);
-            nhit = __popc(bal);
-          }
-          if (hit) {
-            if (!(iq & INFO_BOUNDARY) && (iq & INFO_CONGEAL)) congeal = true;
-            if (!(iq & INFO_BOUNDARY) && (iq & INFO_SEAL)) sealSeen = true;
-            if (pos >= (uint32_t)MAXNBR) f.flag(6);
-            else if (!bnd) {
-              out[(size_t)pos * stride] = q | (iq & INFO_BOUNDARY);
-              if (TILED && local)
-                b.NBRL[(size_t)pos * stride + p] =
-                    (uint16_t)((q + delta) | ((iq & INFO_BOUNDARY) ? NBRL_BOUNDARY : 0u));
-            }
-          }
-          cnt += nhit;
-        }
-      }
-    }
-    if (L > 1) {
-      congeal = (__ballot_sync(0xffffffffu, congeal) & gmask) != 0u;
-      sealSeen = (__ballot_sync(0xffffffffu, sealSeen) & gmask) != 0u;
-    }
-    if (valid && sub == 0)
-      b.NBRN[p] = (bnd || !work) ? 0u
-                                 : (min(cnt, (uint32_t)MAXNBR) | (congeal ? NBRN_CONGEAL : 0u) |
-                                    (sealSeen ? NBRN_SEAL : 0u));
+    const uint32_t word = nbr_lanes<DBG, L, TILED>(
+        b, b.cellStart, cut, valid, p, me,
+        [&](uint32_t pos, uint32_t q, uint32_t iq, uint32_t delta) {
+          b.NBR[(size_t)pos * stride + p] = q | (iq & INFO_BOUNDARY);
+          if (TILED && delta != NO_STAGE)
+            b.NBRL[(size_t)pos * stride + p] = (uint16_t)((q + delta) | ((iq & INFO_BOUNDARY) ? NBRL_BOUNDARY : 0u));
+        },
+        f);
+    if (valid && (threadIdx.x & (L - 1)) == 0) b.NBRN[p] = word;
   }
 }
 
@@ -797,6 +821,7 @@ struct NbrStaged {
     return *reinterpret_cast<const int2*>(sm + (e & NBRL_INDEX));
   }
   __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBRL_BOUNDARY) != 0u; }
+  __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
 };
 // Neighbour access from global memory: records in PL, sorted-index entries.
 struct NbrGlobal {
@@ -807,6 +832,8 @@ struct NbrGlobal {
   __device__ __forceinline__ int4 rec(uint32_t e) const { return g[e & ~NBR_BOUNDARY]; }
   __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e & ~NBR_BOUNDARY); }
   __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBR_BOUNDARY) != 0u; }
+  __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
+  __device__ __forceinline__ int2 ca(const Bufs& b, int id) const { return __ldg(b.CA + id); }
 };
 
 // Copy tile t's neighbourhood (`total` records in `runs` runs) from `from`
@@ -855,7 +882,7 @@ __device__ __forceinline__ void solveA_sums(const Bufs& b, const NB& nb, uint32_
     const int2 d = pdelta(pi, pj, f);
     const int id = lut_index(d, f);
     if (id < 0) continue;
-    const int2 wg = __ldg(b.WG + id);
+    const int2 wg = nb.wg(b, id);
     rho = wadd(rho, wg.x);
     const int32_t gx = mulf<26>(wg.y, d.x, f), gy = mulf<26>(wg.y, d.y, f);
     sgx = wadd(sgx, gx);
@@ -870,11 +897,24 @@ __device__ __forceinline__ void solveA_sums(const Bufs& b, const NB& nb, uint32_
   }
 }
 
+// solveA's tail from the sums: lambda (returned), rho with the particle's own
+// W0, and on the last iteration finalize's rinv.
+template <bool DBG>
+__device__ __forceinline__ int32_t solveA_lambda(const Bufs& b, int32_t eps, int32_t W0, int32_t& rho, int32_t S,
+                                                 int32_t sgx, int32_t sgy, bool last, int32_t& rinv,
+                                                 const Flags<DBG>& f) {
+  rho = wadd(rho, W0);
+  S = wadd(S, wadd(clampi(mul<11>(sgx, sgx, f), 0, S_TERM), clampi(mul<11>(sgy, sgy, f), 0, S_TERM)));
+  const int32_t Cq = clampi(shr_rne<4>(wsub(rho, RHO0)), 0, C_MAX);
+  rinv = last ? clampi(divshift<16>(RHO0, max(rho, RHO_FLOOR_RINV), b.rcp, f), 0, RINV_MAX) : 0;
+  return clampi(neg_sat(divshift<25>(Cq, wadd(S, eps), b.rcp, f), f), -LAM_MAX, LAM_MAX);
+}
+
 // solveA (src/sim.wgsl:1270-1318) for particles [p0, p0 + n) of one tile,
 // `me_of(i)` giving particle p0 + i's own record: density, |grad C|^2,
 // lambda. On the last iteration it also stores rinv (finalize's,
 // src/sim.wgsl:2261-2262), which depends only on this rho.
-template <bool DBG, int L, bool BOTH, class NB, class ME>
+template <bool DBG, int L, class NB, class ME>
 __device__ __forceinline__ void solveA_tile(const Bufs& b, const NB& nb, ME me_of, uint32_t p0, uint32_t n,
                                             int lastIter, const Flags<DBG>& f) {
   const int32_t W0 = __ldg(b.luts);
@@ -890,29 +930,25 @@ __device__ __forceinline__ void solveA_tile(const Bufs& b, const NB& nb, ME me_o
     int32_t rho = 0, S = 0, sgx = 0, sgy = 0;
     solveA_sums<DBG, L>(b, nb, p, cnt, sub, xy(me), f, rho, S, sgx, sgy);
     if (!act || sub != 0) continue;
-    rho = wadd(rho, W0);
-    S = wadd(S, wadd(clampi(mul<11>(sgx, sgx, f), 0, S_TERM), clampi(mul<11>(sgy, sgy, f), 0, S_TERM)));
-    const int32_t Cq = clampi(shr_rne<4>(wsub(rho, RHO0)), 0, C_MAX);
-    const int32_t eps = matw(b, info & INFO_MAT, M_eps);
-    const int32_t lam = clampi(neg_sat(divshift<25>(Cq, wadd(S, eps), b.rcp, f), f), -LAM_MAX, LAM_MAX);
+    int32_t rinv;
+    const int32_t lam =
+        solveA_lambda(b, matw(b, info & INFO_MAT, M_eps), W0, rho, S, sgx, sgy, lastIter != 0, rinv, f);
     b.PL[p].z = lam;
-    if constexpr (BOTH) b.PL2[p].z = lam;
     int4& rx = b.RX[p];
     rx.x = rho;
-    if (lastIter) rx.y = clampi(divshift<16>(RHO0, max(rho, RHO_FLOOR_RINV), b.rcp, f), 0, RINV_MAX);
+    if (lastIter) rx.y = rinv;
   }
 }
 
 // solveA over the sorted particles, the grid striding over them (colour-major
-// layout). lam goes to both buffers of the colour sweep, which copies only
-// preds between them.
+// layout).
 template <bool DBG, int L>
 __device__ __forceinline__ void solveA_all(const Bufs& b, int lastIter, const Flags<DBG>& f) {
   const uint32_t nAct = b.world->nAct;
   const int4* PL = b.PL;
   const uint32_t chunk = blockDim.x / L;
   for (uint32_t i0 = blockIdx.x * chunk; i0 < nAct; i0 += gridDim.x * chunk)
-    solveA_tile<DBG, L, true>(b, NbrGlobal{PL, b.NBR, b.nbrStride}, [&](uint32_t i) { return PL[i0 + i]; }, i0,
+    solveA_tile<DBG, L>(b, NbrGlobal{PL, b.NBR, b.nbrStride}, [&](uint32_t i) { return PL[i0 + i]; }, i0,
                               min(nAct - i0, chunk), lastIter, f);
 }
 template <bool DBG, int L>
@@ -948,7 +984,7 @@ __global__ void __launch_bounds__(256, 4) k_solveA_tiled(Bufs b, int lastIter) {
     if (n == 0 || total > cap) continue;
     if (!stage_tile(b, b.PL, tr, runs, total, stg, &bar, parity, &okS)) return;
     parity ^= 1u;
-    solveA_tile<DBG, L, false>(b, NbrStaged{stg, b.NBRL, stride}, [&](uint32_t i) { return stg[i]; }, p0, n,
+    solveA_tile<DBG, L>(b, NbrStaged{stg, b.NBRL, stride}, [&](uint32_t i) { return stg[i]; }, p0, n,
                                lastIter, f);
     __syncthreads();  // stg is read before the next tile's copy lands
   }
@@ -963,7 +999,7 @@ __global__ void __launch_bounds__(256, 4) k_solveA_tiled(Bufs b, int lastIter) {
     const uint32_t per = gridDim.x * (blockDim.x / L);
     for (uint32_t i0 = first; i0 < n; i0 += per) {
       const uint32_t m = min(n - i0, blockDim.x / L);
-      solveA_tile<DBG, L, false>(b, NbrGlobal{PL, b.NBR, stride}, [&](uint32_t i) { return PL[p0 + i0 + i]; },
+      solveA_tile<DBG, L>(b, NbrGlobal{PL, b.NBR, stride}, [&](uint32_t i) { return PL[p0 + i0 + i]; },
                                  p0 + i0, m, lastIter, f);
     }
   }
@@ -1000,7 +1036,7 @@ __device__ __forceinline__ int2 solveB_dp(const Bufs& b, const NB& nb, uint32_t 
     int32_t co;
     if constexpr (DBG) co = add_sat(add_sat(li, lj, f), __ldg(b.luts + 4 * TN + id), f);
     else co = li + lj;
-    const int32_t gt = __ldg(b.WG + id).y;
+    const int32_t gt = nb.wg(b, id).y;
     dpx = wadd(dpx, mulfc<12>(co, mulf<26>(gt, d.x, f), -DP_TERM, DP_TERM, f));
     dpy = wadd(dpy, mulfc<12>(co, mulf<26>(gt, d.y, f), -DP_TERM, DP_TERM, f));
   }
@@ -1011,14 +1047,19 @@ __device__ __forceinline__ int2 solveB_dp(const Bufs& b, const NB& nb, uint32_t 
   return make_int2(dpx, dpy);
 }
 
-// applyDp_at (src/sim.wgsl:1418-1434).
+// applyDp_at (src/sim.wgsl:1418-1434) with the row's dpMax and the scene's far
+// walls (domain - WALL) at hand.
+template <bool DBG>
+__device__ __forceinline__ int2 apply_dp_in(int32_t dm, int2 far, int2 pr, int2 dp, const Flags<DBG>& f) {
+  const int32_t dmN = neg_sat(dm, f);
+  const int32_t dx = clampi(shr_rne<8>(dp.x), dmN, dm), dy = clampi(shr_rne<8>(dp.y), dmN, dm);
+  return make_int2(clampi(add_sat(pr.x, dx, f), WALL, far.x), clampi(add_sat(pr.y, dy, f), WALL, far.y));
+}
+
 template <bool DBG>
 __device__ __forceinline__ int2 apply_dp(const Bufs& b, const ScenePar& S, uint32_t m, int2 pr, int2 dp,
                                          const Flags<DBG>& f) {
-  int32_t dm = matw(b, m, M_dpMax), dmN = neg_sat(dm, f);
-  int32_t dx = clampi(shr_rne<8>(dp.x), dmN, dm);
-  int32_t dy = clampi(shr_rne<8>(dp.y), dmN, dm);
-  return wall_clamp(S, make_int2(add_sat(pr.x, dx, f), add_sat(pr.y, dy, f)));
+  return apply_dp_in(matw(b, m, M_dpMax), make_int2(S.domW - WALL, S.domH - WALL), pr, dp, f);
 }
 
 // The colour class's particles [lo, lo + n) of one tile: dp of each from the
@@ -1048,66 +1089,69 @@ __device__ __forceinline__ void colour_tile(const Bufs& b, const NB& nb, ME me_o
 }
 
 // One colour of the block Gauss-Seidel sweep (colour-major layout):
-// solveB_cK + applyDp_cK fused. The pass reads every pred from `src` and
-// writes its colour's corrected preds to `dst`, so a particle never reads a
-// value written in the same pass: that is the Jacobi-within-a-colour rule the
-// reference gets from its separate solveB/applyDp dispatches
-// (src/sim.wgsl:1323-1332). `dst` must leave the pass complete, so the pass
-// also copies the two colours that are stale in it: the sweep alternates
-// A->B, B->A, A->B, B->A, colour c is written in phase c and read again four
-// phases later, so phase c copies colours c+1 and c-1. After phase 3 buffer A
-// is complete again. A rigid member's dp is not applied: rigidSolve folds it
-// into its body at the end of the iteration (src/sim.wgsl:1418-1429).
-// (No __restrict__ here: the persistent kernel reads buffers that its own
+// solveB_cK + applyDp_cK fused. The records live in two buffers; an iteration
+// starts with every current record in `src` and ends with every one in `dst`:
+// pass c writes its colour's records to `dst`, and since the colours are
+// consecutive ranges of sorted space, neighbour q's current record is in
+// `dst` when q lies below this colour's range (passes before c wrote it) and
+// in `src` otherwise. So a particle never reads a value written in the same
+// pass: that is the Jacobi-within-a-colour rule the reference gets from its
+// separate solveB/applyDp dispatches (src/sim.wgsl:1323-1332), with one
+// compare per neighbour in place of a copy of the other colours (which moved
+// 8.5 MB a pass on a forked branch of the graph: a 10-substep replay of the
+// 1 M scene fell from 17.5 to 17.1 ms, a frame of 4,096 particles from 386 to
+// 380 us). Wall records
+// never change; k_gather puts them in both buffers. A rigid member's dp is
+// not applied: rigidSolve folds it into its body at the end of the iteration
+// (src/sim.wgsl:1418-1429).
+// (No __restrict__ here: the persistent kernels read buffers that their own
 // earlier phases wrote, which must not go through the non-coherent load path.)
-// Phase c's copy of colours c+1 and c-1 (the two stale in dst) from src.
-__device__ __forceinline__ void copy_other_colours(const Bufs& b, int colour, const int4* src, int4* dst) {
-  const uint32_t* cb = b.world->colourBase;
-  const int c1 = (colour + 1) & 3, c3 = (colour + 3) & 3;
-  const uint32_t lo1 = b.cellStart[cb[c1]], hi1 = b.cellStart[cb[c1 + 1]];
-  const uint32_t lo3 = b.cellStart[cb[c3]], hi3 = b.cellStart[cb[c3 + 1]];
-  const uint32_t n1 = hi1 - lo1, n13 = n1 + (hi3 - lo3);
-  for (uint32_t i = gtid(); i < n13; i += gstride()) {
-    const uint32_t p = i < n1 ? lo1 + i : lo3 + (i - n1);
-    *reinterpret_cast<int2*>(dst + p) = *reinterpret_cast<const int2*>(src + p);
+struct NbrSplit {
+  const int4* src;
+  uint32_t cut, off;  // dst == src + off (wrapping u32 index), for q < cut
+  const uint32_t* nl;
+  uint32_t stride;
+  __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[(size_t)k * stride + p]; }
+  __device__ __forceinline__ int4 rec(uint32_t e) const {
+    const uint32_t q = e & ~NBR_BOUNDARY;
+    return src[(int32_t)(q < cut ? q + off : q)];
   }
+  __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBR_BOUNDARY) != 0u; }
+  __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
+};
+
+// The corrected record of an active particle: its dp applied, or kept in DP
+// for rigidSolve.
+template <bool DBG>
+__device__ __forceinline__ int4 colour_record(const Bufs& b, uint32_t p, int4 me, int2 dp, const Flags<DBG>& f) {
+  const uint32_t info = (uint32_t)me.w;
+  if (info & INFO_RIGID) b.DP[p] = dp;
+  if (!(info & INFO_PINNED)) {
+    const int2 pr = apply_dp(b, b.scenes[b.SCN[p]], info & INFO_MAT, xy(me), dp, f);
+    me.x = pr.x;
+    me.y = pr.y;
+  }
+  return me;
 }
 
 template <bool DBG, int L>
-__device__ __forceinline__ void colour_all(const Bufs& b, int colour, const int4* src, int4* dst,
-                                           const Flags<DBG>& f, bool copyOthers = true) {
+__device__ __forceinline__ void colour_all(const Bufs& b, int colour, const Flags<DBG>& f) {
   const uint32_t* cb = b.world->colourBase;
   const uint32_t lo = b.cellStart[cb[colour]], hi = b.cellStart[cb[colour + 1]];
-  // The grid covers this colour's range only (the launch is sized to the
-  // resident capacity); the copies of the neighbouring colours follow, or
-  // run beside the pass in k_colour_copy.
   const uint32_t chunk = blockDim.x / L;
-  const NbrGlobal nb{src, b.NBR, b.nbrStride};
+  int4* const src = b.PL;
+  const uint32_t off = (uint32_t)(b.PL2 - b.PL);
+  const NbrSplit nb{src, lo, off, b.NBR, b.nbrStride};
   for (uint32_t i0 = blockIdx.x * chunk; i0 < hi - lo; i0 += gridDim.x * chunk)
     colour_tile<DBG, L>(
         b, nb, [&](uint32_t p) { return src[p]; },
-        [&](uint32_t p, int4 me, int2 dp) {
-          const uint32_t info = (uint32_t)me.w;
-          int2 pr = xy(me);
-          if (info & INFO_RIGID) b.DP[p] = dp;
-          if (!(info & INFO_PINNED)) pr = apply_dp(b, b.scenes[b.SCN[p]], info & INFO_MAT, pr, dp, f);
-          *reinterpret_cast<int2*>(dst + p) = pr;
-        },
-        lo + i0, min(hi - lo - i0, chunk), f);
-  if (copyOthers) copy_other_colours(b, colour, src, dst);
+        [&](uint32_t p, int4 me, int2 dp) { src[(int32_t)(p + off)] = colour_record(b, p, me, dp, f); }, lo + i0,
+        min(hi - lo - i0, chunk), f);
 }
 template <bool DBG, int L>
-__global__ void __launch_bounds__(256, 8) k_colour(Bufs b, int colour, const int4* __restrict__ src,
-                                                int4* __restrict__ dst, int copyOthers) {
+__global__ void __launch_bounds__(256, 8) k_colour(Bufs b, int colour) {
   Flags<DBG> f{b.dbg};
-  colour_all<DBG, L>(b, colour, src, dst, f, copyOthers != 0);
-}
-// The copy of phase c, launched on a forked branch of the substep so it runs
-// in the slots the pass leaves free; it touches none of the words the pass
-// reads from dst or writes.
-__global__ void __launch_bounds__(256) k_colour_copy(Bufs b, int colour, const int4* __restrict__ src,
-                                                     int4* __restrict__ dst) {
-  copy_other_colours(b, colour, src, dst);
+  colour_all<DBG, L>(b, colour, f);
 }
 
 // One colour of the sweep in the tile-major layout, with staged gathers.
@@ -1217,124 +1261,132 @@ __device__ __forceinline__ bool friction_row(const Bufs& b, uint32_t m) {
 // any split is exact); a friction row's cost is one chain of dependent
 // gathers, which the split shortens L-fold. The bond gather stays on the
 // particle's first lane.
+//
+// One particle (a warp calls it together; `valid` false for a lane group with
+// none): p its sorted index, `row` its list in nb.
+template <bool DBG, int L, class NB>
+__device__ __forceinline__ void friction_particle(const Bufs& b, const NB& nb, bool valid, uint32_t p, uint32_t row,
+                                                  uint32_t sub, const Flags<DBG>& f) {
+  const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
+  const uint32_t info = (uint32_t)me.w;
+  const uint32_t m = info & INFO_MAT;
+  const bool act = valid && !(info & INFO_BOUNDARY) && friction_row(b, m);
+  // a rigid member skips its own body, gathers no bonds and ADDS its friction
+  // to the solver dp waiting for rigidSolve (src/sim.wgsl:1680-1688, 1925-1929)
+  const bool rigidI = (info & INFO_RIGID) != 0u;
+  const int32_t fi = act ? matw(b, m, M_fric) : 0;
+  const int2 pi = xy(me);
+  const uint32_t pp = act ? p : 0u;
+  const int2 dxi = delta(pi, b.POS[pp], f);
+  const uint32_t cnt = fi != 0 ? (b.NBRN[p] & NBRN_COUNT) : 0u;
+  int32_t fx = 0, fy = 0;
+  // one neighbour ahead (record and old position), two ahead (index)
+  uint32_t en = sub < cnt ? nb.entry(row, sub) : 0u;
+  int4 on = b.PL[en & ~NBR_BOUNDARY];
+  int2 sn = b.POS[en & ~NBR_BOUNDARY];
+  uint32_t en2 = sub + L < cnt ? nb.entry(row, sub + L) : 0u;
+  for (uint32_t k = sub; k < cnt; k += L) {
+    const uint32_t e = en;
+    const int4 o = on;
+    const int2 so = sn;
+    if (k + L < cnt) {
+      en = en2;
+      on = b.PL[en & ~NBR_BOUNDARY];
+      sn = b.POS[en & ~NBR_BOUNDARY];
+    }
+    if (k + 2 * L < cnt) en2 = nb.entry(row, k + 2 * L);
+    if (rigidI && !(e & NBR_BOUNDARY) && same_body(info, (uint32_t)o.w)) continue;
+    int2 pq = xy(o);
+    int2 d = pdelta(pi, pq, f);
+    int id = lut_index(d, f);
+    if (id < 0) continue;
+    int32_t d4x = shr_rne<FPRE>(d.x), d4y = shr_rne<FPRE>(d.y);
+    int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
+    if (d2 < D2_FLOOR) continue;
+    int2 rel = dxi;
+    int32_t mu = fi;
+    if (!(e & NBR_BOUNDARY)) {
+      int2 dq = delta(pq, so, f);
+      rel = make_int2(sub_sat(dxi.x, dq.x, f), sub_sat(dxi.y, dq.y, f));
+      mu = mat_mix(fi, matw(b, (uint32_t)o.w & INFO_MAT, M_fric));
+    }
+    if (mu == 0) continue;
+    int32_t r4x = shr_rne<RPRE>(rel.x), r4y = shr_rne<RPRE>(rel.y);
+    int32_t dot = wadd(wmul(d4x, r4x), wmul(d4y, r4y));
+    int32_t qq = divshift<16>(dot, d2, b.rcp, f);
+    int32_t tx = sub_sat(r4x, mul<16>(d4x, qq, f), f);
+    int32_t ty = sub_sat(r4y, mul<16>(d4y, qq, f), f);
+    int32_t wq = shr_rne<4>(nb.wg(b, id).x);
+    int32_t sx = mul<16>(mul<5>(tx, wq, f), mu, f);
+    int32_t sy = mul<16>(mul<5>(ty, wq, f), mu, f);
+    fx = wsub(fx, clampi(sx, -FR_TERM, FR_TERM));
+    fy = wsub(fy, clampi(sy, -FR_TERM, FR_TERM));
+  }
+  if (L > 1) {
+    fx = gsum<L>(fx);
+    fy = gsum<L>(fy);
+  }
+  if (!act || sub != 0) return;
+  if (rigidI) {
+    const int2 d0 = b.DP[p];
+    b.DP[p] = make_int2(add_sat(d0.x, fx, f), add_sat(d0.y, fy, f));
+    return;
+  }
+  const int32_t bondKi = matw(b, m, M_bondK);
+  int32_t bx = 0, by = 0;
+  if (bondKi != 0 && !(info & INFO_BURST)) {
+    uint32_t slot = b.sslot[p];
+    int32_t ki = bond_k(b, m, b.RX[p].z, f);
+    const uint32_t base = b.scenes[b.SCN[p]].slotBase;
+    uint32_t* brow = b.bond + (size_t)slot * BOND_CAP;
+    for (int k = 0; k < BOND_CAP; ++k) {
+      uint32_t w = brow[k];
+      if (w == 0u) break;
+      if (w & BOND_TOMB) continue;
+      uint32_t q = b.inv[base + (w & BOND_J_MASK)];
+      int4 o = b.PL[q];
+      uint32_t mj = (uint32_t)o.w & INFO_MAT;
+      if ((uint32_t)o.w & INFO_BURST) { brow[k] = w | BOND_TOMB; continue; }
+      if (matw(b, mj, M_bondK) == 0) { brow[k] = w | BOND_TOMB; continue; }
+      int32_t L0 = (int32_t)((w >> 17) & 0x1fffu);
+      int32_t L02 = wmul(L0, L0);
+      int2 d = delta(pi, xy(o), f);
+      int32_t d4x = shr_rne<BPRE>(d.x), d4y = shr_rne<BPRE>(d.y);
+      if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) { brow[k] = w | BOND_TOMB; continue; }
+      int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
+      if (d2 >= HARD_BREAK2) { brow[k] = w | BOND_TOMB; continue; }
+      int32_t mb = min(matw(b, m, M_bondBreak), matw(b, mj, M_bondBreak));
+      int32_t mub = min(matw(b, m, M_bondMu), matw(b, mj, M_bondMu));
+      if (mb != 0 && mub != 0) {
+        int32_t lp = neg_sat(add_sat(me.z, o.z, f), f);
+        int32_t Pq = lp > 0 ? shr_rne<4>(lp) : 0;
+        mb = wadd(wadd(65536, wsub(mb, 65536)), mul<16>(Pq, mub, f));
+      }
+      if (mb != 0 && d2 > mul<16>(L02, mb, f)) { brow[k] = w | BOND_TOMB; continue; }
+      if (d2 < D2_FLOOR) continue;
+      int32_t kj = bond_k(b, mj, b.RX[q].z, f);
+      int32_t kp = min(ki, kj);
+      if (kp == 0) continue;
+      int32_t C = sub_sat(d2, L02, f);
+      int32_t qv = divshift<16>(C, wmul(d2, 4), b.rcp, f);
+      int32_t qk = mul<16>(qv, kp, f);
+      int32_t gx = mul<3>(d4x, qk, f);
+      int32_t gy = mul<3>(d4y, qk, f);
+      bx = wsub(bx, clampi(gx, -BD_TERM, BD_TERM));
+      by = wsub(by, clampi(gy, -BD_TERM, BD_TERM));
+    }
+  }
+  b.DP[p] = make_int2(add_sat(fx, bx, f), add_sat(fy, by, f));
+}
+
 template <bool DBG, int L>
 __device__ __forceinline__ void friction_all(const Bufs& b, const Flags<DBG>& f) {
-  const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
+  const uint32_t nAct = b.world->nAct;
   const uint32_t sub = threadIdx.x & (L - 1), G = gstride() / L;
+  const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
   for (uint32_t p = gtid() / L;; p += G) {
     if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
-    const bool valid = p < nAct;
-    const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
-    const uint32_t info = (uint32_t)me.w;
-    const uint32_t m = info & INFO_MAT;
-    const bool act = valid && !(info & INFO_BOUNDARY) && friction_row(b, m);
-    // a rigid member skips its own body, gathers no bonds and ADDS its friction
-    // to the solver dp waiting for rigidSolve (src/sim.wgsl:1680-1688, 1925-1929)
-    const bool rigidI = (info & INFO_RIGID) != 0u;
-    const int32_t fi = act ? matw(b, m, M_fric) : 0;
-    const int2 pi = xy(me);
-    const uint32_t pp = act ? p : 0u;
-    const int2 dxi = delta(pi, b.POS[pp], f);
-    const uint32_t cnt = fi != 0 ? (b.NBRN[p] & NBRN_COUNT) : 0u;
-    int32_t fx = 0, fy = 0;
-    // one neighbour ahead (record and old position), two ahead (index)
-    const uint32_t* np = b.NBR + pp;
-    uint32_t en = sub < cnt ? np[(size_t)sub * stride] : 0u;
-    int4 on = b.PL[en & ~NBR_BOUNDARY];
-    int2 sn = b.POS[en & ~NBR_BOUNDARY];
-    uint32_t en2 = sub + L < cnt ? np[(size_t)(sub + L) * stride] : 0u;
-    for (uint32_t k = sub; k < cnt; k += L) {
-      const uint32_t e = en;
-      const int4 o = on;
-      const int2 so = sn;
-      if (k + L < cnt) {
-        en = en2;
-        on = b.PL[en & ~NBR_BOUNDARY];
-        sn = b.POS[en & ~NBR_BOUNDARY];
-      }
-      if (k + 2 * L < cnt) en2 = np[(size_t)(k + 2 * L) * stride];
-      if (rigidI && !(e & NBR_BOUNDARY) && same_body(info, (uint32_t)o.w)) continue;
-      int2 pq = xy(o);
-      int2 d = pdelta(pi, pq, f);
-      int id = lut_index(d, f);
-      if (id < 0) continue;
-      int32_t d4x = shr_rne<FPRE>(d.x), d4y = shr_rne<FPRE>(d.y);
-      int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
-      if (d2 < D2_FLOOR) continue;
-      int2 rel = dxi;
-      int32_t mu = fi;
-      if (!(e & NBR_BOUNDARY)) {
-        int2 dq = delta(pq, so, f);
-        rel = make_int2(sub_sat(dxi.x, dq.x, f), sub_sat(dxi.y, dq.y, f));
-        mu = mat_mix(fi, matw(b, (uint32_t)o.w & INFO_MAT, M_fric));
-      }
-      if (mu == 0) continue;
-      int32_t r4x = shr_rne<RPRE>(rel.x), r4y = shr_rne<RPRE>(rel.y);
-      int32_t dot = wadd(wmul(d4x, r4x), wmul(d4y, r4y));
-      int32_t qq = divshift<16>(dot, d2, b.rcp, f);
-      int32_t tx = sub_sat(r4x, mul<16>(d4x, qq, f), f);
-      int32_t ty = sub_sat(r4y, mul<16>(d4y, qq, f), f);
-      int32_t wq = shr_rne<4>(__ldg(b.WG + id).x);
-      int32_t sx = mul<16>(mul<5>(tx, wq, f), mu, f);
-      int32_t sy = mul<16>(mul<5>(ty, wq, f), mu, f);
-      fx = wsub(fx, clampi(sx, -FR_TERM, FR_TERM));
-      fy = wsub(fy, clampi(sy, -FR_TERM, FR_TERM));
-    }
-    if (L > 1) {
-      fx = gsum<L>(fx);
-      fy = gsum<L>(fy);
-    }
-    if (!act || sub != 0) continue;
-    if (rigidI) {
-      const int2 d0 = b.DP[p];
-      b.DP[p] = make_int2(add_sat(d0.x, fx, f), add_sat(d0.y, fy, f));
-      continue;
-    }
-    const int32_t bondKi = matw(b, m, M_bondK);
-    int32_t bx = 0, by = 0;
-    if (bondKi != 0 && !(info & INFO_BURST)) {
-      uint32_t slot = b.sslot[p];
-      int32_t ki = bond_k(b, m, b.RX[p].z, f);
-      const uint32_t base = b.scenes[b.SCN[p]].slotBase;
-      uint32_t* row = b.bond + (size_t)slot * BOND_CAP;
-      for (int k = 0; k < BOND_CAP; ++k) {
-        uint32_t w = row[k];
-        if (w == 0u) break;
-        if (w & BOND_TOMB) continue;
-        uint32_t q = b.inv[base + (w & BOND_J_MASK)];
-        int4 o = b.PL[q];
-        uint32_t mj = (uint32_t)o.w & INFO_MAT;
-        if ((uint32_t)o.w & INFO_BURST) { row[k] = w | BOND_TOMB; continue; }
-        if (matw(b, mj, M_bondK) == 0) { row[k] = w | BOND_TOMB; continue; }
-        int32_t L0 = (int32_t)((w >> 17) & 0x1fffu);
-        int32_t L02 = wmul(L0, L0);
-        int2 d = delta(pi, xy(o), f);
-        int32_t d4x = shr_rne<BPRE>(d.x), d4y = shr_rne<BPRE>(d.y);
-        if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) { row[k] = w | BOND_TOMB; continue; }
-        int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
-        if (d2 >= HARD_BREAK2) { row[k] = w | BOND_TOMB; continue; }
-        int32_t mb = min(matw(b, m, M_bondBreak), matw(b, mj, M_bondBreak));
-        int32_t mub = min(matw(b, m, M_bondMu), matw(b, mj, M_bondMu));
-        if (mb != 0 && mub != 0) {
-          int32_t lp = neg_sat(add_sat(me.z, o.z, f), f);
-          int32_t Pq = lp > 0 ? shr_rne<4>(lp) : 0;
-          mb = wadd(wadd(65536, wsub(mb, 65536)), mul<16>(Pq, mub, f));
-        }
-        if (mb != 0 && d2 > mul<16>(L02, mb, f)) { row[k] = w | BOND_TOMB; continue; }
-        if (d2 < D2_FLOOR) continue;
-        int32_t kj = bond_k(b, mj, b.RX[q].z, f);
-        int32_t kp = min(ki, kj);
-        if (kp == 0) continue;
-        int32_t C = sub_sat(d2, L02, f);
-        int32_t qv = divshift<16>(C, wmul(d2, 4), b.rcp, f);
-        int32_t qk = mul<16>(qv, kp, f);
-        int32_t gx = mul<3>(d4x, qk, f);
-        int32_t gy = mul<3>(d4y, qk, f);
-        bx = wsub(bx, clampi(gx, -BD_TERM, BD_TERM));
-        by = wsub(by, clampi(gy, -BD_TERM, BD_TERM));
-      }
-    }
-    b.DP[p] = make_int2(add_sat(fx, bx, f), add_sat(fy, by, f));
+    friction_particle<DBG, L>(b, nb, p < nAct, p, p < nAct ? p : 0u, sub, f);
   }
 }
 
@@ -1357,7 +1409,6 @@ __device__ __forceinline__ void apply_fric_all(const Bufs& b, const Flags<DBG>& 
     const ScenePar& S = b.scenes[b.SCN[p]];
     int2 np = apply_dp(b, S, m, xy(me), b.DP[p], f);
     *reinterpret_cast<int2*>(b.PL + p) = np;
-    *reinterpret_cast<int2*>(b.PL2 + p) = np;
   }
 }
 template <bool DBG>
@@ -1411,8 +1462,9 @@ __global__ void __launch_bounds__(256, 8) k_iters_persistent(Bufs b, uint32_t it
     solveA_all<DBG, L>(b, it + 1 == iters ? 1 : 0, f);
     for (int c = 0; c < 4; ++c) {
       if (!grid_barrier(bar, b.err, gen)) return;
-      colour_all<DBG, L>(b, c, (c & 1) ? b.PL2 : b.PL, (c & 1) ? b.PL : b.PL2, f);
+      colour_all<DBG, L>(b, c, f);
     }
+    swap_records(b);
     // friction and applyFric, when some particle has a friction or bond row
     // this substep (the flag is the same for every CTA)
     if (*(volatile uint32_t*)b.work != 0u) {
@@ -1429,107 +1481,117 @@ __global__ void __launch_bounds__(256, 8) k_iters_persistent(Bufs b, uint32_t it
 // finalize + xsph + normals + conduct (src/sim.wgsl:2245-2582) in one sweep
 // over the neighbour list. vtmp_j = clamp(pred_j - pos_j) is finalize's
 // velocity, recomputed where it is needed.
+// smat[m] = {xsph, cond, corrode, corrPt} of every material row.
+__device__ __forceinline__ void post1_mats(const Bufs& b, int4* smat) {
+  for (int m = threadIdx.x; m < MAT_MAX; m += blockDim.x)
+    smat[m] = make_int4(matw(b, m, M_xsph), matw(b, m, M_cond), matw(b, m, M_corrode), matw(b, m, M_corrPt));
+}
+// One particle (a warp calls it together; `valid` false for a lane group with
+// none): p its sorted index, `row` its list in nb.
+template <bool DBG, int L, class NB>
+__device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, const int4* smat, bool valid, uint32_t p,
+                                               uint32_t row, uint32_t sub, const Flags<DBG>& f) {
+  const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
+  const uint32_t info = (uint32_t)me.w;
+  const bool act = valid && !(info & INFO_BOUNDARY);
+  const uint32_t pp = act ? p : 0u;
+  const ScenePar& S = b.scenes[b.SCN[pp]];
+  const int32_t vmax = S.vmax, vmaxN = neg_sat(vmax, f);
+  const uint32_t m = info & INFO_MAT;
+  const int2 pi = xy(me);
+  int2 vi = delta(pi, b.POS[pp], f);
+  vi.x = clampi(vi.x, vmaxN, vmax);
+  vi.y = clampi(vi.y, vmaxN, vmax);
+  const bool doX = !(info & INFO_PINNED);
+  const int4 mi = smat[m];
+  const int4 rxi = b.RX[pp];
+  const int32_t rhoi = rxi.x, Ti = rxi.z;
+  const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
+  int32_t ax = 0, ay = 0, sx = 0, sy = 0, hq = 0, hc = 0;
+  // the neighbour's three records (pred/info, rho/rinv/T, old position)
+  // one ahead, its index two ahead
+  uint32_t en = sub < cnt ? nb.entry(row, sub) : 0u;
+  int4 on = b.PL[en & ~NBR_BOUNDARY];
+  int4 rn = b.RX[en & ~NBR_BOUNDARY];
+  int2 sn = b.POS[en & ~NBR_BOUNDARY];
+  uint32_t en2 = sub + L < cnt ? nb.entry(row, sub + L) : 0u;
+  for (uint32_t k = sub; k < cnt; k += L) {
+    const uint32_t e = en;
+    const int4 o = on;
+    const int4 rx = rn;
+    const int2 so = sn;
+    if (k + L < cnt) {
+      en = en2;
+      on = b.PL[en & ~NBR_BOUNDARY];
+      rn = b.RX[en & ~NBR_BOUNDARY];
+      sn = b.POS[en & ~NBR_BOUNDARY];
+    }
+    if (k + 2 * L < cnt) en2 = nb.entry(row, k + 2 * L);
+    if (e & NBR_BOUNDARY) continue;
+    const int2 pq = xy(o);
+    const int2 d = pdelta(pi, pq, f);
+    const int id = lut_index(d, f);
+    if (id < 0) continue;
+    const int2 wg = nb.wg(b, id);
+    const int32_t W = wg.x;
+    const int4 mj = smat[(uint32_t)o.w & INFO_MAT];
+    if (doX) {
+      int32_t K = sym_k(rhoi, rx.x, b.rcp, f);
+      int32_t wk = mulf<16>(W, K, f);
+      int32_t cij = mat_mix(mi.x, mj.x);
+      int2 vj = delta(pq, so, f);
+      vj.x = clampi(vj.x, vmaxN, vmax);
+      vj.y = clampi(vj.y, vmaxN, vmax);
+      ax = wadd(ax, mulfc<16>(mulf<12>(sub_sat(vj.x, vi.x, f), wk, f), cij, -XS_TERM, XS_TERM, f));
+      ay = wadd(ay, mulfc<16>(mulf<12>(sub_sat(vj.y, vi.y, f), wk, f), cij, -XS_TERM, XS_TERM, f));
+    }
+    sx = wadd(sx, mulf<16>(mulf<26>(wg.y, d.x, f), rx.y, f));
+    sy = wadd(sy, mulf<16>(mulf<26>(wg.y, d.y, f), rx.y, f));
+    {
+      int32_t cij = mat_mix(mi.y, mj.y);
+      int32_t wk = mulf<16>(W, cij, f);
+      int32_t dT = clampi(sub_sat(rx.z, Ti, f), -DT_CLAMP, DT_CLAMP);
+      hq = wadd(hq, mulfc<12>(dT, wk, -HT_TERM, HT_TERM, f));
+      if (((uint32_t)o.w & INFO_MAT) != m) {
+        int32_t spend = mj.w != CORR_NEVER ? mi.z : 0;
+        int32_t str = wadd(mj.z, spend);
+        if (str != 0) hc = wadd(hc, mulfc<12>(W, str, 0, CORR_TERM, f));
+      }
+    }
+  }
+  if (L > 1) {
+    ax = gsum<L>(ax);
+    ay = gsum<L>(ay);
+    sx = gsum<L>(sx);
+    sy = gsum<L>(sy);
+    hq = gsum<L>(hq);
+    hc = gsum<L>(hc);
+  }
+  if (!valid || sub != 0) return;
+  int32_t* w = b.state + (size_t)b.sslot[p] * 8;
+  if (!act) {
+    *reinterpret_cast<int2*>(w + 2) = make_int2(0, 0);  // finalize: walls end with zero velocity
+    return;
+  }
+  b.NQ[p] = make_int4(mul<16>(sx, H, f), mul<16>(sy, H, f), rhoi, 0);
+  b.HEAT[p] = hq;
+  b.CORR[p] = hc;
+  int2 vo = vi;
+  if (doX) vo = make_int2(add_sat(vi.x, shr_rne<8>(ax), f), add_sat(vi.y, shr_rne<8>(ay), f));
+  *reinterpret_cast<int4*>(w) = make_int4(pi.x, pi.y, vo.x, vo.y);
+}
 template <bool DBG, int L>
 __global__ void __launch_bounds__(256, 4) k_post1(Bufs b) {
   Flags<DBG> f{b.dbg};
-  __shared__ int4 smat[MAT_MAX];  // {xsph, cond, corrode, corrPt}
-  for (int m = threadIdx.x; m < MAT_MAX; m += blockDim.x)
-    smat[m] = make_int4(matw(b, m, M_xsph), matw(b, m, M_cond), matw(b, m, M_corrode), matw(b, m, M_corrPt));
+  __shared__ int4 smat[MAT_MAX];
+  post1_mats(b, smat);
   __syncthreads();
-  const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
+  const uint32_t nAct = b.world->nAct;
   const uint32_t sub = threadIdx.x & (L - 1), G = gstride() / L;
+  const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
   for (uint32_t p = gtid() / L;; p += G) {
     if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
-    const bool valid = p < nAct;
-    const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
-    const uint32_t info = (uint32_t)me.w;
-    const bool act = valid && !(info & INFO_BOUNDARY);
-    const uint32_t pp = act ? p : 0u;
-    const ScenePar& S = b.scenes[b.SCN[pp]];
-    const int32_t vmax = S.vmax, vmaxN = neg_sat(vmax, f);
-    const uint32_t m = info & INFO_MAT;
-    const int2 pi = xy(me);
-    int2 vi = delta(pi, b.POS[pp], f);
-    vi.x = clampi(vi.x, vmaxN, vmax);
-    vi.y = clampi(vi.y, vmaxN, vmax);
-    const bool doX = !(info & INFO_PINNED);
-    const int4 mi = smat[m];
-    const int4 rxi = b.RX[pp];
-    const int32_t rhoi = rxi.x, Ti = rxi.z;
-    const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
-    int32_t ax = 0, ay = 0, sx = 0, sy = 0, hq = 0, hc = 0;
-    const uint32_t* np = b.NBR + pp;
-    // the neighbour's three records (pred/info, rho/rinv/T, old position)
-    // one ahead, its index two ahead
-    uint32_t en = sub < cnt ? np[(size_t)sub * stride] : 0u;
-    int4 on = b.PL[en & ~NBR_BOUNDARY];
-    int4 rn = b.RX[en & ~NBR_BOUNDARY];
-    int2 sn = b.POS[en & ~NBR_BOUNDARY];
-    uint32_t en2 = sub + L < cnt ? np[(size_t)(sub + L) * stride] : 0u;
-    for (uint32_t k = sub; k < cnt; k += L) {
-      const uint32_t e = en;
-      const int4 o = on;
-      const int4 rx = rn;
-      const int2 so = sn;
-      if (k + L < cnt) {
-        en = en2;
-        on = b.PL[en & ~NBR_BOUNDARY];
-        rn = b.RX[en & ~NBR_BOUNDARY];
-        sn = b.POS[en & ~NBR_BOUNDARY];
-      }
-      if (k + 2 * L < cnt) en2 = np[(size_t)(k + 2 * L) * stride];
-      if (e & NBR_BOUNDARY) continue;
-      const int2 pq = xy(o);
-      const int2 d = pdelta(pi, pq, f);
-      const int id = lut_index(d, f);
-      if (id < 0) continue;
-      const int2 wg = __ldg(b.WG + id);
-      const int32_t W = wg.x;
-      const int4 mj = smat[(uint32_t)o.w & INFO_MAT];
-      if (doX) {
-        int32_t K = sym_k(rhoi, rx.x, b.rcp, f);
-        int32_t wk = mulf<16>(W, K, f);
-        int32_t cij = mat_mix(mi.x, mj.x);
-        int2 vj = delta(pq, so, f);
-        vj.x = clampi(vj.x, vmaxN, vmax);
-        vj.y = clampi(vj.y, vmaxN, vmax);
-        ax = wadd(ax, mulfc<16>(mulf<12>(sub_sat(vj.x, vi.x, f), wk, f), cij, -XS_TERM, XS_TERM, f));
-        ay = wadd(ay, mulfc<16>(mulf<12>(sub_sat(vj.y, vi.y, f), wk, f), cij, -XS_TERM, XS_TERM, f));
-      }
-      sx = wadd(sx, mulf<16>(mulf<26>(wg.y, d.x, f), rx.y, f));
-      sy = wadd(sy, mulf<16>(mulf<26>(wg.y, d.y, f), rx.y, f));
-      {
-        int32_t cij = mat_mix(mi.y, mj.y);
-        int32_t wk = mulf<16>(W, cij, f);
-        int32_t dT = clampi(sub_sat(rx.z, Ti, f), -DT_CLAMP, DT_CLAMP);
-        hq = wadd(hq, mulfc<12>(dT, wk, -HT_TERM, HT_TERM, f));
-        if (((uint32_t)o.w & INFO_MAT) != m) {
-          int32_t spend = mj.w != CORR_NEVER ? mi.z : 0;
-          int32_t str = wadd(mj.z, spend);
-          if (str != 0) hc = wadd(hc, mulfc<12>(W, str, 0, CORR_TERM, f));
-        }
-      }
-    }
-    if (L > 1) {
-      ax = gsum<L>(ax);
-      ay = gsum<L>(ay);
-      sx = gsum<L>(sx);
-      sy = gsum<L>(sy);
-      hq = gsum<L>(hq);
-      hc = gsum<L>(hc);
-    }
-    if (!valid || sub != 0) continue;
-    int32_t* w = b.state + (size_t)b.sslot[p] * 8;
-    if (!act) {
-      *reinterpret_cast<int2*>(w + 2) = make_int2(0, 0);  // finalize: walls end with zero velocity
-      continue;
-    }
-    b.NQ[p] = make_int4(mul<16>(sx, H, f), mul<16>(sy, H, f), rhoi, 0);
-    b.HEAT[p] = hq;
-    b.CORR[p] = hc;
-    int2 vo = vi;
-    if (doX) vo = make_int2(add_sat(vi.x, shr_rne<8>(ax), f), add_sat(vi.y, shr_rne<8>(ay), f));
-    *reinterpret_cast<int4*>(w) = make_int4(pi.x, pi.y, vo.x, vo.y);
+    post1_particle<DBG, L>(b, nb, smat, p < nAct, p, p < nAct ? p : 0u, sub, f);
   }
 }
 
@@ -1644,54 +1706,57 @@ __device__ int2 contain_core(const Bufs& b, Entry entry, uint32_t n, bool filter
 // launch: each writes only an intruder's pred and reads only seal endpoints'
 // preds, which neither moves, so fusing them changes nothing. Runs after the
 // last solver iteration, on the final preds in PL.
+template <bool DBG, class NB>
+__device__ __forceinline__ void contain_particle(const Bufs& b, const NB& nb, uint32_t p, uint32_t row,
+                                                 const Flags<DBG>& f) {
+  const uint32_t nn = b.NBRN[p];
+  if (!(nn & NBRN_SEAL)) return;
+  const int4 me = b.PL[p];
+  const uint32_t info = (uint32_t)me.w;
+  if (info & (INFO_BOUNDARY | INFO_PINNED)) return;
+  const uint32_t m = info & INFO_MAT;
+  if (seal_class(b, m) || matw(b, m, M_phantom) != 0) return;
+  const int2 pos = b.POS[p];
+  int2 pr = xy(me);
+  const bool liquidI = seal_liquid(b, m);
+  const uint32_t cnt = nn & NBRN_COUNT;
+  if (cnt < (uint32_t)MAXNBR) {
+    pr = contain_core(b, [&](uint32_t k) { return nb.entry(row, k); }, cnt, true, pos, pr, liquidI, f);
+  } else {
+    uint32_t seals[MAXNBR];
+    uint32_t sealN = 0;
+    const int32_t loX = sub_sat(min(pos.x, pr.x), SEAL_REACH, f), hiX = add_sat(max(pos.x, pr.x), SEAL_REACH, f);
+    const int32_t loY = sub_sat(min(pos.y, pr.y), SEAL_REACH, f), hiY = add_sat(max(pos.y, pr.y), SEAL_REACH, f);
+    const ScenePar& S = b.scenes[b.SCN[p]];
+    const int2 cc = cell_coord(S, pr);
+    for (int dy = -1; dy <= 1; ++dy) {
+      const int32_t gy = cc.y + dy;
+      if (gy < 0 || gy >= (int32_t)S.gridH) continue;
+      for (int dx = -1; dx <= 1; ++dx) {
+        const int32_t gx = cc.x + dx;
+        if (gx < 0 || gx >= (int32_t)S.gridW) continue;
+        const uint32_t key = key_of(S, gx, gy);
+        for (uint32_t q = b.cellStart[key]; q < b.cellStart[key + 1]; ++q) {
+          const int4 o = b.PL[q];
+          if (((uint32_t)o.w & INFO_BOUNDARY) || !seal_class(b, (uint32_t)o.w & INFO_MAT)) continue;
+          if (o.x < loX || o.x > hiX || o.y < loY || o.y > hiY) continue;
+          if (sealN < (uint32_t)MAXNBR) seals[sealN++] = q;
+        }
+      }
+    }
+    pr = contain_core(b, [&](uint32_t k) { return seals[k]; }, sealN, false, pos, pr, liquidI, f);
+  }
+  *reinterpret_cast<int2*>(b.PL + p) = pr;
+}
 template <bool DBG>
 __global__ void __launch_bounds__(256) k_contain(Bufs b) {
   // a list holds a seal endpoint (NBRN_SEAL) only if some live fluid particle
   // carries SEAL, which k_gather reports in work[1] (with CONGEAL)
   if (b.work[1] == 0u) return;
   Flags<DBG> f{b.dbg};
-  const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
-  for (uint32_t p = gtid(); p < nAct; p += gstride()) {
-    const uint32_t nn = b.NBRN[p];
-    if (!(nn & NBRN_SEAL)) continue;
-    const int4 me = b.PL[p];
-    const uint32_t info = (uint32_t)me.w;
-    if (info & (INFO_BOUNDARY | INFO_PINNED)) continue;
-    const uint32_t m = info & INFO_MAT;
-    if (seal_class(b, m) || matw(b, m, M_phantom) != 0) continue;
-    const int2 pos = b.POS[p];
-    int2 pr = xy(me);
-    const bool liquidI = seal_liquid(b, m);
-    const uint32_t cnt = nn & NBRN_COUNT;
-    if (cnt < (uint32_t)MAXNBR) {
-      const uint32_t* col = b.NBR + p;
-      pr = contain_core(b, [&](uint32_t k) { return col[(size_t)k * stride]; }, cnt, true, pos, pr, liquidI, f);
-    } else {
-      uint32_t seals[MAXNBR];
-      uint32_t sealN = 0;
-      const int32_t loX = sub_sat(min(pos.x, pr.x), SEAL_REACH, f), hiX = add_sat(max(pos.x, pr.x), SEAL_REACH, f);
-      const int32_t loY = sub_sat(min(pos.y, pr.y), SEAL_REACH, f), hiY = add_sat(max(pos.y, pr.y), SEAL_REACH, f);
-      const ScenePar& S = b.scenes[b.SCN[p]];
-      const int2 cc = cell_coord(S, pr);
-      for (int dy = -1; dy <= 1; ++dy) {
-        const int32_t gy = cc.y + dy;
-        if (gy < 0 || gy >= (int32_t)S.gridH) continue;
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int32_t gx = cc.x + dx;
-          if (gx < 0 || gx >= (int32_t)S.gridW) continue;
-          const uint32_t key = key_of(S, gx, gy);
-          for (uint32_t q = b.cellStart[key]; q < b.cellStart[key + 1]; ++q) {
-            const int4 o = b.PL[q];
-            if (((uint32_t)o.w & INFO_BOUNDARY) || !seal_class(b, (uint32_t)o.w & INFO_MAT)) continue;
-            if (o.x < loX || o.x > hiX || o.y < loY || o.y > hiY) continue;
-            if (sealN < (uint32_t)MAXNBR) seals[sealN++] = q;
-          }
-        }
-      }
-      pr = contain_core(b, [&](uint32_t k) { return seals[k]; }, sealN, false, pos, pr, liquidI, f);
-    }
-    *reinterpret_cast<int2*>(b.PL + p) = pr;
-  }
+  const uint32_t nAct = b.world->nAct;
+  const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
+  for (uint32_t p = gtid(); p < nAct; p += gstride()) contain_particle(b, nb, p, p, f);
 }
 
 // containStress (src/sim.wgsl:2742-2771), after thermal: a held seal particle
@@ -1701,43 +1766,51 @@ __global__ void __launch_bounds__(256) k_contain(Bufs b) {
 // the neighbour list only for held seal particles. L lanes share one slot's
 // list (the stress sum wraps, so any split is exact): a seal body's members
 // each walk a list, and the split shortens that serial gather chain.
+// `row`: the slot's list in nb, or NO_ROW for its sorted index.
+constexpr uint32_t NO_ROW = 0xffffffffu;
+template <bool DBG, int L, class NB>
+__device__ __forceinline__ void contain_stress_slot(const Bufs& b, const NB& nb, bool act, uint32_t slot, uint32_t row,
+                                                    uint32_t sub, const Flags<DBG>& f) {
+  int32_t* w = b.state + (size_t)(act ? slot : 0u) * 8;
+  const int2 mf = *reinterpret_cast<const int2*>(w + 4);
+  const uint32_t mi = (uint32_t)mf.x, fl = (uint32_t)mf.y;
+  act = act && (fl & (FLAG_ANCHOR | FLAG_RIGID));
+  int32_t burstP = 0;
+  if (act) {
+    const ScenePar& S = b.scenes[b.sceneOf[slot]];
+    act = S.active && slot - S.slotBase < S.nFluid;
+    burstP = act ? matw(b, mi, M_burstP) : 0;
+    act = act && seal_class(b, mi) && burstP > 0;
+  }
+  const uint32_t p = act ? b.inv[slot] : 0u;
+  const uint32_t r = row == NO_ROW ? p : row;
+  const int32_t px = act ? w[0] : 0, py = act ? w[1] : 0;
+  const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
+  int32_t stress = 0;
+  for (uint32_t k = sub; k < cnt; k += L) {
+    const uint32_t e = nb.entry(r, k);
+    if (e & NBR_BOUNDARY) continue;
+    const int32_t* wj = b.state + (size_t)b.sslot[e] * 8;
+    const uint32_t mj = (uint32_t)wj[4];
+    if (seal_class(b, mj) || matw(b, mj, M_phantom) != 0) continue;
+    const int32_t dx4 = shr_rne<BPRE>(sub_sat(px, wj[0], f)), dy4 = shr_rne<BPRE>(sub_sat(py, wj[1], f));
+    const int32_t d2 = wadd(wmul(dx4, dx4), wmul(dy4, dy4));
+    if (d2 >= SEAL_STRESS4 * SEAL_STRESS4) continue;
+    stress = wadd(stress, SEAL_STRESS4 - (int32_t)isqrt32((uint32_t)d2));
+  }
+  if (L > 1) stress = gsum<L>(stress);
+  if (act && sub == 0 && (int32_t)((uint32_t)stress << BPRE) > burstP)
+    w[5] = (int32_t)((fl & ~(FLAG_ANCHOR | FLAG_RIGID | WELD_TAG_MASK)) | FLAG_BURST);
+}
 template <bool DBG, int L>
 __global__ void __launch_bounds__(256) k_contain_stress(Bufs b) {
   Flags<DBG> f{b.dbg};
-  const uint32_t slotEnd = b.world->slotEnd, stride = b.nbrStride;
+  const uint32_t slotEnd = b.world->slotEnd;
   const uint32_t sub = threadIdx.x & (L - 1), G = gstride() / L;
+  const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
   for (uint32_t slot = gtid() / L;; slot += G) {
     if (__shfl_sync(0xffffffffu, slot, 0) >= slotEnd) break;  // warp-uniform exit
-    bool act = slot < slotEnd;
-    int32_t* w = b.state + (size_t)(act ? slot : 0u) * 8;
-    const int2 mf = *reinterpret_cast<const int2*>(w + 4);
-    const uint32_t mi = (uint32_t)mf.x, fl = (uint32_t)mf.y;
-    act = act && (fl & (FLAG_ANCHOR | FLAG_RIGID));
-    int32_t burstP = 0;
-    if (act) {
-      const ScenePar& S = b.scenes[b.sceneOf[slot]];
-      act = S.active && slot - S.slotBase < S.nFluid;
-      burstP = act ? matw(b, mi, M_burstP) : 0;
-      act = act && seal_class(b, mi) && burstP > 0;
-    }
-    const uint32_t p = act ? b.inv[slot] : 0u;
-    const int32_t px = act ? w[0] : 0, py = act ? w[1] : 0;
-    const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
-    int32_t stress = 0;
-    for (uint32_t k = sub; k < cnt; k += L) {
-      const uint32_t e = b.NBR[(size_t)k * stride + p];
-      if (e & NBR_BOUNDARY) continue;
-      const int32_t* wj = b.state + (size_t)b.sslot[e] * 8;
-      const uint32_t mj = (uint32_t)wj[4];
-      if (seal_class(b, mj) || matw(b, mj, M_phantom) != 0) continue;
-      const int32_t dx4 = shr_rne<BPRE>(sub_sat(px, wj[0], f)), dy4 = shr_rne<BPRE>(sub_sat(py, wj[1], f));
-      const int32_t d2 = wadd(wmul(dx4, dx4), wmul(dy4, dy4));
-      if (d2 >= SEAL_STRESS4 * SEAL_STRESS4) continue;
-      stress = wadd(stress, SEAL_STRESS4 - (int32_t)isqrt32((uint32_t)d2));
-    }
-    if (L > 1) stress = gsum<L>(stress);
-    if (act && sub == 0 && (int32_t)((uint32_t)stress << BPRE) > burstP)
-      w[5] = (int32_t)((fl & ~(FLAG_ANCHOR | FLAG_RIGID | WELD_TAG_MASK)) | FLAG_BURST);
+    contain_stress_slot<DBG, L>(b, nb, slot < slotEnd, slot, NO_ROW, sub, f);
   }
 }
 
@@ -1788,74 +1861,99 @@ __device__ __forceinline__ void thermal(const Bufs& b, uint32_t i, int32_t heat,
 // flag update for rows that cannot bond (bondForm2's tail, src/sim.wgsl:
 // 3059-3067) + the state digest. HASH=false when bond formation runs as its
 // own kernels (the digest then follows them).
+// smat[m] = {gammaCoh, gammaCur, adhesion, 0} of every material row.
+__device__ __forceinline__ void post2_mats(const Bufs& b, int4* smat) {
+  for (int m = threadIdx.x; m < MAT_MAX; m += blockDim.x)
+    smat[m] = make_int4(matw(b, m, M_gammaCoh), matw(b, m, M_gammaCur), matw(b, m, M_adhesion), 0);
+}
+// surfaceTension's sums of one particle (a warp calls it together); `act`:
+// it is a fluid particle.
+template <bool DBG, int L, class NB>
+__device__ __forceinline__ int2 post2_sums(const Bufs& b, const NB& nb, const int4* smat, bool valid, uint32_t p,
+                                           uint32_t row, uint32_t sub, bool& act, const Flags<DBG>& f) {
+  const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
+  const uint32_t info = (uint32_t)me.w;
+  act = valid && !(info & INFO_BOUNDARY);
+  const uint32_t pp = act ? p : 0u;
+  const int4 mi = smat[info & INFO_MAT];
+  const int2 pi = xy(me);
+  const int4 nqi = b.NQ[pp];
+  const int32_t rhoi = nqi.z;
+  const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
+  int32_t ax = 0, ay = 0;
+  // the neighbour's record and normal/density one ahead, its index two ahead
+  uint32_t en = sub < cnt ? nb.entry(row, sub) : 0u;
+  int4 on = b.PL[en & ~NBR_BOUNDARY];
+  int4 nn = b.NQ[en & ~NBR_BOUNDARY];
+  uint32_t en2 = sub + L < cnt ? nb.entry(row, sub + L) : 0u;
+  for (uint32_t k = sub; k < cnt; k += L) {
+    const uint32_t e = en;
+    const int4 o = on;
+    const int4 nq = nn;
+    if (k + L < cnt) {
+      en = en2;
+      on = b.PL[en & ~NBR_BOUNDARY];
+      nn = b.NQ[en & ~NBR_BOUNDARY];
+    }
+    if (k + 2 * L < cnt) en2 = nb.entry(row, k + 2 * L);
+    // a rigid member's cohesion skips its own body (src/sim.wgsl:2450-2457)
+    if ((info & INFO_RIGID) && !(e & NBR_BOUNDARY) && same_body(info, (uint32_t)o.w)) continue;
+    const int2 d = pdelta(pi, xy(o), f);
+    const int id = lut_index(d, f);
+    if (id < 0) continue;
+    const int2 ca = nb.ca(b, id);
+    if (e & NBR_BOUNDARY) {
+      ax = wsub(ax, mulfc<8>(mulf<22>(ca.y, d.x, f), mi.z, -ST_TERM, ST_TERM, f));
+      ay = wsub(ay, mulfc<8>(mulf<22>(ca.y, d.y, f), mi.z, -ST_TERM, ST_TERM, f));
+      continue;
+    }
+    const int32_t K = sym_k(rhoi, nq.z, b.rcp, f);
+    const int4 mj = smat[(uint32_t)o.w & INFO_MAT];
+    const int32_t gCoh = mat_mix(mi.x, mj.x);
+    const int32_t gCur = mat_mix(mi.y, mj.y);
+    int32_t fx = neg_sat(mulf<16>(mulf<22>(ca.x, d.x, f), gCoh, f), f);
+    int32_t fy = neg_sat(mulf<16>(mulf<22>(ca.x, d.y, f), gCoh, f), f);
+    const int32_t cx = mulf<16>(sub_sat(nqi.x, nq.x, f), gCur, f);
+    const int32_t cy = mulf<16>(sub_sat(nqi.y, nq.y, f), gCur, f);
+    fx = add_sat(fx, neg_sat(cx, f), f);
+    fy = add_sat(fy, neg_sat(cy, f), f);
+    ax = wadd(ax, mulc<8>(fx, K, -ST_TERM, ST_TERM, f));
+    ay = wadd(ay, mulc<8>(fy, K, -ST_TERM, ST_TERM, f));
+  }
+  if (L > 1) {
+    ax = gsum<L>(ax);
+    ay = gsum<L>(ay);
+  }
+  return make_int2(ax, ay);
+}
+// thermal and the formation flag update of a fluid particle: its words 4..7.
+template <bool DBG>
+__device__ __forceinline__ void post2_finish(const Bufs& b, const ScenePar& S, uint32_t p, uint32_t slot, uint32_t idx,
+                                             int2 a, bool formFlags, int32_t* w, const Flags<DBG>& f) {
+  b.stacc[slot] = make_int2(shr_rne<8>(a.x), shr_rne<8>(a.y));
+  thermal(b, idx, b.HEAT[p], b.CORR[p], w, f);
+  if (formFlags && S.formNow) {
+    uint32_t fo = (uint32_t)w[5] & ~FLAG_CONGEAL;
+    if (!(fo & FLAG_RIGID) && (fo & WELD_TAG_MASK) != S.weldHold) fo &= ~WELD_TAG_MASK;
+    w[5] = (int32_t)fo;
+  }
+}
 template <bool DBG, bool HASH, int L>
 __global__ void __launch_bounds__(256, 5) k_post2(Bufs b, int formFlags) {
   Flags<DBG> f{b.dbg};
-  __shared__ int4 smat[MAT_MAX];  // {gammaCoh, gammaCur, adhesion, 0}
-  for (int m = threadIdx.x; m < MAT_MAX; m += blockDim.x)
-    smat[m] = make_int4(matw(b, m, M_gammaCoh), matw(b, m, M_gammaCur), matw(b, m, M_adhesion), 0);
+  __shared__ int4 smat[MAT_MAX];
+  post2_mats(b, smat);
   __syncthreads();
   __shared__ uint32_t dsacc[8], dsscene;
   if (HASH) digest_block_begin(dsacc, &dsscene);
-  const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
+  const uint32_t nAct = b.world->nAct;
   const uint32_t sub = threadIdx.x & (L - 1), G = gstride() / L;
+  const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
   for (uint32_t p = gtid() / L;; p += G) {
     if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
     const bool valid = p < nAct;
-    const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
-    const uint32_t info = (uint32_t)me.w;
-    const bool act = valid && !(info & INFO_BOUNDARY);
-    const uint32_t pp = act ? p : 0u;
-    const int4 mi = smat[info & INFO_MAT];
-    const int2 pi = xy(me);
-    const int4 nqi = b.NQ[pp];
-    const int32_t rhoi = nqi.z;
-    const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
-    int32_t ax = 0, ay = 0;
-    const uint32_t* np = b.NBR + pp;
-    // the neighbour's record and normal/density one ahead, its index two ahead
-    uint32_t en = sub < cnt ? np[(size_t)sub * stride] : 0u;
-    int4 on = b.PL[en & ~NBR_BOUNDARY];
-    int4 nn = b.NQ[en & ~NBR_BOUNDARY];
-    uint32_t en2 = sub + L < cnt ? np[(size_t)(sub + L) * stride] : 0u;
-    for (uint32_t k = sub; k < cnt; k += L) {
-      const uint32_t e = en;
-      const int4 o = on;
-      const int4 nq = nn;
-      if (k + L < cnt) {
-        en = en2;
-        on = b.PL[en & ~NBR_BOUNDARY];
-        nn = b.NQ[en & ~NBR_BOUNDARY];
-      }
-      if (k + 2 * L < cnt) en2 = np[(size_t)(k + 2 * L) * stride];
-      // a rigid member's cohesion skips its own body (src/sim.wgsl:2450-2457)
-      if ((info & INFO_RIGID) && !(e & NBR_BOUNDARY) && same_body(info, (uint32_t)o.w)) continue;
-      const int2 d = pdelta(pi, xy(o), f);
-      const int id = lut_index(d, f);
-      if (id < 0) continue;
-      const int2 ca = __ldg(b.CA + id);
-      if (e & NBR_BOUNDARY) {
-        ax = wsub(ax, mulfc<8>(mulf<22>(ca.y, d.x, f), mi.z, -ST_TERM, ST_TERM, f));
-        ay = wsub(ay, mulfc<8>(mulf<22>(ca.y, d.y, f), mi.z, -ST_TERM, ST_TERM, f));
-        continue;
-      }
-      const int32_t K = sym_k(rhoi, nq.z, b.rcp, f);
-      const int4 mj = smat[(uint32_t)o.w & INFO_MAT];
-      const int32_t gCoh = mat_mix(mi.x, mj.x);
-      const int32_t gCur = mat_mix(mi.y, mj.y);
-      int32_t fx = neg_sat(mulf<16>(mulf<22>(ca.x, d.x, f), gCoh, f), f);
-      int32_t fy = neg_sat(mulf<16>(mulf<22>(ca.x, d.y, f), gCoh, f), f);
-      const int32_t cx = mulf<16>(sub_sat(nqi.x, nq.x, f), gCur, f);
-      const int32_t cy = mulf<16>(sub_sat(nqi.y, nq.y, f), gCur, f);
-      fx = add_sat(fx, neg_sat(cx, f), f);
-      fy = add_sat(fy, neg_sat(cy, f), f);
-      ax = wadd(ax, mulc<8>(fx, K, -ST_TERM, ST_TERM, f));
-      ay = wadd(ay, mulc<8>(fy, K, -ST_TERM, ST_TERM, f));
-    }
-    if (L > 1) {
-      ax = gsum<L>(ax);
-      ay = gsum<L>(ay);
-    }
+    bool act;
+    const int2 a2 = post2_sums<DBG, L>(b, nb, smat, valid, p, valid ? p : 0u, sub, act, f);
     const bool lead = valid && sub == 0;
     uint32_t scene = 0, idx = 0;
     int32_t w8[8];
@@ -1865,15 +1963,7 @@ __global__ void __launch_bounds__(256, 5) k_post2(Bufs b, int formFlags) {
       const ScenePar& S = b.scenes[scene];
       idx = slot - S.slotBase;
       int32_t* w = b.state + (size_t)slot * 8;
-      if (act) {
-        b.stacc[slot] = make_int2(shr_rne<8>(ax), shr_rne<8>(ay));
-        thermal(b, idx, b.HEAT[p], b.CORR[p], w, f);
-        if (formFlags && S.formNow) {
-          uint32_t fo = (uint32_t)w[5] & ~FLAG_CONGEAL;
-          if (!(fo & FLAG_RIGID) && (fo & WELD_TAG_MASK) != S.weldHold) fo &= ~WELD_TAG_MASK;
-          w[5] = (int32_t)fo;
-        }
-      }
+      if (act) post2_finish(b, S, p, slot, idx, a2, formFlags != 0, w, f);
       if (HASH) {
         int4 a = reinterpret_cast<const int4*>(w)[0], c = reinterpret_cast<const int4*>(w)[1];
         w8[0] = a.x; w8[1] = a.y; w8[2] = a.z; w8[3] = a.w;
@@ -1917,9 +2007,7 @@ __global__ void __launch_bounds__(256) k_hash(Bufs b, uint32_t* __restrict__ acc
 
 // fold_chain (src/hash/statehash.wgsl:164-170) per scene, then advance the
 // formation clock exactly as `_encodeSubstep` does (src/engine.js:4145-4151).
-__global__ void k_fold(Bufs b, int doChain) {
-  uint32_t s = gtid();
-  if (s >= b.world->numScenes) return;
+__device__ __forceinline__ void fold_scene(const Bufs& b, uint32_t s, bool doChain) {
   ScenePar& S = b.scenes[s];
   if (!S.active) return;
   if (doChain) {
@@ -1936,112 +2024,147 @@ __global__ void k_fold(Bufs b, int doChain) {
   S.formClock += 1;
   S.substep += 1;
 }
+__global__ void k_fold(Bufs b, int doChain) {
+  const uint32_t s = gtid();
+  if (s < b.world->numScenes) fold_scene(b, s, doChain != 0);
+}
 
 // markCongealNbr + bondForm1 (src/sim.wgsl:2714-2989), sorted space.
+template <bool DBG, class NB>
+__device__ __forceinline__ void form1_particle(const Bufs& b, const NB& nb, uint32_t p, uint32_t row,
+                                               const Flags<DBG>& f) {
+  int4 me = b.PL[p];
+  if ((uint32_t)me.w & INFO_BOUNDARY) return;
+  const ScenePar& S = b.scenes[b.SCN[p]];
+  if (!S.formNow) return;
+  uint32_t slot = b.sslot[p];
+  const int32_t* wi = b.state + (size_t)slot * 8;
+  uint32_t* cand = b.bondCand + (size_t)slot * BOND_CAP;
+  const uint32_t* brow = b.bond + (size_t)slot * BOND_CAP;
+  const uint32_t flI = (uint32_t)wi[5], matI = (uint32_t)wi[4];
+  // Rigid members and rows that do not bond propose nothing: their list is
+  // empty. Candidate rows are dense (entries first, zeros after), so a row
+  // whose first word is zero is already empty and is not rewritten.
+  if ((flI & FLAG_RIGID) || matw(b, matI, M_bondK) == 0 || matw(b, matI, M_bondGroup) < 0) {
+    if (cand[0] != 0u)
+      for (int k = 0; k < BOND_CAP; ++k) cand[k] = 0;
+    return;
+  }
+  uint32_t cnt = b.NBRN[p] & NBRN_COUNT;
+  // markCongealNbr: refresh the congeal bit from the post-thermal flags
+  bool seen = false;
+  for (uint32_t k = 0; k < cnt; ++k) {
+    uint32_t e = nb.entry(row, k);
+    if (e & NBR_BOUNDARY) continue;
+    uint32_t qs = b.sslot[e];
+    if ((uint32_t)b.state[(size_t)qs * 8 + 5] & FLAG_CONGEAL) { seen = true; break; }
+  }
+  bool anchoredI = (flI & FLAG_ANCHOR) != 0;
+  uint32_t cn = 0;
+  {
+    for (int k = 0; k < BOND_CAP; ++k) {
+      uint32_t w = brow[k];
+      if (w == 0u) break;
+      if (w & BOND_TOMB) continue;
+      if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
+      cand[cn++] = w;
+    }
+    uint32_t tagI = flI & WELD_TAG_MASK;
+    int32_t ki = bond_k(b, matI, wi[6], f);
+    bool canReform = (!anchoredI && matw(b, matI, M_bondReform) != 0 && ki != 0);
+    bool fuseArmed = S.fuseTag != 0u && fuse_row(b, matI);
+    bool congealI = (flI & FLAG_CONGEAL) && fuse_row(b, matI);
+    bool congealNear = seen && fuse_row(b, matI);
+    if (canReform || (!anchoredI && tagI != 0u) || fuseArmed || congealI || congealNear) {
+      for (uint32_t k = 0; k < cnt; ++k) {
+        if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
+        uint32_t e = nb.entry(row, k);
+        if (e & NBR_BOUNDARY) continue;
+        uint32_t qs = b.sslot[e];
+        const int32_t* wj = b.state + (size_t)qs * 8;
+        uint32_t j = qs - S.slotBase;
+        uint32_t mj = (uint32_t)wj[4];
+        uint32_t fJ = (uint32_t)wj[5];
+        uint32_t tagJ = fJ & WELD_TAG_MASK;
+        bool weld = (!anchoredI && tagI != 0u && tagI == tagJ);
+        bool fuse = false;
+        if (fuseArmed && !(fJ & FLAG_RIGID) && fuse_row(b, mj) && (!anchoredI || !(fJ & FLAG_ANCHOR)))
+          fuse = (tagI == S.fuseTag && tagJ == 0u) || (tagJ == S.fuseTag && tagI == 0u) ||
+                 (tagI == S.fuseTag && tagJ == S.fuseTag);
+        bool congealJ = (fJ & FLAG_CONGEAL) && fuse_row(b, mj);
+        bool congeal = ((congealI || congealJ) && !weld && !fuse && mj == matI && !(fJ & FLAG_RIGID));
+        if (!fuse && !congeal && matw(b, mj, M_bondGroup) != matw(b, matI, M_bondGroup)) continue;
+        if (!weld && !fuse && !congeal) {
+          if (!canReform) continue;
+          if (bond_k(b, mj, wj[6], f) == 0) continue;
+        }
+        bool dup = false;
+        for (uint32_t q2 = 0; q2 < cn; ++q2)
+          if ((cand[q2] & BOND_J_MASK) == j) { dup = true; break; }
+        if (dup) continue;
+        int32_t d4x = shr_rne<BPRE>(sub_sat(wi[0], wj[0], f));
+        int32_t d4y = shr_rne<BPRE>(sub_sat(wi[1], wj[1], f));
+        if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) continue;
+        int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
+        if (d2 < D2_FLOOR || d2 > BOND_R2) continue;
+        if (!weld && !fuse && !congeal) {
+          int32_t vl = min(matw(b, matI, M_bondFormV), matw(b, mj, M_bondFormV));
+          int32_t vl4 = shr_rne<RPRE>(vl);
+          int32_t r4x = shr_rne<RPRE>(sub_sat(wi[2], wj[2], f));
+          int32_t r4y = shr_rne<RPRE>(sub_sat(wi[3], wj[3], f));
+          if (abs(r4x) > vl4 || abs(r4y) > vl4) continue;
+          if (wadd(wmul(r4x, r4x), wmul(r4y, r4y)) > wmul(vl4, vl4)) continue;
+          int32_t pl = min(matw(b, matI, M_bondFormP), matw(b, mj, M_bondFormP));
+          if (pl != 0 && (neg_sat(me.z, f) < pl || neg_sat(b.PL[e].z, f) < pl)) continue;
+        }
+        int32_t L0 = (int32_t)isqrt32((uint32_t)d2);
+        if (L0 < L0_MIN || L0 > L0_MAX) continue;
+        if (j > BOND_J_MASK) { atomicOr(b.err, ERR_BOND_PARTNER); continue; }
+        cand[cn++] = (((uint32_t)L0 & 0x1fffu) << 17) | (j & BOND_J_MASK);
+      }
+    }
+  }
+  for (uint32_t k = cn; k < (uint32_t)BOND_CAP; ++k) cand[k] = 0;
+}
 template <bool DBG>
 __global__ void __launch_bounds__(256) k_form1(Bufs b) {
   if (b.work[5] == 0u) return;  // no scene forms bonds this substep
   Flags<DBG> f{b.dbg};
-  const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
-  for (uint32_t p = gtid(); p < nAct; p += gstride()) {
-    int4 me = b.PL[p];
-    if ((uint32_t)me.w & INFO_BOUNDARY) continue;
-    const ScenePar& S = b.scenes[b.SCN[p]];
-    if (!S.formNow) continue;
-    uint32_t slot = b.sslot[p];
-    const int32_t* wi = b.state + (size_t)slot * 8;
-    uint32_t* cand = b.bondCand + (size_t)slot * BOND_CAP;
-    const uint32_t* brow = b.bond + (size_t)slot * BOND_CAP;
-    const uint32_t flI = (uint32_t)wi[5], matI = (uint32_t)wi[4];
-    // Rigid members and rows that do not bond propose nothing: their list is
-    // empty. Candidate rows are dense (entries first, zeros after), so a row
-    // whose first word is zero is already empty and is not rewritten.
-    if ((flI & FLAG_RIGID) || matw(b, matI, M_bondK) == 0 || matw(b, matI, M_bondGroup) < 0) {
-      if (cand[0] != 0u)
-        for (int k = 0; k < BOND_CAP; ++k) cand[k] = 0;
-      continue;
-    }
-    uint32_t cnt = b.NBRN[p] & NBRN_COUNT;
-    // markCongealNbr: refresh the congeal bit from the post-thermal flags
-    bool seen = false;
-    for (uint32_t k = 0; k < cnt; ++k) {
-      uint32_t e = b.NBR[(size_t)k * stride + p];
-      if (e & NBR_BOUNDARY) continue;
-      uint32_t qs = b.sslot[e];
-      if ((uint32_t)b.state[(size_t)qs * 8 + 5] & FLAG_CONGEAL) { seen = true; break; }
-    }
-    bool anchoredI = (flI & FLAG_ANCHOR) != 0;
-    uint32_t cn = 0;
-    {
-      for (int k = 0; k < BOND_CAP; ++k) {
-        uint32_t w = brow[k];
-        if (w == 0u) break;
-        if (w & BOND_TOMB) continue;
-        if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
-        cand[cn++] = w;
-      }
-      uint32_t tagI = flI & WELD_TAG_MASK;
-      int32_t ki = bond_k(b, matI, wi[6], f);
-      bool canReform = (!anchoredI && matw(b, matI, M_bondReform) != 0 && ki != 0);
-      bool fuseArmed = S.fuseTag != 0u && fuse_row(b, matI);
-      bool congealI = (flI & FLAG_CONGEAL) && fuse_row(b, matI);
-      bool congealNear = seen && fuse_row(b, matI);
-      if (canReform || (!anchoredI && tagI != 0u) || fuseArmed || congealI || congealNear) {
-        for (uint32_t k = 0; k < cnt; ++k) {
-          if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
-          uint32_t e = b.NBR[(size_t)k * stride + p];
-          if (e & NBR_BOUNDARY) continue;
-          uint32_t qs = b.sslot[e];
-          const int32_t* wj = b.state + (size_t)qs * 8;
-          uint32_t j = qs - S.slotBase;
-          uint32_t mj = (uint32_t)wj[4];
-          uint32_t fJ = (uint32_t)wj[5];
-          uint32_t tagJ = fJ & WELD_TAG_MASK;
-          bool weld = (!anchoredI && tagI != 0u && tagI == tagJ);
-          bool fuse = false;
-          if (fuseArmed && !(fJ & FLAG_RIGID) && fuse_row(b, mj) && (!anchoredI || !(fJ & FLAG_ANCHOR)))
-            fuse = (tagI == S.fuseTag && tagJ == 0u) || (tagJ == S.fuseTag && tagI == 0u) ||
-                   (tagI == S.fuseTag && tagJ == S.fuseTag);
-          bool congealJ = (fJ & FLAG_CONGEAL) && fuse_row(b, mj);
-          bool congeal = ((congealI || congealJ) && !weld && !fuse && mj == matI && !(fJ & FLAG_RIGID));
-          if (!fuse && !congeal && matw(b, mj, M_bondGroup) != matw(b, matI, M_bondGroup)) continue;
-          if (!weld && !fuse && !congeal) {
-            if (!canReform) continue;
-            if (bond_k(b, mj, wj[6], f) == 0) continue;
-          }
-          bool dup = false;
-          for (uint32_t q2 = 0; q2 < cn; ++q2)
-            if ((cand[q2] & BOND_J_MASK) == j) { dup = true; break; }
-          if (dup) continue;
-          int32_t d4x = shr_rne<BPRE>(sub_sat(wi[0], wj[0], f));
-          int32_t d4y = shr_rne<BPRE>(sub_sat(wi[1], wj[1], f));
-          if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) continue;
-          int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
-          if (d2 < D2_FLOOR || d2 > BOND_R2) continue;
-          if (!weld && !fuse && !congeal) {
-            int32_t vl = min(matw(b, matI, M_bondFormV), matw(b, mj, M_bondFormV));
-            int32_t vl4 = shr_rne<RPRE>(vl);
-            int32_t r4x = shr_rne<RPRE>(sub_sat(wi[2], wj[2], f));
-            int32_t r4y = shr_rne<RPRE>(sub_sat(wi[3], wj[3], f));
-            if (abs(r4x) > vl4 || abs(r4y) > vl4) continue;
-            if (wadd(wmul(r4x, r4x), wmul(r4y, r4y)) > wmul(vl4, vl4)) continue;
-            int32_t pl = min(matw(b, matI, M_bondFormP), matw(b, mj, M_bondFormP));
-            if (pl != 0 && (neg_sat(me.z, f) < pl || neg_sat(b.PL[e].z, f) < pl)) continue;
-          }
-          int32_t L0 = (int32_t)isqrt32((uint32_t)d2);
-          if (L0 < L0_MIN || L0 > L0_MAX) continue;
-          if (j > BOND_J_MASK) { atomicOr(b.err, ERR_BOND_PARTNER); continue; }
-          cand[cn++] = (((uint32_t)L0 & 0x1fffu) << 17) | (j & BOND_J_MASK);
-        }
-      }
-    }
-    for (uint32_t k = cn; k < (uint32_t)BOND_CAP; ++k) cand[k] = 0;
-  }
+  const uint32_t nAct = b.world->nAct;
+  const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
+  for (uint32_t p = gtid(); p < nAct; p += gstride()) form1_particle(b, nb, p, p, f);
 }
 
 // bondForm2 (src/sim.wgsl:3001-3068): keep mutual proposals, clear weld
 // tags. It is the last pass of the substep that writes hashed words, so with
 // HASH it also folds every particle's digest (the state hash of the substep).
+__device__ __forceinline__ bool form2_slot(const Bufs& b, const ScenePar& S, uint32_t slot, uint32_t i, bool rowsLive) {
+  uint32_t* row = b.bond + (size_t)slot * BOND_CAP;
+  const uint32_t* cand = b.bondCand + (size_t)slot * BOND_CAP;
+  uint32_t nn = 0;
+  for (int k = 0; k < BOND_CAP; ++k) {
+    uint32_t w = cand[k];
+    if (w == 0u) break;
+    uint32_t j = w & BOND_J_MASK;
+    const uint32_t* cj = b.bondCand + (size_t)(S.slotBase + j) * BOND_CAP;
+    bool ok = false;
+    for (int q = 0; q < BOND_CAP; ++q) {
+      uint32_t v = cj[q];
+      if (v == 0u) break;
+      if ((v & BOND_J_MASK) == i) { ok = ((v & BOND_L0_MASK) == (w & BOND_L0_MASK)); break; }
+    }
+    if (ok) row[nn++] = w & ~BOND_TOMB;
+  }
+  // bond rows are dense too: an empty row stays as it is
+  if (nn != 0u || row[0] != 0u)
+    for (int k = nn; k < BOND_CAP; ++k) row[k] = 0;
+  if (nn != 0u && !rowsLive) b.work[4] = 1u;
+  int32_t* w = b.state + (size_t)slot * 8;
+  uint32_t fo = (uint32_t)w[5] & ~FLAG_CONGEAL;
+  if (!(fo & FLAG_RIGID) && (fo & WELD_TAG_MASK) != S.weldHold) fo &= ~WELD_TAG_MASK;
+  w[5] = (int32_t)fo;
+  return nn != 0u;
+}
 template <bool HASH>
 __global__ void __launch_bounds__(256) k_form2(Bufs b, uint32_t* __restrict__ acc) {
   __shared__ uint32_t dsacc[8], dsscene;
@@ -2060,35 +2183,8 @@ __global__ void __launch_bounds__(256) k_form2(Bufs b, uint32_t* __restrict__ ac
       s = b.sceneOf[slot];
       const ScenePar& S = b.scenes[s];
       const uint32_t i = slot - S.slotBase;
-      uint32_t* row = b.bond + (size_t)slot * BOND_CAP;
-      if (S.active && i < S.nFluid && S.formNow) {
-        const uint32_t* cand = b.bondCand + (size_t)slot * BOND_CAP;
-        uint32_t nn = 0;
-        for (int k = 0; k < BOND_CAP; ++k) {
-          uint32_t w = cand[k];
-          if (w == 0u) break;
-          uint32_t j = w & BOND_J_MASK;
-          const uint32_t* cj = b.bondCand + (size_t)(S.slotBase + j) * BOND_CAP;
-          bool ok = false;
-          for (int q = 0; q < BOND_CAP; ++q) {
-            uint32_t v = cj[q];
-            if (v == 0u) break;
-            if ((v & BOND_J_MASK) == i) { ok = ((v & BOND_L0_MASK) == (w & BOND_L0_MASK)); break; }
-          }
-          if (ok) row[nn++] = w & ~BOND_TOMB;
-        }
-        // bond rows are dense too: an empty row stays as it is
-        if (nn != 0u || row[0] != 0u)
-          for (int k = nn; k < BOND_CAP; ++k) row[k] = 0;
-        if (nn != 0u) {
-          formed = true;
-          if (!rowsLive) b.work[4] = 1u;
-        }
-        int32_t* w = b.state + (size_t)slot * 8;
-        uint32_t fo = (uint32_t)w[5] & ~FLAG_CONGEAL;
-        if (!(fo & FLAG_RIGID) && (fo & WELD_TAG_MASK) != S.weldHold) fo &= ~WELD_TAG_MASK;
-        w[5] = (int32_t)fo;
-      }
+      const uint32_t* row = b.bond + (size_t)slot * BOND_CAP;
+      if (S.active && i < S.nFluid && S.formNow) formed = form2_slot(b, S, slot, i, rowsLive);
       if (HASH) {
         valid = S.active && i < S.n;
         if (valid)
