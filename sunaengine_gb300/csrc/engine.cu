@@ -17,8 +17,7 @@
 #include "../../include/suna.h"
 #include "ckptpool.h"
 #include "radix.cuh"
-#include "sim2d.cuh"
-#include "rigid.cuh"
+#include "fused2d.cuh"
 #include <cmath>
 
 using namespace sn;
@@ -429,7 +428,7 @@ struct World {
                     b.NBRL, b.NBRN, (void*)b.tiles, b.TR, b.OVF, b.CB,
                     (void*)b.luts, (void*)b.WG, (void*)b.CA, (void*)b.mats, (void*)b.rcp,
                     b.scenes, b.world, b.acc, b.accLast, b.chain, b.dbg, b.err, b.work, tmpK, tmpV, hist,
-                    hits, accTmp, devEv, devEp, boxChunks, upl, uplRes, barBuf, eraseBuf, initPos};
+                    hits, accTmp, devEv, devEp, boxChunks, upl, uplRes, barBuf, fuBar, fuCount, eraseBuf, initPos};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     if (ev0) cudaEventDestroy(ev0);
@@ -520,6 +519,7 @@ struct World {
     b.err = dalloc<uint32_t>(4, err);
     b.work = dalloc<uint32_t>(8, err);
     barBuf = dalloc<uint32_t>(2, err);
+    fuBar = dalloc<uint32_t>(2, err);
     tmpK = dalloc<uint32_t>(C, err);
     tmpV = dalloc<uint32_t>(C, err);
     hist = dalloc<uint32_t>(radix::hist_words((uint32_t)C), err);
@@ -732,10 +732,12 @@ struct World {
     if (K + 1 > keyCap) {
       if (b.cellStart) cudaFree(b.cellStart);
       if (b.CB) cudaFree(b.CB);
+      if (fuCount) cudaFree(fuCount);
       keyCap = std::max<uint32_t>(K + 1, keyCap + keyCap / 2);
       b.cellStart = dalloc<uint32_t>(keyCap, err);
       b.CB = dalloc<int4>(keyCap, err);
-      if (!b.cellStart || !b.CB) return false;
+      fuCount = dalloc<uint32_t>(keyCap, err);
+      if (!b.cellStart || !b.CB || !fuCount) return false;
     }
     if (tiles > tileCap || !b.tiles) {
       if (b.tiles) cudaFree(const_cast<TileInfo*>(b.tiles));
@@ -927,6 +929,8 @@ struct World {
     cudaMemcpyAsync(b.accLast + s * 8, zero8, 32, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b.dbg, 0, 64, st);
     cudaMemsetAsync(b.err, 0, 16, st);
+    cudaMemsetAsync(fuBar, 0, 8, st);  // a launch that gave up leaves its counts behind
+    if (fuCount) cudaMemsetAsync(fuCount, 0, (size_t)keyCap * 4, st);
     freshScene = s;
     bool ok2 = relayout();
     freshScene = 0xffffffffu;
@@ -1068,6 +1072,85 @@ struct World {
     case 4: { constexpr int L_ = 4; CALL; } break; \
     case 2: { constexpr int L_ = 2; CALL; } break; \
     default: { constexpr int L_ = 1; CALL; } break; \
+  }
+
+  // ---- the fused substep of small worlds (fused2d.cuh) ----
+  uint32_t* fuBar = nullptr;    // barrier words, zero between launches
+  uint32_t* fuCount = nullptr;  // [keyCap] cell counts, zero between launches
+  bool graphFused = false;      // what the captured graph launches, and the
+  uint32_t graphOwn = 0;        // particles a CTA it was sized for
+  // One past the last slot that can hold an active particle.
+  uint32_t slots_used() const {
+    uint32_t e = 0;
+    for (const SceneHost& h : sh)
+      if (h.used && h.loaded) e = std::max(e, h.slotBase + h.n);
+    return e;
+  }
+  // Shared words for the cell ranges (later the CA table), and the particles
+  // a CTA can own in what is left of `bytes`.
+  uint32_t fused_x_words() const { return std::max((hw.K + 1 + 3) & ~3u, 2u * (uint32_t)TN); }
+  static constexpr uint32_t FU_SMEM = 222 * 1024;  // dynamic at most; the static arrays take about 3 KB of the 227
+  uint32_t fused_fixed() const { return (uint32_t)TN * 8 + fused_x_words() * 4; }
+  uint32_t fused_own_cap() const {
+    return fused_fixed() < FU_SMEM ? ((FU_SMEM - fused_fixed()) / FU_OWN_BYTES & ~1u) : 0u;
+  }
+  // Particles a CTA owns at most: an equal share of each colour, rounded up.
+  uint32_t fused_own() const { return hw.nAct / (uint32_t)numSMs + 5; }
+  // Worlds the fused kernel takes: everything it keeps on an SM fits (each
+  // slot a thread, the cell ranges, the owned particles' lists).
+  bool fused_fits() const {
+    const uint64_t G = (uint64_t)numSMs;
+    return !debug && !staged && !persistent && autoLanes && bodies.empty() && hw.nAct > 0 &&
+           slots_used() <= G * FU_T && fused_own() <= fused_own_cap();
+  }
+  template <int L, int LC>
+  void launch_fused_as() {
+    FusedPar P;
+    P.iters = iters;
+    P.friction = hasFriction ? 1u : 0u;
+    P.bonds = hasBonds ? 1u : 0u;
+    P.seal = hasSeal ? 1u : 0u;
+    P.chain = chainOn ? 1u : 0u;
+    // constant under spawns (a slot without a particle is skipped), so a
+    // captured launch stays valid
+    P.slots = std::min(hw.slotEnd, (uint32_t)numSMs * FU_T);
+    P.xWords = fused_x_words();
+    // room for an eighth more than the scene has (spawns), and no more: what
+    // the launch does not take is L1
+    P.ownCap = graphOwn = std::min(fused_own_cap(), (fused_own() + fused_own() / 8 + 1) & ~1u);
+    const uint32_t smem = fused_fixed() + P.ownCap * FU_OWN_BYTES;
+    P.count = fuCount;
+    P.tmp = tmpV;
+    P.bar = fuBar;
+    Bufs bb = b;
+    if (iters & 1u) swap_records(bb);  // so that the last iteration ends in PL
+    const auto fn = k_substep_fused<L, LC>;
+    cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FU_SMEM);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)numSMs);
+    cfg.blockDim = dim3(FU_T);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, fn, bb, P);
+  }
+  void launch_fused() {
+    uint64_t Lc = 1;
+    if (anyEvents) {
+      k_impulse_sched<<<hw.numScenes, IMPULSE_THREADS, 0, st>>>(b, devEv, devEp);
+      ++Lc;
+    }
+    // as many lanes a particle as leave one round of a CTA's threads
+    const uint32_t own = fused_own();
+    if (own <= 128) launch_fused_as<8, 8>();
+    else if (own <= 256) launch_fused_as<4, 8>();
+    else if (own <= 512) launch_fused_as<2, 8>();
+    else launch_fused_as<2, 4>();
+    launchesPerSubstep = Lc;
   }
 
   template <bool DBG>
@@ -1327,8 +1410,9 @@ struct World {
     return ok;
   }
 
-  void launch_one() {
-    if (debug) launch_substep<true>();
+  void launch_one(bool fused = false) {
+    if (fused) launch_fused();
+    else if (debug) launch_substep<true>();
     else launch_substep<false>();
   }
 
@@ -1377,11 +1461,14 @@ struct World {
     if (count == 0) return true;
     if (layoutDirty && !relayout()) return false;
     if (eventsDirty && !upload_events()) return false;
+    const bool fused = fused_fits();
+    if (fused != graphFused || (fused && fused_own() > graphOwn)) graphValid = false;
     if (useGraph && !graphValid) {
       if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
       if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
       if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture")) return false;
-      launch_one();
+      launch_one(fused);
+      graphFused = fused;
       if (!cuda_ok(cudaStreamEndCapture(st, &graph), "endCapture")) return false;
       if (!cuda_ok(cudaGraphInstantiate(&gexec, graph, 0), "instantiate")) return false;
       graphValid = true;
@@ -1391,7 +1478,7 @@ struct World {
       if (useGraph) {
         if (!cuda_ok(cudaGraphLaunch(gexec, st), "graphLaunch")) return false;
       } else {
-        launch_one();
+        launch_one(fused);
       }
     }
     cudaEventRecord(ev1, st);
@@ -1636,7 +1723,7 @@ struct World {
                   "the reference's");
     if (e[0] & ERR_BOND_PARTNER) return fail("a bond partner slot exceeds the 17-bit bond word");
     if (e[0] & ERR_BARRIER)
-      return fail("a grid barrier of the persistent solver loop timed out; results past it are not valid");
+      return fail("a grid barrier timed out; results past it are not valid");
     if (e[0] & ERR_STAGE_TIMEOUT)
       return fail("a tile's staged copy did not complete within the bounded wait; results past it are not valid");
     return true;

@@ -109,38 +109,26 @@ __device__ __forceinline__ void digest_block_begin(uint32_t* sacc, uint32_t* ssc
 }
 __device__ __forceinline__ void digest_add_block(uint32_t* acc, uint32_t* sacc, uint32_t* sscene, bool valid,
                                                  uint32_t scene, const uint32_t h[8]) {
-  uint32_t key = valid ? scene : DIGEST_NO_SCENE;
-  uint32_t peers = __match_any_sync(0xffffffffu, key);
-  int lane = threadIdx.x & 31;
-  bool leader = lane == __ffs(peers) - 1;
-  uint32_t t[8];
-  if (peers == 0xffffffffu) {
+  // one round per scene the warp holds (almost always one): its lanes' sum,
+  // the other lanes adding zero
+  uint32_t left = __ballot_sync(0xffffffffu, valid);
+  while (left) {
+    const int src = __ffs(left) - 1;
+    const uint32_t sc = __shfl_sync(0xffffffffu, scene, src);
+    const bool in = valid && scene == sc;
+    left &= ~__ballot_sync(0xffffffffu, in);
+    uint32_t t[8];
 #pragma unroll
-    for (int l = 0; l < 8; ++l) t[l] = __reduce_add_sync(0xffffffffu, h[l]);
-  } else {
-#pragma unroll
-    for (int l = 0; l < 8; ++l) {
-      uint32_t v = h[l], total = 0, m = peers;
-      while (m) {
-        int src = __ffs(m) - 1;
-        m &= m - 1;
-        total += __shfl_sync(peers, v, src);
-      }
-      t[l] = total;
+    for (int l = 0; l < 8; ++l) t[l] = __reduce_add_sync(0xffffffffu, in ? h[l] : 0u);
+    if ((threadIdx.x & 31u) != (unsigned)src) continue;
+    uint32_t owner = *(volatile uint32_t*)sscene;
+    if (owner == DIGEST_NO_SCENE) {
+      const uint32_t prev = atomicCAS(sscene, DIGEST_NO_SCENE, sc);
+      owner = prev == DIGEST_NO_SCENE ? sc : prev;
     }
-  }
-  if (!(leader && valid)) return;
-  uint32_t owner = *(volatile uint32_t*)sscene;
-  if (owner == DIGEST_NO_SCENE) {
-    const uint32_t prev = atomicCAS(sscene, DIGEST_NO_SCENE, scene);
-    owner = prev == DIGEST_NO_SCENE ? scene : prev;
-  }
-  if (owner == scene) {
+    uint32_t* to = owner == sc ? sacc : acc + (size_t)sc * 8;
 #pragma unroll
-    for (int l = 0; l < 8; ++l) atomicAdd(sacc + l, t[l]);
-  } else {
-#pragma unroll
-    for (int l = 0; l < 8; ++l) atomicAdd(acc + scene * 8 + l, t[l]);
+    for (int l = 0; l < 8; ++l) atomicAdd(to + l, t[l]);
   }
 }
 __device__ __forceinline__ void digest_block_end(uint32_t* acc, uint32_t* sacc, uint32_t* sscene) {
