@@ -424,7 +424,7 @@ struct World {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
     void* ptrs[] = {b.state, b.stacc, b.predSlot, b.sceneOf, b.keys, b.inv, b.bond, b.bondCand, b.skey,
-                    b.sslot, b.cellStart, recBuf, b.RX, b.NQ, b.POS, b.SCN, b.DP, b.HEAT, b.CORR, b.NBR,
+                    b.sslot, b.cellStart, recBuf, b.QC, b.RX, b.NQ, b.POS, b.SCN, b.DP, b.HEAT, b.CORR, b.NBR,
                     b.NBRL, b.NBRN, (void*)b.tiles, b.TR, b.OVF, b.CB,
                     (void*)b.luts, (void*)b.WG, (void*)b.CA, (void*)b.mats, (void*)b.rcp,
                     b.scenes, b.world, b.acc, b.accLast, b.chain, b.dbg, b.err, b.work, tmpK, tmpV, hist,
@@ -496,6 +496,7 @@ struct World {
     b.PL2 = b.PL + C;
     b.RX = dalloc<int4>(C, err);
     b.NQ = dalloc<int4>(C, err);
+    b.QC = dalloc<uint32_t>((C + 7) & ~(size_t)3, err);
     b.POS = dalloc<int2>(C, err);
     b.SCN = dalloc<uint32_t>(C, err);
     b.DP = dalloc<int2>(C, err);

@@ -81,11 +81,9 @@ struct NbrOwned {
   uint32_t cut, off;
   __device__ __forceinline__ uint32_t entry(uint32_t row, uint32_t k) const { return rows[row * FU_ROW + k]; }
   __device__ __forceinline__ int4 rec(uint32_t e) const {
-    const uint32_t q = e & ~NBR_BOUNDARY;
-    return g[(int32_t)(q < cut ? q + off : q)];
+    return g[(int32_t)(e < cut ? e + off : e)];
   }
-  __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e & ~NBR_BOUNDARY); }
-  __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBR_BOUNDARY) != 0u; }
+  __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e); }
   __device__ __forceinline__ int2 wg(const Bufs&, int id) const { return swg[id]; }
   __device__ __forceinline__ int2 ca(const Bufs&, int id) const { return sca[id]; }
 };
@@ -194,6 +192,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     const int4 r = make_int4(pred.x, pred.y, 0, (int32_t)info);
     b.PL[p] = r;
     if (info & INFO_BOUNDARY) b.PL2[p] = r;
+    b.QC[p] = (info & INFO_DEAD) ? CAND_DEAD : cand_code(b.scenes[sc], pred);
     b.RX[p] = make_int4(0, 0, temp, 0);
     b.POS[p] = pos;
     b.SCN[p] = sc;
@@ -255,7 +254,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     const uint32_t r = valid ? i : 0u, p = pOf[r];
     const uint32_t w = nbr_lanes<false, L, false>(
         b, X, cutLists, valid, p, rec[r],
-        [&](uint32_t at, uint32_t q, uint32_t iq, uint32_t) { rows[r * FU_ROW + at] = q | (iq & INFO_BOUNDARY); }, f);
+        [&](uint32_t at, uint32_t q, uint32_t, uint32_t) { rows[r * FU_ROW + at] = q; }, f);
     if (valid && sub == 0) {
       word[r] = w;
       b.NBRN[p] = w;

@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
       const uint32_t p = b.inv[slot], cnt = b.NBRN[p] & NBRN_COUNT;
       for (uint32_t k = 0; k < cnt && !touched; ++k) {
         const uint32_t e = b.NBR[(size_t)k * stride + p];
-        if (e & NBR_BOUNDARY) continue;
+        if (is_wall(b.PL[e].w)) continue;
         const uint32_t js = b.sslot[e];
         if (!rg_member(b, js, tag)) continue;
         const int32_t* wj = b.state + (size_t)js * 8;

@@ -127,12 +127,13 @@ struct Bufs {
   int4* PL2;            // the other buffer of the colour sweep (one allocation with PL)
   int4* RX;             // {rho, rinv, temp, 0}
   int4* NQ;             // {nrm.x, nrm.y, rho, 0}
+  uint32_t* QC;         // candidate codes (cand_code), padded to whole 16-byte vectors
   int2* POS;
   uint32_t* SCN;
   int2* DP;
   int32_t* HEAT;
   int32_t* CORR;
-  uint32_t* NBR;        // [MAXNBR][nbrStride] sorted indices | NBR_BOUNDARY
+  uint32_t* NBR;        // [MAXNBR][nbrStride] sorted indices
   uint16_t* NBRL;       // [MAXNBR][nbrStride] the same neighbours as tile-local indices | NBRL_BOUNDARY
   uint32_t* NBRN;
   uint32_t nbrStride;
@@ -320,6 +321,8 @@ __device__ __forceinline__ uint32_t info_of(uint32_t matId, uint32_t flags, bool
 __device__ __forceinline__ bool same_body(uint32_t infoI, uint32_t infoJ) {
   return (infoI & infoJ & INFO_RIGID) != 0u && ((infoI ^ infoJ) & INFO_TAG) == 0u && (infoI & INFO_TAG) != 0u;
 }
+// The info word of a wall particle (INFO_BOUNDARY is its sign bit).
+__device__ __forceinline__ bool is_wall(int32_t info) { return info < 0; }
 __device__ __forceinline__ int2 xy(int4 v) { return make_int2(v.x, v.y); }
 __device__ __forceinline__ int2 ld_pred(const int4* PL, uint32_t q) {
   return *reinterpret_cast<const int2*>(PL + q);
@@ -405,6 +408,84 @@ __global__ void __launch_bounds__(256) k_cellstart(Bufs b) {
   cell_starts(b.skey, b.world->slotEnd, b.world->K, b.cellStart);
 }
 
+// ---- the candidate filter of the list build ----------------------------------
+//
+// About a quarter of the candidates of the 3 x 3 cells are neighbours, and an
+// exact test costs a 16-byte record and some 20 instructions. QC holds each
+// sorted particle's place inside its cell in 64ths of a cell, x in byte 0 and
+// y in byte 2, so a lane tests a candidate against its own place with an add
+// and a byte dot product, four candidates to one 16-byte load, and only the
+// survivors (about 28 %) go through the exact test. The list pass of the 1 M
+// scene fell from 261 to 190 us (2.1 k thread instructions a particle at 14
+// active lanes: what bounds it now is the lanes' uneven survivor counts), a
+// 262 k one from 117 to 84, a fused 40 k world's from 30 to 15.
+//
+// The filter never drops a neighbour. Quantised places are clamped to the
+// scene's cells as cell_coord is, and clamping brings no two points further
+// apart; with q ticks to the 64th, each axis' difference is off by less than
+// one step from flooring, y by one more where x borrows from its half, and
+// the two sign bytes add at most 2: a pair within CAND_R ticks has a dot
+// product of at most (CAND_R / q + sqrt(5))^2 + 2. A dead particle's code puts
+// 64 into byte 1, whose square alone (63^2 at least, after the add) is above
+// that for every cell size allowed (q >= 4096).
+constexpr int32_t CAND_R = (HS + 1) * 16;  // lut_index accepts only |d| < (HS + 0.7) * 16
+constexpr uint32_t CAND_DEAD = 0x4000u;
+__device__ __forceinline__ uint32_t cand_code(const ScenePar& S, int2 p) {
+  const uint32_t sh = S.cellShift - 6u;
+  const uint32_t x = (uint32_t)clampi(p.x >> sh, 0, (int32_t)(S.gridW * 64u) - 1) & 63u;
+  const uint32_t y = (uint32_t)clampi(p.y >> sh, 0, (int32_t)(S.gridH * 64u) - 1) & 63u;
+  return x | y << 16;
+}
+// What to add to the code of a candidate in the cell (dx, dy) from one's own.
+__device__ __forceinline__ uint32_t cand_bias(uint32_t own, int dx, int dy) {
+  return (uint32_t)(dx * 64 + dy * (64 << 16)) - own;
+}
+// The accumulator start that leaves a survivor's dot product negative.
+__device__ __forceinline__ int32_t cand_threshold(const ScenePar& S) {
+  const int32_t r4 = ((4 * CAND_R) >> (S.cellShift - 6u)) + 1;  // >= 4 CAND_R / q, and 9 / 4 >= sqrt(5)
+  return -((r4 + 9) * (r4 + 9) / 16 + 4);
+}
+// Survivors among the candidates [base, base + 32) that lie in [lo, hi), base a
+// multiple of 4: candidate base + j at bit 31 - j. NV vectors are in flight.
+template <int NV>
+__device__ __forceinline__ uint32_t cand_mask(const uint32_t* QC, uint32_t base, uint32_t lo, uint32_t hi,
+                                              uint32_t bias, int32_t thr) {
+  const uint32_t nv = min((hi - base + 3u) >> 2, 8u);
+  const uint4* src = reinterpret_cast<const uint4*>(QC + base);
+  uint32_t m = 0;
+  for (uint32_t v = 0; v < nv; v += NV) {
+    uint4 w[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) w[j] = src[min(v + j, nv - 1u)];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int d0 = (int)(w[j].x + bias), d1 = (int)(w[j].y + bias), d2 = (int)(w[j].z + bias),
+                d3 = (int)(w[j].w + bias);
+      m = __funnelshift_l((uint32_t)__dp4a(d0, d0, thr), m, 1);
+      m = __funnelshift_l((uint32_t)__dp4a(d1, d1, thr), m, 1);
+      m = __funnelshift_l((uint32_t)__dp4a(d2, d2, thr), m, 1);
+      m = __funnelshift_l((uint32_t)__dp4a(d3, d3, thr), m, 1);
+    }
+  }
+  const uint32_t done = 4u * ((nv + NV - 1u) / NV * NV);  // codes shifted in (a repeated vector's lie past hi)
+  m <<= 32u - done;
+  if (lo > base) m &= 0xffffffffu >> (lo - base);
+  if (hi - base < 32u) m &= ~(0xffffffffu >> (hi - base));
+  return m;
+}
+// The survivors that are in the kernel.
+template <bool DBG>
+__device__ __forceinline__ uint32_t cand_test(const int4* PL, uint32_t base, uint32_t m, int2 pi,
+                                              const Flags<DBG>& f) {
+  uint32_t keep = m;
+  while (m) {
+    const uint32_t j = (uint32_t)__clz((int)m), bit = 0x80000000u >> j;
+    m &= ~bit;
+    if (!in_kernel(pdelta(pi, ld_pred(PL, base + j), f))) keep &= ~bit;
+  }
+  return keep;
+}
+
 // The per-substep world flags one particle raises (see Bufs::work): some lanes
 // of the warp may be absent.
 __device__ __forceinline__ void raise_work(const Bufs& b, int k, bool raise) {
@@ -436,6 +517,7 @@ __global__ void __launch_bounds__(256) k_gather(Bufs b) {
     int4 rec = make_int4(pr.x, pr.y, 0, (int32_t)info_of((uint32_t)c.x, (uint32_t)c.y, i >= S.nFluid));
     b.PL[p] = rec;
     if ((uint32_t)rec.w & INFO_BOUNDARY) b.PL2[p] = rec;  // walls never move: the colour passes do not write them
+    b.QC[p] = ((uint32_t)rec.w & INFO_DEAD) ? CAND_DEAD : cand_code(S, pr);
     b.RX[p] = make_int4(0, 0, c.z, 0);
     b.POS[p] = make_int2(a.x, a.y);
     b.SCN[p] = s;
@@ -622,6 +704,12 @@ constexpr uint32_t NO_STAGE = 0x7fffffffu;  // a candidate whose tile is not sta
 // The list of one particle by L lanes (a warp calls it together; `valid` false
 // for a lane group with none): p its sorted index, `me` its record. The hits go
 // to out(position, sorted index, info, staged offset); returns the NBRN word.
+//
+// The stopping scan (`cut`) deals the particle's cells in reach to its lanes,
+// in order: each lane filters and tests its cell's candidates, a prefix over
+// the lanes gives its hits their places, and round after round the cells
+// follow in the reference's order. A cell of more candidates than two filter
+// words sends the warp to the general scan below.
 template <bool DBG, int L, bool TILED, class OUT>
 __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cellStart, bool cut, bool valid,
                                               uint32_t p, int4 me, OUT out, const Flags<DBG>& f) {
@@ -640,6 +728,62 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
   const uint32_t ts = S.tileShift, tx = (uint32_t)cc.x >> ts, ty = (uint32_t)cc.y >> ts;
   const uint32_t* tr = (TILED && work) ? b.TR + (size_t)tile_of(S, cc.x, cc.y) * TR_STRIDE : b.TR;
   const bool local = TILED && work && !bnd && tr[TR_BASE + tile_runs(ts)] <= b.world->stageCap;
+  if (!TILED && L > 1 && cut) {
+    // the cells in reach: bit 3 (dy + 1) + dx + 1
+    const uint32_t cols = ((skip & SKIP_LEFT) || cc.x == 0 ? 0u : 1u) | 2u |
+                          ((skip & SKIP_RIGHT) || cc.x + 1 >= (int32_t)S.gridW ? 0u : 4u);
+    uint32_t cells = ((skip & SKIP_DOWN) || cc.y == 0 ? 0u : cols) | cols << 3 |
+                     ((skip & SKIP_UP) || cc.y + 1 >= (int32_t)S.gridH ? 0u : cols << 6);
+    if (!work) cells = 0u;
+    const uint32_t cq = cand_code(S, pi);
+    const int32_t thr = cand_threshold(S);
+    // this lane's cells are every L-th set bit from the sub-th on
+    for (uint32_t t = 0; t < sub; ++t) cells &= cells - 1u;
+    bool fits = true;
+    uint32_t n = 0;
+    for (;;) {
+      uint32_t base = 0, m0 = 0, m1 = 0;
+      if (cells) {
+        const int k = __ffs((int)cells) - 1, dy = k / 3 - 1, dx = k - 3 * (k / 3) - 1;
+        const uint32_t key = key_of(S, cc.x + dx, cc.y + dy), lo = cellStart[key], hi = cellStart[key + 1];
+        base = lo & ~3u;
+        if (hi - base > 64u) {
+          fits = false;
+        } else {
+          const uint32_t bias = cand_bias(cq, dx, dy);
+          if (base < hi) m0 = cand_mask<4>(b.QC, base, lo, hi, bias, thr);
+          if (base + 32 < hi) m1 = cand_mask<4>(b.QC, base + 32, lo, hi, bias, thr);
+          if (k == 4 && p - base < 32u) m0 &= ~(0x80000000u >> (p - base));
+          if (k == 4 && p - base - 32u < 32u) m1 &= ~(0x80000000u >> (p - base - 32u));
+          m0 = cand_test(b.PL, base, m0, pi, f);
+          m1 = cand_test(b.PL, base + 32, m1, pi, f);
+        }
+      }
+      if (__any_sync(0xffffffffu, !fits)) break;
+      const uint32_t mine = (uint32_t)(__popc(m0) + __popc(m1));
+      uint32_t inc = mine;
+#pragma unroll
+      for (int o = 1; o < L; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o, L);
+        if (sub >= (uint32_t)o) inc += v;
+      }
+      uint32_t at = n + inc - mine;
+      n += __shfl_sync(0xffffffffu, inc, L - 1, L);
+      for (; m0 && at < (uint32_t)MAXNBR; ++at) {
+        const uint32_t j = (uint32_t)__clz((int)m0);
+        m0 &= ~(0x80000000u >> j);
+        out(at, base + j, 0u, NO_STAGE);
+      }
+      for (; m1 && at < (uint32_t)MAXNBR; ++at) {
+        const uint32_t j = (uint32_t)__clz((int)m1);
+        m1 &= ~(0x80000000u >> j);
+        out(at, base + 32u + j, 0u, NO_STAGE);
+      }
+#pragma unroll
+      for (int t = 0; t < L; ++t) cells &= cells - 1u;
+      if (!__any_sync(0xffffffffu, cells != 0u && n < (uint32_t)MAXNBR)) return work ? min(n, (uint32_t)MAXNBR) : 0u;
+    }
+  }
   for (int dy = -1; dy <= 1; ++dy) {
     for (int dx = -1; dx <= 1; ++dx) {
       const int32_t gy = cc.y + dy, gx = cc.x + dx;
@@ -704,7 +848,7 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
 // once and place the hits with a ballot prefix, so the list keeps exactly the
 // sequential order (and the same MAXNBR cut) whatever L is.
 template <bool DBG, int L, bool TILED>
-__global__ void __launch_bounds__(256, TILED ? 6 : 8) k_nbr(Bufs b) {
+__global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
   // Once a list is full, a later candidate can only raise a flag bit or the
   // overflow counter. With no live SEAL/CONGEAL fluid particle in the world
   // and no counters kept, nothing it could change remains, so the scan stops:
@@ -723,6 +867,8 @@ __global__ void __launch_bounds__(256, TILED ? 6 : 8) k_nbr(Bufs b) {
       int2 pi = xy(me);
       int2 cc = cell_coord(S, pi);
       const uint32_t skip = far_sides(S, pi, cc);
+      const uint32_t cq = cand_code(S, pi);
+      const int32_t thr = cand_threshold(S);
       uint32_t cnt = 0;
       bool congeal = false, sealSeen = false;
       uint32_t* out = b.NBR + p;
@@ -745,16 +891,18 @@ __global__ void __launch_bounds__(256, TILED ? 6 : 8) k_nbr(Bufs b) {
           if (!TILED && cut) {
             // The stopping scan: no live fluid particle carries SEAL or
             // CONGEAL (so neither flag can be raised) and the list ends at
-            // MAXNBR (so nothing overflows); the next record is loaded one
-            // candidate ahead.
-            int4 nx = lo < hi ? b.PL[lo] : make_int4(0, 0, 0, 0);
-            for (uint32_t q = lo; q < hi; ++q) {
-              const int4 o = nx;
-              if (q + 1 < hi) nx = b.PL[q + 1];
-              const uint32_t iq = (uint32_t)o.w;
-              if (q == p || (iq & INFO_DEAD) || !in_kernel(pdelta(pi, xy(o), f))) continue;
-              out[(size_t)cnt * stride] = q | (iq & INFO_BOUNDARY);
-              if (++cnt >= (uint32_t)MAXNBR) goto listed;
+            // MAXNBR (so nothing overflows).
+            const uint32_t bias = cand_bias(cq, dx, dy);
+            for (uint32_t base = lo & ~3u; base < hi; base += 32) {
+              uint32_t m = cand_mask<2>(b.QC, base, lo, hi, bias, thr);
+              if (dx == 0 && dy == 0 && p - base < 32u) m &= ~(0x80000000u >> (p - base));
+              while (m) {
+                const uint32_t j = (uint32_t)__clz((int)m), q = base + j;
+                m &= ~(0x80000000u >> j);
+                if (!in_kernel(pdelta(pi, ld_pred(b.PL, q), f))) continue;
+                out[(size_t)cnt * stride] = q;
+                if (++cnt >= (uint32_t)MAXNBR) goto listed;
+              }
             }
             continue;
           }
@@ -768,7 +916,7 @@ __global__ void __launch_bounds__(256, TILED ? 6 : 8) k_nbr(Bufs b) {
             if (!(iq & INFO_BOUNDARY) && (iq & INFO_CONGEAL)) congeal = true;
             if (!(iq & INFO_BOUNDARY) && (iq & INFO_SEAL)) sealSeen = true;
             if (cnt >= (uint32_t)MAXNBR) { f.flag(6); continue; }
-            if (!bnd) out[(size_t)cnt * stride] = q | (iq & INFO_BOUNDARY);
+            if (!bnd) out[(size_t)cnt * stride] = q;
             if (TILED && local)
               outl[(size_t)cnt * stride] = (uint16_t)((q + delta) | ((iq & INFO_BOUNDARY) ? NBRL_BOUNDARY : 0u));
             cnt++;
@@ -791,7 +939,7 @@ __global__ void __launch_bounds__(256, TILED ? 6 : 8) k_nbr(Bufs b) {
     const uint32_t word = nbr_lanes<DBG, L, TILED>(
         b, b.cellStart, cut, valid, p, me,
         [&](uint32_t pos, uint32_t q, uint32_t iq, uint32_t delta) {
-          b.NBR[(size_t)pos * stride + p] = q | (iq & INFO_BOUNDARY);
+          b.NBR[(size_t)pos * stride + p] = q;
           if (TILED && delta != NO_STAGE)
             b.NBRL[(size_t)pos * stride + p] = (uint16_t)((q + delta) | ((iq & INFO_BOUNDARY) ? NBRL_BOUNDARY : 0u));
         },
@@ -820,7 +968,6 @@ struct NbrStaged {
   __device__ __forceinline__ int2 pred(uint32_t e) const {
     return *reinterpret_cast<const int2*>(sm + (e & NBRL_INDEX));
   }
-  __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBRL_BOUNDARY) != 0u; }
   __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
 };
 // Neighbour access from global memory: records in PL, sorted-index entries.
@@ -829,9 +976,8 @@ struct NbrGlobal {
   const uint32_t* nl;
   uint32_t stride;
   __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[(size_t)k * stride + p]; }
-  __device__ __forceinline__ int4 rec(uint32_t e) const { return g[e & ~NBR_BOUNDARY]; }
-  __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e & ~NBR_BOUNDARY); }
-  __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBR_BOUNDARY) != 0u; }
+  __device__ __forceinline__ int4 rec(uint32_t e) const { return g[e]; }
+  __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e); }
   __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
   __device__ __forceinline__ int2 ca(const Bufs& b, int id) const { return __ldg(b.CA + id); }
 };
@@ -1025,7 +1171,7 @@ __device__ __forceinline__ int2 solveB_dp(const Bufs& b, const NB& nb, uint32_t 
       on = nb.rec(en);
     }
     if (k + 2 * L < cnt) en2 = nb.entry(p, k + 2 * L);
-    const bool wall = nb.wall(e);
+    const bool wall = is_wall(o.w);
     if constexpr (RIG) {
       if (!wall && same_body(infoI, (uint32_t)o.w)) continue;
     }
@@ -1113,10 +1259,8 @@ struct NbrSplit {
   uint32_t stride;
   __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[(size_t)k * stride + p]; }
   __device__ __forceinline__ int4 rec(uint32_t e) const {
-    const uint32_t q = e & ~NBR_BOUNDARY;
-    return src[(int32_t)(q < cut ? q + off : q)];
+    return src[(int32_t)(e < cut ? e + off : e)];
   }
-  __device__ __forceinline__ bool wall(uint32_t e) const { return (e & NBR_BOUNDARY) != 0u; }
   __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
 };
 
@@ -1282,8 +1426,8 @@ __device__ __forceinline__ void friction_particle(const Bufs& b, const NB& nb, b
   int32_t fx = 0, fy = 0;
   // one neighbour ahead (record and old position), two ahead (index)
   uint32_t en = sub < cnt ? nb.entry(row, sub) : 0u;
-  int4 on = b.PL[en & ~NBR_BOUNDARY];
-  int2 sn = b.POS[en & ~NBR_BOUNDARY];
+  int4 on = b.PL[en];
+  int2 sn = b.POS[en];
   uint32_t en2 = sub + L < cnt ? nb.entry(row, sub + L) : 0u;
   for (uint32_t k = sub; k < cnt; k += L) {
     const uint32_t e = en;
@@ -1291,11 +1435,11 @@ __device__ __forceinline__ void friction_particle(const Bufs& b, const NB& nb, b
     const int2 so = sn;
     if (k + L < cnt) {
       en = en2;
-      on = b.PL[en & ~NBR_BOUNDARY];
-      sn = b.POS[en & ~NBR_BOUNDARY];
+      on = b.PL[en];
+      sn = b.POS[en];
     }
     if (k + 2 * L < cnt) en2 = nb.entry(row, k + 2 * L);
-    if (rigidI && !(e & NBR_BOUNDARY) && same_body(info, (uint32_t)o.w)) continue;
+    if (rigidI && !is_wall(o.w) && same_body(info, (uint32_t)o.w)) continue;
     int2 pq = xy(o);
     int2 d = pdelta(pi, pq, f);
     int id = lut_index(d, f);
@@ -1305,7 +1449,7 @@ __device__ __forceinline__ void friction_particle(const Bufs& b, const NB& nb, b
     if (d2 < D2_FLOOR) continue;
     int2 rel = dxi;
     int32_t mu = fi;
-    if (!(e & NBR_BOUNDARY)) {
+    if (!is_wall(o.w)) {
       int2 dq = delta(pq, so, f);
       rel = make_int2(sub_sat(dxi.x, dq.x, f), sub_sat(dxi.y, dq.y, f));
       mu = mat_mix(fi, matw(b, (uint32_t)o.w & INFO_MAT, M_fric));
@@ -1511,9 +1655,9 @@ __device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, cons
   // the neighbour's three records (pred/info, rho/rinv/T, old position)
   // one ahead, its index two ahead
   uint32_t en = sub < cnt ? nb.entry(row, sub) : 0u;
-  int4 on = b.PL[en & ~NBR_BOUNDARY];
-  int4 rn = b.RX[en & ~NBR_BOUNDARY];
-  int2 sn = b.POS[en & ~NBR_BOUNDARY];
+  int4 on = b.PL[en];
+  int4 rn = b.RX[en];
+  int2 sn = b.POS[en];
   uint32_t en2 = sub + L < cnt ? nb.entry(row, sub + L) : 0u;
   for (uint32_t k = sub; k < cnt; k += L) {
     const uint32_t e = en;
@@ -1522,12 +1666,12 @@ __device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, cons
     const int2 so = sn;
     if (k + L < cnt) {
       en = en2;
-      on = b.PL[en & ~NBR_BOUNDARY];
-      rn = b.RX[en & ~NBR_BOUNDARY];
-      sn = b.POS[en & ~NBR_BOUNDARY];
+      on = b.PL[en];
+      rn = b.RX[en];
+      sn = b.POS[en];
     }
     if (k + 2 * L < cnt) en2 = nb.entry(row, k + 2 * L);
-    if (e & NBR_BOUNDARY) continue;
+    if (is_wall(o.w)) continue;
     const int2 pq = xy(o);
     const int2 d = pdelta(pi, pq, f);
     const int id = lut_index(d, f);
@@ -1642,20 +1786,21 @@ __device__ __forceinline__ int seal_cross_sign(int32_t ax, int32_t ay, int32_t b
 // The geometry contain and containOverflow share: a keep-out push from each
 // seal endpoint, then the swept-segment test against every pair of seal
 // endpoints, where a crossing reverts this substep's motion. `entry(k)` gives
-// the k-th candidate's sorted index with NBR_BOUNDARY set for wall particles;
+// the k-th candidate's sorted index;
 // `filter` means the list still holds entries that are not seal endpoints.
 template <bool DBG, typename Entry>
 __device__ int2 contain_core(const Bufs& b, Entry entry, uint32_t n, bool filter, int2 pos, int2 pr, bool liquidI,
                              const Flags<DBG>& f) {
   auto seal_at = [&](uint32_t e) {
-    return !(e & NBR_BOUNDARY) && seal_class(b, (uint32_t)b.PL[e & ~NBR_BOUNDARY].w & INFO_MAT);
+    const int32_t w = b.PL[e].w;
+    return !is_wall(w) && seal_class(b, (uint32_t)w & INFO_MAT);
   };
   bool touched = false;
   for (uint32_t k = 0; k < n; ++k) {
     const uint32_t e = entry(k);
     if (filter && !seal_at(e)) continue;
     touched = true;
-    const int2 pj = ld_pred(b.PL, e & ~NBR_BOUNDARY);
+    const int2 pj = ld_pred(b.PL, e);
     const int32_t dx4 = shr_rne<BPRE>(sub_sat(pr.x, pj.x, f)), dy4 = shr_rne<BPRE>(sub_sat(pr.y, pj.y, f));
     const int32_t d2 = wadd(wmul(dx4, dx4), wmul(dy4, dy4));
     if (d2 > 0 && d2 < SEAL_KEEP4 * SEAL_KEEP4) {
@@ -1672,14 +1817,13 @@ __device__ int2 contain_core(const Bufs& b, Entry entry, uint32_t n, bool filter
   for (uint32_t k = 0; k < n; ++k) {
     const uint32_t e = entry(k);
     if (filter && !seal_at(e)) continue;
-    const uint32_t j = e & ~NBR_BOUNDARY;
-    const int4 oj = b.PL[j];
+    const int4 oj = b.PL[e];
     const int32_t sealModeJ = matw(b, (uint32_t)oj.w & INFO_MAT, M_sealMode);
     const int2 pj = xy(oj);
     for (uint32_t q = k + 1; q < n; ++q) {
       const uint32_t e2 = entry(q);
       if (filter && !seal_at(e2)) continue;
-      const int4 ok = b.PL[e2 & ~NBR_BOUNDARY];
+      const int4 ok = b.PL[e2];
       if (liquidI && sealModeJ != 0 && matw(b, (uint32_t)ok.w & INFO_MAT, M_sealMode) != 0) continue;
       const int2 pk = xy(ok);
       const int32_t ex4 = shr_rne<BPRE>(sub_sat(pk.x, pj.x, f)), ey4 = shr_rne<BPRE>(sub_sat(pk.y, pj.y, f));
@@ -1789,7 +1933,7 @@ __device__ __forceinline__ void contain_stress_slot(const Bufs& b, const NB& nb,
   int32_t stress = 0;
   for (uint32_t k = sub; k < cnt; k += L) {
     const uint32_t e = nb.entry(r, k);
-    if (e & NBR_BOUNDARY) continue;
+    if (is_wall(b.PL[e].w)) continue;
     const int32_t* wj = b.state + (size_t)b.sslot[e] * 8;
     const uint32_t mj = (uint32_t)wj[4];
     if (seal_class(b, mj) || matw(b, mj, M_phantom) != 0) continue;
@@ -1883,8 +2027,8 @@ __device__ __forceinline__ int2 post2_sums(const Bufs& b, const NB& nb, const in
   int32_t ax = 0, ay = 0;
   // the neighbour's record and normal/density one ahead, its index two ahead
   uint32_t en = sub < cnt ? nb.entry(row, sub) : 0u;
-  int4 on = b.PL[en & ~NBR_BOUNDARY];
-  int4 nn = b.NQ[en & ~NBR_BOUNDARY];
+  int4 on = b.PL[en];
+  int4 nn = b.NQ[en];
   uint32_t en2 = sub + L < cnt ? nb.entry(row, sub + L) : 0u;
   for (uint32_t k = sub; k < cnt; k += L) {
     const uint32_t e = en;
@@ -1892,17 +2036,17 @@ __device__ __forceinline__ int2 post2_sums(const Bufs& b, const NB& nb, const in
     const int4 nq = nn;
     if (k + L < cnt) {
       en = en2;
-      on = b.PL[en & ~NBR_BOUNDARY];
-      nn = b.NQ[en & ~NBR_BOUNDARY];
+      on = b.PL[en];
+      nn = b.NQ[en];
     }
     if (k + 2 * L < cnt) en2 = nb.entry(row, k + 2 * L);
     // a rigid member's cohesion skips its own body (src/sim.wgsl:2450-2457)
-    if ((info & INFO_RIGID) && !(e & NBR_BOUNDARY) && same_body(info, (uint32_t)o.w)) continue;
+    if ((info & INFO_RIGID) && !is_wall(o.w) && same_body(info, (uint32_t)o.w)) continue;
     const int2 d = pdelta(pi, xy(o), f);
     const int id = lut_index(d, f);
     if (id < 0) continue;
     const int2 ca = nb.ca(b, id);
-    if (e & NBR_BOUNDARY) {
+    if (is_wall(o.w)) {
       ax = wsub(ax, mulfc<8>(mulf<22>(ca.y, d.x, f), mi.z, -ST_TERM, ST_TERM, f));
       ay = wsub(ay, mulfc<8>(mulf<22>(ca.y, d.y, f), mi.z, -ST_TERM, ST_TERM, f));
       continue;
@@ -2055,7 +2199,7 @@ __device__ __forceinline__ void form1_particle(const Bufs& b, const NB& nb, uint
   bool seen = false;
   for (uint32_t k = 0; k < cnt; ++k) {
     uint32_t e = nb.entry(row, k);
-    if (e & NBR_BOUNDARY) continue;
+    if (is_wall(b.PL[e].w)) continue;
     uint32_t qs = b.sslot[e];
     if ((uint32_t)b.state[(size_t)qs * 8 + 5] & FLAG_CONGEAL) { seen = true; break; }
   }
@@ -2079,7 +2223,7 @@ __device__ __forceinline__ void form1_particle(const Bufs& b, const NB& nb, uint
       for (uint32_t k = 0; k < cnt; ++k) {
         if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
         uint32_t e = nb.entry(row, k);
-        if (e & NBR_BOUNDARY) continue;
+        if (is_wall(b.PL[e].w)) continue;
         uint32_t qs = b.sslot[e];
         const int32_t* wj = b.state + (size_t)qs * 8;
         uint32_t j = qs - S.slotBase;

@@ -37,8 +37,7 @@ constexpr int MAT_WORDS = 48;
 constexpr int MAT_MAX = 64;
 constexpr int TN = 3202;
 constexpr int LUT_WORDS = 5 * TN;
-constexpr uint32_t NBR_BOUNDARY = 0x80000000u;  // set in a neighbour entry when it is a wall particle
-constexpr uint16_t NBRL_BOUNDARY = 0x8000u;     // the same flag in a tile-local (16-bit) entry
+constexpr uint16_t NBRL_BOUNDARY = 0x8000u;  // set in a tile-local (16-bit) entry when it is a wall particle
 constexpr uint16_t NBRL_INDEX = 0x7fffu;
 
 // Tiles: side 2^tileShift cells, tileShift in [TILE_SHIFT_MIN, TILE_SHIFT_MAX].
