@@ -462,6 +462,8 @@ struct World {
     std::memcpy(hmats, o->mats, sizeof(int32_t) * MAT_WORDS * o->mat_count);
     std::memcpy(hauth, hmats, sizeof(hauth));
     matCount = authoredCount = o->mat_count;
+    tablesOk = tables_in_range(o->luts);
+    inRange = tablesOk && rows_in_range(hmats, matCount);
     for (uint32_t m = 0; m < matCount; ++m) {
       const int32_t* r = hmats + m * MAT_WORDS;
       if (r[M_eps] < 32768) return fail("mats[%u].eps < 32768", m);
@@ -1078,6 +1080,9 @@ struct World {
   // ---- the fused substep of small worlds (fused2d.cuh) ----
   uint32_t* fuBar = nullptr;    // barrier words, zero between launches
   uint32_t* fuCount = nullptr;  // [keyCap] cell counts, zero between launches
+  // the tables and every row lie in the ranges the release kernels are built
+  // for; else the debug kernels, which assume none, run
+  bool inRange = true, tablesOk = true;
   bool graphFused = false;      // what the captured graph launches, and the
   uint32_t graphOwn = 0;        // particles a CTA it was sized for
   // One past the last slot that can hold an active particle.
@@ -1101,7 +1106,7 @@ struct World {
   // slot a thread, the cell ranges, the owned particles' lists).
   bool fused_fits() const {
     const uint64_t G = (uint64_t)numSMs;
-    return !debug && !staged && !persistent && autoLanes && bodies.empty() && hw.nAct > 0 &&
+    return !debug && inRange && !staged && !persistent && autoLanes && bodies.empty() && hw.nAct > 0 &&
            slots_used() <= G * FU_T && fused_own() <= fused_own_cap();
   }
   template <int L, int LC>
@@ -1413,7 +1418,7 @@ struct World {
 
   void launch_one(bool fused = false) {
     if (fused) launch_fused();
-    else if (debug) launch_substep<true>();
+    else if (debug || !inRange) launch_substep<true>();
     else launch_substep<false>();
   }
 
@@ -2385,6 +2390,7 @@ struct World {
   // baked from its ramp, grav scaled by the world gravity. `row` may be the
   // next free row (the table grows) or an existing row past the authored ones.
   bool upload_mats(uint32_t lo, uint32_t hi) {
+    inRange = tablesOk && rows_in_range(hmats, matCount);
     if (hi <= lo) return true;
     graphValid = false;
     accFresh = false;

@@ -34,8 +34,13 @@
 // [0, 2^27] and wall particles lie in [-2^27, 2^27], so pred differences never
 // overflow; an accepted neighbour has |d| <= 163848 < 2^18; |G| < 2^27, so a
 // gradient term is < 2^19; |lambda| <= 2^22; |vel| <= 2^16; K_ij <= 2^18;
-// |T| <= 2^29. Under these bounds every per-pair product below either fits in
-// i32 after its shift (mulf) or is clamped at once into an i32 range (mulc).
+// |T| <= 2^29; a gradient |G d| >> 26 is below
+// 2^15 and |C d| >> 22, |A d| >> 22 below 2^17 (tables_in_range); a normal sum is
+// below 2^24; |gammaCoh| <= 2^19 and |gammaCur| < 2^11 (rows_in_range). Under
+// these bounds every per-pair product below either fits in i32 after its shift
+// (mulf) or is clamped at once into an i32 range (mulc). The host checks the
+// tables and rows it is given and runs the debug build's kernels, which need
+// none of this, where they lie outside.
 #pragma once
 #include <cstdint>
 #include "fixed.cuh"
@@ -106,6 +111,30 @@ enum : int {
   M_burstP = 46, M_sealMode = 47
 };
 constexpr int32_t SOLID_RIGID = 2;
+
+// What the release build's arithmetic takes from the kernel tables and the
+// material rows (see above); host.
+inline bool tables_in_range(const int32_t* luts) {
+  for (int i = 0; i < TN; ++i) {
+    // the largest |d| on one axis with table index i: 16 * sqrt((i + 1) * 2^15) + 8
+    int64_t d = 0;
+    for (int64_t step = 1 << 18; step; step >>= 1)
+      if ((d + step) * (d + step) <= 256ll * 32768 * (i + 1)) d += step;
+    d += 9;
+    auto mag = [](int32_t v) { return v < 0 ? -(int64_t)v : (int64_t)v; };
+    if (luts[i] < 0 || luts[i] >= 1 << 18) return false;
+    if ((mag(luts[TN + i]) * d >> 26) + 1 >= 1 << 15) return false;
+    if ((mag(luts[2 * TN + i]) * d >> 22) + 1 >= 1 << 17 || (mag(luts[3 * TN + i]) * d >> 22) + 1 >= 1 << 17) return false;
+  }
+  return true;
+}
+inline bool rows_in_range(const int32_t* mats, uint32_t count) {
+  for (uint32_t m = 0; m < count; ++m) {
+    const int32_t coh = mats[m * MAT_WORDS + M_gammaCoh], cur = mats[m * MAT_WORDS + M_gammaCur];
+    if (coh > 1 << 19 || coh < -(1 << 19) || cur > 2047 || cur < -2047) return false;
+  }
+  return true;
+}
 
 // All device buffers of a world, passed by value.
 struct Bufs {
@@ -218,8 +247,19 @@ __device__ __forceinline__ int2 wall_clamp(const ScenePar& S, int2 p) {
   return make_int2(clampi(p.x, WALL, S.domW - WALL), clampi(p.y, WALL, S.domH - WALL));
 }
 __device__ __forceinline__ int32_t mat_mix(int32_t a, int32_t b) { return wadd(a, b) >> 1; }
+// rho is a sum of at most 49 table values below 2^18, so the release build's
+// den lies in [2^16, 2^25): divshift's shift of 2^21 * Rn is by 14 + e with e in
+// 1..9, that is Rn * 2^(7 - e), rounded only for e = 8 and 9 (a mean density
+// above 4 rho0).
 template <bool DBG>
 __device__ __forceinline__ int32_t sym_k(int32_t ri, int32_t rj, const uint16_t* rcp, const Flags<DBG>& f) {
+  if constexpr (!DBG) {
+    const int32_t den = max(RHO_FLOOR_K, ri + rj), e = 16 - __clz(den);
+    const int32_t Rn = (int32_t)__ldg(rcp + ((den >> e) - 32768));
+    if (e <= 7) return min(Rn << (7 - e), RINV_MAX);
+    const int32_t q = Rn >> (e - 7), r = Rn - (q << (e - 7)), half = 1 << (e - 8);
+    return q + ((r > half || (r == half && (q & 1))) ? 1 : 0);
+  }
   int32_t den = max(RHO_FLOOR_K, add_sat(ri, rj, f));
   return clampi(divshift<16>(TWO_RHO0, den, rcp, f), 0, RINV_MAX);
 }
@@ -1011,6 +1051,32 @@ __device__ __forceinline__ bool stage_tile(const Bufs& b, const int4* from, cons
   return *okS != 0u;
 }
 
+// One axis of solveA's |grad C|^2 term: clamp(RNE(g * g / 2^11), 0, S_TERM).
+// |g| < 2^15 (tables_in_range), so the square fits i32 and stays below
+// S_TERM * 2^11; and a square is never an odd multiple of 2^11 away from a tie:
+// g * g = 1024 mod 2048 only for g = 32 * odd, where g * g = 1024 mod 8192, so
+// the tie's floor is even and it rounds down.
+template <bool DBG>
+__device__ __forceinline__ int32_t grad_sq(int32_t g, const Flags<DBG>& f) {
+  if constexpr (DBG) return mulfc<11>(g, g, 0, S_TERM, f);
+  else return (g * g + 1023) >> 11;
+}
+
+// One neighbour's terms of solveA's sums.
+template <bool DBG, class NB>
+__device__ __forceinline__ void solveA_pair(const Bufs& b, const NB& nb, int2 pi, int2 pj, const Flags<DBG>& f,
+                                            int32_t& rho, int32_t& S, int32_t& sgx, int32_t& sgy) {
+  const int2 d = pdelta(pi, pj, f);
+  const int id = lut_index(d, f);
+  if (id < 0) return;
+  const int2 wg = nb.wg(b, id);
+  rho = wadd(rho, wg.x);
+  const int32_t gx = mulf<26>(wg.y, d.x, f), gy = mulf<26>(wg.y, d.y, f);
+  sgx = wadd(sgx, gx);
+  sgy = wadd(sgy, gy);
+  S = wadd(S, wadd(grad_sq<DBG>(gx, f), grad_sq<DBG>(gy, f)));
+}
+
 // solveA's neighbour sums for one particle (L lanes share its list).
 template <bool DBG, int L, class NB>
 __device__ __forceinline__ void solveA_sums(const Bufs& b, const NB& nb, uint32_t p, uint32_t cnt, uint32_t sub,
@@ -1025,15 +1091,7 @@ __device__ __forceinline__ void solveA_sums(const Bufs& b, const NB& nb, uint32_
     const int2 pj = pn;
     if (k + L < cnt) pn = nb.pred(en2);
     if (k + 2 * L < cnt) en2 = nb.entry(p, k + 2 * L);
-    const int2 d = pdelta(pi, pj, f);
-    const int id = lut_index(d, f);
-    if (id < 0) continue;
-    const int2 wg = nb.wg(b, id);
-    rho = wadd(rho, wg.x);
-    const int32_t gx = mulf<26>(wg.y, d.x, f), gy = mulf<26>(wg.y, d.y, f);
-    sgx = wadd(sgx, gx);
-    sgy = wadd(sgy, gy);
-    S = wadd(S, wadd(mulfc<11>(gx, gx, 0, S_TERM, f), mulfc<11>(gy, gy, 0, S_TERM, f)));
+    solveA_pair<DBG>(b, nb, pi, pj, f, rho, S, sgx, sgy);
   }
   if (L > 1) {
     rho = gsum<L>(rho);
@@ -1151,9 +1209,25 @@ __global__ void __launch_bounds__(256, 4) k_solveA_tiled(Bufs b, int lastIter) {
   }
 }
 
-// solveB_at (src/sim.wgsl:1337-1372) for one particle. The S table is all
-// zeros in the frozen tables (scorrK = 0, checked at load), so the release
+// One neighbour's terms of solveB_at (src/sim.wgsl:1337-1372). The S table is
+// all zeros in the frozen tables (scorrK = 0, checked at load), so the release
 // build drops its term; debug builds still read it.
+template <bool DBG, class NB>
+__device__ __forceinline__ void solveB_pair(const Bufs& b, const NB& nb, int2 pi, int32_t li, int4 o,
+                                            const Flags<DBG>& f, int32_t& dpx, int32_t& dpy) {
+  const int2 d = pdelta(pi, xy(o), f);
+  const int id = lut_index(d, f);
+  if (id < 0) return;
+  const int32_t lj = is_wall(o.w) ? li : o.z;
+  int32_t co;
+  if constexpr (DBG) co = add_sat(add_sat(li, lj, f), __ldg(b.luts + 4 * TN + id), f);
+  else co = li + lj;
+  const int32_t gt = nb.wg(b, id).y;
+  dpx = wadd(dpx, mulfc<12>(co, mulf<26>(gt, d.x, f), -DP_TERM, DP_TERM, f));
+  dpy = wadd(dpy, mulfc<12>(co, mulf<26>(gt, d.y, f), -DP_TERM, DP_TERM, f));
+}
+
+// solveB_at for one particle.
 // RIG: the warp holds a rigid member, whose own correction skips the members
 // of its body (src/sim.wgsl:1355-1358).
 template <bool DBG, int L, bool RIG, class NB>
@@ -1171,20 +1245,10 @@ __device__ __forceinline__ int2 solveB_dp(const Bufs& b, const NB& nb, uint32_t 
       on = nb.rec(en);
     }
     if (k + 2 * L < cnt) en2 = nb.entry(p, k + 2 * L);
-    const bool wall = is_wall(o.w);
     if constexpr (RIG) {
-      if (!wall && same_body(infoI, (uint32_t)o.w)) continue;
+      if (!is_wall(o.w) && same_body(infoI, (uint32_t)o.w)) continue;
     }
-    const int2 d = pdelta(pi, xy(o), f);
-    const int id = lut_index(d, f);
-    if (id < 0) continue;
-    const int32_t lj = wall ? li : o.z;
-    int32_t co;
-    if constexpr (DBG) co = add_sat(add_sat(li, lj, f), __ldg(b.luts + 4 * TN + id), f);
-    else co = li + lj;
-    const int32_t gt = nb.wg(b, id).y;
-    dpx = wadd(dpx, mulfc<12>(co, mulf<26>(gt, d.x, f), -DP_TERM, DP_TERM, f));
-    dpy = wadd(dpy, mulfc<12>(co, mulf<26>(gt, d.y, f), -DP_TERM, DP_TERM, f));
+    solveB_pair<DBG>(b, nb, pi, li, o, f, dpx, dpy);
   }
   if (L > 1) {
     dpx = gsum<L>(dpx);
@@ -1683,11 +1747,16 @@ __device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, cons
       int32_t K = sym_k(rhoi, rx.x, b.rcp, f);
       int32_t wk = mulf<16>(W, K, f);
       int32_t cij = mat_mix(mi.x, mj.x);
-      int2 vj = delta(pq, so, f);
-      vj.x = clampi(vj.x, vmaxN, vmax);
-      vj.y = clampi(vj.y, vmaxN, vmax);
-      ax = wadd(ax, mulfc<16>(mulf<12>(sub_sat(vj.x, vi.x, f), wk, f), cij, -XS_TERM, XS_TERM, f));
-      ay = wadd(ay, mulfc<16>(mulf<12>(sub_sat(vj.y, vi.y, f), wk, f), cij, -XS_TERM, XS_TERM, f));
+      int2 vj;
+      if constexpr (DBG) {
+        vj = delta(pq, so, f);
+        vj = make_int2(clampi(vj.x, vmaxN, vmax), clampi(vj.y, vmaxN, vmax));
+      } else {  // the same for any old position: pq lies within the kernel of a particle in the domain
+        vj = make_int2(pq.x - clampi(so.x, pq.x - vmax, pq.x + vmax), pq.y - clampi(so.y, pq.y - vmax, pq.y + vmax));
+      }
+      const int2 dv = pdelta(vj, vi, f);
+      ax = wadd(ax, mulfc<16>(mulf<12>(dv.x, wk, f), cij, -XS_TERM, XS_TERM, f));
+      ay = wadd(ay, mulfc<16>(mulf<12>(dv.y, wk, f), cij, -XS_TERM, XS_TERM, f));
     }
     sx = wadd(sx, mulf<16>(mulf<26>(wg.y, d.x, f), rx.y, f));
     sy = wadd(sy, mulf<16>(mulf<26>(wg.y, d.y, f), rx.y, f));
@@ -2055,14 +2124,20 @@ __device__ __forceinline__ int2 post2_sums(const Bufs& b, const NB& nb, const in
     const int4 mj = smat[(uint32_t)o.w & INFO_MAT];
     const int32_t gCoh = mat_mix(mi.x, mj.x);
     const int32_t gCur = mat_mix(mi.y, mj.y);
-    int32_t fx = neg_sat(mulf<16>(mulf<22>(ca.x, d.x, f), gCoh, f), f);
-    int32_t fy = neg_sat(mulf<16>(mulf<22>(ca.x, d.y, f), gCoh, f), f);
-    const int32_t cx = mulf<16>(sub_sat(nqi.x, nq.x, f), gCur, f);
-    const int32_t cy = mulf<16>(sub_sat(nqi.y, nq.y, f), gCur, f);
-    fx = add_sat(fx, neg_sat(cx, f), f);
-    fy = add_sat(fy, neg_sat(cy, f), f);
-    ax = wadd(ax, mulc<8>(fx, K, -ST_TERM, ST_TERM, f));
-    ay = wadd(ay, mulc<8>(fy, K, -ST_TERM, ST_TERM, f));
+    const int32_t hx = mulf<16>(mulf<22>(ca.x, d.x, f), gCoh, f);
+    const int32_t hy = mulf<16>(mulf<22>(ca.x, d.y, f), gCoh, f);
+    const int2 dn = pdelta(make_int2(nqi.x, nqi.y), make_int2(nq.x, nq.y), f);
+    const int32_t cx = mulf<16>(dn.x, gCur, f), cy = mulf<16>(dn.y, gCur, f);
+    if constexpr (DBG) {
+      const int32_t fx = add_sat(neg_sat(hx, f), neg_sat(cx, f), f), fy = add_sat(neg_sat(hy, f), neg_sat(cy, f), f);
+      ax = wadd(ax, mulc<8>(fx, K, -ST_TERM, ST_TERM, f));
+      ay = wadd(ay, mulc<8>(fy, K, -ST_TERM, ST_TERM, f));
+    } else {
+      // |h| < 2^19.1 and |c| < 2^20 (rows_in_range), K <= 2^18: the product's
+      // shift fits i32
+      ax = wadd(ax, mulfc<8>(-hx - cx, K, -ST_TERM, ST_TERM, f));
+      ay = wadd(ay, mulfc<8>(-hy - cy, K, -ST_TERM, ST_TERM, f));
+    }
   }
   if (L > 1) {
     ax = gsum<L>(ax);
