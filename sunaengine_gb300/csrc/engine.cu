@@ -1152,8 +1152,8 @@ struct World {
     }
     // as many lanes a particle as leave one round of a CTA's threads
     const uint32_t own = fused_own();
-    if (own <= 128) launch_fused_as<8, 8>();
-    else if (own <= 256) launch_fused_as<4, 8>();
+    if (own <= 128) launch_fused_as<8, 16>();
+    else if (own <= 256) launch_fused_as<4, 16>();
     else if (own <= 512) launch_fused_as<2, 8>();
     else launch_fused_as<2, 4>();
     launchesPerSubstep = Lc;
