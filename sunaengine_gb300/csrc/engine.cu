@@ -1152,7 +1152,8 @@ struct World {
     }
     // as many lanes a particle as leave one round of a CTA's threads
     const uint32_t own = fused_own();
-    if (own <= 128) launch_fused_as<8, 16>();
+    if (own <= 64) launch_fused_as<16, 16>();
+    else if (own <= 128) launch_fused_as<8, 16>();
     else if (own <= 256) launch_fused_as<4, 16>();
     else if (own <= 512) launch_fused_as<2, 8>();
     else launch_fused_as<2, 4>();
@@ -1252,7 +1253,8 @@ struct World {
         k_rigid_member<DBG><<<nB, RG_THREADS, 0, st>>>(b);
         ++Lc;
       }
-      k_form1<DBG><<<ga, 256, 0, st>>>(b);
+      if constexpr (DBG) k_form1<true, 1><<<ga, 256, 0, st>>>(b);
+      else SN_LANES(lc.n, (k_form1<false, L_><<<grid_for((uint64_t)hw.nAct * L_), 256, 0, st>>>(b)));
       if (chainOn) k_form2<true><<<gs, 256, 0, st>>>(b, b.acc);
       else k_form2<false><<<gs, 256, 0, st>>>(b, nullptr);
       Lc += 3;

@@ -416,13 +416,20 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   }
   if (P.bonds && *(volatile uint32_t*)(b.work + 5) != 0u) {
     if (!grid_wait(P.bar, b.err, target)) return;
-    for (uint32_t i = tid; i < own[4]; i += FU_T) form1_particle(b, nb, pOf[i], i, f);
+    for (uint32_t i = tid / L;; i += FU_T / L) {
+      if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+      const bool valid = i < own[4];
+      const uint32_t r = valid ? i : 0u;
+      form1_particle<false, L>(b, nb, valid, pOf[r], r, sub, f);
+    }
     if (!grid_wait(P.bar, b.err, target)) return;
     const bool live = *(volatile uint32_t*)(b.work + 4) != 0u;
-    for (uint32_t i = tid; i < own[4]; i += FU_T) {
-      const uint32_t sl = b.sslot[pOf[i]];
-      const ScenePar& S = b.scenes[b.SCN[pOf[i]]];
-      if (sl - S.slotBase < S.nFluid && S.formNow) form2_slot(b, S, sl, sl - S.slotBase, live);
+    for (uint32_t i = tid / L;; i += FU_T / L) {
+      if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+      const bool valid = i < own[4];
+      const uint32_t r = valid ? i : 0u, p = pOf[r], sl = b.sslot[p];
+      const ScenePar& S = b.scenes[b.SCN[p]];
+      form2_slot<L>(b, S, valid && !is_wall(rec[r].w) && S.formNow, sl, sl - S.slotBase, sub, live);
     }
   }
 

@@ -88,6 +88,7 @@ constexpr int32_t L0_MAX = 5120, L0_MIN = 512;
 constexpr uint32_t BOND_J_MASK = 0x0001ffffu, BOND_L0_MASK = 0x3ffe0000u, BOND_TOMB = 0x40000000u;
 constexpr int32_t BD_TERM = 16777216;
 constexpr uint32_t MAT_PHOTO_ROW = 15;
+constexpr uint32_t FORM_FAR = 0xffffffffu;  // a proposal whose partner does not fit the bond word
 // info word bits (sorted space)
 constexpr uint32_t INFO_MAT = 0xffu;
 constexpr uint32_t INFO_BOUNDARY = 0x80000000u;  // a wall particle (slot >= nFluid)
@@ -1465,10 +1466,52 @@ __global__ void __launch_bounds__(256, 6) k_colour_tiled(Bufs b, int colour, con
 __device__ __forceinline__ bool friction_row(const Bufs& b, uint32_t m) {
   return matw(b, m, M_fric) != 0 || matw(b, m, M_bondK) != 0;
 }
+// One live bond of particle i (word w at `entry`): its correction's terms, or its
+// tombstone. `base`: the scene's first slot; m, ki: the particle's row and
+// stiffness; lamI: its lambda.
+template <bool DBG>
+__device__ __forceinline__ void bond_term(const Bufs& b, uint32_t* entry, uint32_t w, uint32_t base, int2 pi,
+                                          int32_t lamI, uint32_t m, int32_t ki, int32_t& bx, int32_t& by,
+                                          const Flags<DBG>& f) {
+  uint32_t q = b.inv[base + (w & BOND_J_MASK)];
+  int4 o = b.PL[q];
+  uint32_t mj = (uint32_t)o.w & INFO_MAT;
+  if ((uint32_t)o.w & INFO_BURST) { *entry = w | BOND_TOMB; return; }
+  if (matw(b, mj, M_bondK) == 0) { *entry = w | BOND_TOMB; return; }
+  int32_t L0 = (int32_t)((w >> 17) & 0x1fffu);
+  int32_t L02 = wmul(L0, L0);
+  int2 d = delta(pi, xy(o), f);
+  int32_t d4x = shr_rne<BPRE>(d.x), d4y = shr_rne<BPRE>(d.y);
+  if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) { *entry = w | BOND_TOMB; return; }
+  int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
+  if (d2 >= HARD_BREAK2) { *entry = w | BOND_TOMB; return; }
+  int32_t mb = min(matw(b, m, M_bondBreak), matw(b, mj, M_bondBreak));
+  int32_t mub = min(matw(b, m, M_bondMu), matw(b, mj, M_bondMu));
+  if (mb != 0 && mub != 0) {
+    int32_t lp = neg_sat(add_sat(lamI, o.z, f), f);
+    int32_t Pq = lp > 0 ? shr_rne<4>(lp) : 0;
+    mb = wadd(wadd(65536, wsub(mb, 65536)), mul<16>(Pq, mub, f));
+  }
+  if (mb != 0 && d2 > mul<16>(L02, mb, f)) { *entry = w | BOND_TOMB; return; }
+  if (d2 < D2_FLOOR) return;
+  int32_t kj = bond_k(b, mj, b.RX[q].z, f);
+  int32_t kp = min(ki, kj);
+  if (kp == 0) return;
+  int32_t C = sub_sat(d2, L02, f);
+  int32_t qv = divshift<16>(C, wmul(d2, 4), b.rcp, f);
+  int32_t qk = mul<16>(qv, kp, f);
+  int32_t gx = mul<3>(d4x, qk, f);
+  int32_t gy = mul<3>(d4y, qk, f);
+  bx = wsub(bx, clampi(gx, -BD_TERM, BD_TERM));
+  by = wsub(by, clampi(gy, -BD_TERM, BD_TERM));
+}
+
 // L lanes share one particle's neighbour list (the friction sums wrap, so
 // any split is exact); a friction row's cost is one chain of dependent
-// gathers, which the split shortens L-fold. The bond gather stays on the
-// particle's first lane.
+// gathers, which the split shortens L-fold, and so is a bonded row's gather of
+// its bonds (each three dependent loads long: the pass over a 6 k gel pool took
+// 13.5 us with the bonds on one lane; with this and the formation passes split
+// too, a substep went from 177 to 124 us).
 //
 // One particle (a warp calls it together; `valid` false for a lane group with
 // none): p its sorted index, `row` its list in nb.
@@ -1534,55 +1577,38 @@ __device__ __forceinline__ void friction_particle(const Bufs& b, const NB& nb, b
     fx = gsum<L>(fx);
     fy = gsum<L>(fy);
   }
+  // the bond gather: L entries of the row at a time, up to its first zero word
+  // (the sums wrap, so any split is exact)
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t gmask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << (lane & ~(uint32_t)(L - 1));
+  const int32_t bondKi = act && !rigidI ? matw(b, m, M_bondK) : 0;
+  bool live = bondKi != 0 && !(info & INFO_BURST);
+  int32_t bx = 0, by = 0;
+  if (__any_sync(0xffffffffu, live)) {
+    const uint32_t slot = live ? b.sslot[p] : 0u;
+    // debug builds count this row's events once
+    const int32_t ki = !live ? 0
+                             : (sub == 0 ? bond_k(b, m, b.RX[p].z, f)
+                                         : bond_k(b, m, b.RX[p].z, Flags<false>{nullptr}));
+    const uint32_t base = live ? b.scenes[b.SCN[p]].slotBase : 0u;
+    uint32_t* brow = b.bond + (size_t)slot * BOND_CAP;
+    for (uint32_t k0 = 0; k0 < (uint32_t)BOND_CAP; k0 += L) {
+      const uint32_t k = k0 + sub;
+      const uint32_t w = live ? brow[k] : 0u;
+      const uint32_t ends = __ballot_sync(0xffffffffu, w == 0u) & gmask;
+      const bool mine = w != 0u && (L == 1 || (ends & ((1u << lane) - 1u)) == 0u);
+      if (ends) live = false;
+      if (mine && !(w & BOND_TOMB)) bond_term<DBG>(b, brow + k, w, base, pi, me.z, m, ki, bx, by, f);
+      if (!__any_sync(0xffffffffu, live)) break;
+    }
+    bx = gsum<L>(bx);
+    by = gsum<L>(by);
+  }
   if (!act || sub != 0) return;
   if (rigidI) {
     const int2 d0 = b.DP[p];
     b.DP[p] = make_int2(add_sat(d0.x, fx, f), add_sat(d0.y, fy, f));
     return;
-  }
-  const int32_t bondKi = matw(b, m, M_bondK);
-  int32_t bx = 0, by = 0;
-  if (bondKi != 0 && !(info & INFO_BURST)) {
-    uint32_t slot = b.sslot[p];
-    int32_t ki = bond_k(b, m, b.RX[p].z, f);
-    const uint32_t base = b.scenes[b.SCN[p]].slotBase;
-    uint32_t* brow = b.bond + (size_t)slot * BOND_CAP;
-    for (int k = 0; k < BOND_CAP; ++k) {
-      uint32_t w = brow[k];
-      if (w == 0u) break;
-      if (w & BOND_TOMB) continue;
-      uint32_t q = b.inv[base + (w & BOND_J_MASK)];
-      int4 o = b.PL[q];
-      uint32_t mj = (uint32_t)o.w & INFO_MAT;
-      if ((uint32_t)o.w & INFO_BURST) { brow[k] = w | BOND_TOMB; continue; }
-      if (matw(b, mj, M_bondK) == 0) { brow[k] = w | BOND_TOMB; continue; }
-      int32_t L0 = (int32_t)((w >> 17) & 0x1fffu);
-      int32_t L02 = wmul(L0, L0);
-      int2 d = delta(pi, xy(o), f);
-      int32_t d4x = shr_rne<BPRE>(d.x), d4y = shr_rne<BPRE>(d.y);
-      if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) { brow[k] = w | BOND_TOMB; continue; }
-      int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
-      if (d2 >= HARD_BREAK2) { brow[k] = w | BOND_TOMB; continue; }
-      int32_t mb = min(matw(b, m, M_bondBreak), matw(b, mj, M_bondBreak));
-      int32_t mub = min(matw(b, m, M_bondMu), matw(b, mj, M_bondMu));
-      if (mb != 0 && mub != 0) {
-        int32_t lp = neg_sat(add_sat(me.z, o.z, f), f);
-        int32_t Pq = lp > 0 ? shr_rne<4>(lp) : 0;
-        mb = wadd(wadd(65536, wsub(mb, 65536)), mul<16>(Pq, mub, f));
-      }
-      if (mb != 0 && d2 > mul<16>(L02, mb, f)) { brow[k] = w | BOND_TOMB; continue; }
-      if (d2 < D2_FLOOR) continue;
-      int32_t kj = bond_k(b, mj, b.RX[q].z, f);
-      int32_t kp = min(ki, kj);
-      if (kp == 0) continue;
-      int32_t C = sub_sat(d2, L02, f);
-      int32_t qv = divshift<16>(C, wmul(d2, 4), b.rcp, f);
-      int32_t qk = mul<16>(qv, kp, f);
-      int32_t gx = mul<3>(d4x, qk, f);
-      int32_t gy = mul<3>(d4y, qk, f);
-      bx = wsub(bx, clampi(gx, -BD_TERM, BD_TERM));
-      by = wsub(by, clampi(gy, -BD_TERM, BD_TERM));
-    }
   }
   b.DP[p] = make_int2(add_sat(fx, bx, f), add_sat(fy, by, f));
 }
@@ -2248,15 +2274,35 @@ __global__ void k_fold(Bufs b, int doChain) {
   if (s < b.world->numScenes) fold_scene(b, s, doChain != 0);
 }
 
-// markCongealNbr + bondForm1 (src/sim.wgsl:2714-2989), sorted space.
-template <bool DBG, class NB>
-__device__ __forceinline__ void form1_particle(const Bufs& b, const NB& nb, uint32_t p, uint32_t row,
-                                               const Flags<DBG>& f) {
-  int4 me = b.PL[p];
-  if ((uint32_t)me.w & INFO_BOUNDARY) return;
-  const ScenePar& S = b.scenes[b.SCN[p]];
-  if (!S.formNow) return;
-  uint32_t slot = b.sslot[p];
+// Which of the L lanes sharing a particle this is, as masks of the warp: the
+// group's lanes and the lanes below.
+template <int L>
+struct LaneGroup {
+  uint32_t group, below;
+  __device__ __forceinline__ LaneGroup() {
+    const uint32_t lane = threadIdx.x & 31u;
+    group = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << (lane & ~(uint32_t)(L - 1));
+    below = group & ((1u << lane) - 1u);
+  }
+  __device__ __forceinline__ uint32_t ballot(bool v) const { return __ballot_sync(0xffffffffu, v) & group; }
+};
+
+// markCongealNbr + bondForm1 (src/sim.wgsl:2714-2989) for one particle: its
+// candidate row. L lanes share it (a warp calls it together): they take L
+// entries of the bond row, then L neighbours at a time, and ballot prefixes
+// keep the row in sequential order. A neighbour is in a list once, so an entry
+// can only repeat one of the particle's own bonds. Debug builds use one lane,
+// whose event counts follow the sequential pass.
+template <bool DBG, int L, class NB>
+__device__ __forceinline__ void form1_particle(const Bufs& b, const NB& nb, bool valid, uint32_t p, uint32_t row,
+                                               uint32_t sub, const Flags<DBG>& f) {
+  static_assert(!DBG || L == 1, "debug builds count events in sequence");
+  const LaneGroup<L> lg;
+  const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
+  bool act = valid && !is_wall(me.w);
+  const ScenePar& S = b.scenes[b.SCN[act ? p : 0u]];
+  act = act && S.formNow;
+  const uint32_t slot = b.sslot[act ? p : 0u];
   const int32_t* wi = b.state + (size_t)slot * 8;
   uint32_t* cand = b.bondCand + (size_t)slot * BOND_CAP;
   const uint32_t* brow = b.bond + (size_t)slot * BOND_CAP;
@@ -2264,124 +2310,157 @@ __device__ __forceinline__ void form1_particle(const Bufs& b, const NB& nb, uint
   // Rigid members and rows that do not bond propose nothing: their list is
   // empty. Candidate rows are dense (entries first, zeros after), so a row
   // whose first word is zero is already empty and is not rewritten.
-  if ((flI & FLAG_RIGID) || matw(b, matI, M_bondK) == 0 || matw(b, matI, M_bondGroup) < 0) {
-    if (cand[0] != 0u)
-      for (int k = 0; k < BOND_CAP; ++k) cand[k] = 0;
-    return;
-  }
-  uint32_t cnt = b.NBRN[p] & NBRN_COUNT;
+  const bool prop = act && !((flI & FLAG_RIGID) || matw(b, matI, M_bondK) == 0 || matw(b, matI, M_bondGroup) < 0);
+  const bool clear = act && !prop && cand[0] != 0u;
+  __syncwarp();
+  if (clear)
+    for (uint32_t k = sub; k < (uint32_t)BOND_CAP; k += L) cand[k] = 0;
+  if (!__any_sync(0xffffffffu, prop)) return;
+  const uint32_t cnt = prop ? (b.NBRN[p] & NBRN_COUNT) : 0u;
   // markCongealNbr: refresh the congeal bit from the post-thermal flags
   bool seen = false;
-  for (uint32_t k = 0; k < cnt; ++k) {
-    uint32_t e = nb.entry(row, k);
-    if (is_wall(b.PL[e].w)) continue;
-    uint32_t qs = b.sslot[e];
-    if ((uint32_t)b.state[(size_t)qs * 8 + 5] & FLAG_CONGEAL) { seen = true; break; }
+  for (uint32_t k = sub; k < cnt && !seen; k += L) {
+    const uint32_t e = nb.entry(row, k);
+    if (!is_wall(b.PL[e].w)) seen = ((uint32_t)b.state[(size_t)b.sslot[e] * 8 + 5] & FLAG_CONGEAL) != 0u;
   }
-  bool anchoredI = (flI & FLAG_ANCHOR) != 0;
+  seen = lg.ballot(seen) != 0u;
+  const bool anchoredI = (flI & FLAG_ANCHOR) != 0;
   uint32_t cn = 0;
-  {
-    for (int k = 0; k < BOND_CAP; ++k) {
-      uint32_t w = brow[k];
-      if (w == 0u) break;
-      if (w & BOND_TOMB) continue;
-      if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
-      cand[cn++] = w;
-    }
-    uint32_t tagI = flI & WELD_TAG_MASK;
-    int32_t ki = bond_k(b, matI, wi[6], f);
-    bool canReform = (!anchoredI && matw(b, matI, M_bondReform) != 0 && ki != 0);
-    bool fuseArmed = S.fuseTag != 0u && fuse_row(b, matI);
-    bool congealI = (flI & FLAG_CONGEAL) && fuse_row(b, matI);
-    bool congealNear = seen && fuse_row(b, matI);
-    if (canReform || (!anchoredI && tagI != 0u) || fuseArmed || congealI || congealNear) {
-      for (uint32_t k = 0; k < cnt; ++k) {
-        if (cn >= (uint32_t)BOND_CAP) { f.flag(8); break; }
-        uint32_t e = nb.entry(row, k);
-        if (is_wall(b.PL[e].w)) continue;
-        uint32_t qs = b.sslot[e];
-        const int32_t* wj = b.state + (size_t)qs * 8;
-        uint32_t j = qs - S.slotBase;
-        uint32_t mj = (uint32_t)wj[4];
-        uint32_t fJ = (uint32_t)wj[5];
-        uint32_t tagJ = fJ & WELD_TAG_MASK;
-        bool weld = (!anchoredI && tagI != 0u && tagI == tagJ);
-        bool fuse = false;
-        if (fuseArmed && !(fJ & FLAG_RIGID) && fuse_row(b, mj) && (!anchoredI || !(fJ & FLAG_ANCHOR)))
-          fuse = (tagI == S.fuseTag && tagJ == 0u) || (tagJ == S.fuseTag && tagI == 0u) ||
-                 (tagI == S.fuseTag && tagJ == S.fuseTag);
-        bool congealJ = (fJ & FLAG_CONGEAL) && fuse_row(b, mj);
-        bool congeal = ((congealI || congealJ) && !weld && !fuse && mj == matI && !(fJ & FLAG_RIGID));
-        if (!fuse && !congeal && matw(b, mj, M_bondGroup) != matw(b, matI, M_bondGroup)) continue;
-        if (!weld && !fuse && !congeal) {
-          if (!canReform) continue;
-          if (bond_k(b, mj, wj[6], f) == 0) continue;
-        }
-        bool dup = false;
-        for (uint32_t q2 = 0; q2 < cn; ++q2)
-          if ((cand[q2] & BOND_J_MASK) == j) { dup = true; break; }
-        if (dup) continue;
-        int32_t d4x = shr_rne<BPRE>(sub_sat(wi[0], wj[0], f));
-        int32_t d4y = shr_rne<BPRE>(sub_sat(wi[1], wj[1], f));
-        if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) continue;
-        int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
-        if (d2 < D2_FLOOR || d2 > BOND_R2) continue;
-        if (!weld && !fuse && !congeal) {
-          int32_t vl = min(matw(b, matI, M_bondFormV), matw(b, mj, M_bondFormV));
-          int32_t vl4 = shr_rne<RPRE>(vl);
-          int32_t r4x = shr_rne<RPRE>(sub_sat(wi[2], wj[2], f));
-          int32_t r4y = shr_rne<RPRE>(sub_sat(wi[3], wj[3], f));
-          if (abs(r4x) > vl4 || abs(r4y) > vl4) continue;
-          if (wadd(wmul(r4x, r4x), wmul(r4y, r4y)) > wmul(vl4, vl4)) continue;
-          int32_t pl = min(matw(b, matI, M_bondFormP), matw(b, mj, M_bondFormP));
-          if (pl != 0 && (neg_sat(me.z, f) < pl || neg_sat(b.PL[e].z, f) < pl)) continue;
-        }
-        int32_t L0 = (int32_t)isqrt32((uint32_t)d2);
-        if (L0 < L0_MIN || L0 > L0_MAX) continue;
-        if (j > BOND_J_MASK) { atomicOr(b.err, ERR_BOND_PARTNER); continue; }
-        cand[cn++] = (((uint32_t)L0 & 0x1fffu) << 17) | (j & BOND_J_MASK);
-      }
-    }
+  // the bonds it has, up to the row's first zero word
+  bool live = prop;
+  for (uint32_t k0 = 0; k0 < (uint32_t)BOND_CAP && __any_sync(0xffffffffu, live); k0 += L) {
+    const uint32_t w = live ? brow[k0 + sub] : 0u;
+    const uint32_t ends = lg.ballot(w == 0u);
+    const bool keep = w != 0u && (ends & lg.below) == 0u && !(w & BOND_TOMB);
+    const uint32_t bal = lg.ballot(keep);
+    if (keep) cand[cn + __popc(bal & lg.below)] = w;
+    cn += __popc(bal);
+    live = live && ends == 0u;
   }
-  for (uint32_t k = cn; k < (uint32_t)BOND_CAP; ++k) cand[k] = 0;
+  __syncwarp();
+  const uint32_t own = cn;
+  const uint32_t tagI = flI & WELD_TAG_MASK;
+  const int32_t ki = prop ? bond_k(b, matI, wi[6], f) : 0;
+  const bool canReform = (!anchoredI && matw(b, matI, M_bondReform) != 0 && ki != 0);
+  const bool fuseArmed = S.fuseTag != 0u && fuse_row(b, matI);
+  const bool congealI = (flI & FLAG_CONGEAL) && fuse_row(b, matI);
+  const bool congealNear = seen && fuse_row(b, matI);
+  // the entry a neighbour proposes, 0 for none
+  auto propose = [&](uint32_t e) -> uint32_t {
+    if (is_wall(b.PL[e].w)) return 0u;
+    const uint32_t qs = b.sslot[e];
+    const int32_t* wj = b.state + (size_t)qs * 8;
+    const uint32_t j = qs - S.slotBase, mj = (uint32_t)wj[4], fJ = (uint32_t)wj[5], tagJ = fJ & WELD_TAG_MASK;
+    const bool weld = (!anchoredI && tagI != 0u && tagI == tagJ);
+    bool fuse = false;
+    if (fuseArmed && !(fJ & FLAG_RIGID) && fuse_row(b, mj) && (!anchoredI || !(fJ & FLAG_ANCHOR)))
+      fuse = (tagI == S.fuseTag && tagJ == 0u) || (tagJ == S.fuseTag && tagI == 0u) ||
+             (tagI == S.fuseTag && tagJ == S.fuseTag);
+    const bool congealJ = (fJ & FLAG_CONGEAL) && fuse_row(b, mj);
+    const bool congeal = ((congealI || congealJ) && !weld && !fuse && mj == matI && !(fJ & FLAG_RIGID));
+    if (!fuse && !congeal && matw(b, mj, M_bondGroup) != matw(b, matI, M_bondGroup)) return 0u;
+    if (!weld && !fuse && !congeal) {
+      if (!canReform) return 0u;
+      if (bond_k(b, mj, wj[6], f) == 0) return 0u;
+    }
+    for (uint32_t q2 = 0; q2 < own; ++q2)
+      if ((cand[q2] & BOND_J_MASK) == j) return 0u;
+    const int32_t d4x = shr_rne<BPRE>(sub_sat(wi[0], wj[0], f)), d4y = shr_rne<BPRE>(sub_sat(wi[1], wj[1], f));
+    if (abs(d4x) > L0_MAX || abs(d4y) > L0_MAX) return 0u;
+    const int32_t d2 = wadd(wmul(d4x, d4x), wmul(d4y, d4y));
+    if (d2 < D2_FLOOR || d2 > BOND_R2) return 0u;
+    if (!weld && !fuse && !congeal) {
+      const int32_t vl = min(matw(b, matI, M_bondFormV), matw(b, mj, M_bondFormV));
+      const int32_t vl4 = shr_rne<RPRE>(vl);
+      const int32_t r4x = shr_rne<RPRE>(sub_sat(wi[2], wj[2], f)), r4y = shr_rne<RPRE>(sub_sat(wi[3], wj[3], f));
+      if (abs(r4x) > vl4 || abs(r4y) > vl4) return 0u;
+      if (wadd(wmul(r4x, r4x), wmul(r4y, r4y)) > wmul(vl4, vl4)) return 0u;
+      const int32_t pl = min(matw(b, matI, M_bondFormP), matw(b, mj, M_bondFormP));
+      if (pl != 0 && (neg_sat(me.z, f) < pl || neg_sat(b.PL[e].z, f) < pl)) return 0u;
+    }
+    const int32_t L0 = (int32_t)isqrt32((uint32_t)d2);
+    if (L0 < L0_MIN || L0 > L0_MAX) return 0u;
+    if (j > BOND_J_MASK) return FORM_FAR;
+    return (((uint32_t)L0 & 0x1fffu) << 17) | (j & BOND_J_MASK);
+  };
+  live = prop && (canReform || (!anchoredI && tagI != 0u) || fuseArmed || congealI || congealNear);
+  for (uint32_t k0 = 0; __any_sync(0xffffffffu, live && k0 < cnt); k0 += L) {
+    if (live && k0 < cnt && cn >= (uint32_t)BOND_CAP) {
+      f.flag(8);
+      live = false;
+    }
+    const uint32_t k = k0 + sub;
+    const uint32_t w = live && k < cnt ? propose(nb.entry(row, k)) : 0u;
+    const uint32_t bal = lg.ballot(w != 0u && w != FORM_FAR);
+    const uint32_t at = cn + __popc(bal & lg.below);
+    if (w != 0u && at < (uint32_t)BOND_CAP) {
+      if (w == FORM_FAR) atomicOr(b.err, ERR_BOND_PARTNER);
+      else cand[at] = w;
+    }
+    cn = min(cn + __popc(bal), (uint32_t)BOND_CAP);
+  }
+  if (prop)
+    for (uint32_t k = cn + sub; k < (uint32_t)BOND_CAP; k += L) cand[k] = 0;
 }
-template <bool DBG>
+template <bool DBG, int L>
 __global__ void __launch_bounds__(256) k_form1(Bufs b) {
   if (b.work[5] == 0u) return;  // no scene forms bonds this substep
   Flags<DBG> f{b.dbg};
   const uint32_t nAct = b.world->nAct;
+  const uint32_t sub = threadIdx.x & (L - 1), G = gstride() / L;
   const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
-  for (uint32_t p = gtid(); p < nAct; p += gstride()) form1_particle(b, nb, p, p, f);
+  for (uint32_t p = gtid() / L;; p += G) {
+    if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
+    form1_particle<DBG, L>(b, nb, p < nAct, p, p < nAct ? p : 0u, sub, f);
+  }
 }
 
 // bondForm2 (src/sim.wgsl:3001-3068): keep mutual proposals, clear weld
 // tags. It is the last pass of the substep that writes hashed words, so with
 // HASH it also folds every particle's digest (the state hash of the substep).
-__device__ __forceinline__ bool form2_slot(const Bufs& b, const ScenePar& S, uint32_t slot, uint32_t i, bool rowsLive) {
+//
+// One slot (L lanes share it; a warp calls it together with `act` false where
+// there is none): L candidates at a time, a ballot prefix keeping their order.
+// Returns whether the slot has bonds now.
+template <int L>
+__device__ __forceinline__ bool form2_slot(const Bufs& b, const ScenePar& S, bool act, uint32_t slot, uint32_t i,
+                                           uint32_t sub, bool rowsLive) {
+  const LaneGroup<L> lg;
   uint32_t* row = b.bond + (size_t)slot * BOND_CAP;
   const uint32_t* cand = b.bondCand + (size_t)slot * BOND_CAP;
+  const uint32_t first = act ? row[0] : 0u;
+  __syncwarp();  // every lane has it before one writes the row
   uint32_t nn = 0;
-  for (int k = 0; k < BOND_CAP; ++k) {
-    uint32_t w = cand[k];
-    if (w == 0u) break;
-    uint32_t j = w & BOND_J_MASK;
-    const uint32_t* cj = b.bondCand + (size_t)(S.slotBase + j) * BOND_CAP;
+  bool live = act;
+  for (uint32_t k0 = 0; k0 < (uint32_t)BOND_CAP; k0 += L) {
+    const uint32_t w = live ? cand[k0 + sub] : 0u;
+    const uint32_t ends = lg.ballot(w == 0u);
     bool ok = false;
-    for (int q = 0; q < BOND_CAP; ++q) {
-      uint32_t v = cj[q];
-      if (v == 0u) break;
-      if ((v & BOND_J_MASK) == i) { ok = ((v & BOND_L0_MASK) == (w & BOND_L0_MASK)); break; }
+    if (w != 0u && (ends & lg.below) == 0u) {
+      const uint32_t* cj = b.bondCand + (size_t)(S.slotBase + (w & BOND_J_MASK)) * BOND_CAP;
+      for (int q = 0; q < BOND_CAP; ++q) {
+        const uint32_t v = cj[q];
+        if (v == 0u) break;
+        if ((v & BOND_J_MASK) == i) { ok = ((v & BOND_L0_MASK) == (w & BOND_L0_MASK)); break; }
+      }
     }
-    if (ok) row[nn++] = w & ~BOND_TOMB;
+    const uint32_t bal = lg.ballot(ok);
+    if (ok) row[nn + __popc(bal & lg.below)] = w & ~BOND_TOMB;
+    nn += __popc(bal);
+    live = live && ends == 0u;
+    if (!__any_sync(0xffffffffu, live)) break;
   }
+  if (!act) return false;
   // bond rows are dense too: an empty row stays as it is
-  if (nn != 0u || row[0] != 0u)
-    for (int k = nn; k < BOND_CAP; ++k) row[k] = 0;
-  if (nn != 0u && !rowsLive) b.work[4] = 1u;
-  int32_t* w = b.state + (size_t)slot * 8;
-  uint32_t fo = (uint32_t)w[5] & ~FLAG_CONGEAL;
-  if (!(fo & FLAG_RIGID) && (fo & WELD_TAG_MASK) != S.weldHold) fo &= ~WELD_TAG_MASK;
-  w[5] = (int32_t)fo;
+  if (nn != 0u || first != 0u)
+    for (uint32_t k = nn + sub; k < (uint32_t)BOND_CAP; k += L) row[k] = 0;
+  if (sub == 0) {
+    if (nn != 0u && !rowsLive) b.work[4] = 1u;
+    int32_t* w = b.state + (size_t)slot * 8;
+    uint32_t fo = (uint32_t)w[5] & ~FLAG_CONGEAL;
+    if (!(fo & FLAG_RIGID) && (fo & WELD_TAG_MASK) != S.weldHold) fo &= ~WELD_TAG_MASK;
+    w[5] = (int32_t)fo;
+  }
   return nn != 0u;
 }
 template <bool HASH>
@@ -2393,22 +2472,19 @@ __global__ void __launch_bounds__(256) k_form2(Bufs b, uint32_t* __restrict__ ac
   // launch forms is read by the thread that formed it.
   const bool rowsLive = b.work[4] != 0u;
   const uint32_t slotEnd = b.world->slotEnd;
-  const uint32_t nIter = HASH ? (slotEnd + gstride() - 1) / gstride() * gstride() : slotEnd;
+  const uint32_t nIter = (slotEnd + 31u) & ~31u;  // whole warps
   for (uint32_t slot = gtid(); slot < nIter; slot += gstride()) {
-    bool valid = false, formed = false;
-    uint32_t s = 0;
     uint32_t h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (slot < slotEnd) {
-      s = b.sceneOf[slot];
-      const ScenePar& S = b.scenes[s];
-      const uint32_t i = slot - S.slotBase;
+    const uint32_t s = slot < slotEnd ? b.sceneOf[slot] : 0u;
+    const ScenePar& S = b.scenes[s];
+    const uint32_t i = slot - S.slotBase;
+    const bool valid = slot < slotEnd && S.active && i < S.n;
+    const bool act = valid && i < S.nFluid && S.formNow;
+    bool formed = false;
+    if (__any_sync(0xffffffffu, act)) formed = form2_slot<1>(b, S, act, slot < slotEnd ? slot : 0u, i, 0u, rowsLive);
+    if (HASH && valid) {
       const uint32_t* row = b.bond + (size_t)slot * BOND_CAP;
-      if (S.active && i < S.nFluid && S.formNow) formed = form2_slot(b, S, slot, i, rowsLive);
-      if (HASH) {
-        valid = S.active && i < S.n;
-        if (valid)
-          particle_digest(b.state + (size_t)slot * 8, i, (i < S.nFluid && (rowsLive || formed)) ? row : nullptr, h);
-      }
+      particle_digest(b.state + (size_t)slot * 8, i, (i < S.nFluid && (rowsLive || formed)) ? row : nullptr, h);
     }
     if (HASH) digest_add_block(acc, dsacc, &dsscene, valid, s, h);
   }
