@@ -455,11 +455,12 @@ __global__ void __launch_bounds__(256) k_cellstart(Bufs b) {
 // exact test costs a 16-byte record and some 20 instructions. QC holds each
 // sorted particle's place inside its cell in 64ths of a cell, x in byte 0 and
 // y in byte 2, so a lane tests a candidate against its own place with an add
-// and a byte dot product, four candidates to one 16-byte load, and only the
-// survivors (about 28 %) go through the exact test. The list pass of the 1 M
-// scene fell from 261 to 190 us (2.1 k thread instructions a particle at 14
-// active lanes: what bounds it now is the lanes' uneven survivor counts), a
-// 262 k one from 117 to 84, a fused 40 k world's from 30 to 15.
+// and a byte dot product, four candidates to one 16-byte load. What is left
+// (about 28 %) is mostly near enough to be a neighbour for sure; only the ring
+// about the kernel's edge (6 %) goes through the exact test. The list pass of
+// the 1 M scene fell from 261 to 165 us (190 with every survivor tested), a
+// 262 k one from 117 to 70, a fused 40 k world's from 30 to 12. What bounds it
+// now is issue (67 %) at 15 active lanes: a warp's cells differ in survivors.
 //
 // The filter never drops a neighbour. Quantised places are clamped to the
 // scene's cells as cell_coord is, and clamping brings no two points further
@@ -481,50 +482,80 @@ __device__ __forceinline__ uint32_t cand_code(const ScenePar& S, int2 p) {
 __device__ __forceinline__ uint32_t cand_bias(uint32_t own, int dx, int dy) {
   return (uint32_t)(dx * 64 + dy * (64 << 16)) - own;
 }
-// The accumulator start that leaves a survivor's dot product negative.
-__device__ __forceinline__ int32_t cand_threshold(const ScenePar& S) {
-  const int32_t r4 = ((4 * CAND_R) >> (S.cellShift - 6u)) + 1;  // >= 4 CAND_R / q, and 9 / 4 >= sqrt(5)
-  return -((r4 + 9) * (r4 + 9) / 16 + 4);
+// Bounds on the dot product, for accumulators that go negative: `far` drops a
+// candidate, `near` accepts it without the exact test. The bounds above read
+// backwards: a pair whose dot product is at most (CAND_IN / q - sqrt(5))^2 lies
+// within CAND_IN ticks, where lut_index accepts every pair. That does not hold
+// for a clamped place, so a particle outside the cells takes nothing as near,
+// and nobody takes anything in a border cell (only those hold such particles).
+constexpr int32_t CAND_IN = HS * 16 - 12;  // |d| <= CAND_IN: (|dx| + 8)^2 + (|dy| + 8)^2 < (16 HS)^2
+struct CandBounds {
+  int32_t far, near;
+};
+__device__ __forceinline__ CandBounds cand_bounds(const ScenePar& S) {
+  const uint32_t sh = S.cellShift - 6u;
+  const int32_t r4 = ((4 * CAND_R) >> sh) + 1;            // >= 4 CAND_R / q, and 9 / 4 >= sqrt(5)
+  const int32_t n4 = max(((4 * CAND_IN) >> sh) - 9, 0);   // <= 4 CAND_IN / q - 4 sqrt(5)
+  return CandBounds{-((r4 + 9) * (r4 + 9) / 16 + 4), -(n4 * n4 / 16)};
 }
-// Survivors among the candidates [base, base + 32) that lie in [lo, hi), base a
-// multiple of 4: candidate base + j at bit 31 - j. NV vectors are in flight.
+__device__ __forceinline__ bool cand_outside(const ScenePar& S, int2 p, int2 cc) {
+  return (p.x >> S.cellShift) != cc.x || (p.y >> S.cellShift) != cc.y;
+}
+__device__ __forceinline__ CandBounds cand_cell(const ScenePar& S, CandBounds cb, int32_t gx, int32_t gy) {
+  const bool border = (uint32_t)(gx - 1) >= S.gridW - 2u || (uint32_t)(gy - 1) >= S.gridH - 2u;
+  return CandBounds{cb.far, border ? 0 : cb.near};
+}
+// Candidates [base, base + 32) that lie in [lo, hi), base a multiple of 4, as two
+// masks with candidate base + j at bit 31 - j: the survivors, and those of them
+// near enough to need no test. NV vectors are in flight.
+struct CandMask {
+  uint32_t hit, near;
+};
 template <int NV>
-__device__ __forceinline__ uint32_t cand_mask(const uint32_t* QC, uint32_t base, uint32_t lo, uint32_t hi,
-                                              uint32_t bias, int32_t thr) {
+__device__ __forceinline__ CandMask cand_mask(const uint32_t* QC, uint32_t base, uint32_t lo, uint32_t hi,
+                                              uint32_t bias, CandBounds cb) {
   const uint32_t nv = min((hi - base + 3u) >> 2, 8u);
   const uint4* src = reinterpret_cast<const uint4*>(QC + base);
-  uint32_t m = 0;
+  const int32_t step = cb.near - cb.far;
+  CandMask m{0u, 0u};
+  auto test = [&](uint32_t code) {
+    const int d = (int)(code + bias);
+    const int32_t acc = __dp4a(d, d, cb.far);
+    m.hit = __funnelshift_l((uint32_t)acc, m.hit, 1);
+    m.near = __funnelshift_l((uint32_t)(acc + step), m.near, 1);
+  };
   for (uint32_t v = 0; v < nv; v += NV) {
     uint4 w[NV];
 #pragma unroll
     for (int j = 0; j < NV; ++j) w[j] = src[min(v + j, nv - 1u)];
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-      const int d0 = (int)(w[j].x + bias), d1 = (int)(w[j].y + bias), d2 = (int)(w[j].z + bias),
-                d3 = (int)(w[j].w + bias);
-      m = __funnelshift_l((uint32_t)__dp4a(d0, d0, thr), m, 1);
-      m = __funnelshift_l((uint32_t)__dp4a(d1, d1, thr), m, 1);
-      m = __funnelshift_l((uint32_t)__dp4a(d2, d2, thr), m, 1);
-      m = __funnelshift_l((uint32_t)__dp4a(d3, d3, thr), m, 1);
+      test(w[j].x);
+      test(w[j].y);
+      test(w[j].z);
+      test(w[j].w);
     }
   }
-  const uint32_t done = 4u * ((nv + NV - 1u) / NV * NV);  // codes shifted in (a repeated vector's lie past hi)
-  m <<= 32u - done;
-  if (lo > base) m &= 0xffffffffu >> (lo - base);
-  if (hi - base < 32u) m &= ~(0xffffffffu >> (hi - base));
+  // codes shifted in so far (a repeated vector's lie past hi), to the top; the
+  // ones outside [lo, hi) dropped
+  const uint32_t done = 4u * ((nv + NV - 1u) / NV * NV);
+  uint32_t in = 0xffffffffu << (32u - done);
+  if (lo > base) in &= 0xffffffffu >> (lo - base);
+  if (hi - base < 32u) in &= ~(0xffffffffu >> (hi - base));
+  m.hit = (m.hit << (32u - done)) & in;
+  m.near = m.near << (32u - done);
   return m;
 }
-// The survivors that are in the kernel.
+// The survivors that are in the kernel: those that are not near enough tested.
 template <bool DBG>
-__device__ __forceinline__ uint32_t cand_test(const int4* PL, uint32_t base, uint32_t m, int2 pi,
+__device__ __forceinline__ uint32_t cand_test(const int4* PL, uint32_t base, CandMask m, int2 pi,
                                               const Flags<DBG>& f) {
-  uint32_t keep = m;
-  while (m) {
-    const uint32_t j = (uint32_t)__clz((int)m), bit = 0x80000000u >> j;
-    m &= ~bit;
-    if (!in_kernel(pdelta(pi, ld_pred(PL, base + j), f))) keep &= ~bit;
+  for (uint32_t t = m.hit & ~m.near; t;) {
+    const uint32_t j = (uint32_t)__clz((int)t), bit = 0x80000000u >> j;
+    t ^= bit;
+    if (!in_kernel(pdelta(pi, ld_pred(PL, base + j), f))) m.hit ^= bit;
   }
-  return keep;
+  return m.hit;
 }
 
 // The per-substep world flags one particle raises (see Bufs::work): some lanes
@@ -777,7 +808,8 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
                      ((skip & SKIP_UP) || cc.y + 1 >= (int32_t)S.gridH ? 0u : cols << 6);
     if (!work) cells = 0u;
     const uint32_t cq = cand_code(S, pi);
-    const int32_t thr = cand_threshold(S);
+    CandBounds cb = cand_bounds(S);
+    if (cand_outside(S, pi, cc)) cb.near = 0;
     // this lane's cells are every L-th set bit from the sub-th on
     for (uint32_t t = 0; t < sub; ++t) cells &= cells - 1u;
     bool fits = true;
@@ -792,12 +824,14 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
           fits = false;
         } else {
           const uint32_t bias = cand_bias(cq, dx, dy);
-          if (base < hi) m0 = cand_mask<4>(b.QC, base, lo, hi, bias, thr);
-          if (base + 32 < hi) m1 = cand_mask<4>(b.QC, base + 32, lo, hi, bias, thr);
-          if (k == 4 && p - base < 32u) m0 &= ~(0x80000000u >> (p - base));
-          if (k == 4 && p - base - 32u < 32u) m1 &= ~(0x80000000u >> (p - base - 32u));
-          m0 = cand_test(b.PL, base, m0, pi, f);
-          m1 = cand_test(b.PL, base + 32, m1, pi, f);
+          const CandBounds ce = cand_cell(S, cb, cc.x + dx, cc.y + dy);
+          CandMask c0{0u, 0u}, c1{0u, 0u};
+          if (base < hi) c0 = cand_mask<4>(b.QC, base, lo, hi, bias, ce);
+          if (base + 32 < hi) c1 = cand_mask<4>(b.QC, base + 32, lo, hi, bias, ce);
+          if (k == 4 && p - base < 32u) c0.hit &= ~(0x80000000u >> (p - base));
+          if (k == 4 && p - base - 32u < 32u) c1.hit &= ~(0x80000000u >> (p - base - 32u));
+          m0 = cand_test(b.PL, base, c0, pi, f);
+          m1 = cand_test(b.PL, base + 32, c1, pi, f);
         }
       }
       if (__any_sync(0xffffffffu, !fits)) break;
@@ -909,7 +943,8 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
       int2 cc = cell_coord(S, pi);
       const uint32_t skip = far_sides(S, pi, cc);
       const uint32_t cq = cand_code(S, pi);
-      const int32_t thr = cand_threshold(S);
+      CandBounds cb = cand_bounds(S);
+      if (cand_outside(S, pi, cc)) cb.near = 0;
       uint32_t cnt = 0;
       bool congeal = false, sealSeen = false;
       uint32_t* out = b.NBR + p;
@@ -935,13 +970,12 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
             // MAXNBR (so nothing overflows).
             const uint32_t bias = cand_bias(cq, dx, dy);
             for (uint32_t base = lo & ~3u; base < hi; base += 32) {
-              uint32_t m = cand_mask<2>(b.QC, base, lo, hi, bias, thr);
-              if (dx == 0 && dy == 0 && p - base < 32u) m &= ~(0x80000000u >> (p - base));
-              while (m) {
-                const uint32_t j = (uint32_t)__clz((int)m), q = base + j;
-                m &= ~(0x80000000u >> j);
-                if (!in_kernel(pdelta(pi, ld_pred(b.PL, q), f))) continue;
-                out[(size_t)cnt * stride] = q;
+              CandMask c = cand_mask<2>(b.QC, base, lo, hi, bias, cand_cell(S, cb, gx, gy));
+              if (dx == 0 && dy == 0 && p - base < 32u) c.hit &= ~(0x80000000u >> (p - base));
+              for (uint32_t m = cand_test(b.PL, base, c, pi, f); m;) {
+                const uint32_t j = (uint32_t)__clz((int)m);
+                m ^= 0x80000000u >> j;
+                out[(size_t)cnt * stride] = base + j;
                 if (++cnt >= (uint32_t)MAXNBR) goto listed;
               }
             }
