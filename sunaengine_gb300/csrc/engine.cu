@@ -1273,15 +1273,23 @@ struct World {
   }
 #undef SN_LANES
 
-  // Lanes before (or without) tuning, from the active particle count: each
-  // class is sized by the particles one launch works on and how heavy its
-  // per-particle epilogue is (measured on the 1 M-particle scene: solveA 1,
-  // colours 4, post1 2, post2 1).
-  static int lanes_for(uint64_t n) {
-    if (n < 40000) return 8;
-    if (n < 80000) return 4;
-    if (n < 160000) return 2;
-    return 1;
+  // Lanes before (or without) tuning, from the active particle count. Fewer
+  // particles need more lanes to fill the GPU; more lanes cost each particle's
+  // prologue and reduction again. The lines lie where uniform splits crossed on
+  // the settled two-fluid scene (phase us at the neighbouring sizes, fewer / more
+  // lanes): solveA 265 k 94 / 94 (1, 2) and 197 k 88 / 76, 103 k 61 / 60 (2, 4);
+  // colours 265 k 203 / 219 and 197 k 181 / 175 (4, 8); post1 265 k 66 / 62,
+  // 363 k 77 / 83, 744 k 155 / 149 (1, 2: its waves come out even or not); post2
+  // 744 k 182 / 175 and 1.05 M 223 / 234 (1, 2); lists 265 k 54 / 62 and 197 k
+  // 50 / 48 (1, 2).
+  static LaneCfg lanes_for(uint64_t n) {
+    LaneCfg l;
+    l.a = n < 40000 ? 8 : n < 110000 ? 4 : n < 265000 ? 2 : 1;
+    l.c = n < 220000 ? 8 : 4;
+    l.p1 = n < 40000 ? 8 : n < 110000 ? 4 : (n < 330000 || n >= 650000) ? 2 : 1;
+    l.p2 = n < 40000 ? 8 : n < 110000 ? 4 : n < 900000 ? 2 : 1;
+    l.n = n < 40000 ? 8 : n < 80000 ? 4 : n < 220000 ? 2 : 1;
+    return l;
   }
   void default_lanes() {
     if (!autoLanes) {
@@ -1291,8 +1299,7 @@ struct World {
     }
     if (lanesTuned && hw.nAct * 2 >= tunedAtN && hw.nAct <= tunedAtN * 2ull) return;
     lanesTuned = false;
-    const uint64_t n = hw.nAct;
-    lanesCfg = LaneCfg{lanes_for(n), lanes_for(n / 16), lanes_for(n / 8), lanes_for(n), lanes_for(n)};
+    lanesCfg = lanes_for(hw.nAct);
   }
 
   // The autotuner: run `per` real substeps under each uniform lane count with
