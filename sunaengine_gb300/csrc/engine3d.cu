@@ -137,6 +137,7 @@ struct Engine3 {
   cudaGraphExec_t gexec = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   uint64_t lastLaunches = 0, launchesPerSubstep = 0;
+  bool inRange = true;  // the tables lie in the ranges the release kernels are built for
   cudaEvent_t* pev = nullptr;
   int npev = 0;
 
@@ -157,7 +158,7 @@ struct Engine3 {
   ~Engine3() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
-    void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.NBR,
+    void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.QC, b.NBR,
                     b.NBRN, (void*)b.WG, (void*)b.PG, (void*)b.mats, (void*)b.rcp, b.scenes, b.world, b.acc,
                     b.accLast, b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes};
     for (void* p : ptrs)
@@ -195,6 +196,7 @@ struct Engine3 {
     maxCells = o->max_cells ? o->max_cells : (1u << 20);
     matCount = o->mat_count;
     hluts.assign(o->luts, o->luts + LUT_WORDS);
+    inRange = tables_in_range(o->luts);
     hmats.assign(o->mats, o->mats + 4 * matCount);
     if (!cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) return false;
     if (!cuda_ok(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking), "stream")) return false;
@@ -216,6 +218,7 @@ struct Engine3 {
     b.PW = dalloc3<int4>(C, err);
     b.PW2 = dalloc3<int4>(C, err);
     b.PL = dalloc3<int4>(C, err);
+    b.QC = dalloc3<uint32_t>((C + 7) & ~(size_t)3, err);
     b.NBR = dalloc3<uint32_t>(C * MAXNBR, err);
     b.NBRN = dalloc3<uint32_t>(C, err);
     b.nbrStride = (uint32_t)C;
@@ -298,12 +301,14 @@ struct Engine3 {
       return;
     }
     if (lanesTuned) return;
-    // Measured on 3D columns (ms per substep with 1 / 2 / 4 lanes): 32,768
-    // particles 0.162 / 0.141 / 0.119, 64,000 0.183 / 0.179 / 0.166,
-    // 85,184 0.209 / 0.211 / 0.206, 97,336 0.226 / 0.237 / 0.238, 262,144
-    // 0.387 / 0.500 / 0.531: two lanes never won.
+    // Measured on settled columns (phase us with 1 / 2 / 4 lanes): density 64,000
+    // particles 77 / 67 / 67, 85,184 85 / 74 / 75, 110,592 90 / 83 / 91, 157,464
+    // 116 / 102 / 109, 262,144 150 / 155 / 169; solve 85,184 82 / 69 / 66, 110,592
+    // 86 / 80 / 82, 157,464 114 / 98 / 100, 262,144 148 / 142 / 156 (but
+    // 1.4 % slower over a whole stirred and bonded replay).
     const uint32_t n = hw.nAct;
-    lanesD = lanesS = n < 90112 ? 4 : 1;
+    lanesD = n < 90112 ? 4 : n < 200000 ? 2 : 1;
+    lanesS = n < 98304 ? 4 : n < 200000 ? 2 : 1;
     lanesN = 1;  // the ballot-split list build measured slower than one lane per particle
   }
 
@@ -427,7 +432,7 @@ struct Engine3 {
     launchesPerSubstep = (uint64_t)launches;
   }
   void launch_one() {
-    if (debug) launch_t<true>(); else launch_t<false>();
+    if (debug || !inRange) launch_t<true>(); else launch_t<false>();
   }
 
   bool any_loaded() const {

@@ -43,6 +43,7 @@
 // none of this, where they lie outside.
 #pragma once
 #include <cstdint>
+#include "filter.cuh"
 #include "fixed.cuh"
 #include "stage.cuh"
 #include "statehash.cuh"
@@ -489,9 +490,6 @@ __device__ __forceinline__ uint32_t cand_bias(uint32_t own, int dx, int dy) {
 // for a clamped place, so a particle outside the cells takes nothing as near,
 // and nobody takes anything in a border cell (only those hold such particles).
 constexpr int32_t CAND_IN = HS * 16 - 12;  // |d| <= CAND_IN: (|dx| + 8)^2 + (|dy| + 8)^2 < (16 HS)^2
-struct CandBounds {
-  int32_t far, near;
-};
 __device__ __forceinline__ CandBounds cand_bounds(const ScenePar& S) {
   const uint32_t sh = S.cellShift - 6u;
   const int32_t r4 = ((4 * CAND_R) >> sh) + 1;            // >= 4 CAND_R / q, and 9 / 4 >= sqrt(5)
@@ -504,47 +502,6 @@ __device__ __forceinline__ bool cand_outside(const ScenePar& S, int2 p, int2 cc)
 __device__ __forceinline__ CandBounds cand_cell(const ScenePar& S, CandBounds cb, int32_t gx, int32_t gy) {
   const bool border = (uint32_t)(gx - 1) >= S.gridW - 2u || (uint32_t)(gy - 1) >= S.gridH - 2u;
   return CandBounds{cb.far, border ? 0 : cb.near};
-}
-// Candidates [base, base + 32) that lie in [lo, hi), base a multiple of 4, as two
-// masks with candidate base + j at bit 31 - j: the survivors, and those of them
-// near enough to need no test. NV vectors are in flight.
-struct CandMask {
-  uint32_t hit, near;
-};
-template <int NV>
-__device__ __forceinline__ CandMask cand_mask(const uint32_t* QC, uint32_t base, uint32_t lo, uint32_t hi,
-                                              uint32_t bias, CandBounds cb) {
-  const uint32_t nv = min((hi - base + 3u) >> 2, 8u);
-  const uint4* src = reinterpret_cast<const uint4*>(QC + base);
-  const int32_t step = cb.near - cb.far;
-  CandMask m{0u, 0u};
-  auto test = [&](uint32_t code) {
-    const int d = (int)(code + bias);
-    const int32_t acc = __dp4a(d, d, cb.far);
-    m.hit = __funnelshift_l((uint32_t)acc, m.hit, 1);
-    m.near = __funnelshift_l((uint32_t)(acc + step), m.near, 1);
-  };
-  for (uint32_t v = 0; v < nv; v += NV) {
-    uint4 w[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) w[j] = src[min(v + j, nv - 1u)];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      test(w[j].x);
-      test(w[j].y);
-      test(w[j].z);
-      test(w[j].w);
-    }
-  }
-  // codes shifted in so far (a repeated vector's lie past hi), to the top; the
-  // ones outside [lo, hi) dropped
-  const uint32_t done = 4u * ((nv + NV - 1u) / NV * NV);
-  uint32_t in = 0xffffffffu << (32u - done);
-  if (lo > base) in &= 0xffffffffu >> (lo - base);
-  if (hi - base < 32u) in &= ~(0xffffffffu >> (hi - base));
-  m.hit = (m.hit << (32u - done)) & in;
-  m.near = m.near << (32u - done);
-  return m;
 }
 // The survivors that are in the kernel: those that are not near enough tested.
 template <bool DBG>

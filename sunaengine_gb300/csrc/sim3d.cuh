@@ -29,12 +29,16 @@
 // are clamped into [MARGIN, 52 * H - MARGIN], so coordinate differences fit
 // easily and the wrapping r2q of any in-world pair is non-negative; a pair
 // that passes r2q < H2Q has |d| < H = 2^17 on every axis (so the reference's
-// per-axis reject is implied); |G| < 2^24, so a gradient term G*d >> 16 is
-// below 2^25 and never saturates; its square may, and is clamped at once into
-// [0, S_TERM]; |lambda| <= 2^22, so lambda_i + lambda_j never saturates and
-// (lambda sum) * gradient >> 20 is below 2^28.
+// per-axis reject is implied); a gradient term |G d| >> 16 is below 2^20
+// (tables_in_range; the tables' largest is 986,224), so its square's shift fits
+// i32; |lambda| <= 2^22, so lambda_i + lambda_j never saturates,
+// (lambda sum) * gradient >> 20 is below 2^23 and 48 of them below 2^29: solveDp's
+// saturating sum never saturates and may be split. The host checks the tables
+// it is given and runs the debug build's kernels, which need none of this, where
+// they lie outside.
 #pragma once
 #include <cstdint>
+#include "filter.cuh"
 #include "fixed.cuh"
 #include "statehash.cuh"
 
@@ -71,6 +75,18 @@ constexpr int32_t BOND3_DP_MAX = 16384;    // a bond moves a particle at most 1/
 constexpr uint32_t NO_SCENE = 0xffffffffu;
 constexpr uint32_t MAX_AXIS_CELLS = 52;  // keeps the reference's wrapping r2q of any in-world pair non-negative
 
+// What the release build takes from the kernel tables (see above); host.
+inline bool tables_in_range(const int32_t* luts) {
+  for (int i = 0; i < LUT_N; ++i) {
+    // the largest |d| on one axis with table index i: r2q < 128 (i + 1), |d| < 256 (sqrt(r2q) + 1)
+    int64_t q = 0;
+    while ((q + 1) * (q + 1) <= 128ll * (i + 1)) ++q;
+    const int64_t g = luts[LUT_N + i] < 0 ? -(int64_t)luts[LUT_N + i] : luts[LUT_N + i];
+    if ((g * (q + 2) * 256 >> 16) + 1 >= 1 << 20) return false;
+  }
+  return true;
+}
+
 struct Scene3 {
   uint32_t slotBase, cap, n, keyOff;
   uint32_t gx, gy, gz, cellTotal;
@@ -100,6 +116,7 @@ struct Bufs3 {
   int4* PRS;
   uint32_t *keys, *skey, *sslot, *cellStart;
   int4 *PW, *PW2, *PL;
+  uint32_t* QC;       // candidate codes (cand_code), padded to whole 16-byte vectors
   uint32_t *NBR, *NBRN;
   uint32_t nbrStride;
   const int2* WG;     // {W, G}, 2049
@@ -188,11 +205,47 @@ __global__ void __launch_bounds__(256) k3_cellstart(Bufs3 b) {
   cell_starts(b.skey, b.world->slotEnd, b.world->K, b.cellStart);
 }
 
+// ---- the candidate filter of the list build (filter.cuh) --------------------------
+//
+// One in six candidates of the 27 cells is a neighbour. A code holds a
+// particle's place in 64ths of a cell (q = 2048 ticks) modulo 256, x, y, z in
+// bytes 0 to 2; cells in reach differ by at most 127 steps, so the bytes of a
+// code's difference are the signed differences, y and z less one where the byte
+// below borrows, and byte 3 adds at most 1 to the dot product. With flooring off
+// by less than one step an axis, a pair at distance R has a dot product of at
+// most (R / q + 3)^2 + 1, and at least (R / q - 3)^2. r2q floors each axis by
+// 256, so it accepts only |d| < 256 (512 + sqrt(3)) and every pair with
+// |d| < 256 (512 - sqrt(3)).
+// The list pass of the 262 k dam break took 74 us with every candidate tested and
+// takes 61.
+constexpr int32_t CAND_FAR = 4520, CAND_NEAR = 3694;
+static_assert((CAND_FAR - 1) * 1ll * 2048 * 2048 > (131516ll + 3 * 2048) * (131516 + 3 * 2048), "no neighbour is dropped");
+static_assert(CAND_NEAR * 1ll * 2048 * 2048 <= (130628ll - 3 * 2048) * (130628 - 3 * 2048), "a near pair is a neighbour");
+__device__ __forceinline__ uint32_t cand_code(int4 p) {
+  return ((uint32_t)p.x >> 11 & 255u) | ((uint32_t)p.y >> 11 & 255u) << 8 | ((uint32_t)p.z >> 11 & 255u) << 16;
+}
+// Particle s's neighbours among the candidates [base, base + 32) in [lo, hi).
+template <int NV>
+__device__ __forceinline__ uint32_t cand_row(const uint32_t* QC, const int4* PW, uint32_t base, uint32_t lo,
+                                             uint32_t hi, uint32_t s, int4 me) {
+  CandMask c = cand_mask<NV>(QC, base, lo, hi, 0u - cand_code(me), CandBounds{-CAND_FAR - 1, -CAND_NEAR});
+  if (s - base < 32u) c.hit &= ~(0x80000000u >> (s - base));
+  for (uint32_t t = c.hit & ~c.near; t;) {
+    const uint32_t j = (uint32_t)__clz((int)t), bit = 0x80000000u >> j;
+    t ^= bit;
+    const int4 o = PW[base + j];
+    if (r2q_of(wsub(o.x, me.x), wsub(o.y, me.y), wsub(o.z, me.z)) >= H2Q) c.hit ^= bit;
+  }
+  return c.hit;
+}
+
 __global__ void __launch_bounds__(256) k3_gather(Bufs3 b) {
   const uint32_t nAct = b.world->nAct;
   for (uint32_t s = gtid3(); s < nAct; s += gstride3()) {
     const uint32_t slot = b.sslot[s];
-    b.PW[s] = b.PRS[slot];
+    const int4 r = b.PRS[slot];
+    b.PW[s] = r;
+    b.QC[s] = cand_code(r);
     b.inv[slot] = s;
   }
 }
@@ -221,12 +274,21 @@ __global__ void __launch_bounds__(256) k3_nbr(Bufs3 b) {
           if (y < 0 || y >= (int32_t)S.gy) continue;
           uint32_t row = S.keyOff + ((uint32_t)z * S.gy + (uint32_t)y) * S.gx;
           uint32_t lo = b.cellStart[row + x0], hi = b.cellStart[row + x1 + 1];
+          if constexpr (!DBG) {
+            for (uint32_t base = lo & ~3u; base < hi; base += 32)
+              for (uint32_t m = cand_row<2>(b.QC, b.PW, base, lo, hi, s, me); m;) {
+                const uint32_t j = (uint32_t)__clz((int)m);
+                m ^= 0x80000000u >> j;
+                b.NBR[(size_t)cnt * stride + s] = base + j;
+                if (++cnt >= MAXNBR) goto listed;  // the rest of the order is dropped
+              }
+            continue;
+          }
           for (uint32_t t = lo; t < hi; ++t) {
             if (t == s) continue;
             int4 o = b.PW[t];
             int32_t dx = wsub(o.x, me.x), dy2 = wsub(o.y, me.y), dz2 = wsub(o.z, me.z);
-            if constexpr (DBG)
-              if (abs_sat(dx, f) >= H || abs_sat(dy2, f) >= H || abs_sat(dz2, f) >= H) continue;
+            if (abs_sat(dx, f) >= H || abs_sat(dy2, f) >= H || abs_sat(dz2, f) >= H) continue;
             if (r2q_of(dx, dy2, dz2) >= H2Q) continue;
             if (cnt >= MAXNBR) { f.flag(6); continue; }
             b.NBR[(size_t)cnt * stride + s] = t;
@@ -234,6 +296,7 @@ __global__ void __launch_bounds__(256) k3_nbr(Bufs3 b) {
           }
         }
       }
+    listed:
       b.NBRN[s] = cnt;
     }
     return;
@@ -313,6 +376,14 @@ __device__ __forceinline__ uint32_t gor3(uint32_t v) {
   return v;
 }
 
+// clamp(RNE(g * g / 2^16), 0, S_TERM) of one pair's gradient component: |g| <
+// 2^20, and no square is an odd multiple of 2^15, so there is no tie to round.
+template <bool DBG>
+__device__ __forceinline__ int32_t grad_sq(int32_t g, const Flags<DBG>& f) {
+  if constexpr (DBG) return mulc<16>(g, g, 0, S_TERM, f);
+  else return min((int32_t)(((int64_t)g * g + 32768) >> 16), S_TERM);
+}
+
 // density (3d/sim3d.wgsl:397-468). L lanes share a particle's neighbour list;
 // every sum here is a wrapping i32 sum (per-term clamps only), so any split is
 // exact.
@@ -344,8 +415,7 @@ __global__ void __launch_bounds__(256) k3_density(Bufs3 b, const int4* __restric
       sgx = wadd(sgx, gx);
       sgy = wadd(sgy, gy);
       sgz = wadd(sgz, gz);
-      St = wadd(St, wadd(wadd(mulc<16>(gx, gx, 0, S_TERM, f), mulc<16>(gy, gy, 0, S_TERM, f)),
-                         mulc<16>(gz, gz, 0, S_TERM, f)));
+      St = wadd(St, wadd(wadd(grad_sq<DBG>(gx, f), grad_sq<DBG>(gy, f)), grad_sq<DBG>(gz, f)));
     }
     if (L > 1) {
       rho = gsum3<L>(rho);
@@ -451,11 +521,11 @@ __device__ __forceinline__ int3 bond_dp(const Bufs3& b, const Scene3& S, uint32_
 // position goes to PWout.
 //
 // solveDp's running sum saturates, which makes it order-dependent in general.
-// The lanes keep wrapping partial sums and an OR of the terms' magnitudes:
-// when cnt x max|term| <= INT_MAX no prefix of the sequential sum can leave
-// i32, every saturating add is an exact add, and the wrapping total IS the
-// sequential result. Otherwise (never seen in practice) lane 0 redoes the sum
-// sequentially with saturation in the canonical order.
+// In the release build's ranges 48 terms cannot leave i32, so the lanes' wrapping
+// sums are it. Debug builds with more than one lane, which assume no range, keep
+// an OR of the terms' magnitudes: when cnt x max|term| <= INT_MAX every
+// saturating add is an exact one; otherwise lane 0 redoes the sum sequentially
+// with saturation in the canonical order.
 template <bool DBG, int L>
 __global__ void __launch_bounds__(256) k3_solve(Bufs3 b, const int4* __restrict__ PWin, int4* __restrict__ PWout) {
   const uint32_t nAct = b.world->nAct, stride = b.nbrStride;
@@ -487,16 +557,16 @@ __global__ void __launch_bounds__(256) k3_solve(Bufs3 b, const int4* __restrict_
       ax = wadd(ax, tx);
       ay = wadd(ay, ty);
       az = wadd(az, tz);
-      mag |= (uint32_t)abs(tx) | (uint32_t)abs(ty) | (uint32_t)abs(tz);
+      if constexpr (DBG) mag |= (uint32_t)abs(tx) | (uint32_t)abs(ty) | (uint32_t)abs(tz);
     }
     if (L > 1) {
       ax = gsum3<L>(ax);
       ay = gsum3<L>(ay);
       az = gsum3<L>(az);
-      mag = gor3<L>(mag);
+      if constexpr (DBG) mag = gor3<L>(mag);
     }
     if (!valid || sub != 0) continue;
-    const bool exact = (DBG && L == 1) || (uint64_t)mag * cnt <= 0x7fffffffull;
+    const bool exact = !DBG || L == 1 || (uint64_t)mag * cnt <= 0x7fffffffull;
     if (!exact) {
       // the terms' own events were counted in the lane pass; recount only the sum's
       const Flags<false> quiet{nullptr};

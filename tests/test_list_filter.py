@@ -45,3 +45,24 @@ def test_filter_bounds(cell_shift, margin):
         exact_only = (pi >> cell_shift != ci).any(1) | ((cj == 0) | (cj == cells - 1)).any(1)
         assert want[(dot + near < 0) & ~exact_only].all()
         assert (_dot((0x4000 + bias) & 0xffffffff) + far >= 0).all()
+
+
+@pytest.mark.parametrize('cells', [1, 2, 7, 52])
+def test_filter_bounds_3d(cells):
+    """The 3D filter: places modulo 256, three bytes, r2q's floored axes."""
+    rng = np.random.default_rng(cells)
+    n, span, margin = 400000, cells << 17, 32768
+    pi = rng.integers(margin, span - margin + 1, (n, 3))
+    v = rng.normal(size=(n, 3))
+    rad = np.where(rng.random(n) < 0.7, 131072 + rng.integers(-9000, 9000, n), rng.uniform(0, 200000, n))
+    pj = pi + (v / np.linalg.norm(v, axis=1)[:, None] * rad[:, None]).astype(np.int64)
+    ok = ((pj >> 17) - (pi >> 17) >= -1).all(1) & ((pj >> 17) - (pi >> 17) <= 1).all(1)
+    ok &= (pj >= margin).all(1) & (pj <= span - margin).all(1)
+    pi, pj = pi[ok], pj[ok]
+    code = lambda p: ((p >> 11) & 255) @ np.array([1, 256, 65536])
+    dot = _dot((code(pj) - code(pi)) & 0xffffffff)
+    q = (pj - pi) >> 8
+    want = (q * q).sum(1) < 262144
+    assert (dot <= 4520)[want].all()
+    assert want[dot < 3694].all()
+    assert want.any()
