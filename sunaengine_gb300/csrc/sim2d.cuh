@@ -1265,8 +1265,9 @@ __device__ __forceinline__ int2 apply_dp(const Bufs& b, const ScenePar& S, uint3
 }
 
 // The colour class's particles [lo, lo + n) of one tile: dp of each from the
-// pre-pass records, then `out(p, me, dp)` stores the result. `me_of(p)` gives
-// particle p's own pre-pass record. Walls are not passed to `out`.
+// pre-pass records, then `out(p, me, dp, act, sub)` stores the result, called by
+// all L lanes (act false for walls and lanes without a particle). `me_of(p)` gives
+// particle p's own pre-pass record.
 template <bool DBG, int L, class NB, class ME, class OUT>
 __device__ __forceinline__ void colour_tile(const Bufs& b, const NB& nb, ME me_of, OUT out, uint32_t lo, uint32_t n,
                                             const Flags<DBG>& f) {
@@ -1285,8 +1286,7 @@ __device__ __forceinline__ void colour_tile(const Bufs& b, const NB& nb, ME me_o
       dp = solveB_dp<DBG, L, true>(b, nb, p, cnt, sub, xy(me), me.z, f, rigidI ? info : 0u);
     else
       dp = solveB_dp<DBG, L, false>(b, nb, p, cnt, sub, xy(me), me.z, f);
-    if (sub != 0 || !act) continue;
-    out(p, me, dp);
+    out(p, me, dp, act, sub);
   }
 }
 
@@ -1320,18 +1320,37 @@ struct NbrSplit {
   __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
 };
 
-// The corrected record of an active particle: its dp applied, or kept in DP
-// for rigidSolve.
-template <bool DBG>
-__device__ __forceinline__ int4 colour_record(const Bufs& b, uint32_t p, int4 me, int2 dp, const Flags<DBG>& f) {
+// The corrected record of an active particle (its dp applied, or kept in DP for
+// rigidSolve) to *to, by its L lanes. With four or more, lane 0 corrects x,
+// lane 1 y, and lanes 0 to 3 store a word each: the tail is executed once a warp
+// whatever its lanes do, and two axes in one pass halve it (four sweeps at 262 k
+// 235 -> 228 us, at 524 k 335 -> 330, at 1 M 541 -> 536; release builds: the sum of
+// a pred inside 2^28 and a dp below 2^23 cannot saturate).
+template <bool DBG, int L>
+__device__ __forceinline__ void colour_store(const Bufs& b, uint32_t p, int4 me, int2 dp, bool act, uint32_t sub,
+                                             int4* to, const Flags<DBG>& f) {
   const uint32_t info = (uint32_t)me.w;
-  if (info & INFO_RIGID) b.DP[p] = dp;
-  if (!(info & INFO_PINNED)) {
-    const int2 pr = apply_dp(b, b.scenes[b.SCN[p]], info & INFO_MAT, xy(me), dp, f);
-    me.x = pr.x;
-    me.y = pr.y;
+  if constexpr (DBG || L < 4) {
+    if (!act || sub != 0) return;
+    if (info & INFO_RIGID) b.DP[p] = dp;
+    if (!(info & INFO_PINNED)) {
+      const int2 pr = apply_dp(b, b.scenes[b.SCN[p]], info & INFO_MAT, xy(me), dp, f);
+      me.x = pr.x;
+      me.y = pr.y;
+    }
+    *to = me;
+  } else {
+    if (!act || sub >= 4) return;
+    int32_t word = sub == 0 ? me.x : sub == 1 ? me.y : sub == 2 ? me.z : me.w;
+    if (!(info & INFO_PINNED)) {
+      const int32_t dm = matw(b, info & INFO_MAT, M_dpMax), far = (&b.scenes[b.SCN[p]].domW)[sub & 1u] - WALL;
+      const int32_t v = clampi(word + clampi(shr_rne<8>(sub & 1u ? dp.y : dp.x), -dm, dm), WALL, far);
+      if (sub < 2) word = v;
+    } else if ((info & INFO_RIGID) && sub == 0) {
+      b.DP[p] = dp;
+    }
+    reinterpret_cast<int32_t*>(to)[sub] = word;
   }
-  return me;
 }
 
 template <bool DBG, int L>
@@ -1345,8 +1364,10 @@ __device__ __forceinline__ void colour_all(const Bufs& b, int colour, const Flag
   for (uint32_t i0 = blockIdx.x * chunk; i0 < hi - lo; i0 += gridDim.x * chunk)
     colour_tile<DBG, L>(
         b, nb, [&](uint32_t p) { return src[p]; },
-        [&](uint32_t p, int4 me, int2 dp) { src[(int32_t)(p + off)] = colour_record(b, p, me, dp, f); }, lo + i0,
-        min(hi - lo - i0, chunk), f);
+        [&](uint32_t p, int4 me, int2 dp, bool act, uint32_t sub) {
+          colour_store<DBG, L>(b, p, me, dp, act, sub, src + (int32_t)(p + off), f);
+        },
+        lo + i0, min(hi - lo - i0, chunk), f);
 }
 template <bool DBG, int L>
 __global__ void __launch_bounds__(256, 8) k_colour(Bufs b, int colour) {
@@ -1412,7 +1433,9 @@ __global__ void __launch_bounds__(256, 6) k_colour_tiled(Bufs b, int colour, con
     parity ^= 1u;
     colour_tile<DBG, L>(
         b, NbrStaged{stg, b.NBRL, stride}, [&](uint32_t p) { return stg[p - p0]; },
-        [&](uint32_t p, int4 me, int2 dp) { moved(S, p, me, dp); }, lo, n, f);
+        [&](uint32_t p, int4 me, int2 dp, bool act, uint32_t sub) {
+          if (act && sub == 0) moved(S, p, me, dp);
+        }, lo, n, f);
     // the rest of the tile (other colours and walls) unchanged
     for (uint32_t i = threadIdx.x; i < n0; i += blockDim.x) {
       const uint32_t p = p0 + i;
@@ -1437,7 +1460,9 @@ __global__ void __launch_bounds__(256, 6) k_colour_tiled(Bufs b, int colour, con
       const uint32_t m = min(n - i0, blockDim.x / L);
       colour_tile<DBG, L>(
           b, NbrGlobal{src, b.NBR, stride}, [&](uint32_t p) { return src[p]; },
-          [&](uint32_t p, int4 me, int2 dp) { moved(S, p, me, dp); }, lo + i0, m, f);
+          [&](uint32_t p, int4 me, int2 dp, bool act, uint32_t sub) {
+          if (act && sub == 0) moved(S, p, me, dp);
+        }, lo + i0, m, f);
     }
     // every other record of the tile, and the class's walls, copied
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n0; i += gridDim.x * blockDim.x) {
