@@ -302,13 +302,11 @@ struct Engine3 {
     }
     if (lanesTuned) return;
     // Measured on settled columns (phase us with 1 / 2 / 4 lanes): density 64,000
-    // particles 77 / 67 / 67, 85,184 85 / 74 / 75, 110,592 90 / 83 / 91, 157,464
-    // 116 / 102 / 109, 262,144 150 / 155 / 169; solve 85,184 82 / 69 / 66, 110,592
-    // 86 / 80 / 82, 157,464 114 / 98 / 100, 262,144 148 / 142 / 156 (but
-    // 1.4 % slower over a whole stirred and bonded replay).
+    // particles 67 / 67 / 66, 110,592 79 / 83 / 92, 262,144 136 / 157 / 175; solve
+    // 64,000 68 / 66 / 60, 110,592 80 / 82 / 86, 262,144 131 / 153 / 163.
     const uint32_t n = hw.nAct;
-    lanesD = n < 90112 ? 4 : n < 200000 ? 2 : 1;
-    lanesS = n < 98304 ? 4 : n < 200000 ? 2 : 1;
+    lanesD = n < 72000 ? 4 : 1;
+    lanesS = n < 90112 ? 4 : 1;
     lanesN = 1;  // the ballot-split list build measured slower than one lane per particle
   }
 

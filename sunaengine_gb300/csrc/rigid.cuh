@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
       bool touched = false;
       const uint32_t p = b.inv[slot], cnt = b.NBRN[p] & NBRN_COUNT;
       for (uint32_t k = 0; k < cnt && !touched; ++k) {
-        const uint32_t e = b.NBR[(size_t)k * stride + p];
+        const uint32_t e = b.NBR[nbr_at(stride, p, k)];
         if (is_wall(b.PL[e].w)) continue;
         const uint32_t js = b.sslot[e];
         if (!rg_member(b, js, tag)) continue;

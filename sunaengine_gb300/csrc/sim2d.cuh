@@ -43,6 +43,7 @@
 // none of this, where they lie outside.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include "filter.cuh"
 #include "fixed.cuh"
 #include "stage.cuh"
@@ -164,7 +165,7 @@ struct Bufs {
   int2* DP;
   int32_t* HEAT;
   int32_t* CORR;
-  uint32_t* NBR;        // [MAXNBR][nbrStride] sorted indices
+  uint32_t* NBR;        // [MAXNBR / 4][nbrStride][4] sorted indices (nbr_at)
   uint16_t* NBRL;       // [MAXNBR][nbrStride] the same neighbours as tile-local indices | NBRL_BOUNDARY
   uint32_t* NBRN;
   uint32_t nbrStride;
@@ -904,7 +905,7 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
       if (cand_outside(S, pi, cc)) cb.near = 0;
       uint32_t cnt = 0;
       bool congeal = false, sealSeen = false;
-      uint32_t* out = b.NBR + p;
+      NbrWriter out(b.NBR, stride, p);
       // the tile-local list: offsets into this particle's tile's staged neighbourhood
       const uint32_t ts = S.tileShift, tx = (uint32_t)cc.x >> ts, ty = (uint32_t)cc.y >> ts;
       const uint32_t* tr = TILED ? b.TR + (size_t)tile_of(S, cc.x, cc.y) * TR_STRIDE : b.TR;
@@ -932,7 +933,7 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
               for (uint32_t m = cand_test(b.PL, base, c, pi, f); m;) {
                 const uint32_t j = (uint32_t)__clz((int)m);
                 m ^= 0x80000000u >> j;
-                out[(size_t)cnt * stride] = base + j;
+                out.put(cnt, base + j);
                 if (++cnt >= (uint32_t)MAXNBR) goto listed;
               }
             }
@@ -948,7 +949,7 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
             if (!(iq & INFO_BOUNDARY) && (iq & INFO_CONGEAL)) congeal = true;
             if (!(iq & INFO_BOUNDARY) && (iq & INFO_SEAL)) sealSeen = true;
             if (cnt >= (uint32_t)MAXNBR) { f.flag(6); continue; }
-            if (!bnd) out[(size_t)cnt * stride] = q;
+            if (!bnd) out.put(cnt, q);
             if (TILED && local)
               outl[(size_t)cnt * stride] = (uint16_t)((q + delta) | ((iq & INFO_BOUNDARY) ? NBRL_BOUNDARY : 0u));
             cnt++;
@@ -971,7 +972,7 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
     const uint32_t word = nbr_lanes<DBG, L, TILED>(
         b, b.cellStart, cut, valid, p, me,
         [&](uint32_t pos, uint32_t q, uint32_t iq, uint32_t delta) {
-          b.NBR[(size_t)pos * stride + p] = q;
+          b.NBR[nbr_at(stride, p, pos)] = q;
           if (TILED && delta != NO_STAGE)
             b.NBRL[(size_t)pos * stride + p] = (uint16_t)((q + delta) | ((iq & INFO_BOUNDARY) ? NBRL_BOUNDARY : 0u));
         },
@@ -1007,7 +1008,10 @@ struct NbrGlobal {
   const int4* g;
   const uint32_t* nl;
   uint32_t stride;
-  __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[(size_t)k * stride + p]; }
+  __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[nbr_at(stride, p, k)]; }
+  __device__ __forceinline__ uint4 four(uint32_t p, uint32_t v) const {
+    return reinterpret_cast<const uint4*>(nl)[(size_t)v * stride + p];
+  }
   __device__ __forceinline__ int4 rec(uint32_t e) const { return g[e]; }
   __device__ __forceinline__ int2 pred(uint32_t e) const { return ld_pred(g, e); }
   __device__ __forceinline__ int2 wg(const Bufs& b, int id) const { return __ldg(b.WG + id); }
@@ -1074,6 +1078,20 @@ template <bool DBG, int L, class NB>
 __device__ __forceinline__ void solveA_sums(const Bufs& b, const NB& nb, uint32_t p, uint32_t cnt, uint32_t sub,
                                             int2 pi, const Flags<DBG>& f, int32_t& rho, int32_t& S, int32_t& sgx,
                                             int32_t& sgy) {
+  if constexpr (L == 1 && !DBG && std::is_same<NB, NbrGlobal>::value) {
+    // four neighbours' positions in flight, the next vector of entries one ahead
+    // (one position ahead: four passes at 1 M 310 us, at 524 k 194; so: 273 and 160)
+    uint4 e = cnt ? nb.four(p, 0) : make_uint4(0, 0, 0, 0);
+    for (uint32_t k = 0; k < cnt; k += 4) {
+      const int2 p0 = nb.pred(e.x), p1 = nb.pred(e.y), p2 = nb.pred(e.z), p3 = nb.pred(e.w);
+      if (k + 4 < cnt) e = nb.four(p, (k >> 2) + 1);
+      solveA_pair<DBG>(b, nb, pi, p0, f, rho, S, sgx, sgy);
+      if (k + 1 < cnt) solveA_pair<DBG>(b, nb, pi, p1, f, rho, S, sgx, sgy);
+      if (k + 2 < cnt) solveA_pair<DBG>(b, nb, pi, p2, f, rho, S, sgx, sgy);
+      if (k + 3 < cnt) solveA_pair<DBG>(b, nb, pi, p3, f, rho, S, sgx, sgy);
+    }
+    return;
+  }
   // one neighbour ahead: its entry and position are in flight while the
   // current pair is computed
   uint32_t en = sub < cnt ? nb.entry(p, sub) : 0u;
@@ -1313,7 +1331,7 @@ struct NbrSplit {
   uint32_t cut, off;  // dst == src + off (wrapping u32 index), for q < cut
   const uint32_t* nl;
   uint32_t stride;
-  __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[(size_t)k * stride + p]; }
+  __device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t k) const { return nl[nbr_at(stride, p, k)]; }
   __device__ __forceinline__ int4 rec(uint32_t e) const {
     return src[(int32_t)(e < cut ? e + off : e)];
   }

@@ -13,7 +13,7 @@
 //   PW[s], PW2[s]= {pr.x, pr.y, pr.z, tag}   sorted space, ping-pong across iterations
 //   PL[s]        = {pr.x, pr.y, pr.z, lambda}                        density output
 //   tag          = (256 + rhoW(mat)) | scene << 12  (the volume-claim weight and the scene)
-//   NBR[k][s]    = sorted index of neighbour k (column-major, coalesced across s)
+//   NBR[k / 4][s][k % 4] = sorted index of neighbour k (nbr_at, coalesced across s)
 // Sorted space is all scenes' particles ordered by (scene key offset + cell,
 // slot): the stable radix sort of slot-ordered keys leaves every cell in
 // ascending particle id, which is the reference's canonical order (its
@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(256) k3_nbr(Bufs3 b) {
       const int32_t cx = me.x >> HSHIFT, cy = me.y >> HSHIFT, cz = me.z >> HSHIFT;
       const int32_t x0 = max(cx - 1, 0), x1 = min(cx + 1, (int32_t)S.gx - 1);
       uint32_t cnt = 0;
+      NbrWriter out(b.NBR, stride, s);
       for (int dz = -1; dz <= 1; ++dz) {
         int32_t z = cz + dz;
         if (z < 0 || z >= (int32_t)S.gz) continue;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(256) k3_nbr(Bufs3 b) {
               for (uint32_t m = cand_row<2>(b.QC, b.PW, base, lo, hi, s, me); m;) {
                 const uint32_t j = (uint32_t)__clz((int)m);
                 m ^= 0x80000000u >> j;
-                b.NBR[(size_t)cnt * stride + s] = base + j;
+                out.put(cnt, base + j);
                 if (++cnt >= MAXNBR) goto listed;  // the rest of the order is dropped
               }
             continue;
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(256) k3_nbr(Bufs3 b) {
             if (abs_sat(dx, f) >= H || abs_sat(dy2, f) >= H || abs_sat(dz2, f) >= H) continue;
             if (r2q_of(dx, dy2, dz2) >= H2Q) continue;
             if (cnt >= MAXNBR) { f.flag(6); continue; }
-            b.NBR[(size_t)cnt * stride + s] = t;
+            out.put(cnt, t);
             ++cnt;
           }
         }
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(256) k3_nbr(Bufs3 b) {
           }
           if (hit) {
             if (pos >= MAXNBR) f.flag(6);
-            else b.NBR[(size_t)pos * stride + s] = t;
+            else b.NBR[nbr_at(stride, s, pos)] = t;
           }
           cnt += nhit;
         }
@@ -376,6 +377,23 @@ __device__ __forceinline__ uint32_t gor3(uint32_t v) {
   return v;
 }
 
+// pair(record) of every neighbour of particle s, four records in flight and the
+// next four entries one ahead (one record ahead: density 149 us a substep at
+// 262 k, solve 147; so: 136 and 131).
+template <class PAIR>
+__device__ __forceinline__ void nbr_fours(const Bufs3& b, uint32_t s, uint32_t cnt, const int4* rec, PAIR pair) {
+  const uint4* list = reinterpret_cast<const uint4*>(b.NBR) + s;
+  uint4 e = cnt ? list[0] : make_uint4(0, 0, 0, 0);
+  for (uint32_t k = 0; k < cnt; k += 4) {
+    const int4 o0 = rec[e.x], o1 = rec[e.y], o2 = rec[e.z], o3 = rec[e.w];
+    if (k + 4 < cnt) e = list[(size_t)((k >> 2) + 1) * b.nbrStride];
+    pair(o0);
+    if (k + 1 < cnt) pair(o1);
+    if (k + 2 < cnt) pair(o2);
+    if (k + 3 < cnt) pair(o3);
+  }
+}
+
 // clamp(RNE(g * g / 2^16), 0, S_TERM) of one pair's gradient component: |g| <
 // 2^20, and no square is an odd multiple of 2^15, so there is no tie to round.
 template <bool DBG>
@@ -399,23 +417,30 @@ __global__ void __launch_bounds__(256) k3_density(Bufs3 b, const int4* __restric
     const int4 me = valid ? PW[s] : make_int4(0, 0, 0, 0);
     int32_t rho = 0, St = 0, sgx = 0, sgy = 0, sgz = 0;
     const uint32_t cnt = valid ? b.NBRN[s] : 0u;
-    // one neighbour record and two indices ahead (as in the 2D sweeps)
-    int4 on = PW[sub < cnt ? b.NBR[(size_t)sub * stride + s] : 0u];
-    uint32_t tn2 = sub + L < cnt ? b.NBR[(size_t)(sub + L) * stride + s] : 0u;
-    for (uint32_t k = sub; k < cnt; k += L) {
-      const int4 o = on;
-      if (k + L < cnt) on = PW[tn2];
-      if (k + 2 * L < cnt) tn2 = b.NBR[(size_t)(k + 2 * L) * stride + s];
-      int32_t dx = wsub(o.x, me.x), dy = wsub(o.y, me.y), dz = wsub(o.z, me.z);
-      int32_t r2q = r2q_of(dx, dy, dz);
-      if (r2q >= H2Q) continue;
-      int2 wg = __ldg(b.WG + ((uint32_t)r2q >> 7));
+    auto pair = [&](const int4& o) {
+      const int32_t dx = wsub(o.x, me.x), dy = wsub(o.y, me.y), dz = wsub(o.z, me.z);
+      const int32_t r2q = r2q_of(dx, dy, dz);
+      if (r2q >= H2Q) return;
+      const int2 wg = __ldg(b.WG + ((uint32_t)r2q >> 7));
       rho = wadd(rho, wmul(wg.x, (int32_t)((uint32_t)o.w & TAG_W)) >> 8);
-      int32_t gx = mulf<16>(wg.y, dx, f), gy = mulf<16>(wg.y, dy, f), gz = mulf<16>(wg.y, dz, f);
+      const int32_t gx = mulf<16>(wg.y, dx, f), gy = mulf<16>(wg.y, dy, f), gz = mulf<16>(wg.y, dz, f);
       sgx = wadd(sgx, gx);
       sgy = wadd(sgy, gy);
       sgz = wadd(sgz, gz);
       St = wadd(St, wadd(wadd(grad_sq<DBG>(gx, f), grad_sq<DBG>(gy, f)), grad_sq<DBG>(gz, f)));
+    };
+    if constexpr (L == 1 && !DBG) {
+      nbr_fours(b, s, cnt, PW, pair);
+    } else {
+      // one neighbour record and two indices ahead
+      int4 on = PW[sub < cnt ? b.NBR[nbr_at(stride, s, sub)] : 0u];
+      uint32_t tn2 = sub + L < cnt ? b.NBR[nbr_at(stride, s, sub + L)] : 0u;
+      for (uint32_t k = sub; k < cnt; k += L) {
+        const int4 o = on;
+        if (k + L < cnt) on = PW[tn2];
+        if (k + 2 * L < cnt) tn2 = b.NBR[nbr_at(stride, s, k + 2 * L)];
+        pair(o);
+      }
     }
     if (L > 1) {
       rho = gsum3<L>(rho);
@@ -538,26 +563,31 @@ __global__ void __launch_bounds__(256) k3_solve(Bufs3 b, const int4* __restrict_
     const uint32_t cnt = valid ? b.NBRN[s] : 0u;
     int32_t ax = 0, ay = 0, az = 0;
     uint32_t mag = 0;
-    int4 on = b.PL[sub < cnt ? b.NBR[(size_t)sub * stride + s] : 0u];
-    uint32_t tn2 = sub + L < cnt ? b.NBR[(size_t)(sub + L) * stride + s] : 0u;
-    for (uint32_t k = sub; k < cnt; k += L) {
-      const int4 o = on;
-      if (k + L < cnt) on = b.PL[tn2];
-      if (k + 2 * L < cnt) tn2 = b.NBR[(size_t)(k + 2 * L) * stride + s];
+    auto pair = [&](const int4& o) {
       int32_t tx, ty, tz;
-      if (!dp_term(b, me, o, tx, ty, tz, f)) continue;
-      if constexpr (DBG) {
-        if (L == 1) {
-          ax = add_sat(ax, tx, f);
-          ay = add_sat(ay, ty, f);
-          az = add_sat(az, tz, f);
-          continue;
-        }
+      if (!dp_term(b, me, o, tx, ty, tz, f)) return;
+      if constexpr (DBG && L == 1) {
+        ax = add_sat(ax, tx, f);
+        ay = add_sat(ay, ty, f);
+        az = add_sat(az, tz, f);
+      } else {
+        ax = wadd(ax, tx);
+        ay = wadd(ay, ty);
+        az = wadd(az, tz);
+        if constexpr (DBG) mag |= (uint32_t)abs(tx) | (uint32_t)abs(ty) | (uint32_t)abs(tz);
       }
-      ax = wadd(ax, tx);
-      ay = wadd(ay, ty);
-      az = wadd(az, tz);
-      if constexpr (DBG) mag |= (uint32_t)abs(tx) | (uint32_t)abs(ty) | (uint32_t)abs(tz);
+    };
+    if constexpr (L == 1 && !DBG) {
+      nbr_fours(b, s, cnt, b.PL, pair);
+    } else {
+      int4 on = b.PL[sub < cnt ? b.NBR[nbr_at(stride, s, sub)] : 0u];
+      uint32_t tn2 = sub + L < cnt ? b.NBR[nbr_at(stride, s, sub + L)] : 0u;
+      for (uint32_t k = sub; k < cnt; k += L) {
+        const int4 o = on;
+        if (k + L < cnt) on = b.PL[tn2];
+        if (k + 2 * L < cnt) tn2 = b.NBR[nbr_at(stride, s, k + 2 * L)];
+        pair(o);
+      }
     }
     if (L > 1) {
       ax = gsum3<L>(ax);
@@ -572,7 +602,7 @@ __global__ void __launch_bounds__(256) k3_solve(Bufs3 b, const int4* __restrict_
       const Flags<false> quiet{nullptr};
       ax = ay = az = 0;
       for (uint32_t k = 0; k < cnt; ++k) {
-        int4 o = b.PL[b.NBR[(size_t)k * stride + s]];
+        int4 o = b.PL[b.NBR[nbr_at(stride, s, k)]];
         int32_t tx, ty, tz;
         if (!dp_term(b, me, o, tx, ty, tz, quiet)) continue;
         ax = add_sat(ax, tx, f);

@@ -32,6 +32,7 @@
 namespace sn {
 
 constexpr int MAXNBR = 48;
+static_assert(MAXNBR % 4 == 0, "lists are stored four entries to a vector");
 constexpr int BOND_CAP = 48;
 constexpr int MAT_WORDS = 48;
 constexpr int MAT_MAX = 64;
@@ -95,6 +96,26 @@ struct TileInfo {
 };
 
 #ifdef __CUDACC__
+// Neighbour lists are stored four entries to a vector: entry k of particle p is
+// component k & 3 of vector [k / 4][p]. A warp with one lane to a particle reads a
+// vector (four entries) as four full lines, one with four lanes a particle as one
+// line, where rows of single entries took four quarter-used ones.
+__device__ __forceinline__ size_t nbr_at(uint32_t stride, uint32_t p, uint32_t k) {
+  return ((size_t)(k >> 2) * stride + p) * 4u + (k & 3u);
+}
+// Writes one particle's entries in order.
+struct NbrWriter {
+  uint32_t* at;    // the next entry
+  uint32_t jump;   // from a vector's last entry to the next vector's first
+  __device__ __forceinline__ NbrWriter(uint32_t* lists, uint32_t stride, uint32_t p)
+      : at(lists + (size_t)p * 4u), jump(stride * 4u - 3u) {}
+  // entry k, the next one
+  __device__ __forceinline__ void put(uint32_t k, uint32_t q) {
+    *at = q;
+    at += (k & 3u) == 3u ? jump : 1u;
+  }
+};
+
 // cellStart[k] = first sorted position whose key is >= k, for k in [0, K],
 // over the n sorted keys. Each CTA (256 threads) first loads 256 pivots,
 // skey[j * n / 256], into shared memory; a key's answer lies between the last
