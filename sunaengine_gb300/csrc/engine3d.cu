@@ -17,7 +17,7 @@
 #include "../../include/suna.h"
 #include "ckptpool.h"
 #include "radix.cuh"
-#include "sim3d.cuh"
+#include "fused3d.cuh"
 
 using namespace sn::d3;
 namespace radix = sn::radix;
@@ -160,9 +160,10 @@ struct Engine3 {
     if (graph) cudaGraphDestroy(graph);
     void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.QC, b.NBR,
                     b.NBRN, (void*)b.WG, (void*)b.PG, (void*)b.mats, (void*)b.rcp, b.scenes, b.world, b.acc,
-                    b.accLast, b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes};
+                    b.accLast, b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes, fuWords, fuCount, fuLocal};
     for (void* p : ptrs)
       if (p) cudaFree(p);
+    if (fuErrHost) cudaFreeHost(fuErrHost);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (evFork) cudaEventDestroy(evFork);
@@ -238,6 +239,13 @@ struct Engine3 {
     hist = dalloc3<uint32_t>(radix::hist_words((uint32_t)C), err);
     accTmp = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
     fnvBuf = dalloc3<uint32_t>(256, err);
+    fuWords = dalloc3<uint32_t>(4 + F3_MAX_GRID, err);
+    fuCount = dalloc3<uint32_t>((size_t)maxCells + 2, err);
+    fuLocal = dalloc3<uint32_t>((size_t)maxCells + 2, err);
+    if (cudaHostAlloc((void**)&fuErrHost, 4, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&fuErrDev, fuErrHost, 0) != cudaSuccess)
+      return fail("cudaHostAlloc failed");
+    *fuErrHost = 0u;
     if (!err.empty()) return false;
     {
       std::vector<int2> wg(LUT_N), pg(PLANE_N);
@@ -429,7 +437,68 @@ struct Engine3 {
     mark(nullptr);
     launchesPerSubstep = (uint64_t)launches;
   }
-  void launch_one() {
+  // ---- the fused substep of small worlds (fused3d.cuh) ----
+  uint32_t* fuWords = nullptr;  // barrier words (2), error word, pad, slice totals
+  uint32_t *fuCount = nullptr, *fuLocal = nullptr;  // [maxCells + 2] each
+  uint32_t *fuErrHost = nullptr, *fuErrDev = nullptr;
+  bool graphFused = false;
+  static constexpr uint32_t F3_SMEM = 216 * 1024;  // dynamic at most; the static arrays take about 6 KB of the 227
+  static constexpr uint32_t F3_FIXED = (LUT_N + PLANE_N) * 8;
+  uint32_t fused_own() const { return (hw.nAct + (uint32_t)numSMs - 1) / (uint32_t)numSMs; }
+  // Worlds the fused kernel takes: everything it keeps on an SM fits (each slot
+  // a thread, each slice a scan, the owned particles' lists).
+  bool fused_fits() const {
+    const uint64_t G = (uint64_t)numSMs;
+    return !debug && inRange && lanesPin == 0 && G <= F3_MAX_GRID && hw.nAct > 0 && hw.slotEnd <= G * sn::FU_T &&
+           hw.K <= G * sn::FU_T && (uint64_t)(fused_own() + 1) * F3_OWN_BYTES + F3_FIXED <= F3_SMEM;
+  }
+  template <int L>
+  void launch_fused_as() {
+    Fused3Par P;
+    P.iters = iters;
+    P.chain = chainOn ? 1u : 0u;
+    P.slots = hw.slotEnd;
+    P.slice = (hw.K + (uint32_t)numSMs - 1) / (uint32_t)numSMs;
+    P.ownCap = (fused_own() + 1) & ~1u;
+    P.count = fuCount;
+    P.local = fuLocal;
+    P.totals = fuWords + 4;
+    P.tmp = tmpV;
+    P.bar = fuWords;
+    P.err = fuWords + 2;
+    P.errHost = fuErrDev;
+    const auto fn = k3_substep_fused<L>;
+    cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F3_SMEM);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)numSMs);
+    cfg.blockDim = dim3(sn::FU_T);
+    cfg.dynamicSmemBytes = F3_FIXED + P.ownCap * F3_OWN_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, fn, b, P);
+  }
+  void launch_fused() {
+    // as many lanes a particle as leave one round of a CTA's threads
+    const uint32_t own = fused_own();
+    if (own <= 64) launch_fused_as<16>();
+    else if (own <= 128) launch_fused_as<8>();
+    else if (own <= 256) launch_fused_as<4>();
+    else launch_fused_as<2>();
+    launchesPerSubstep = 1;
+  }
+  // The error a fused launch left, after the stream was waited for.
+  bool synced(const char* what) {
+    if (!cuda_ok(cudaStreamSynchronize(st), what)) return false;
+    if (*(volatile uint32_t*)fuErrHost)
+      return fail("%s: a grid barrier timed out; results past it are not valid", what);
+    return true;
+  }
+  void launch_one(bool fused = false) {
+    if (fused) return launch_fused();
     if (debug || !inRange) launch_t<true>(); else launch_t<false>();
   }
 
@@ -455,11 +524,14 @@ struct Engine3 {
     if (count == 0) return true;
     if (layoutDirty && !relayout()) return false;
     if (anyStir && !upload_phase()) return false;
+    const bool fused = fused_fits();
+    if (fused != graphFused) graphValid = false;
     if (useGraph && !graphValid) {
       if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
       if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
       if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture")) return false;
-      launch_one();
+      launch_one(fused);
+      graphFused = fused;
       if (!cuda_ok(cudaStreamEndCapture(st, &graph), "endCapture")) return false;
       if (!cuda_ok(cudaGraphInstantiate(&gexec, graph, 0), "instantiate")) return false;
       graphValid = true;
@@ -469,7 +541,7 @@ struct Engine3 {
       if (useGraph) {
         if (!cuda_ok(cudaGraphLaunch(gexec, st), "graphLaunch")) return false;
       } else {
-        launch_one();
+        launch_one(fused);
       }
     }
     cudaEventRecord(ev1, st);
@@ -578,6 +650,12 @@ struct Engine3 {
                                            0xa4093822u, 0x299f31d0u, 0x082efa98u, 0xec4e6c89u};
     cudaMemcpyAsync(b.chain + (size_t)s * 8, CHAIN_INIT, 32, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b.acc + (size_t)s * 8, 0, 32, st);
+    if (*(volatile uint32_t*)fuErrHost) {  // a launch that gave up leaves its counts behind
+      cudaMemsetAsync(fuWords, 0, 12, st);
+      cudaMemsetAsync(fuCount, 0, ((size_t)maxCells + 2) * 4, st);
+      if (!cuda_ok(cudaStreamSynchronize(st), "load")) return false;
+      *fuErrHost = 0u;
+    }
     if (!clear_bonds(s)) return false;
     h.n = sc->n;
     h.gx = sc->gx;
@@ -740,13 +818,13 @@ struct Engine3 {
     if (!check_scene(s)) return false;
     if (accFresh && !layoutDirty) {
       cudaMemcpyAsync(out, b.accLast + (size_t)s * 8, 32, cudaMemcpyDeviceToHost, st);
-      return cuda_ok(cudaStreamSynchronize(st), "digest");
+      return synced("digest");
     }
     if (layoutDirty && !relayout()) return false;
     cudaMemsetAsync(accTmp, 0, sizeof(uint32_t) * 8 * maxScenes, st);
     k3_hash<<<grid_for(hw.slotEnd), 256, 0, st>>>(b, accTmp);
     cudaMemcpyAsync(out, accTmp + s * 8, 32, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "digest");
+    return synced("digest");
   }
 
   // chain() (3d/app.js:717-744): stripe words on the device, the 8-lane fold
@@ -756,7 +834,7 @@ struct Engine3 {
     uint32_t words[256];
     k3_fnv<<<1, 256, 0, st>>>(b.state, sh[s].slotBase, sh[s].n, fnvBuf);
     cudaMemcpyAsync(words, fnvBuf, sizeof(words), cudaMemcpyDeviceToHost, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "fnv")) return false;
+    if (!synced("fnv")) return false;
     for (uint32_t L = 0; L < 8; ++L) out[L] = 2166136261u ^ (L * 0x9e3779b9u);
     for (uint32_t k = 0; k < 256; ++k)
       for (uint32_t L = 0; L < 8; ++L) {
@@ -769,7 +847,7 @@ struct Engine3 {
   bool chain(uint32_t s, uint32_t out[8]) {
     if (!check_scene(s)) return false;
     cudaMemcpyAsync(out, b.chain + (size_t)s * 8, 32, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "chain");
+    return synced("chain");
   }
 
   bool read_state(uint32_t s, int32_t* out, size_t words) {
@@ -777,7 +855,7 @@ struct Engine3 {
     size_t need = (size_t)sh[s].n * 8;
     if (!out || words < need) return fail("read_state needs %zu words", need);
     cudaMemcpyAsync(out, b.state + (size_t)sh[s].slotBase * 8, need * 4, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "read_state");
+    return synced("read_state");
   }
 
   // A keyframe: the state words fully determine every later substep (the
@@ -966,7 +1044,7 @@ int sn3_debug_counters(sn3_engine* e, uint32_t out[16]) {
 }
 int sn3_sync(sn3_engine* e) {
   if (!e) return SN_E_INVALID;
-  return rc3(e->w, e->w.cuda_ok(cudaStreamSynchronize(e->w.st), "sync"));
+  return rc3(e->w, e->w.synced("sync"));
 }
 int sn3_get_info(sn3_engine* e, uint32_t scene, sn3_info* out) {
   if (!e || !out) return SN_E_INVALID;

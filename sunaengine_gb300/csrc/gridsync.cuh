@@ -1,0 +1,69 @@
+// What the fused substeps (fused2d.cuh, fused3d.cuh) share: the grid barrier of a
+// cooperative launch and a CTA's prefix sum.
+#pragma once
+#include <cstdint>
+
+namespace sn {
+
+constexpr int FU_T = 1024;  // threads of a fused substep's CTA, one CTA to an SM
+constexpr uint32_t ERR_BARRIER = 8u;
+constexpr long long BARRIER_WAIT_CYCLES = 1ll << 31;  // about a second
+
+// Grid barrier of a cooperative launch: `target` counts the arrivals every CTA
+// waits for (monotonic over the launch). A CTA that waits longer than
+// BARRIER_WAIT_CYCLES raises ERR_BARRIER; false sends the whole CTA out.
+__device__ __forceinline__ bool grid_wait(uint32_t* bar, uint32_t* err, uint32_t& target) {
+  __syncthreads();
+  int bad = 0;
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    const long long t0 = clock64();
+    for (;;) {
+      uint32_t v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if ((int32_t)(v - target) >= 0) break;
+      if (clock64() - t0 > BARRIER_WAIT_CYCLES) {
+        atomicOr(err, ERR_BARRIER);
+        bad = 1;
+        break;
+      }
+    }
+  }
+  return __syncthreads_or(bad) == 0;
+}
+
+// Exclusive prefix of x[0, n) in place by the whole CTA, the total in x[n];
+// returns the largest element (to every thread).
+__device__ __forceinline__ uint32_t cta_scan(uint32_t* x, uint32_t n, uint32_t* ws) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t per = (n + FU_T - 1) / FU_T, lo = min(tid * per, n), hi = min(lo + per, n);
+  uint32_t sum = 0, most = 0;
+  for (uint32_t k = lo; k < hi; ++k) {
+    sum += x[k];
+    most = max(most, x[k]);
+  }
+  uint32_t inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += v;
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 31) ws[warp] = inc;
+  if (lane == 0) ws[32 + warp] = most;
+  __syncthreads();
+  uint32_t run = inc - sum;
+  for (uint32_t w = 0; w < warp; ++w) run += ws[w];
+  for (uint32_t k = lo; k < hi; ++k) {
+    const uint32_t v = x[k];
+    x[k] = run;
+    run += v;
+  }
+  if (tid == FU_T - 1) x[n] = run;
+  most = __reduce_max_sync(0xffffffffu, ws[32 + lane]);
+  __syncthreads();
+  return most;
+}
+
+}  // namespace sn

@@ -46,6 +46,7 @@
 #include <type_traits>
 #include "filter.cuh"
 #include "fixed.cuh"
+#include "gridsync.cuh"
 #include "stage.cuh"
 #include "statehash.cuh"
 #include "world.cuh"
@@ -202,7 +203,7 @@ struct Bufs {
   uint32_t* rmark;      // [cap] rigidMember's leave marks, slot space
 };
 
-enum : uint32_t { ERR_UNSUPPORTED_ROW = 1u, ERR_BOND_PARTNER = 2u, ERR_STAGE_TIMEOUT = 4u, ERR_BARRIER = 8u };
+enum : uint32_t { ERR_UNSUPPORTED_ROW = 1u, ERR_BOND_PARTNER = 2u, ERR_STAGE_TIMEOUT = 4u };  // and ERR_BARRIER
 
 __device__ __forceinline__ int32_t matw(const Bufs& b, uint32_t m, int w) { return __ldg(b.mats + m * MAT_WORDS + w); }
 
@@ -1696,7 +1697,6 @@ __global__ void __launch_bounds__(256) k_apply_fric(Bufs b) {
 // before each launch) and releases generation g by writing g + 1 to bar[1];
 // a CTA that waits longer than BARRIER_WAIT_CYCLES raises ERR_BARRIER and the
 // kernel returns (its results are then not valid; sn_check_errors reports it).
-constexpr long long BARRIER_WAIT_CYCLES = 1ll << 31;  // about a second
 __device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t* err, uint32_t& gen) {
   __shared__ uint32_t okS;
   __syncthreads();

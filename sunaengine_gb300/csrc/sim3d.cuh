@@ -167,6 +167,34 @@ __device__ __forceinline__ bool ball_term(const Bufs3& b, const Scene3& S, uint3
   return true;
 }
 
+// predict (3d/sim3d.wgsl:188-215) of one slot: the record of its predicted position.
+template <bool DBG>
+__device__ __forceinline__ int4 predict_record(const Bufs3& b, const Scene3& S, uint32_t sc, uint32_t slot,
+                                               const Flags<DBG>& f) {
+  const int4* w4 = reinterpret_cast<const int4*>(b.state + (size_t)slot * 8);
+  int4 p = w4[0], v4 = w4[1];
+  uint32_t m = (uint32_t)p.w;
+  const int32_t grav = __ldg(b.mats + m * 4 + 0), rhoW = __ldg(b.mats + m * 4 + 1), damp = __ldg(b.mats + m * 4 + 2);
+  int32_t vx = v4.x, vy = sub_sat(v4.y, grav, f), vz = v4.z;
+  if (S.stirAmp != 0) {
+    const int32_t phase =
+        S.frame ? (int32_t)(((S.substep - S.substep % S.frame) * 384u) & 131071u) : S.stirPhase;
+    int32_t t0 = ((phase + 32768) & 131071) - 65536;
+    int32_t tri = (t0 < 0 ? -t0 : t0) - 32768;
+    vx = add_sat(vx, mul<16>(tri, S.stirAmp, f), f);
+  }
+  vx = mul<16>(vx, damp, f);
+  vy = mul<16>(vy, damp, f);
+  vz = mul<16>(vz, damp, f);
+  int3 pr = clamp_world(S, add_sat(p.x, vx, f), add_sat(p.y, vy, f), add_sat(p.z, vz, f));
+  const uint32_t bonded = b.bflag[slot] ? TAG_BONDED : 0u;
+  return make_int4(pr.x, pr.y, pr.z, (int32_t)((uint32_t)(256 + rhoW) | (sc << TAG_SHIFT) | bonded));
+}
+__device__ __forceinline__ uint32_t key_of(const Scene3& S, int4 pr) {
+  const uint32_t cx = (uint32_t)pr.x >> HSHIFT, cy = (uint32_t)pr.y >> HSHIFT, cz = (uint32_t)pr.z >> HSHIFT;
+  return S.keyOff + (cz * S.gy + cy) * S.gx + cx;
+}
+
 // predict (3d/sim3d.wgsl:188-215) and the grid key of the predicted position.
 template <bool DBG>
 __global__ void __launch_bounds__(256) k3_predict(Bufs3 b) {
@@ -177,26 +205,9 @@ __global__ void __launch_bounds__(256) k3_predict(Bufs3 b) {
     if (sc == NO_SCENE) { b.keys[slot] = W.K; continue; }
     const Scene3& S = b.scenes[sc];
     if (slot - S.slotBase >= S.n) { b.keys[slot] = W.K; continue; }
-    const int4* w4 = reinterpret_cast<const int4*>(b.state + (size_t)slot * 8);
-    int4 p = w4[0], v4 = w4[1];
-    uint32_t m = (uint32_t)p.w;
-    const int32_t grav = __ldg(b.mats + m * 4 + 0), rhoW = __ldg(b.mats + m * 4 + 1), damp = __ldg(b.mats + m * 4 + 2);
-    int32_t vx = v4.x, vy = sub_sat(v4.y, grav, f), vz = v4.z;
-    if (S.stirAmp != 0) {
-      const int32_t phase =
-          S.frame ? (int32_t)(((S.substep - S.substep % S.frame) * 384u) & 131071u) : S.stirPhase;
-      int32_t t0 = ((phase + 32768) & 131071) - 65536;
-      int32_t tri = (t0 < 0 ? -t0 : t0) - 32768;
-      vx = add_sat(vx, mul<16>(tri, S.stirAmp, f), f);
-    }
-    vx = mul<16>(vx, damp, f);
-    vy = mul<16>(vy, damp, f);
-    vz = mul<16>(vz, damp, f);
-    int3 pr = clamp_world(S, add_sat(p.x, vx, f), add_sat(p.y, vy, f), add_sat(p.z, vz, f));
-    const uint32_t bonded = b.bflag[slot] ? TAG_BONDED : 0u;
-    b.PRS[slot] = make_int4(pr.x, pr.y, pr.z, (int32_t)((uint32_t)(256 + rhoW) | (sc << TAG_SHIFT) | bonded));
-    uint32_t cx = (uint32_t)pr.x >> HSHIFT, cy = (uint32_t)pr.y >> HSHIFT, cz = (uint32_t)pr.z >> HSHIFT;
-    b.keys[slot] = S.keyOff + (cz * S.gy + cy) * S.gx + cx;
+    const int4 pr = predict_record(b, S, sc, slot, f);
+    b.PRS[slot] = pr;
+    b.keys[slot] = key_of(S, pr);
   }
 }
 
@@ -402,6 +413,58 @@ __device__ __forceinline__ int32_t grad_sq(int32_t g, const Flags<DBG>& f) {
   else return min((int32_t)(((int64_t)g * g + 32768) >> 16), S_TERM);
 }
 
+// One neighbour's terms of density's sums. WG: the kernel table (global or a
+// shared copy).
+template <bool DBG>
+__device__ __forceinline__ void density_pair(const int2* WG, const int4& me, const int4& o, int32_t& rho, int32_t& St,
+                                             int32_t& sgx, int32_t& sgy, int32_t& sgz, const Flags<DBG>& f) {
+  const int32_t dx = wsub(o.x, me.x), dy = wsub(o.y, me.y), dz = wsub(o.z, me.z);
+  const int32_t r2q = r2q_of(dx, dy, dz);
+  if (r2q >= H2Q) return;
+  const int2 wg = WG[(uint32_t)r2q >> 7];
+  rho = wadd(rho, wmul(wg.x, (int32_t)((uint32_t)o.w & TAG_W)) >> 8);
+  const int32_t gx = mulf<16>(wg.y, dx, f), gy = mulf<16>(wg.y, dy, f), gz = mulf<16>(wg.y, dz, f);
+  sgx = wadd(sgx, gx);
+  sgy = wadd(sgy, gy);
+  sgz = wadd(sgz, gz);
+  St = wadd(St, wadd(wadd(grad_sq<DBG>(gx, f), grad_sq<DBG>(gy, f)), grad_sq<DBG>(gz, f)));
+}
+
+// density's tail from the pair sums: the own, wall and ball terms, then lambda.
+// PG: the plane table (global or a shared copy).
+template <bool DBG>
+__device__ __forceinline__ int32_t density_lambda(const Bufs3& b, const int2* PG, int32_t W0, const int4& me,
+                                                  int32_t rho, int32_t St, int32_t sgx, int32_t sgy, int32_t sgz,
+                                                  const Flags<DBG>& f) {
+  const uint32_t sc = scene_of_tag((uint32_t)me.w);
+  const Scene3& S = b.scenes[sc];
+  rho = wadd(rho, wmul(W0, (int32_t)((uint32_t)me.w & TAG_W)) >> 8);
+#pragma unroll
+  for (int w = 0; w < 6; ++w) {
+    int32_t dist = wall_dist(S, me.x, me.y, me.z, w);
+    if (dist >= H) continue;
+    int2 pg = PG[(uint32_t)dist >> 8];
+    rho = wadd(rho, pg.x);
+    int32_t gm = (w & 1) ? pg.y : neg_sat(pg.y, f);
+    if (w & 1) (void)neg_sat(pg.y, f);  // select() evaluates both arms
+    int axis = w >> 1;
+    if (axis == 0) sgx = wadd(sgx, gm); else if (axis == 1) sgy = wadd(sgy, gm); else sgz = wadd(sgz, gm);
+    St = wadd(St, s_term(gm, f));  // the two zero components contribute clamp(0) = 0
+  }
+  int32_t bw;
+  int3 bg;
+  if (ball_term(b, S, sc, me.x, me.y, me.z, bw, bg, f)) {
+    rho = wadd(rho, bw);
+    sgx = wadd(sgx, bg.x);
+    sgy = wadd(sgy, bg.y);
+    sgz = wadd(sgz, bg.z);
+    St = wadd(St, wadd(wadd(s_term(bg.x, f), s_term(bg.y, f)), s_term(bg.z, f)));
+  }
+  St = wadd(St, wadd(wadd(s_term(sgx, f), s_term(sgy, f)), s_term(sgz, f)));
+  int32_t Cq = clampi(shr_rne<4>(wsub(rho, RHO0)), 0, C_MAX);
+  return clampi(neg_sat(divshift<24>(Cq, wadd(St, EPS_S), b.rcp, f), f), -LAM_MAX, LAM_MAX);
+}
+
 // density (3d/sim3d.wgsl:397-468). L lanes share a particle's neighbour list;
 // every sum here is a wrapping i32 sum (per-term clamps only), so any split is
 // exact.
@@ -417,18 +480,7 @@ __global__ void __launch_bounds__(256) k3_density(Bufs3 b, const int4* __restric
     const int4 me = valid ? PW[s] : make_int4(0, 0, 0, 0);
     int32_t rho = 0, St = 0, sgx = 0, sgy = 0, sgz = 0;
     const uint32_t cnt = valid ? b.NBRN[s] : 0u;
-    auto pair = [&](const int4& o) {
-      const int32_t dx = wsub(o.x, me.x), dy = wsub(o.y, me.y), dz = wsub(o.z, me.z);
-      const int32_t r2q = r2q_of(dx, dy, dz);
-      if (r2q >= H2Q) return;
-      const int2 wg = __ldg(b.WG + ((uint32_t)r2q >> 7));
-      rho = wadd(rho, wmul(wg.x, (int32_t)((uint32_t)o.w & TAG_W)) >> 8);
-      const int32_t gx = mulf<16>(wg.y, dx, f), gy = mulf<16>(wg.y, dy, f), gz = mulf<16>(wg.y, dz, f);
-      sgx = wadd(sgx, gx);
-      sgy = wadd(sgy, gy);
-      sgz = wadd(sgz, gz);
-      St = wadd(St, wadd(wadd(grad_sq<DBG>(gx, f), grad_sq<DBG>(gy, f)), grad_sq<DBG>(gz, f)));
-    };
+    auto pair = [&](const int4& o) { density_pair(b.WG, me, o, rho, St, sgx, sgy, sgz, f); };
     if constexpr (L == 1 && !DBG) {
       nbr_fours(b, s, cnt, PW, pair);
     } else {
@@ -450,33 +502,7 @@ __global__ void __launch_bounds__(256) k3_density(Bufs3 b, const int4* __restric
       sgz = gsum3<L>(sgz);
     }
     if (!valid || sub != 0) continue;
-    const uint32_t sc = scene_of_tag((uint32_t)me.w);
-    const Scene3& S = b.scenes[sc];
-    rho = wadd(rho, wmul(W0, (int32_t)((uint32_t)me.w & TAG_W)) >> 8);
-#pragma unroll
-    for (int w = 0; w < 6; ++w) {
-      int32_t dist = wall_dist(S, me.x, me.y, me.z, w);
-      if (dist >= H) continue;
-      int2 pg = __ldg(b.PG + ((uint32_t)dist >> 8));
-      rho = wadd(rho, pg.x);
-      int32_t gm = (w & 1) ? pg.y : neg_sat(pg.y, f);
-      if (w & 1) (void)neg_sat(pg.y, f);  // select() evaluates both arms
-      int axis = w >> 1;
-      if (axis == 0) sgx = wadd(sgx, gm); else if (axis == 1) sgy = wadd(sgy, gm); else sgz = wadd(sgz, gm);
-      St = wadd(St, s_term(gm, f));  // the two zero components contribute clamp(0) = 0
-    }
-    int32_t bw;
-    int3 bg;
-    if (ball_term(b, S, sc, me.x, me.y, me.z, bw, bg, f)) {
-      rho = wadd(rho, bw);
-      sgx = wadd(sgx, bg.x);
-      sgy = wadd(sgy, bg.y);
-      sgz = wadd(sgz, bg.z);
-      St = wadd(St, wadd(wadd(s_term(bg.x, f), s_term(bg.y, f)), s_term(bg.z, f)));
-    }
-    St = wadd(St, wadd(wadd(s_term(sgx, f), s_term(sgy, f)), s_term(sgz, f)));
-    int32_t Cq = clampi(shr_rne<4>(wsub(rho, RHO0)), 0, C_MAX);
-    int32_t lam = clampi(neg_sat(divshift<24>(Cq, wadd(St, EPS_S), b.rcp, f), f), -LAM_MAX, LAM_MAX);
+    const int32_t lam = density_lambda(b, b.PG, W0, me, rho, St, sgx, sgy, sgz, f);
     b.PL[s] = make_int4(me.x, me.y, me.z, lam);
   }
 }
@@ -484,12 +510,12 @@ __global__ void __launch_bounds__(256) k3_density(Bufs3 b, const int4* __restric
 // One solveDp pair term (3d/sim3d.wgsl:493-509); false when the pair is out
 // of range (it adds nothing).
 template <bool DBG>
-__device__ __forceinline__ bool dp_term(const Bufs3& b, const int4& me, const int4& o, int32_t& tx, int32_t& ty,
+__device__ __forceinline__ bool dp_term(const int2* WG, const int4& me, const int4& o, int32_t& tx, int32_t& ty,
                                         int32_t& tz, const Flags<DBG>& f) {
   int32_t dx = wsub(o.x, me.x), dy = wsub(o.y, me.y), dz = wsub(o.z, me.z);
   int32_t r2q = r2q_of(dx, dy, dz);
   if (r2q >= H2Q) return false;
-  int32_t gt = __ldg(&b.WG[(uint32_t)r2q >> 7].y);
+  int32_t gt = WG[(uint32_t)r2q >> 7].y;
   int32_t lsum = DBG ? add_sat(me.w, o.w, f) : wadd(me.w, o.w);
   tx = mulf<20>(lsum, mulf<16>(gt, dx, f), f);
   ty = mulf<20>(lsum, mulf<16>(gt, dy, f), f);
@@ -541,6 +567,42 @@ __device__ __forceinline__ int3 bond_dp(const Bufs3& b, const Scene3& S, uint32_
                    clampi(shr_rne<8>(bz), -BOND3_DP_MAX, BOND3_DP_MAX));
 }
 
+// solveDp's tail and applyDp from the pair sums: the wall, ball and bond terms,
+// then the corrected position of sorted particle s. me: {position, lambda}.
+template <bool DBG>
+__device__ __forceinline__ int3 solve_place(const Bufs3& b, const int2* PG, const int4& me, int32_t tag, uint32_t s,
+                                            int32_t ax, int32_t ay, int32_t az, const Flags<DBG>& f) {
+  const uint32_t sc = scene_of_tag((uint32_t)tag);
+  const Scene3& S = b.scenes[sc];
+  const int32_t lami = me.w;
+#pragma unroll
+  for (int w = 0; w < 6; ++w) {
+    int32_t dist = wall_dist(S, me.x, me.y, me.z, w);
+    if (dist >= H) continue;
+    int32_t pg = PG[(uint32_t)dist >> 8].y;
+    int32_t gm = (w & 1) ? pg : neg_sat(pg, f);
+    if (w & 1) (void)neg_sat(pg, f);
+    int axis = w >> 1;
+    // the zero components add fp_mul_s(lami, 0) = 0
+    int32_t c = mul<20>(lami, gm, f);
+    if (axis == 0) ax = add_sat(ax, c, f); else if (axis == 1) ay = add_sat(ay, c, f); else az = add_sat(az, c, f);
+  }
+  int32_t bw;
+  int3 bg;
+  if (ball_term(b, S, sc, me.x, me.y, me.z, bw, bg, f)) {
+    ax = add_sat(ax, mul<20>(lami, bg.x, f), f);
+    ay = add_sat(ay, mul<20>(lami, bg.y, f), f);
+    az = add_sat(az, mul<20>(lami, bg.z, f), f);
+  }
+  if ((uint32_t)tag & TAG_BONDED) {
+    const int3 bd = bond_dp(b, S, b.sslot[s], me, f);
+    ax = add_sat(ax, bd.x, f);
+    ay = add_sat(ay, bd.y, f);
+    az = add_sat(az, bd.z, f);
+  }
+  return clamp_world(S, add_sat(me.x, ax, f), add_sat(me.y, ay, f), add_sat(me.z, az, f));
+}
+
 // solveDp + applyDp (3d/sim3d.wgsl:476-537), fused over a double buffer:
 // every read is of the PL / PW written by the previous kernel, the new
 // position goes to PWout.
@@ -565,7 +627,7 @@ __global__ void __launch_bounds__(256) k3_solve(Bufs3 b, const int4* __restrict_
     uint32_t mag = 0;
     auto pair = [&](const int4& o) {
       int32_t tx, ty, tz;
-      if (!dp_term(b, me, o, tx, ty, tz, f)) return;
+      if (!dp_term(b.WG, me, o, tx, ty, tz, f)) return;
       if constexpr (DBG && L == 1) {
         ax = add_sat(ax, tx, f);
         ay = add_sat(ay, ty, f);
@@ -604,42 +666,14 @@ __global__ void __launch_bounds__(256) k3_solve(Bufs3 b, const int4* __restrict_
       for (uint32_t k = 0; k < cnt; ++k) {
         int4 o = b.PL[b.NBR[nbr_at(stride, s, k)]];
         int32_t tx, ty, tz;
-        if (!dp_term(b, me, o, tx, ty, tz, quiet)) continue;
+        if (!dp_term(b.WG, me, o, tx, ty, tz, quiet)) continue;
         ax = add_sat(ax, tx, f);
         ay = add_sat(ay, ty, f);
         az = add_sat(az, tz, f);
       }
     }
     const int32_t tag = PWin[s].w;
-    const uint32_t sc = scene_of_tag((uint32_t)tag);
-    const Scene3& S = b.scenes[sc];
-    const int32_t lami = me.w;
-#pragma unroll
-    for (int w = 0; w < 6; ++w) {
-      int32_t dist = wall_dist(S, me.x, me.y, me.z, w);
-      if (dist >= H) continue;
-      int32_t pg = __ldg(&b.PG[(uint32_t)dist >> 8].y);
-      int32_t gm = (w & 1) ? pg : neg_sat(pg, f);
-      if (w & 1) (void)neg_sat(pg, f);
-      int axis = w >> 1;
-      // the zero components add fp_mul_s(lami, 0) = 0
-      int32_t c = mul<20>(lami, gm, f);
-      if (axis == 0) ax = add_sat(ax, c, f); else if (axis == 1) ay = add_sat(ay, c, f); else az = add_sat(az, c, f);
-    }
-    int32_t bw;
-    int3 bg;
-    if (ball_term(b, S, sc, me.x, me.y, me.z, bw, bg, f)) {
-      ax = add_sat(ax, mul<20>(lami, bg.x, f), f);
-      ay = add_sat(ay, mul<20>(lami, bg.y, f), f);
-      az = add_sat(az, mul<20>(lami, bg.z, f), f);
-    }
-    if ((uint32_t)tag & TAG_BONDED) {
-      const int3 bd = bond_dp(b, S, b.sslot[s], me, f);
-      ax = add_sat(ax, bd.x, f);
-      ay = add_sat(ay, bd.y, f);
-      az = add_sat(az, bd.z, f);
-    }
-    int3 pr = clamp_world(S, add_sat(me.x, ax, f), add_sat(me.y, ay, f), add_sat(me.z, az, f));
+    const int3 pr = solve_place(b, b.PG, me, tag, s, ax, ay, az, f);
     PWout[s] = make_int4(pr.x, pr.y, pr.z, tag);
   }
 }
@@ -705,9 +739,8 @@ __global__ void __launch_bounds__(256) k3_hash(Bufs3 b, uint32_t* __restrict__ a
 
 // Per-scene chain fold of this substep's digest (src/engine.js:4154 semantics)
 // and the scene's substep counter.
-__global__ void k3_fold(Bufs3 b, int doChain) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= b.world->numScenes || !b.scenes[s].active) return;
+__device__ __forceinline__ void fold_scene3(const Bufs3& b, uint32_t s, bool doChain) {
+  if (!b.scenes[s].active) return;
   b.scenes[s].substep += 1u;
   if (!doChain) return;
   uint32_t a[8], nx[8];
@@ -721,6 +754,10 @@ __global__ void k3_fold(Bufs3 b, int doChain) {
     b.accLast[s * 8 + j] = a[j];
     b.acc[s * 8 + j] = 0u;
   }
+}
+__global__ void k3_fold(Bufs3 b, int doChain) {
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < b.world->numScenes) fold_scene3(b, s, doChain != 0);
 }
 
 // digestStripe (3d/sim3d.wgsl:555-590): 256 fixed contiguous stripes of
