@@ -326,6 +326,33 @@ __global__ void __launch_bounds__(256) k_fill_u32(uint32_t* __restrict__ out, ui
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = v;
 }
 
+// A checkpoint's copy of a scene's bond rows (words of 8 bytes, `n` of them).
+// While no row of the world has ever been non-empty (*live == 0, see Bufs::work)
+// the copy is four marker words, which no bond row holds (bit 31 is not part of a
+// bond word): 200 MB less to copy at 1 M particles.
+__device__ constexpr uint32_t ROWS_EMPTY[4] = {0x80000000u, 0xfeedbeefu, 0x80000000u, 0xfeedbeefu};
+__global__ void __launch_bounds__(256) k_rows_save(const uint2* __restrict__ rows, size_t n, const uint32_t* live,
+                                                   uint2* __restrict__ copy) {
+  if (*live == 0u) {
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+      copy[threadIdx.x] = make_uint2(ROWS_EMPTY[2 * threadIdx.x], ROWS_EMPTY[2 * threadIdx.x + 1]);
+    return;
+  }
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    copy[i] = rows[i];
+}
+// The rows back; `live` is raised when they may be non-empty (never lowered: other
+// scenes' rows, and these, may already be).
+__global__ void __launch_bounds__(256) k_rows_load(const uint2* __restrict__ copy, size_t n, uint32_t* live,
+                                                   uint2* __restrict__ rows) {
+  const uint2 a = copy[0], c = copy[1];
+  const bool empty = a.x == ROWS_EMPTY[0] && a.y == ROWS_EMPTY[1] && c.x == ROWS_EMPTY[2] && c.y == ROWS_EMPTY[3];
+  if (empty && *(volatile uint32_t*)live == 0u) return;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    rows[i] = empty ? make_uint2(0u, 0u) : copy[i];
+  if (!empty && blockIdx.x == 0 && threadIdx.x == 0) *live = 1u;
+}
+
 template <typename T>
 T* dalloc(size_t count, std::string& err) {
   if (count == 0) count = 1;
@@ -431,6 +458,7 @@ struct World {
                     hits, accTmp, devEv, devEp, boxChunks, upl, uplRes, barBuf, fuBar, fuCount, eraseBuf, initPos};
     for (void* p : ptrs)
       if (p) cudaFree(p);
+    if (mirror) cudaFreeHost(mirror);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (evFork) cudaEventDestroy(evFork);
@@ -518,6 +546,9 @@ struct World {
     b.acc = dalloc<uint32_t>((size_t)scenesCap * 8, err);
     b.accLast = dalloc<uint32_t>((size_t)scenesCap * 8, err);
     b.chain = dalloc<uint32_t>((size_t)scenesCap * 8, err);
+    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)scenesCap * 64, cudaHostAllocMapped), "mirror") ||
+        !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
+      return false;
     b.dbg = dalloc<uint32_t>(16, err);
     b.err = dalloc<uint32_t>(4, err);
     b.work = dalloc<uint32_t>(8, err);
@@ -941,6 +972,7 @@ struct World {
   }
 
   bool reset_chain(uint32_t s) {
+    chainFresh = false;
     static const uint32_t CHAIN_INIT[8] = {0x243f6a88u, 0x85a308d3u, 0x13198a2eu, 0x03707344u,
                                            0xa4093822u, 0x299f31d0u, 0x082efa98u, 0xec4e6c89u};
     return cuda_ok(cudaMemcpyAsync(b.chain + s * 8, CHAIN_INIT, 32, cudaMemcpyHostToDevice, st), "chain");
@@ -1392,7 +1424,7 @@ struct World {
         for (auto& s2 : sh)
           if (s2.used && s2.loaded) s2.substeps += 1;
         paramsStale = true;
-        accFresh = chainOn;
+        accFresh = chainFresh = chainOn;
         ++n;
         if (r == 0) continue;
         auto span = [&](int k) {
@@ -1434,6 +1466,8 @@ struct World {
   bool upload_events() {
     std::vector<ImpulseEv> all;
     std::vector<EvPar> ep(maxScenes, EvPar{0, 0, 0, 0});
+    const bool had = anyEvents;
+    const ImpulseEv* const before = devEv;
     anyEvents = false;
     for (uint32_t s = 0; s < maxScenes; ++s) {
       SceneHost& h = sh[s];
@@ -1450,6 +1484,12 @@ struct World {
       }
       ep[s].end = (uint32_t)all.size();
     }
+    // the graph holds the impulse kernel only while some event is ahead
+    if (anyEvents != had) graphValid = false;
+    if (!anyEvents) {
+      eventsDirty = false;
+      return true;
+    }
     if (all.size() > devEvCap) {
       if (devEv) cudaFree(devEv);
       devEvCap = std::max<size_t>(all.size(), 256);
@@ -1463,7 +1503,7 @@ struct World {
     if (!cuda_ok(cudaMemcpyAsync(devEp, ep.data(), ep.size() * sizeof(EvPar), cudaMemcpyHostToDevice, st), "ep"))
       return false;
     eventsDirty = false;
-    graphValid = false;
+    if (devEv != before) graphValid = false;
     return true;
   }
 
@@ -1479,13 +1519,12 @@ struct World {
     const bool fused = fused_fits();
     if (fused != graphFused || (fused && fused_own() > graphOwn)) graphValid = false;
     if (useGraph && !graphValid) {
-      if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
-      if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
+      cudaGraph_t fresh = nullptr;
       if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture")) return false;
       launch_one(fused);
       graphFused = fused;
-      if (!cuda_ok(cudaStreamEndCapture(st, &graph), "endCapture")) return false;
-      if (!cuda_ok(cudaGraphInstantiate(&gexec, graph, 0), "instantiate")) return false;
+      if (!cuda_ok(cudaStreamEndCapture(st, &fresh), "endCapture")) return false;
+      if (!cuda_ok(refresh_graph(fresh, graph, gexec), "instantiate")) return false;
       graphValid = true;
     }
     cudaEventRecord(ev0, st);
@@ -1501,7 +1540,7 @@ struct World {
       if (s.used && s.loaded) s.substeps += count;
     lastLaunches = launchesPerSubstep * count;
     paramsStale = true;
-    accFresh = chainOn;
+    accFresh = chainFresh = chainOn;
     sortedFresh = true;
     // step() (src/engine.js:3990-3997): an armed fusion outlives its gesture
     // only until the formation pass after release, i.e. this call.
@@ -1537,7 +1576,7 @@ struct World {
       for (auto& s2 : sh)
         if (s2.used && s2.loaded) s2.substeps += 1;
       paramsStale = true;
-      accFresh = chainOn;
+      accFresh = chainFresh = chainOn;
       sortedFresh = true;
     }
     for (auto& e : evs) cudaEventDestroy(e);
@@ -1563,14 +1602,26 @@ struct World {
   bool sortedFresh = false;
   bool digest(uint32_t s, uint32_t out[8]) {
     if (accFresh && !layoutDirty) {
-      cudaMemcpyAsync(out, b.accLast + s * 8, 32, cudaMemcpyDeviceToHost, st);
-      return cuda_ok(cudaStreamSynchronize(st), "digest");
+      if (!cuda_ok(cudaStreamSynchronize(st), "digest")) return false;
+      std::memcpy(out, mirror + (size_t)s * 16, 32);
+      return true;
     }
     if (layoutDirty && !relayout()) return false;
     cudaMemsetAsync(accTmp, 0, sizeof(uint32_t) * 8 * maxScenes, st);
     k_hash<<<grid_for(hw.slotEnd), 256, 0, st>>>(b, accTmp);
     cudaMemcpyAsync(out, accTmp + s * 8, 32, cudaMemcpyDeviceToHost, st);
     return cuda_ok(cudaStreamSynchronize(st), "digest");
+  }
+  // mirror: the last fold's digests and chains in host memory, where the fold
+  // wrote them (a read of 32 bytes from the device costs 12 us). chainFresh: no
+  // chain has been written from elsewhere since.
+  uint32_t* mirror = nullptr;
+  bool chainFresh = false;
+  bool read_chain(uint32_t s, uint32_t out[8]) {
+    if (!chainFresh) return read_words(b.chain + (size_t)s * 8, out, 32);
+    if (!cuda_ok(cudaStreamSynchronize(st), "chain")) return false;
+    std::memcpy(out, mirror + (size_t)s * 16 + 8, 32);
+    return true;
   }
   bool read_words(const void* dsrc, void* out, size_t bytes) {
     cudaMemcpyAsync(out, dsrc, bytes, cudaMemcpyDeviceToHost, st);
@@ -2567,9 +2618,12 @@ struct World {
     bool ok = cuda_ok(cudaMemcpyAsync(d, b.state + (size_t)h.slotBase * 8, n * 32, cudaMemcpyDeviceToDevice, st), "ckpt") &&
               cuda_ok(cudaMemcpyAsync(d + n * 32, b.stacc + h.slotBase, n * 8, cudaMemcpyDeviceToDevice, st), "ckpt") &&
               cuda_ok(cudaMemcpyAsync(d + n * 40, b.chain + (size_t)s * 8, 32, cudaMemcpyDeviceToDevice, st), "ckpt");
-    if (ok && hasBonds)
-      ok = cuda_ok(cudaMemcpyAsync(d + n * 40 + 32, b.bond + (size_t)h.slotBase * BOND_CAP,
-                                   (size_t)h.nFluid * BOND_CAP * 4, cudaMemcpyDeviceToDevice, st), "ckpt");
+    if (ok && hasBonds && h.nFluid) {
+      k_rows_save<<<grid_for((uint64_t)h.nFluid * (BOND_CAP / 2)), 256, 0, st>>>(
+          reinterpret_cast<const uint2*>(b.bond + (size_t)h.slotBase * BOND_CAP), (size_t)h.nFluid * (BOND_CAP / 2),
+          b.work + 4, reinterpret_cast<uint2*>(d + n * 40 + 32));
+      ok = cuda_ok(cudaGetLastError(), "ckpt");
+    }
     r->nBodies = scene_bodies(s);
     r->bodyRec.clear();
     r->bodyDrv.clear();
@@ -2600,6 +2654,7 @@ struct World {
   }
   bool ckpt_load(uint32_t s, sn_ckpt_pool* pool, uint64_t handle) {
     accFresh = false;
+    chainFresh = false;
     sortedFresh = false;
     SceneHost& h = sh[s];
     if (!h.loaded) return fail("checkpoint load into a scene that is not loaded");
@@ -2609,7 +2664,8 @@ struct World {
       return fail("checkpoint holds n = %u, n_fluid = %u; the scene has n = %u, n_fluid = %u", r->n, r->nFluid, h.n,
                   h.nFluid);
     if (layoutDirty && !relayout()) return false;
-    if (!pull_params()) return false;
+    // the clocks, all that the device changes in the parameters, are the
+    // checkpoint's: nothing to fetch, and nothing to wait for
     cudaStreamWaitEvent(st, r->done, 0);
     const char* d = pool->base + r->off;
     const size_t n = h.n;
@@ -2618,11 +2674,13 @@ struct World {
               cuda_ok(cudaMemcpyAsync(b.chain + (size_t)s * 8, d + n * 40, 32, cudaMemcpyDeviceToDevice, st), "load");
     uint32_t* bondRows = b.bond + (size_t)h.slotBase * BOND_CAP;
     if (ok && r->hasBonds) {
-      ok = cuda_ok(cudaMemcpyAsync(bondRows, d + n * 40 + 32, (size_t)h.nFluid * BOND_CAP * 4,
-                                   cudaMemcpyDeviceToDevice, st), "load");
-      mark_bonds_live();
-    }
-    else if (ok)
+      if (h.nFluid) {
+        k_rows_load<<<grid_for((uint64_t)h.nFluid * (BOND_CAP / 2)), 256, 0, st>>>(
+            reinterpret_cast<const uint2*>(d + n * 40 + 32), (size_t)h.nFluid * (BOND_CAP / 2), b.work + 4,
+            reinterpret_cast<uint2*>(bondRows));
+        ok = cuda_ok(cudaGetLastError(), "load");
+      }
+    } else if (ok)
       ok = cuda_ok(cudaMemsetAsync(bondRows, 0, (size_t)h.nFluid * BOND_CAP * 4, st), "load");
     if (ok && r->nBodies) {
       const size_t restOff = n * 40 + 32 + (r->hasBonds ? (size_t)h.nFluid * BOND_CAP * 4 : 0);
@@ -2637,7 +2695,7 @@ struct World {
     hpar[s].bondDirty = r->dirty;
     hpar[s].substep = (uint32_t)r->substeps;
     eventsDirty = true;
-    return push_scene(s) && cuda_ok(cudaStreamSynchronize(st), "load");
+    return push_scene(s);
   }
 
   // Slot allocation for a new scene: first fit over released ranges.
@@ -2711,7 +2769,7 @@ int sn_digest(sn_engine* e, uint32_t acc[8]) {
 }
 int sn_chain(sn_engine* e, uint32_t chain[8]) {
   if (!e || !chain) return SN_E_INVALID;
-  return rc_of(e->w, e->w.read_words(e->w.b.chain, chain, 32));
+  return rc_of(e->w, e->w.read_chain(0, chain));
 }
 int sn_reset_chain(sn_engine* e) {
   if (!e) return SN_E_INVALID;
@@ -2910,7 +2968,7 @@ int sn_batch_digest(sn_batch* b, uint32_t id, uint32_t acc[8]) {
 }
 int sn_batch_chain(sn_batch* b, uint32_t id, uint32_t chain[8]) {
   if (!b || !chain || id >= b->w.maxScenes || !b->w.sh[id].loaded) return SN_E_INVALID;
-  return rc_of(b->w, b->w.read_words(b->w.b.chain + id * 8, chain, 32));
+  return rc_of(b->w, b->w.read_chain(id, chain));
 }
 int sn_batch_read_state(sn_batch* b, uint32_t id, int32_t* out, size_t words) {
   if (!b || !out || id >= b->w.maxScenes || !b->w.sh[id].loaded) return SN_E_INVALID;

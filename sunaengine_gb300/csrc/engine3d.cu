@@ -164,6 +164,7 @@ struct Engine3 {
     for (void* p : ptrs)
       if (p) cudaFree(p);
     if (fuErrHost) cudaFreeHost(fuErrHost);
+    if (mirror) cudaFreeHost(mirror);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (evFork) cudaEventDestroy(evFork);
@@ -246,6 +247,9 @@ struct Engine3 {
         cudaHostGetDevicePointer((void**)&fuErrDev, fuErrHost, 0) != cudaSuccess)
       return fail("cudaHostAlloc failed");
     *fuErrHost = 0u;
+    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)maxScenes * 64, cudaHostAllocMapped), "mirror") ||
+        !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
+      return false;
     if (!err.empty()) return false;
     {
       std::vector<int2> wg(LUT_N), pg(PLANE_N);
@@ -527,13 +531,12 @@ struct Engine3 {
     const bool fused = fused_fits();
     if (fused != graphFused) graphValid = false;
     if (useGraph && !graphValid) {
-      if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
-      if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
+      cudaGraph_t fresh = nullptr;
       if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture")) return false;
       launch_one(fused);
       graphFused = fused;
-      if (!cuda_ok(cudaStreamEndCapture(st, &graph), "endCapture")) return false;
-      if (!cuda_ok(cudaGraphInstantiate(&gexec, graph, 0), "instantiate")) return false;
+      if (!cuda_ok(cudaStreamEndCapture(st, &fresh), "endCapture")) return false;
+      if (!cuda_ok(sn::refresh_graph(fresh, graph, gexec), "instantiate")) return false;
       graphValid = true;
     }
     cudaEventRecord(ev0, st);
@@ -548,7 +551,7 @@ struct Engine3 {
     for (auto& s : sh)
       if (s.used && s.loaded) s.substeps += count;
     lastLaunches = launchesPerSubstep * count;
-    accFresh = chainOn;
+    accFresh = chainFresh = chainOn;
     return cuda_ok(cudaGetLastError(), "step");
   }
 
@@ -577,7 +580,7 @@ struct Engine3 {
       }
       for (auto& s2 : sh)
         if (s2.used && s2.loaded) s2.substeps += 1;
-      accFresh = chainOn;
+      accFresh = chainFresh = chainOn;
     }
     for (auto& e : evs) cudaEventDestroy(e);
     uint32_t n = (uint32_t)std::max(0, used - 1);
@@ -619,6 +622,7 @@ struct Engine3 {
 
   bool load(uint32_t s, const sn3_scene* sc) {
     accFresh = false;
+    chainFresh = false;
     if (!check_scene(s, false)) return false;
     if (!sc) return fail("scene is NULL");
     Scene3Host& h = sh[s];
@@ -814,11 +818,17 @@ struct Engine3 {
   // accFresh: the fold's last digest is the digest of the current state (set
   // by stepping with the chain on, cleared by any change made outside a substep).
   bool accFresh = false;
+  // mirror: the last fold's digests and chains in host memory, where the fold
+  // wrote them (a read of 32 bytes from the device costs 12 us). chainFresh: no
+  // chain has been written from elsewhere since.
+  uint32_t* mirror = nullptr;
+  bool chainFresh = false;
   bool digest(uint32_t s, uint32_t out[8]) {
     if (!check_scene(s)) return false;
     if (accFresh && !layoutDirty) {
-      cudaMemcpyAsync(out, b.accLast + (size_t)s * 8, 32, cudaMemcpyDeviceToHost, st);
-      return synced("digest");
+      if (!synced("digest")) return false;
+      memcpy(out, mirror + (size_t)s * 16, 32);
+      return true;
     }
     if (layoutDirty && !relayout()) return false;
     cudaMemsetAsync(accTmp, 0, sizeof(uint32_t) * 8 * maxScenes, st);
@@ -846,6 +856,11 @@ struct Engine3 {
 
   bool chain(uint32_t s, uint32_t out[8]) {
     if (!check_scene(s)) return false;
+    if (chainFresh) {
+      if (!synced("chain")) return false;
+      memcpy(out, mirror + (size_t)s * 16 + 8, 32);
+      return true;
+    }
     cudaMemcpyAsync(out, b.chain + (size_t)s * 8, 32, cudaMemcpyDeviceToHost, st);
     return synced("chain");
   }
@@ -863,6 +878,7 @@ struct Engine3 {
   // substep count (for the stir phase) and the chain.
   bool write_state(uint32_t s, const int32_t* state, uint32_t n, uint64_t substeps, const uint32_t* chainIn) {
     accFresh = false;
+    chainFresh = false;
     if (!check_scene(s)) return false;
     Scene3Host& h = sh[s];
     if (n > h.cap) return fail("state has %u particles, above capacity %u", n, h.cap);
@@ -903,6 +919,7 @@ struct Engine3 {
   }
   bool ckpt_load(uint32_t s, sn_ckpt_pool* pool, uint64_t handle) {
     accFresh = false;
+    chainFresh = false;
     if (!check_scene(s)) return false;
     sn_ckpt_pool::Rec* r = pool->find(handle);
     if (!r || r->kind != 3) return fail("no 3D checkpoint %llu in the pool", (unsigned long long)handle);
@@ -925,7 +942,7 @@ struct Engine3 {
     if (!layoutDirty &&
         !cuda_ok(cudaMemcpyAsync(b.scenes + s, &hpar[s], sizeof(Scene3), cudaMemcpyHostToDevice, st), "load"))
       return false;
-    return cuda_ok(cudaStreamSynchronize(st), "load");
+    return true;
   }
 
   bool timing(float* ms) {

@@ -1,9 +1,26 @@
-// What the fused substeps (fused2d.cuh, fused3d.cuh) share: the grid barrier of a
-// cooperative launch and a CTA's prefix sum.
+// What the 2D and 3D engines share around a substep's launch: the graph's refresh,
+// the grid barrier of a cooperative launch and a CTA's prefix sum.
 #pragma once
+#include <cuda_runtime.h>
 #include <cstdint>
 
 namespace sn {
+
+// The captured substep graph after a change: an update of the executable graph where
+// the topology allows it (a new scene size does), a new one where it does not.
+inline cudaError_t refresh_graph(cudaGraph_t fresh, cudaGraph_t& graph, cudaGraphExec_t& exec) {
+  if (exec) {
+    cudaGraphExecUpdateResultInfo info;
+    if (cudaGraphExecUpdate(exec, fresh, &info) != cudaSuccess) {
+      cudaGetLastError();  // refused: not an error of the stream
+      cudaGraphExecDestroy(exec);
+      exec = nullptr;
+    }
+  }
+  if (graph) cudaGraphDestroy(graph);
+  graph = fresh;
+  return exec ? cudaSuccess : cudaGraphInstantiate(&exec, graph, 0);
+}
 
 constexpr int FU_T = 1024;  // threads of a fused substep's CTA, one CTA to an SM
 constexpr uint32_t ERR_BARRIER = 8u;

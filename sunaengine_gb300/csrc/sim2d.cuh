@@ -182,6 +182,7 @@ struct Bufs {
   WorldPar* world;
   uint32_t* acc;        // [S * 8]
   uint32_t* accLast;    // [S * 8]
+  uint32_t* mirror;     // [S * 16] {digest, chain} of the last substep, in host memory
   uint32_t* chain;      // [S * 8]
   uint32_t* dbg;        // [16]
   uint32_t* err;        // [4]
@@ -2297,6 +2298,8 @@ __device__ __forceinline__ void fold_scene(const Bufs& b, uint32_t s, bool doCha
       b.chain[s * 8 + j] = next[j];
       b.accLast[s * 8 + j] = a[j];
       b.acc[s * 8 + j] = 0;
+      b.mirror[s * 16 + j] = a[j];
+      b.mirror[s * 16 + 8 + j] = next[j];
     }
   }
   if (S.formNow) S.bondDirty = 0;

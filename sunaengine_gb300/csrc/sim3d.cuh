@@ -127,6 +127,7 @@ struct Bufs3 {
   Scene3* scenes;
   World3* world;
   uint32_t *acc, *accLast, *chain, *dbg;
+  uint32_t* mirror;   // [S * 16] {digest, chain} of the last substep, in host memory
 };
 
 __device__ __forceinline__ uint32_t gstride3() { return gridDim.x * blockDim.x; }
@@ -753,6 +754,8 @@ __device__ __forceinline__ void fold_scene3(const Bufs3& b, uint32_t s, bool doC
     b.chain[s * 8 + j] = nx[j];
     b.accLast[s * 8 + j] = a[j];
     b.acc[s * 8 + j] = 0u;
+    b.mirror[s * 16 + j] = a[j];
+    b.mirror[s * 16 + 8 + j] = nx[j];
   }
 }
 __global__ void k3_fold(Bufs3 b, int doChain) {
