@@ -1138,15 +1138,16 @@ struct World {
   // slot a thread, the cell ranges, the owned particles' lists).
   bool fused_fits() const {
     const uint64_t G = (uint64_t)numSMs;
-    return !debug && inRange && !staged && !persistent && autoLanes && bodies.empty() && hw.nAct > 0 &&
+    return !debug && inRange && !staged && !persistent && autoLanes && hw.nAct > 0 &&
            slots_used() <= G * FU_T && fused_own() <= fused_own_cap();
   }
-  template <int L, int LC>
+  template <int L, int LC, bool RIG>
   void launch_fused_as() {
     FusedPar P;
     P.iters = iters;
     P.friction = hasFriction ? 1u : 0u;
-    P.bonds = hasBonds ? 1u : 0u;
+    P.bodies = (uint32_t)bodies.size();
+    P.bonds = hasBonds || P.bodies ? 1u : 0u;
     P.seal = hasSeal ? 1u : 0u;
     P.chain = chainOn ? 1u : 0u;
     // constant under spawns (a slot without a particle is skipped), so a
@@ -1162,7 +1163,7 @@ struct World {
     P.bar = fuBar;
     Bufs bb = b;
     if (iters & 1u) swap_records(bb);  // so that the last iteration ends in PL
-    const auto fn = k_substep_fused<L, LC>;
+    const auto fn = k_substep_fused<L, LC, RIG>;
     cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FU_SMEM);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)numSMs);
@@ -1176,6 +1177,14 @@ struct World {
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, fn, bb, P);
   }
+  template <bool RIG>
+  void launch_fused_for(uint32_t own) {
+    if (own <= 64) launch_fused_as<16, 16, RIG>();
+    else if (own <= 128) launch_fused_as<8, 16, RIG>();
+    else if (own <= 256) launch_fused_as<4, 16, RIG>();
+    else if (own <= 512) launch_fused_as<2, 8, RIG>();
+    else launch_fused_as<2, 4, RIG>();
+  }
   void launch_fused() {
     uint64_t Lc = 1;
     if (anyEvents) {
@@ -1184,11 +1193,8 @@ struct World {
     }
     // as many lanes a particle as leave one round of a CTA's threads
     const uint32_t own = fused_own();
-    if (own <= 64) launch_fused_as<16, 16>();
-    else if (own <= 128) launch_fused_as<8, 16>();
-    else if (own <= 256) launch_fused_as<4, 16>();
-    else if (own <= 512) launch_fused_as<2, 8>();
-    else launch_fused_as<2, 4>();
+    if (bodies.empty()) launch_fused_for<false>(own);
+    else launch_fused_for<true>(own);
     launchesPerSubstep = Lc;
   }
 

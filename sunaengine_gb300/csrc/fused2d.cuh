@@ -41,6 +41,7 @@ struct FusedPar {
   uint32_t slots;    // slots that can be active: [0, slots)
   uint32_t xWords;   // shared words for the cell ranges, then the CA table
   uint32_t ownCap;   // particles a CTA can own
+  uint32_t bodies;   // rigid bodies, one CTA each in turn
   uint32_t* count;   // [K] cell counts, zero between launches
   uint32_t* tmp;     // slots by cell in arrival order
   uint32_t* bar;     // [2] barrier arrivals and finished CTAs, zero between launches
@@ -88,9 +89,11 @@ __device__ __forceinline__ void solveA_owned(const Bufs& b, const NbrOwned& nb, 
   sgx = gsum<L>(sgx);
   sgy = gsum<L>(sgy);
 }
-template <int L>
+// RIG: infoI is a rigid member's info, whose correction skips its own body, or 0.
+template <int L, bool RIG>
 __device__ __forceinline__ int2 solveB_owned(const Bufs& b, const NbrOwned& nb, uint32_t row, uint32_t cnt,
-                                             uint32_t sub, int2 pi, int32_t li, const Flags<false>& f) {
+                                             uint32_t sub, int2 pi, int32_t li, uint32_t infoI,
+                                             const Flags<false>& f) {
   int32_t dpx = 0, dpy = 0;
   for (uint32_t k = sub; k < cnt; k += L * FU_B) {
     int4 o[FU_B];
@@ -98,14 +101,20 @@ __device__ __forceinline__ int2 solveB_owned(const Bufs& b, const NbrOwned& nb, 
     for (int j = 0; j < FU_B; ++j) o[j] = nb.rec(k + j * L < cnt ? nb.entry(row, k + j * L) : 0u);
 #pragma unroll
     for (int j = 0; j < FU_B; ++j)
-      if (k + j * L < cnt) solveB_pair<false>(b, nb, pi, li, o[j], f, dpx, dpy);
+      if (k + j * L < cnt && !(RIG && !is_wall(o[j].w) && same_body(infoI, (uint32_t)o[j].w)))
+        solveB_pair<false>(b, nb, pi, li, o[j], f, dpx, dpy);
   }
   return make_int2(gsum<L>(dpx), gsum<L>(dpy));
 }
 
 // L lanes share a particle's list in the sweeps over every owned particle, LC
-// in the colour passes (a quarter of the particles each).
-template <int L, int LC>
+// in the colour passes (a quarter of the particles each). RIG: the world has
+// rigid bodies. A body's passes run on one CTA (the bodies dealt round), between
+// barriers of their own: rigidStep before the keys, rigidSolve beside the
+// friction correction, which touches other particles, rigidMember after the
+// owners, who have the lists, have marked the members that leave. Twins of this
+// kernel without RIG keep the bodies out of worlds that have none.
+template <int L, int LC, bool RIG>
 __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   extern __shared__ int4 dyn[];
   int4* rec = dyn;                                              // [ownCap] records
@@ -119,6 +128,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   __shared__ int4 smat1[MAT_MAX], smat2[MAT_MAX];
   __shared__ int2 scol[MAT_MAX];  // {eps, dpMax}
   __shared__ uint32_t dsacc[8], dsscene, lastCta;
+  __shared__ int32_t rsum[RIG ? FU_T / 32 : 1][RG_SUMS];
   const Flags<false> f{b.dbg};
   const uint32_t tid = threadIdx.x, lane = tid & 31u, G = gridDim.x, cta = blockIdx.x;
   const uint32_t K = b.world->K;
@@ -146,10 +156,21 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       temp = c.z;
       info = info_of((uint32_t)c.x, (uint32_t)c.y, i >= S.nFluid);
       pred = predict_pos(b, S, slot, i, a, c, f);
-      const int2 cc = cell_coord(S, pred);
-      key = key_of(S, cc.x, cc.y);
-      arrival = atomicAdd(P.count + key, 1u);
     }
+  }
+  if constexpr (RIG) {
+    const bool member = on && (info & INFO_RIGID);
+    if (member) b.predSlot[slot] = pred;
+    if (!grid_wait(P.bar, b.err, target)) return;
+    for (uint32_t k = cta; k < P.bodies; k += G) rigid_step_body<false, FU_T, false>(b, k, rsum, f);
+    if (!grid_wait(P.bar, b.err, target)) return;
+    if (member) pred = b.predSlot[slot];
+  }
+  if (on) {
+    const ScenePar& S = b.scenes[sc];
+    const int2 cc = cell_coord(S, pred);
+    key = key_of(S, cc.x, cc.y);
+    arrival = atomicAdd(P.count + key, 1u);
   }
   for (uint32_t k = tid; k < (uint32_t)TN; k += FU_T) swg[k] = __ldg(b.WG + k);
   post1_mats(b, smat1);
@@ -286,8 +307,10 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
         const uint32_t inf = (uint32_t)me.w;
         const bool act = valid && !(inf & INFO_BOUNDARY);
         const uint32_t cnt = act ? (word[r] & NBRN_COUNT) : 0u;
-        const int2 dp = solveB_owned<LC>(b, nb, r, cnt, subC, xy(me), me.z, f);
+        const int2 dp =
+            solveB_owned<LC, RIG>(b, nb, r, cnt, subC, xy(me), me.z, (inf & INFO_RIGID) ? inf : 0u, f);
         if (!act || subC != 0) continue;
+        if (RIG && (inf & INFO_RIGID)) b.DP[pOf[r]] = dp;
         if (!(inf & INFO_PINNED)) {
           const int2 pr = apply_dp_in(scol[inf & INFO_MAT].y, wall[r], xy(me), dp, f);
           me.x = pr.x;
@@ -319,7 +342,20 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
         rec[i] = me;
         b.PL[p] = me;
       }
+    }
+    if constexpr (RIG)
+      for (uint32_t k = cta; k < P.bodies; k += G) rigid_solve_body<false, FU_T>(b, k, P.seal != 0u, rsum, f);
+    if (RIG || fric) {
       if (!grid_wait(P.bar, b.err, target)) return;
+    }
+    if constexpr (RIG) {
+      for (uint32_t i = tid; i < own[4]; i += FU_T) {
+        if (!((uint32_t)rec[i].w & INFO_RIGID)) continue;
+        const int2 pr = ld_pred(b.PL, pOf[i]);
+        rec[i].x = pr.x;
+        rec[i].y = pr.y;
+      }
+      __syncthreads();
     }
   }
 
@@ -348,8 +384,12 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       post2_finish(b, S, p, sl, sl - S.slotBase, a2, !P.bonds, b.state + (size_t)sl * 8, f);
     }
   }
-  if (P.seal && *(volatile uint32_t*)(b.work + 6) != 0u) {
+  const bool stress = P.seal && *(volatile uint32_t*)(b.work + 6) != 0u;
+  const bool forming = P.bonds && *(volatile uint32_t*)(b.work + 5) != 0u;
+  if (RIG || stress) {
     if (!grid_wait(P.bar, b.err, target)) return;
+  }
+  if (stress) {
     for (uint32_t i = tid / L;; i += FU_T / L) {
       if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
       const bool valid = i < own[4];
@@ -357,7 +397,19 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       contain_stress_slot<false, L>(b, nb, valid, b.sslot[pOf[r]], r, sub, f);
     }
   }
-  if (P.bonds && *(volatile uint32_t*)(b.work + 5) != 0u) {
+  if constexpr (RIG) {
+    for (uint32_t i = tid; i < own[4]; i += FU_T) {
+      const uint32_t inf = (uint32_t)rec[i].w;
+      if (!(inf & INFO_RIGID) || is_wall(rec[i].w)) continue;
+      const uint32_t p = pOf[i], sl = b.sslot[p];
+      const int32_t tag = (int32_t)((uint32_t)b.state[(size_t)sl * 8 + 5] & WELD_TAG_MASK);
+      b.rmark[sl] = rigid_leaves(b, nb, sl, p, i, tag, f) ? 1u : 0u;
+    }
+    if (!grid_wait(P.bar, b.err, target)) return;
+    for (uint32_t k = cta; k < P.bodies; k += G) rigid_member_body<false, FU_T, true>(b, k, rsum, f);
+    if (!forming && !grid_wait(P.bar, b.err, target)) return;
+  }
+  if (forming) {
     if (!grid_wait(P.bar, b.err, target)) return;
     for (uint32_t i = tid / L;; i += FU_T / L) {
       if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;

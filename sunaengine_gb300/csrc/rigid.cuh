@@ -43,6 +43,7 @@ constexpr int32_t RIGID_MIN_MEMBERS = 4;
 constexpr int32_t RG_IQ_MIN = 16, RG_IQ_MAX = 31;
 constexpr int32_t SEAL_R4 = 1126;  // 0.55 wu
 constexpr int RG_THREADS = 256;
+constexpr int RG_SUMS = 7;  // a body's sums at most, per warp of its CTA
 
 // fp_shr_rne with a per-body shift; WGSL shift amounts wrap modulo 32, so
 // s = 0 leaves x unchanged.
@@ -138,8 +139,8 @@ __device__ __forceinline__ bool rg_member(const Bufs& b, uint32_t slot, int32_t 
 }
 
 // Sum K wrapping i32 values over the CTA; every thread gets the totals.
-template <int K>
-__device__ __forceinline__ void rg_block_sum(int32_t (&v)[K], int32_t (*sh)[K]) {
+template <int NT, int K>
+__device__ __forceinline__ void rg_block_sum(int32_t (&v)[K], int32_t (*sh)[RG_SUMS]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < K; ++k)
@@ -151,7 +152,7 @@ __device__ __forceinline__ void rg_block_sum(int32_t (&v)[K], int32_t (*sh)[K]) 
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     int32_t t = 0;
-    for (int w = 0; w < RG_THREADS / 32; ++w) t = wadd(t, sh[w][k]);
+    for (int w = 0; w < NT / 32; ++w) t = wadd(t, sh[w][k]);
     v[k] = t;
   }
   __syncthreads();
@@ -165,13 +166,17 @@ __device__ __forceinline__ int2 rg_at(int32_t cx, int32_t cy, int32_t c, int32_t
 }
 
 // rigidStep (src/sim.wgsl:3226-3440). Runs after k_predict_key, which gave
-// every member pred = pos; the placement overwrites predSlot and the grid key.
-template <bool DBG>
-__global__ void __launch_bounds__(RG_THREADS) k_rigid_step(Bufs b) {
-  Flags<DBG> f{b.dbg};
-  __shared__ int32_t sh[RG_THREADS / 32][4];
-  int32_t* R = b.rbody + (size_t)blockIdx.x * RG_BODY_WORDS;
-  const int32_t* D = b.rdrv + (size_t)blockIdx.x * RG_DRIVER_WORDS;
+// every member pred = pos; the placement overwrites predSlot and the grid key
+// (KEYS; the fused substep takes its keys from predSlot).
+//
+// The three passes are device functions of one CTA of NT threads and a body; a
+// CTA may call them for several bodies in turn (each ends past its last use of
+// `sh`).
+template <bool DBG, int NT, bool KEYS>
+__device__ __forceinline__ void rigid_step_body(const Bufs& b, uint32_t body, int32_t (*sh)[RG_SUMS],
+                                                const Flags<DBG>& f) {
+  int32_t* R = b.rbody + (size_t)body * RG_BODY_WORDS;
+  const int32_t* D = b.rdrv + (size_t)body * RG_DRIVER_WORDS;
   const ScenePar& S = b.scenes[R[RB_SCENE]];
   const int32_t tag = R[RB_TAG], n = R[RB_N], axis = R[RB_AXIS], dmask = D[RD_MASK];
   if (!(R[RB_LIVE] != 0 && n >= RIGID_MIN_MEMBERS) || !S.active) return;
@@ -180,7 +185,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_step(Bufs b) {
   if (dmask & RD_HAS_PX) cx = D[RD_PX];
   if (dmask & RD_HAS_PY) cy = D[RD_PY];
   int32_t v[4] = {0, 0, 0, 0};  // fx, fy, thi, tlo
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
+  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
     const int32_t* w = b.state + (size_t)slot * 8;
@@ -201,7 +206,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_step(Bufs b) {
     v[2] = wadd(v[2], hi);
     v[3] = wadd(v[3], wsub(t, (int32_t)((uint32_t)hi << TQ_HI_SH)));
   }
-  rg_block_sum<4>(v, sh);
+  rg_block_sum<NT>(v, sh);
   if (threadIdx.x == 0) {
     const int32_t invI = R[RB_INVI], iq = R[RB_IQ], gS = R[RB_GSUM];
     const bool holdX = axis != 0 || (dmask & RD_HAS_PX), holdY = axis != 0 || (dmask & RD_HAS_PY);
@@ -252,21 +257,29 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_step(Bufs b) {
   __syncthreads();
   const int32_t qx = R[RB_CQX], qy = R[RB_CQY], th = R[RB_THETAQ];
   const int32_t c = rg_cos(b.cosT, th, f), s = rg_sin(b.cosT, th, f);
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
+  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
     const int2 pr = rg_at(qx, qy, c, s, b.rest[slot], f);
     b.predSlot[slot] = pr;
-    const int2 cc = cell_coord(S, pr);
-    b.keys[slot] = key_of(S, cc.x, cc.y);
+    if constexpr (KEYS) {
+      const int2 cc = cell_coord(S, pr);
+      b.keys[slot] = key_of(S, cc.x, cc.y);
+    }
   }
+}
+template <bool DBG>
+__global__ void __launch_bounds__(RG_THREADS) k_rigid_step(Bufs b) {
+  __shared__ int32_t sh[RG_THREADS / 32][RG_SUMS];
+  rigid_step_body<DBG, RG_THREADS, true>(b, blockIdx.x, sh, Flags<DBG>{b.dbg});
 }
 
 // rigid_seal_delta (src/sim.wgsl:2001-2051): the member's swept segment
 // against held seal particles in the cells its expanded AABB touches. Every
 // hit returns the same reversion (pos - pred), so the scan is an existence
-// test and its order does not matter: lane `sub` of a group of L lanes tests
-// every L-th candidate of each cell, and the group ORs the answers.
+// test and its order does not matter: a group of L lanes takes the cells, two
+// lanes to a cell from L = 4 up (a cell's range and its records are dependent
+// loads, other cells' are not), and ORs the answers.
 template <bool DBG>
 __device__ bool rigid_seal_hit(const Bufs& b, const ScenePar& S, uint32_t p, int2 pos, int2 pr, int32_t tag,
                                uint32_t sub, uint32_t L, const Flags<DBG>& f) {
@@ -274,47 +287,47 @@ __device__ bool rigid_seal_hit(const Bufs& b, const ScenePar& S, uint32_t p, int
   const int32_t ml2 = wadd(wmul(mx4, mx4), wmul(my4, my4));
   const int2 lo = cell_coord(S, make_int2(sub_sat(min(pos.x, pr.x), SEAL_REACH, f), sub_sat(min(pos.y, pr.y), SEAL_REACH, f)));
   const int2 hi = cell_coord(S, make_int2(add_sat(max(pos.x, pr.x), SEAL_REACH, f), add_sat(max(pos.y, pr.y), SEAL_REACH, f)));
-  for (int32_t gy = lo.y; gy <= hi.y; ++gy)
-    for (int32_t gx = lo.x; gx <= hi.x; ++gx) {
-      const uint32_t key = key_of(S, gx, gy);
-      for (uint32_t t = b.cellStart[key] + sub; t < b.cellStart[key + 1]; t += L) {
-        if (t == p) continue;
-        const int4 o = b.PL[t];
-        const uint32_t info = (uint32_t)o.w;
-        // a held seal particle wears FLAG_SEAL and FLAG_ANCHOR, so its sorted
-        // record carries INFO_SEAL and INFO_PINNED; only those read their flags
-        if ((info & INFO_BOUNDARY) || !(info & INFO_SEAL) || !(info & INFO_PINNED)) continue;
-        const uint32_t fj = (uint32_t)b.state[(size_t)b.sslot[t] * 8 + 5];
-        if ((fj & (FLAG_ANCHOR | FLAG_SEAL)) != (FLAG_ANCHOR | FLAG_SEAL) || !seal_class(b, info & INFO_MAT)) continue;
-        if ((fj & FLAG_RIGID) && (int32_t)(fj & WELD_TAG_MASK) == tag) continue;
-        const int32_t px4 = shr_rne<BPRE>(sub_sat(o.x, pos.x, f)), py4 = shr_rne<BPRE>(sub_sat(o.y, pos.y, f));
-        int32_t dx4 = px4, dy4 = py4;
-        if (ml2 > 0) {
-          const int32_t dot = wadd(wmul(px4, mx4), wmul(py4, my4));
-          if (dot >= ml2) {
-            dx4 = wsub(px4, mx4);
-            dy4 = wsub(py4, my4);
-          } else if (dot > 0) {
-            const int32_t tq = div_s(dot, ml2, 16u, f);
-            dx4 = wsub(px4, mul<16>(mx4, tq, f));
-            dy4 = wsub(py4, mul<16>(my4, tq, f));
-          }
+  const uint32_t two = L >= 4u ? 1u : 0u;
+  const uint32_t wide = (uint32_t)(hi.x - lo.x + 1), cells = wide * (uint32_t)(hi.y - lo.y + 1);
+  for (uint32_t c = sub >> two; c < cells; c += L >> two) {
+    const uint32_t key = key_of(S, lo.x + (int32_t)(c % wide), lo.y + (int32_t)(c / wide));
+    for (uint32_t t = b.cellStart[key] + (sub & two); t < b.cellStart[key + 1]; t += 1u + two) {
+      if (t == p) continue;
+      const int4 o = b.PL[t];
+      const uint32_t info = (uint32_t)o.w;
+      // a held seal particle wears FLAG_SEAL and FLAG_ANCHOR, so its sorted
+      // record carries INFO_SEAL and INFO_PINNED; only those read their flags
+      if ((info & INFO_BOUNDARY) || !(info & INFO_SEAL) || !(info & INFO_PINNED)) continue;
+      const uint32_t fj = (uint32_t)b.state[(size_t)b.sslot[t] * 8 + 5];
+      if ((fj & (FLAG_ANCHOR | FLAG_SEAL)) != (FLAG_ANCHOR | FLAG_SEAL) || !seal_class(b, info & INFO_MAT)) continue;
+      if ((fj & FLAG_RIGID) && (int32_t)(fj & WELD_TAG_MASK) == tag) continue;
+      const int32_t px4 = shr_rne<BPRE>(sub_sat(o.x, pos.x, f)), py4 = shr_rne<BPRE>(sub_sat(o.y, pos.y, f));
+      int32_t dx4 = px4, dy4 = py4;
+      if (ml2 > 0) {
+        const int32_t dot = wadd(wmul(px4, mx4), wmul(py4, my4));
+        if (dot >= ml2) {
+          dx4 = wsub(px4, mx4);
+          dy4 = wsub(py4, my4);
+        } else if (dot > 0) {
+          const int32_t tq = div_s(dot, ml2, 16u, f);
+          dx4 = wsub(px4, mul<16>(mx4, tq, f));
+          dy4 = wsub(py4, mul<16>(my4, tq, f));
         }
-        if (wadd(wmul(dx4, dx4), wmul(dy4, dy4)) < SEAL_R4 * SEAL_R4)
-          return true;
       }
+      if (wadd(wmul(dx4, dx4), wmul(dy4, dy4)) < SEAL_R4 * SEAL_R4)
+        return true;
     }
+  }
   return false;
 }
 
 // rigidSolve (src/sim.wgsl:3459-3573), after each iteration's friction pass.
 // `seal`: the world has seal-class rows (else no contact can exist).
-template <bool DBG>
-__global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal) {
-  Flags<DBG> f{b.dbg};
-  __shared__ int32_t sh[RG_THREADS / 32][7];
-  int32_t* R = b.rbody + (size_t)blockIdx.x * RG_BODY_WORDS;
-  const int32_t* D = b.rdrv + (size_t)blockIdx.x * RG_DRIVER_WORDS;
+template <bool DBG, int NT>
+__device__ __forceinline__ void rigid_solve_body(const Bufs& b, uint32_t body, bool seal, int32_t (*sh)[RG_SUMS],
+                                                 const Flags<DBG>& f) {
+  int32_t* R = b.rbody + (size_t)body * RG_BODY_WORDS;
+  const int32_t* D = b.rdrv + (size_t)body * RG_DRIVER_WORDS;
   const ScenePar& S = b.scenes[R[RB_SCENE]];
   const int32_t tag = R[RB_TAG], n = R[RB_N], axis = R[RB_AXIS], dmask = D[RD_MASK];
   if (!(R[RB_LIVE] != 0 && n >= RIGID_MIN_MEMBERS) || !S.active) return;
@@ -327,10 +340,10 @@ __global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal)
   const uint32_t span = last >= first ? last - first + 1u : 0u;
   uint32_t L = 1;
   if (!DBG && seal)
-    while (L < 8u && span * (L * 2u) <= (uint32_t)RG_THREADS) L *= 2u;
+    while (L < 8u && span * (L * 2u) <= (uint32_t)NT) L *= 2u;
   const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x & (L - 1u);
   const uint32_t gmask = ((1u << L) - 1u) << (lane & ~(L - 1u));
-  for (uint32_t base = first; base <= last && base < S.nFluid; base += RG_THREADS / L) {
+  for (uint32_t base = first; base <= last && base < S.nFluid; base += NT / L) {
     const uint32_t i = base + threadIdx.x / L;
     const uint32_t slot = S.slotBase + i;
     const bool mem = i <= last && i < S.nFluid && rg_member(b, slot, tag);
@@ -361,7 +374,7 @@ __global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal)
     v[2] = wadd(v[2], hi);
     v[3] = wadd(v[3], wsub(t, (int32_t)((uint32_t)hi << TQ_HI_SH)));
   }
-  rg_block_sum<7>(v, sh);
+  rg_block_sum<NT>(v, sh);
   if (threadIdx.x == 0) {
     const int32_t invI = R[RB_INVI], iq = R[RB_IQ];
     if (axis == 0) {
@@ -385,7 +398,7 @@ __global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal)
   __syncthreads();
   const int32_t qx = R[RB_CQX], qy = R[RB_CQY], th = R[RB_THETAQ];
   const int32_t c = rg_cos(b.cosT, th, f), s = rg_sin(b.cosT, th, f);
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
+  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
     const uint32_t p = b.inv[slot];
@@ -393,22 +406,49 @@ __global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal)
     *reinterpret_cast<int2*>(b.PL + p) = pr;
   }
 }
+template <bool DBG>
+__global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal) {
+  __shared__ int32_t sh[RG_THREADS / 32][RG_SUMS];
+  rigid_solve_body<DBG, RG_THREADS>(b, blockIdx.x, seal != 0, sh, Flags<DBG>{b.dbg});
+}
 
 // rigidMember (src/sim.wgsl:3610-3747), after thermal and containStress.
 // Leave decisions read the membership the pass began with (marks first, then
 // the clears, across a CTA barrier); the reference's single loop clears
 // FLAG_RIGID while other lanes of its workgroup read it.
-template <bool DBG>
-__global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
-  Flags<DBG> f{b.dbg};
-  __shared__ int32_t sh[RG_THREADS / 32][5];
-  int32_t* R = b.rbody + (size_t)blockIdx.x * RG_BODY_WORDS;
+//
+// Whether the member in `slot` leaves; row: its list in nb.
+template <bool DBG, class NB>
+__device__ __forceinline__ bool rigid_leaves(const Bufs& b, const NB& nb, uint32_t slot, uint32_t p, uint32_t row,
+                                             int32_t tag, const Flags<DBG>& f) {
+  const int32_t* w = b.state + (size_t)slot * 8;
+  const uint32_t m = (uint32_t)w[4];
+  if (matw(b, m, M_solidMode) != SOLID_RIGID || matw(b, m, M_phantom) != 0) return true;
+  const uint32_t cnt = b.NBRN[p] & NBRN_COUNT;
+  for (uint32_t k = 0; k < cnt; ++k) {
+    const uint32_t e = nb.entry(row, k);
+    if (is_wall(b.PL[e].w)) continue;
+    const uint32_t js = b.sslot[e];
+    if (!rg_member(b, js, tag)) continue;
+    const int32_t* wj = b.state + (size_t)js * 8;
+    const int32_t dx = shr_rne<BPRE>(sub_sat(w[0], wj[0], f)), dy = shr_rne<BPRE>(sub_sat(w[1], wj[1], f));
+    if (abs(dx) > L0_MAX || abs(dy) > L0_MAX) continue;
+    if (wadd(wmul(dx, dx), wmul(dy, dy)) <= BOND_R2) return false;
+  }
+  return true;
+}
+
+// MARKED: rmark already holds every member's decision (the fused substep, where
+// the lists are with the particles' owners).
+template <bool DBG, int NT, bool MARKED>
+__device__ __forceinline__ void rigid_member_body(const Bufs& b, uint32_t body, int32_t (*sh)[RG_SUMS],
+                                                  const Flags<DBG>& f) {
+  int32_t* R = b.rbody + (size_t)body * RG_BODY_WORDS;
   const ScenePar& S = b.scenes[R[RB_SCENE]];
   if (R[RB_LIVE] == 0 || !S.active) return;
   const int32_t tag = R[RB_TAG], axis = R[RB_AXIS];
   const uint32_t first = (uint32_t)R[RB_FIRST], last = (uint32_t)R[RB_LAST];
   const uint32_t ish = (uint32_t)R[RB_ISH], osh = (uint32_t)R[RB_OSH];
-  const uint32_t stride = b.nbrStride;
   if (threadIdx.x == 0) {  // 1. close the substep
     const int32_t vmaxN = neg_sat(S.vmax, f);
     R[RB_VX] = clampi(sub_sat(R[RB_CQX], R[RB_CX], f), vmaxN, S.vmax);
@@ -420,31 +460,17 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
   }
   // 2. leave: a member whose row is no longer rigid (or retired), or with no
   // same-body neighbour within bond range
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
-    const uint32_t slot = S.slotBase + i;
-    if (!rg_member(b, slot, tag)) continue;
-    const int32_t* w = b.state + (size_t)slot * 8;
-    const uint32_t m = (uint32_t)w[4];
-    bool leave = matw(b, m, M_solidMode) != SOLID_RIGID || matw(b, m, M_phantom) != 0;
-    if (!leave) {
-      bool touched = false;
-      const uint32_t p = b.inv[slot], cnt = b.NBRN[p] & NBRN_COUNT;
-      for (uint32_t k = 0; k < cnt && !touched; ++k) {
-        const uint32_t e = b.NBR[nbr_at(stride, p, k)];
-        if (is_wall(b.PL[e].w)) continue;
-        const uint32_t js = b.sslot[e];
-        if (!rg_member(b, js, tag)) continue;
-        const int32_t* wj = b.state + (size_t)js * 8;
-        const int32_t dx = shr_rne<BPRE>(sub_sat(w[0], wj[0], f)), dy = shr_rne<BPRE>(sub_sat(w[1], wj[1], f));
-        if (abs(dx) > L0_MAX || abs(dy) > L0_MAX) continue;
-        if (wadd(wmul(dx, dx), wmul(dy, dy)) <= BOND_R2) touched = true;
-      }
-      leave = !touched;
+  if constexpr (!MARKED) {
+    const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
+    for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
+      const uint32_t slot = S.slotBase + i;
+      if (!rg_member(b, slot, tag)) continue;
+      const uint32_t p = b.inv[slot];
+      b.rmark[slot] = rigid_leaves(b, nb, slot, p, p, tag, f) ? 1u : 0u;
     }
-    b.rmark[slot] = leave ? 1u : 0u;
   }
   __syncthreads();
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
+  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
     if (b.rmark[slot]) b.state[(size_t)slot * 8 + 5] &= ~(int32_t)FLAG_RIGID;
@@ -452,7 +478,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
   __syncthreads();
   // 3. recount and re-base
   int32_t v[5] = {0, 0, 0, 0, 0};  // n, sum ox>>osh, sum oy>>osh, sum (o>>ish)^2, sum grav
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
+  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
     const int2 o = b.rest[slot];
@@ -463,7 +489,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
     v[3] = wadd(v[3], wadd(wmul(a, a), wmul(c, c)));
     v[4] = wadd(v[4], matw(b, (uint32_t)b.state[(size_t)slot * 8 + 4], M_grav));
   }
-  rg_block_sum<5>(v, sh);
+  rg_block_sum<NT>(v, sh);
   const int32_t nLive = v[0];
   const bool dissolve = nLive < RIGID_MIN_MEMBERS;
   int32_t dx = 0, dy = 0;
@@ -492,7 +518,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
     }
   }
   if (!dissolve && dx == 0 && dy == 0) return;
-  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += RG_THREADS) {
+  for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
     if (dissolve) {
@@ -502,6 +528,11 @@ __global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
       b.rest[slot] = make_int2(wsub(o.x, dx), wsub(o.y, dy));
     }
   }
+}
+template <bool DBG>
+__global__ void __launch_bounds__(RG_THREADS) k_rigid_member(Bufs b) {
+  __shared__ int32_t sh[RG_THREADS / 32][RG_SUMS];
+  rigid_member_body<DBG, RG_THREADS, false>(b, blockIdx.x, sh, Flags<DBG>{b.dbg});
 }
 
 }  // namespace d2
