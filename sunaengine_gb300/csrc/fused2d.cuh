@@ -72,6 +72,7 @@ struct NbrOwned {
 // colour's particle a substep of 4.7 k particles went from 94 to 86 us, of 40 k
 // from 145 to 128.
 constexpr int FU_B = 3;
+constexpr uint32_t FU_CHUNK = 16;  // particles of a colour dealt to a CTA at a time, in worlds with bodies
 template <int L>
 __device__ __forceinline__ void solveA_owned(const Bufs& b, const NbrOwned& nb, uint32_t row, uint32_t cnt,
                                              uint32_t sub, int2 pi, const Flags<false>& f, int32_t& rho, int32_t& S,
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   __shared__ uint32_t ws[64];
   __shared__ int4 smat1[MAT_MAX], smat2[MAT_MAX];
   __shared__ int2 scol[MAT_MAX];  // {eps, dpMax}
+  __shared__ bool sfric[MAT_MAX];  // the row rubs or bonds
   __shared__ uint32_t dsacc[8], dsscene, lastCta;
   __shared__ int32_t rsum[RIG ? FU_T / 32 : 1][RG_SUMS];
   const Flags<false> f{b.dbg};
@@ -175,7 +177,10 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   for (uint32_t k = tid; k < (uint32_t)TN; k += FU_T) swg[k] = __ldg(b.WG + k);
   post1_mats(b, smat1);
   post2_mats(b, smat2);
-  if (tid < (uint32_t)MAT_MAX) scol[tid] = make_int2(matw(b, tid, M_eps), matw(b, tid, M_dpMax));
+  if (tid < (uint32_t)MAT_MAX) {
+    scol[tid] = make_int2(matw(b, tid, M_eps), matw(b, tid, M_dpMax));
+    if (RIG) sfric[tid] = friction_row(b, tid);
+  }
   if (!grid_wait(P.bar, b.err, target)) return;
 
   // ---- cell ranges (every CTA its own copy), slots to their cells
@@ -208,21 +213,30 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   if (!grid_wait(P.bar, b.err, target)) return;
 
   // ---- the owned share of each colour class
-  uint32_t own[5], first[4], lo4[4];
+  // One contiguous share, which has the best of L1, but in worlds with bodies
+  // whole rounds of a chunk to each CTA first: their members, who rub and are
+  // marked, lie together, on 8 of 152 CTAs. us a substep, contiguous / chunks of
+  // 32, 16, 8: the site 304 / 286, 277, 279; worlds without bodies lose (40 k
+  // 139 / 141, 142, 146, 16 twins 145 / 153, 162, 178).
+  uint32_t own[5], first[4], lo4[4], dealt[4];
   own[0] = 0;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     lo4[c] = X[b.world->colourBase[c]];
-    const uint32_t n = X[b.world->colourBase[c + 1]] - lo4[c], per = (n + G - 1) / G;
-    const uint32_t s0 = min(cta * per, n), e0 = min(s0 + per, n);
-    first[c] = lo4[c] + s0;
-    own[c + 1] = own[c] + (e0 - s0);
+    const uint32_t n = X[b.world->colourBase[c + 1]] - lo4[c];
+    dealt[c] = RIG ? n / (FU_CHUNK * G) * FU_CHUNK : 0u;
+    const uint32_t rest = n - dealt[c] * G, per = (rest + G - 1) / G;
+    const uint32_t s0 = min(cta * per, rest), e0 = min(s0 + per, rest);
+    first[c] = lo4[c] + dealt[c] * G + s0;
+    own[c + 1] = own[c] + dealt[c] + (e0 - s0);
   }
   for (uint32_t i = tid; i < own[4]; i += FU_T) {
-    const uint32_t p = i < own[1]   ? first[0] + i
-                       : i < own[2] ? first[1] + (i - own[1])
-                       : i < own[3] ? first[2] + (i - own[2])
-                                    : first[3] + (i - own[3]);
+    const int c = i < own[1] ? 0 : i < own[2] ? 1 : i < own[3] ? 2 : 3;
+    const uint32_t k = i - (c == 0 ? 0u : c == 1 ? own[1] : c == 2 ? own[2] : own[3]);
+    const uint32_t lo = c == 0 ? lo4[0] : c == 1 ? lo4[1] : c == 2 ? lo4[2] : lo4[3];
+    const uint32_t d = c == 0 ? dealt[0] : c == 1 ? dealt[1] : c == 2 ? dealt[2] : dealt[3];
+    const uint32_t f0 = c == 0 ? first[0] : c == 1 ? first[1] : c == 2 ? first[2] : first[3];
+    const uint32_t p = RIG && k < d ? lo + (k / FU_CHUNK * G + cta) * FU_CHUNK + k % FU_CHUNK : f0 + (k - d);
     pOf[i] = p;
     rec[i] = b.PL[p];
     const ScenePar& S = b.scenes[b.SCN[p]];
@@ -251,18 +265,22 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   // ---- neighbour lists
   const uint32_t sub = tid & (L - 1);
   const bool cutLists = *(volatile uint32_t*)(b.work + 1) == 0u;
-  for (uint32_t i = tid / L;; i += FU_T / L) {
-    if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;  // warp-uniform exit
-    const bool valid = i < own[4];
-    const uint32_t r = valid ? i : 0u, p = pOf[r];
-    const uint32_t w = nbr_lanes<false, L, false>(
-        b, X, cutLists, valid, p, rec[r],
-        [&](uint32_t at, uint32_t q, uint32_t, uint32_t) { rows[r * FU_ROW + at] = q; }, f);
-    if (valid && sub == 0) {
-      word[r] = w;
-      b.NBRN[p] = w;
+  const auto lists = [&](auto cut) {  // the stopping scan without the other's flags
+    for (uint32_t i = tid / L;; i += FU_T / L) {
+      if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;  // warp-uniform exit
+      const bool valid = i < own[4];
+      const uint32_t r = valid ? i : 0u, p = pOf[r];
+      const uint32_t w = nbr_lanes<false, L, false>(
+          b, X, decltype(cut)::value, valid, p, rec[r],
+          [&](uint32_t at, uint32_t q, uint32_t, uint32_t) { rows[r * FU_ROW + at] = q; }, f);
+      if (valid && sub == 0) {
+        word[r] = w;
+        b.NBRN[p] = w;
+      }
     }
-  }
+  };
+  if (cutLists) lists(std::true_type{});
+  else lists(std::false_type{});
   __syncthreads();
   int2* sca = reinterpret_cast<int2*>(X);  // the cell ranges are not read again
   for (uint32_t k = tid; k < (uint32_t)TN; k += FU_T) sca[k] = __ldg(b.CA + k);
@@ -324,11 +342,15 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     if (!grid_wait(P.bar, b.err, target)) return;
     if (fric) {
       const NbrOwned nf{b.PL, rows, swg, sca, 0u, 0u};
-      for (uint32_t i = tid / L;; i += FU_T / L) {
+      // beside bodies few rows rub: their lists over as many lanes as a colour pass
+      // takes, warps without one go on
+      constexpr int LF = RIG ? LC : L;
+      for (uint32_t i = tid / LF;; i += FU_T / LF) {
         if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
-        const bool valid = i < own[4];
-        const uint32_t r = valid ? i : 0u;
-        friction_particle<false, L>(b, nf, valid, pOf[r], r, sub, f);
+        const uint32_t r = i < own[4] ? i : 0u;
+        const bool valid = i < own[4] && !(RIG && (is_wall(rec[r].w) || !sfric[(uint32_t)rec[r].w & INFO_MAT]));
+        if (!RIG || __any_sync(0xffffffffu, valid))
+          friction_particle<false, LF>(b, nf, valid, pOf[r], r, tid & (LF - 1), f);
       }
       if (!grid_wait(P.bar, b.err, target)) return;
       for (uint32_t i = tid; i < own[4]; i += FU_T) {
@@ -390,20 +412,27 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     if (!grid_wait(P.bar, b.err, target)) return;
   }
   if (stress) {
-    for (uint32_t i = tid / L;; i += FU_T / L) {
+    const uint32_t subC = tid & (LC - 1);
+    for (uint32_t i = tid / LC;; i += FU_T / LC) {
       if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
-      const bool valid = i < own[4];
-      const uint32_t r = valid ? i : 0u;
-      contain_stress_slot<false, L>(b, nb, valid, b.sslot[pOf[r]], r, sub, f);
+      const uint32_t r = i < own[4] ? i : 0u;
+      const bool held = i < own[4] && !is_wall(rec[r].w) && ((uint32_t)rec[r].w & INFO_PINNED);
+      if (__any_sync(0xffffffffu, held)) contain_stress_slot<false, LC>(b, nb, held, b.sslot[pOf[r]], r, subC, f);
     }
+    // a burst takes a member out of its body: the marks below see it
+    if (RIG && !grid_wait(P.bar, b.err, target)) return;
   }
   if constexpr (RIG) {
-    for (uint32_t i = tid; i < own[4]; i += FU_T) {
-      const uint32_t inf = (uint32_t)rec[i].w;
-      if (!(inf & INFO_RIGID) || is_wall(rec[i].w)) continue;
-      const uint32_t p = pOf[i], sl = b.sslot[p];
+    const uint32_t subC = tid & (LC - 1);
+    for (uint32_t i = tid / LC;; i += FU_T / LC) {
+      if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
+      const uint32_t r = i < own[4] ? i : 0u;
+      const bool member = i < own[4] && !is_wall(rec[r].w) && ((uint32_t)rec[r].w & INFO_RIGID);
+      if (!__any_sync(0xffffffffu, member)) continue;
+      const uint32_t p = pOf[r], sl = b.sslot[p];
       const int32_t tag = (int32_t)((uint32_t)b.state[(size_t)sl * 8 + 5] & WELD_TAG_MASK);
-      b.rmark[sl] = rigid_leaves(b, nb, sl, p, i, tag, f) ? 1u : 0u;
+      const bool leaves = rigid_leaves<false, LC>(b, nb, member, sl, p, r, subC, tag, f);
+      if (member && subC == 0) b.rmark[sl] = leaves ? 1u : 0u;
     }
     if (!grid_wait(P.bar, b.err, target)) return;
     for (uint32_t k = cta; k < P.bodies; k += G) rigid_member_body<false, FU_T, true>(b, k, rsum, f);

@@ -143,18 +143,21 @@ template <int NT, int K>
 __device__ __forceinline__ void rg_block_sum(int32_t (&v)[K], int32_t (*sh)[RG_SUMS]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < K; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] = wadd(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-  if (lane == 0)
+  for (int k = 0; k < K; ++k) {
+    v[k] = __reduce_add_sync(0xffffffffu, v[k]);
+    if (lane == 0) sh[warp][k] = v[k];
+  }
+  __syncthreads();
+  if (warp == 0) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) sh[warp][k] = v[k];
+    for (int k = 0; k < K; ++k) {
+      const int32_t t = __reduce_add_sync(0xffffffffu, lane < NT / 32 ? sh[lane][k] : 0);
+      if (lane == 0) sh[0][k] = t;
+    }
+  }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    int32_t t = 0;
-    for (int w = 0; w < NT / 32; ++w) t = wadd(t, sh[w][k]);
-    v[k] = t;
-  }
+  for (int k = 0; k < K; ++k) v[k] = sh[0][k];
   __syncthreads();
 }
 
@@ -343,19 +346,27 @@ __device__ __forceinline__ void rigid_solve_body(const Bufs& b, uint32_t body, b
     while (L < 8u && span * (L * 2u) <= (uint32_t)NT) L *= 2u;
   const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x & (L - 1u);
   const uint32_t gmask = ((1u << L) - 1u) << (lane & ~(L - 1u));
+  // (a slot's words, its index and its rest offset in one round of loads, what
+  // they lead to in the next; a body of one round keeps them for the placement)
+  const bool once = span <= (uint32_t)NT / L;
+  bool mem = false;
+  uint32_t p = 0;
+  int2 rest = make_int2(0, 0);
   for (uint32_t base = first; base <= last && base < S.nFluid; base += NT / L) {
     const uint32_t i = base + threadIdx.x / L;
-    const uint32_t slot = S.slotBase + i;
-    const bool mem = i <= last && i < S.nFluid && rg_member(b, slot, tag);
-    const int32_t* w = b.state + (size_t)(mem ? slot : S.slotBase) * 8;
-    const uint32_t p = mem ? b.inv[slot] : 0u;
-    const int2 pr = ld_pred(b.PL, p);
-    const int2 pos = make_int2(w[0], w[1]);
+    const bool in = i <= last && i < S.nFluid;
+    const uint32_t slot = S.slotBase + (in ? i : first);
+    const int4* w4 = reinterpret_cast<const int4*>(b.state + (size_t)slot * 8);
+    const int4 w0 = w4[0], w1 = w4[1];
+    p = b.inv[slot];
+    rest = b.rest[slot];
+    const int2 pr = ld_pred(b.PL, p), dp = b.DP[p];
+    mem = in && ((uint32_t)w1.y & FLAG_RIGID) && (int32_t)((uint32_t)w1.y & WELD_TAG_MASK) == tag;
+    const int2 pos = xy(w0);
     bool hit = seal && mem && rigid_seal_hit(b, S, p, pos, pr, tag, sub, L, f);
     if (L > 1u) hit = (__ballot_sync(0xffffffffu, hit) & gmask) != 0u;
     if (!mem || sub != 0u) continue;
-    const int32_t dm = matw(b, (uint32_t)w[4], M_dpMax), dmN = neg_sat(dm, f);
-    const int2 dp = b.DP[p];
+    const int32_t dm = matw(b, (uint32_t)w1.x, M_dpMax), dmN = neg_sat(dm, f);
     const int2 sd = hit ? make_int2(sub_sat(pos.x, pr.x, f), sub_sat(pos.y, pr.y, f)) : make_int2(0, 0);
     const int32_t dx = clampi(shr_rne<8>(dp.x), dmN, dm), dy = clampi(shr_rne<8>(dp.y), dmN, dm);
     v[0] = wadd(v[0], dx);
@@ -398,12 +409,15 @@ __device__ __forceinline__ void rigid_solve_body(const Bufs& b, uint32_t body, b
   __syncthreads();
   const int32_t qx = R[RB_CQX], qy = R[RB_CQY], th = R[RB_THETAQ];
   const int32_t c = rg_cos(b.cosT, th, f), s = rg_sin(b.cosT, th, f);
+  if (once) {
+    if (mem && sub == 0u) *reinterpret_cast<int2*>(b.PL + p) = rg_at(qx, qy, c, s, rest, f);
+    return;
+  }
   for (uint32_t i = first + threadIdx.x; i <= last && i < S.nFluid; i += NT) {
     const uint32_t slot = S.slotBase + i;
     if (!rg_member(b, slot, tag)) continue;
-    const uint32_t p = b.inv[slot];
-    const int2 pr = rg_at(qx, qy, c, s, b.rest[slot], f);
-    *reinterpret_cast<int2*>(b.PL + p) = pr;
+    const uint32_t q = b.inv[slot];
+    *reinterpret_cast<int2*>(b.PL + q) = rg_at(qx, qy, c, s, b.rest[slot], f);
   }
 }
 template <bool DBG>
@@ -417,25 +431,31 @@ __global__ void __launch_bounds__(RG_THREADS, 1) k_rigid_solve(Bufs b, int seal)
 // the clears, across a CTA barrier); the reference's single loop clears
 // FLAG_RIGID while other lanes of its workgroup read it.
 //
-// Whether the member in `slot` leaves; row: its list in nb.
-template <bool DBG, class NB>
-__device__ __forceinline__ bool rigid_leaves(const Bufs& b, const NB& nb, uint32_t slot, uint32_t p, uint32_t row,
-                                             int32_t tag, const Flags<DBG>& f) {
+// Whether the member in `slot` leaves; row: its list in nb, walked by L lanes (a
+// warp calls it together where L > 1; `mem` false for lanes without a member).
+template <bool DBG, int L, class NB>
+__device__ __forceinline__ bool rigid_leaves(const Bufs& b, const NB& nb, bool mem, uint32_t slot, uint32_t p,
+                                             uint32_t row, uint32_t sub, int32_t tag, const Flags<DBG>& f) {
   const int32_t* w = b.state + (size_t)slot * 8;
   const uint32_t m = (uint32_t)w[4];
-  if (matw(b, m, M_solidMode) != SOLID_RIGID || matw(b, m, M_phantom) != 0) return true;
-  const uint32_t cnt = b.NBRN[p] & NBRN_COUNT;
-  for (uint32_t k = 0; k < cnt; ++k) {
+  const bool walk = mem && matw(b, m, M_solidMode) == SOLID_RIGID && matw(b, m, M_phantom) == 0;
+  const uint32_t cnt = walk ? (b.NBRN[p] & NBRN_COUNT) : 0u;
+  bool touched = false;
+  for (uint32_t k = sub; k < cnt && !touched; k += L) {
     const uint32_t e = nb.entry(row, k);
-    if (is_wall(b.PL[e].w)) continue;
-    const uint32_t js = b.sslot[e];
-    if (!rg_member(b, js, tag)) continue;
+    const uint32_t infoJ = (uint32_t)b.PL[e].w, js = b.sslot[e];
+    // nothing becomes a member inside a substep
+    if ((infoJ & INFO_BOUNDARY) || !(infoJ & INFO_RIGID) || !rg_member(b, js, tag)) continue;
     const int32_t* wj = b.state + (size_t)js * 8;
     const int32_t dx = shr_rne<BPRE>(sub_sat(w[0], wj[0], f)), dy = shr_rne<BPRE>(sub_sat(w[1], wj[1], f));
     if (abs(dx) > L0_MAX || abs(dy) > L0_MAX) continue;
-    if (wadd(wmul(dx, dx), wmul(dy, dy)) <= BOND_R2) return false;
+    if (wadd(wmul(dx, dx), wmul(dy, dy)) <= BOND_R2) touched = true;
   }
-  return true;
+  if constexpr (L > 1) {
+    const uint32_t gmask = ((1u << L) - 1u) << (threadIdx.x & 31u & ~(uint32_t)(L - 1));
+    touched = (__ballot_sync(0xffffffffu, touched) & gmask) != 0u;
+  }
+  return !touched;
 }
 
 // MARKED: rmark already holds every member's decision (the fused substep, where
@@ -466,7 +486,7 @@ __device__ __forceinline__ void rigid_member_body(const Bufs& b, uint32_t body, 
       const uint32_t slot = S.slotBase + i;
       if (!rg_member(b, slot, tag)) continue;
       const uint32_t p = b.inv[slot];
-      b.rmark[slot] = rigid_leaves(b, nb, slot, p, p, tag, f) ? 1u : 0u;
+      b.rmark[slot] = rigid_leaves<DBG, 1>(b, nb, true, slot, p, p, 0u, tag, f) ? 1u : 0u;
     }
   }
   __syncthreads();

@@ -518,6 +518,21 @@ __device__ __forceinline__ uint32_t cand_test(const int4* PL, uint32_t base, Can
   return m.hit;
 }
 
+// Whether a live fluid particle with CONGEAL or SEAL is among the hits `m` of the
+// candidates from base on (no hit is dead). Worlds that hold one used to test
+// every candidate's record; a hit's info word alone is a third of those loads.
+__device__ __forceinline__ void raise_kinds(const int4* PL, uint32_t base, uint32_t m, bool& congeal, bool& seal) {
+#pragma unroll 4
+  while (m) {
+    const uint32_t j = (uint32_t)__clz((int)m);
+    m ^= 0x80000000u >> j;
+    const uint32_t info = (uint32_t)PL[base + j].w;
+    if (info & INFO_BOUNDARY) continue;
+    congeal |= (info & INFO_CONGEAL) != 0u;
+    seal |= (info & INFO_SEAL) != 0u;
+  }
+}
+
 // The per-substep world flags one particle raises (see Bufs::work): some lanes
 // of the warp may be absent.
 __device__ __forceinline__ void raise_work(const Bufs& b, int k, bool raise) {
@@ -737,7 +752,7 @@ constexpr uint32_t NO_STAGE = 0x7fffffffu;  // a candidate whose tile is not sta
 // for a lane group with none): p its sorted index, `me` its record. The hits go
 // to out(position, sorted index, info, staged offset); returns the NBRN word.
 //
-// The stopping scan (`cut`) deals the particle's cells in reach to its lanes,
+// Release builds deal the particle's cells in reach to its lanes,
 // in order: each lane filters and tests its cell's candidates, a prefix over
 // the lanes gives its hits their places, and round after round the cells
 // follow in the reference's order. A cell of more candidates than two filter
@@ -760,7 +775,7 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
   const uint32_t ts = S.tileShift, tx = (uint32_t)cc.x >> ts, ty = (uint32_t)cc.y >> ts;
   const uint32_t* tr = (TILED && work) ? b.TR + (size_t)tile_of(S, cc.x, cc.y) * TR_STRIDE : b.TR;
   const bool local = TILED && work && !bnd && tr[TR_BASE + tile_runs(ts)] <= b.world->stageCap;
-  if (!TILED && L > 1 && cut) {
+  if (!TILED && !DBG && L > 1) {
     // the cells in reach: bit 3 (dy + 1) + dx + 1
     const uint32_t cols = ((skip & SKIP_LEFT) || cc.x == 0 ? 0u : 1u) | 2u |
                           ((skip & SKIP_RIGHT) || cc.x + 1 >= (int32_t)S.gridW ? 0u : 4u);
@@ -804,6 +819,10 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
       }
       uint32_t at = n + inc - mine;
       n += __shfl_sync(0xffffffffu, inc, L - 1, L);
+      if (!cut) {
+        raise_kinds(b.PL, base, m0, congeal, sealSeen);
+        raise_kinds(b.PL, base + 32, m1, congeal, sealSeen);
+      }
       for (; m0 && at < (uint32_t)MAXNBR; ++at) {
         const uint32_t j = (uint32_t)__clz((int)m0);
         m0 &= ~(0x80000000u >> j);
@@ -816,8 +835,13 @@ __device__ __forceinline__ uint32_t nbr_lanes(const Bufs& b, const uint32_t* cel
       }
 #pragma unroll
       for (int t = 0; t < L; ++t) cells &= cells - 1u;
-      if (!__any_sync(0xffffffffu, cells != 0u && n < (uint32_t)MAXNBR)) return work ? min(n, (uint32_t)MAXNBR) : 0u;
+      if (!__any_sync(0xffffffffu, cells != 0u && !(cut && n >= (uint32_t)MAXNBR))) {
+        congeal = (__ballot_sync(0xffffffffu, congeal) & gmask) != 0u;
+        sealSeen = (__ballot_sync(0xffffffffu, sealSeen) & gmask) != 0u;
+        return work ? min(n, (uint32_t)MAXNBR) | (congeal ? NBRN_CONGEAL : 0u) | (sealSeen ? NBRN_SEAL : 0u) : 0u;
+      }
     }
+    congeal = sealSeen = false;
   }
   for (int dy = -1; dy <= 1; ++dy) {
     for (int dx = -1; dx <= 1; ++dx) {
@@ -924,20 +948,21 @@ __global__ void __launch_bounds__(256, 6) k_nbr(Bufs b) {
           uint32_t key = key_of(S, gx, gy);
           uint32_t lo = b.cellStart[key], hi = b.cellStart[key + 1];
           if (!DBG && hi - lo > CELL_BIG && !box_reaches(b.CB[key], pi)) continue;
-          if (!TILED && cut) {
-            // The stopping scan: no live fluid particle carries SEAL or
-            // CONGEAL (so neither flag can be raised) and the list ends at
-            // MAXNBR (so nothing overflows).
+          if (!TILED && !DBG) {
+            // The stopping scan (cut) ends with the list; the other goes on for
+            // the flags of the hits past it.
             const uint32_t bias = cand_bias(cq, dx, dy);
             for (uint32_t base = lo & ~3u; base < hi; base += 32) {
               CandMask c = cand_mask<2>(b.QC, base, lo, hi, bias, cand_cell(S, cb, gx, gy));
               if (dx == 0 && dy == 0 && p - base < 32u) c.hit &= ~(0x80000000u >> (p - base));
-              for (uint32_t m = cand_test(b.PL, base, c, pi, f); m;) {
+              uint32_t m = cand_test(b.PL, base, c, pi, f);
+              if (!cut) raise_kinds(b.PL, base, m, congeal, sealSeen);
+              while (m && cnt < (uint32_t)MAXNBR) {
                 const uint32_t j = (uint32_t)__clz((int)m);
                 m ^= 0x80000000u >> j;
-                out.put(cnt, base + j);
-                if (++cnt >= (uint32_t)MAXNBR) goto listed;
+                out.put(cnt++, base + j);
               }
+              if (cut && cnt >= (uint32_t)MAXNBR) goto listed;
             }
             continue;
           }
@@ -2062,9 +2087,9 @@ __device__ __forceinline__ void contain_stress_slot(const Bufs& b, const NB& nb,
   const uint32_t cnt = act ? (b.NBRN[p] & NBRN_COUNT) : 0u;
   int32_t stress = 0;
   for (uint32_t k = sub; k < cnt; k += L) {
-    const uint32_t e = nb.entry(r, k);
+    const uint32_t e = nb.entry(r, k), sj = b.sslot[e];
     if (is_wall(b.PL[e].w)) continue;
-    const int32_t* wj = b.state + (size_t)b.sslot[e] * 8;
+    const int32_t* wj = b.state + (size_t)sj * 8;
     const uint32_t mj = (uint32_t)wj[4];
     if (seal_class(b, mj) || matw(b, mj, M_phantom) != 0) continue;
     const int32_t dx4 = shr_rne<BPRE>(sub_sat(px, wj[0], f)), dy4 = shr_rne<BPRE>(sub_sat(py, wj[1], f));
