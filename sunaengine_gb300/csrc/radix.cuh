@@ -13,7 +13,7 @@
 // of tile counts (one CTA per digit) -> scatter, whose prologue scans the
 // digit totals itself (one thread per digit). The tile (512 threads x IT
 // items) is picked per sort so that even a few hundred thousand keys spread
-// over ~128 CTAs.
+// over the GPU (items_for).
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -29,7 +29,7 @@ constexpr int RADIX = 1 << RBITS;
 constexpr int TPB = 512;                 // threads per tile
 constexpr int WARPS = TPB / 32;
 constexpr int MAX_ITEMS = 16;            // items per thread, largest tile
-constexpr int MIN_TILES = 128;           // a sort spreads over at least this many tiles when it can
+constexpr int MIN_TILES = 256;           // a sort spreads over at least this many tiles when it can
 static_assert(TPB == RADIX, "one thread per digit in the histogram and scatter prologues");
 
 __device__ __forceinline__ uint32_t digit_of(const uint32_t* keys, uint32_t idx, uint32_t n, int shift) {
@@ -149,11 +149,16 @@ __global__ void __launch_bounds__(TPB) k_scatter(const uint32_t* __restrict__ ke
   }
 }
 
-// Items per thread for n keys: the smallest power of two (1..16) that keeps
-// the tile count at or below MIN_TILES, so small sorts still fill the GPU.
+// Items per thread for n keys: the largest power of two (1..16) that leaves at
+// least MIN_TILES tiles, three CTAs to two SMs. A tile's items are one serial
+// chain of match rounds, so fewer tiles than SMs is the worst case: 265 k keys in
+// 65 tiles of 8 items (at most 128 tiles, the rule before) took 46 us a substep.
+// us a substep with at most 128 tiles / at least 128, 256, 512: 265 k particles
+// 616 / 607, 597, 603, 756 k in 48 scenes 1366 /
+// 1355, 1330, 1340.
 inline int items_for(uint32_t n) {
   int it = 1;
-  while (it < MAX_ITEMS && (uint64_t)TPB * it * MIN_TILES < n) it <<= 1;
+  while (it < MAX_ITEMS && (uint64_t)TPB * 2 * it * MIN_TILES <= n) it <<= 1;
   return it;
 }
 
@@ -198,10 +203,11 @@ inline void sort_pairs(uint32_t* keys0, uint32_t n, int keyBits, uint32_t* outKe
 
 constexpr int LAUNCHES_PER_PASS = 3;
 
-// Words of `hist` a sort of up to n keys needs (tile counts plus the digit totals).
+// Words of `hist` a sort of up to n keys needs (tile counts plus the digit totals);
+// below MAX_ITEMS a smaller sort may have more tiles, but fewer than 2 MIN_TILES.
 inline size_t hist_words(uint32_t n) {
   const uint32_t tiles = (n + TPB * items_for(n) - 1) / (TPB * items_for(n));
-  return (size_t)RADIX * (std::max<uint32_t>(tiles, MIN_TILES) + 2);
+  return (size_t)RADIX * (std::max<uint32_t>(tiles, 2 * MIN_TILES) + 2);
 }
 
 }  // namespace

@@ -1265,12 +1265,37 @@ __device__ __forceinline__ void solveB_pair(const Bufs& b, const NB& nb, int2 pi
 }
 
 // solveB_at for one particle.
+// The colour passes (NbrSplit) keep two neighbours' records in flight. More do
+// not fit 32 registers, and the pass wants all its warps: us a substep at 265 k /
+// 1 M one ahead 607 / 1337, two 600 / 1322, two or three with 6 CTAs an SM 603 /
+// 1347 and 600 / 1333, three with 5 607 / 1367.
 // RIG: the warp holds a rigid member, whose own correction skips the members
 // of its body (src/sim.wgsl:1355-1358).
+struct NbrSplit;
 template <bool DBG, int L, bool RIG, class NB>
 __device__ __forceinline__ int2 solveB_dp(const Bufs& b, const NB& nb, uint32_t p, uint32_t cnt, uint32_t sub,
                                           int2 pi, int32_t li, const Flags<DBG>& f, uint32_t infoI = 0u) {
   int32_t dpx = 0, dpy = 0;
+  if constexpr (!DBG && std::is_same<NB, NbrSplit>::value) {
+    constexpr int B = 2;
+    uint32_t e[B];
+#pragma unroll
+    for (int j = 0; j < B; ++j) e[j] = sub + j * L < cnt ? nb.entry(p, sub + j * L) : 0u;
+    for (uint32_t k = sub; k < cnt; k += L * B) {
+      int4 o[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) o[j] = nb.rec(e[j]);
+#pragma unroll
+      for (int j = 0; j < B; ++j) e[j] = k + (B + j) * L < cnt ? nb.entry(p, k + (B + j) * L) : 0u;
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        if (k + j * L >= cnt) break;
+        if (RIG && !is_wall(o[j].w) && same_body(infoI, (uint32_t)o[j].w)) continue;
+        solveB_pair<DBG>(b, nb, pi, li, o[j], f, dpx, dpy);
+      }
+    }
+    return make_int2(gsum<L>(dpx), gsum<L>(dpy));
+  }
   uint32_t en = sub < cnt ? nb.entry(p, sub) : 0u;
   int4 on = nb.rec(en);
   uint32_t en2 = sub + L < cnt ? nb.entry(p, sub + L) : 0u;
