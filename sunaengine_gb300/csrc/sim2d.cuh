@@ -2268,8 +2268,11 @@ __device__ __forceinline__ void post2_finish(const Bufs& b, const ScenePar& S, u
     w[5] = (int32_t)fo;
   }
 }
+// Six CTAs an SM (40 registers): us at 262 k / 757 k / 1 M particles with five 84 /
+// 195 / 217, six 78 / 176 / 214, seven 82 / 190 / 245 (spills). The digest's
+// registers make that five.
 template <bool DBG, bool HASH, int L>
-__global__ void __launch_bounds__(256, 5) k_post2(Bufs b, int formFlags) {
+__global__ void __launch_bounds__(256, HASH ? 5 : 6) k_post2(Bufs b, int formFlags) {
   Flags<DBG> f{b.dbg};
   __shared__ int4 smat[MAT_MAX];
   post2_mats(b, smat);
