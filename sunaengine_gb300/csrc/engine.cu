@@ -1315,18 +1315,21 @@ struct World {
   // particles need more lanes to fill the GPU; more lanes cost each particle's
   // prologue and reduction again. The lines lie where uniform splits crossed on
   // the settled two-fluid scene (phase us at the neighbouring sizes, fewer / more
-  // lanes): solveA 265 k 94 / 94 (1, 2) and 197 k 88 / 76, 103 k 61 / 60 (2, 4);
-  // colours 265 k 203 / 219 and 197 k 181 / 175 (4, 8); post1 265 k 66 / 62,
-  // 363 k 77 / 83, 744 k 155 / 149 (1, 2: its waves come out even or not); post2
-  // 744 k 182 / 175 and 1.05 M 223 / 234 (1, 2); lists 265 k 54 / 62 and 197 k
-  // 50 / 48 (1, 2).
+  // lanes): solveA 179 k 74 / 75 (1, 2), 133 k 66 / 66 and 104 k 60 / 59 (1, 4);
+  // colours 1.05 M 437 / 446 and 927 k 412 / 372 (1, 2), 762 k 335 / 349 and 529 k
+  // 273 / 271 (2, 4), 133 k 166 / 172 and 104 k 157 / 153 (4, 8); post1 364 k 77 / 84
+  // and 265 k 67 / 63 (1, 2), 179 k 46 / 47 and 133 k 41 / 39 (2, 4); post2 529 k 114
+  // / 123 and 364 k 94 / 94 (1, 2; at 265 k 72 / 74, but 7.5 us slower once the scene
+  // has settled 200 substeps), 179 k 57 / 60 and 133 k 49 / 48 (2, 4); lists 133 k 38
+  // / 39 and 104 k 34 / 34 (1, 2). Where two tie the line leans to the side of the
+  // clear one.
   static LaneCfg lanes_for(uint64_t n) {
     LaneCfg l;
-    l.a = n < 40000 ? 8 : n < 110000 ? 4 : n < 265000 ? 2 : 1;
-    l.c = n < 220000 ? 8 : 4;
-    l.p1 = n < 40000 ? 8 : n < 110000 ? 4 : (n < 330000 || n >= 650000) ? 2 : 1;
-    l.p2 = n < 40000 ? 8 : n < 110000 ? 4 : n < 900000 ? 2 : 1;
-    l.n = n < 40000 ? 8 : n < 80000 ? 4 : n < 220000 ? 2 : 1;
+    l.a = n < 40000 ? 8 : n < 110000 ? 4 : n < 150000 ? 2 : 1;
+    l.c = n < 120000 ? 8 : n < 600000 ? 4 : n < 1000000 ? 2 : 1;
+    l.p1 = n < 40000 ? 8 : n < 150000 ? 4 : n < 300000 ? 2 : 1;
+    l.p2 = n < 40000 ? 8 : n < 140000 ? 4 : n < 400000 ? 2 : 1;
+    l.n = n < 40000 ? 8 : n < 80000 ? 4 : n < 110000 ? 2 : 1;
     return l;
   }
   void default_lanes() {
