@@ -17,7 +17,8 @@
  *     must be driven from one host thread at a time (the reference's engine is
  *     single-threaded JS);
  *   - GPU-side failures are deferred and reported by sn_check_errors(), like
- *     the reference's checkErrors() (src/engine.js:3689-3696).
+ *     the reference's checkErrors() (src/engine.js:3689-3696); a launch that gave
+ *     up half way is reported by every read as well (sn_set_barrier_wait).
  *
  * State words are the reference's Particle struct (src/sim.wgsl:181-188):
  * 8 int32 per particle, [pos.x, pos.y, vel.x, vel.y, matId, flags, temp, fuel],
@@ -377,10 +378,19 @@ int sn_batch_autotune_layout(sn_batch* b, uint32_t reps, uint32_t* substeps_run,
  * kernel with grid barriers between the phases, instead of one launch per
  * phase. Applies to worlds with no rigid body in the default layout; others
  * keep the per-phase launches. Results are identical (measured slower
- * on GB300 than the captured per-phase graph; off by default). A barrier that
- * waits past its bound raises an error that sn_check_errors reports. */
+ * on GB300 than the captured per-phase graph; off by default). */
 int sn_set_persistent(sn_engine* e, uint32_t on);
 int sn_batch_set_persistent(sn_batch* b, uint32_t on);
+/* (no counterpart) How long a grid barrier of a cooperative launch (the
+ * persistent form above, and the substep of small worlds, which is one launch)
+ * waits, in SM cycles; 2^31, about a second, by default, 2^40 at most. A launch
+ * whose barrier runs out ends its substep half way: from then on every call that
+ * steps a scene of this world or gives out its words, clocks, chain or digest
+ * returns SN_E_DEVICE, sn_sync and sn_check_errors too, until the scene is loaded
+ * again or takes a checkpoint (one scene of a batch at a time; the others stay
+ * refused). */
+int sn_set_barrier_wait(sn_engine* e, uint64_t cycles);
+int sn_batch_set_barrier_wait(sn_batch* b, uint64_t cycles);
 
 /* ---- digest without device allocation ------------------------------------ */
 /* No counterpart in the reference. For callers that cannot allocate device
@@ -498,6 +508,9 @@ int sn3_get_info(sn3_engine* e, uint32_t scene, sn3_info* out);
 int sn3_last_timing(sn3_engine* e, float* ms, uint64_t* launches);
 /* Phases: predict, sort, cellstart+gather, neighbour lists, then density and
  * solve per iteration, integrate(+hash), fold. */
+/* sn_set_barrier_wait for the 3D engine (a keyframe with its chain restores a
+ * scene too). */
+int sn3_set_barrier_wait(sn3_engine* e, uint64_t cycles);
 int sn3_profile_substep(sn3_engine* e, uint32_t reps, float* ms, uint32_t max_phases, uint32_t* n_phases);
 
 /* ---- device checkpoints ------------------------------------------------------

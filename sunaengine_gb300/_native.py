@@ -237,6 +237,9 @@ SIGNATURES = {
     'sn_batch_set_staged': (ctypes.c_int, [P, u32]),
     'sn_set_persistent': (ctypes.c_int, [P, u32]),
     'sn_batch_set_persistent': (ctypes.c_int, [P, u32]),
+    'sn_set_barrier_wait': (ctypes.c_int, [P, u64]),
+    'sn_batch_set_barrier_wait': (ctypes.c_int, [P, u64]),
+    'sn3_set_barrier_wait': (ctypes.c_int, [P, u64]),
     'sn_lanes': (ctypes.c_int, [P, P]),
     'sn_batch_lanes': (ctypes.c_int, [P, P]),
     'sn_ckpt_pool_create': (ctypes.c_int, [ctypes.c_size_t, ctypes.c_int32, ctypes.POINTER(P)]),

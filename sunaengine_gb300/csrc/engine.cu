@@ -389,6 +389,7 @@ struct SceneHost {
   bool wallsOn = true;
   std::vector<ImpulseEv> events;
   uint32_t consumed = 0;  // events already applied (at < substeps)
+  bool lost = false;      // a substep of it was left half done (World::recover)
 };
 
 }  // namespace
@@ -546,13 +547,16 @@ struct World {
     b.acc = dalloc<uint32_t>((size_t)scenesCap * 8, err);
     b.accLast = dalloc<uint32_t>((size_t)scenesCap * 8, err);
     b.chain = dalloc<uint32_t>((size_t)scenesCap * 8, err);
-    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)scenesCap * 64, cudaHostAllocMapped), "mirror") ||
+    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)scenesCap * 64 + 4, cudaHostAllocMapped), "mirror") ||
         !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
       return false;
+    std::memset(mirror, 0, (size_t)scenesCap * 64 + 4);
+    gaveUp = mirror + (size_t)scenesCap * 16;
+    gaveUpDev = b.mirror + (size_t)scenesCap * 16;
     b.dbg = dalloc<uint32_t>(16, err);
     b.err = dalloc<uint32_t>(4, err);
     b.work = dalloc<uint32_t>(8, err);
-    barBuf = dalloc<uint32_t>(2, err);
+    barBuf = dalloc<uint32_t>(1, err);
     fuBar = dalloc<uint32_t>(2, err);
     tmpK = dalloc<uint32_t>(C, err);
     tmpV = dalloc<uint32_t>(C, err);
@@ -796,6 +800,7 @@ struct World {
                  "pull"))
       return false;
     if (!cuda_ok(cudaStreamSynchronize(st), "pull")) return false;
+    if (gave_up()) return fail("%s", BARRIER_TEXT);
     paramsStale = false;
     return true;
   }
@@ -963,11 +968,11 @@ struct World {
     cudaMemcpyAsync(b.accLast + s * 8, zero8, 32, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b.dbg, 0, 64, st);
     cudaMemsetAsync(b.err, 0, 16, st);
-    cudaMemsetAsync(fuBar, 0, 8, st);  // a launch that gave up leaves its counts behind
-    if (fuCount) cudaMemsetAsync(fuCount, 0, (size_t)keyCap * 4, st);
     freshScene = s;
-    bool ok2 = relayout();
+    bool ok2 = relayout();  // waits for the stream
     freshScene = 0xffffffffu;
+    if (gave_up()) ok2 = recover() && ok2;
+    h.lost = false;
     return ok2;
   }
 
@@ -1062,7 +1067,7 @@ struct World {
     const void* fn = (const void*)k_iters_persistent<DBG, L>;
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, 0);
-    cudaMemsetAsync(barBuf, 0, 8, st);
+    cudaMemsetAsync(barBuf, 0, 4, st);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(std::max(per, 1) * numSMs));
     cfg.blockDim = dim3(256);
@@ -1073,7 +1078,7 @@ struct World {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_iters_persistent<DBG, L>, b, iters, barBuf);
+    cudaLaunchKernelEx(&cfg, k_iters_persistent<DBG, L>, b, iters, grid_bar(barBuf));
   }
   template <bool DBG, int L>
   void launch_contain_stress() {
@@ -1111,6 +1116,41 @@ struct World {
 
   // ---- the fused substep of small worlds (fused2d.cuh) ----
   uint32_t* fuBar = nullptr;    // barrier words, zero between launches
+  uint32_t *gaveUp = nullptr, *gaveUpDev = nullptr;  // ERR_BARRIER for the host (mapped)
+  long long waitLimit = BARRIER_WAIT_CYCLES;
+  GridBar grid_bar(uint32_t* count) const { return GridBar{count, b.err, gaveUpDev, waitLimit}; }
+  // A launch whose grid barrier ran out leaves its substep half done in every
+  // scene, and its counts behind; the fused launches after it return at once.
+  // From then on no word of these scenes is given out until they are loaded
+  // again or take a checkpoint's words. (gave_up is looked at once the stream has
+  // been waited for; it costs no copy.)
+  bool gave_up() const { return *(volatile uint32_t*)gaveUp != 0u; }
+  bool whole(uint32_t s, const char* what) {
+    return !gave_up() && !sh[s].lost ? true : fail("%s: %s", what, BARRIER_TEXT);
+  }
+  bool sync() {
+    return cuda_ok(cudaStreamSynchronize(st), "sync") && (!gave_up() ? true : fail("sync: %s", BARRIER_TEXT));
+  }
+  bool synced(uint32_t s, const char* what) { return cuda_ok(cudaStreamSynchronize(st), what) && whole(s, what); }
+  // The world can be stepped again; the scenes that were in it are lost.
+  bool recover() {
+    if (!cuda_ok(cudaStreamSynchronize(st), "recover")) return false;
+    accFresh = chainFresh = sortedFresh = false;
+    for (SceneHost& h : sh) h.lost = h.lost || (h.used && h.loaded);
+    const bool ok = cuda_ok(cudaMemsetAsync(b.err, 0, 16, st), "recover") &&
+                    cuda_ok(cudaMemsetAsync(fuBar, 0, 8, st), "recover") &&
+                    (!fuCount || cuda_ok(cudaMemsetAsync(fuCount, 0, (size_t)keyCap * 4, st), "recover")) &&
+                    cuda_ok(cudaMemsetAsync(b.acc, 0, (size_t)maxScenes * 32, st), "recover") &&
+                    cuda_ok(cudaStreamSynchronize(st), "recover");
+    if (ok) *(volatile uint32_t*)gaveUp = 0u;
+    return ok;
+  }
+  bool set_barrier_wait(uint64_t cycles) {
+    if (cycles > 1ull << 40) return fail("a barrier waits 2^40 cycles at most");
+    waitLimit = (long long)cycles;
+    graphValid = false;
+    return true;
+  }
   uint32_t* fuCount = nullptr;  // [keyCap] cell counts, zero between launches
   // the tables and every row lie in the ranges the release kernels are built
   // for; else the debug kernels, which assume none, run
@@ -1160,7 +1200,7 @@ struct World {
     const uint32_t smem = fused_fixed() + P.ownCap * FU_OWN_BYTES;
     P.count = fuCount;
     P.tmp = tmpV;
-    P.bar = fuBar;
+    P.bar = grid_bar(fuBar);
     Bufs bb = b;
     if (iters & 1u) swap_records(bb);  // so that the last iteration ends in PL
     const auto fn = k_substep_fused<L, LC, RIG>;
@@ -1523,6 +1563,7 @@ struct World {
       if (!any) return fail("step() called before loadScene()");
     }
     if (count == 0) return true;
+    if (gave_up()) return fail("step: %s", BARRIER_TEXT);
     if (layoutDirty && !relayout()) return false;
     if (eventsDirty && !upload_events()) return false;
     const bool fused = fused_fits();
@@ -1611,7 +1652,7 @@ struct World {
   bool sortedFresh = false;
   bool digest(uint32_t s, uint32_t out[8]) {
     if (accFresh && !layoutDirty) {
-      if (!cuda_ok(cudaStreamSynchronize(st), "digest")) return false;
+      if (!synced(s, "digest")) return false;
       std::memcpy(out, mirror + (size_t)s * 16, 32);
       return true;
     }
@@ -1619,7 +1660,7 @@ struct World {
     cudaMemsetAsync(accTmp, 0, sizeof(uint32_t) * 8 * maxScenes, st);
     k_hash<<<grid_for(hw.slotEnd), 256, 0, st>>>(b, accTmp);
     cudaMemcpyAsync(out, accTmp + s * 8, 32, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "digest");
+    return synced(s, "digest");
   }
   // mirror: the last fold's digests and chains in host memory, where the fold
   // wrote them (a read of 32 bytes from the device costs 12 us). chainFresh: no
@@ -1627,14 +1668,18 @@ struct World {
   uint32_t* mirror = nullptr;
   bool chainFresh = false;
   bool read_chain(uint32_t s, uint32_t out[8]) {
-    if (!chainFresh) return read_words(b.chain + (size_t)s * 8, out, 32);
-    if (!cuda_ok(cudaStreamSynchronize(st), "chain")) return false;
+    if (!chainFresh) return read_words(s, b.chain + (size_t)s * 8, out, 32);
+    if (!synced(s, "chain")) return false;
     std::memcpy(out, mirror + (size_t)s * 16 + 8, 32);
     return true;
   }
   bool read_words(const void* dsrc, void* out, size_t bytes) {
     cudaMemcpyAsync(out, dsrc, bytes, cudaMemcpyDeviceToHost, st);
     return cuda_ok(cudaStreamSynchronize(st), "read");
+  }
+  // words that scene s's substeps write
+  bool read_words(uint32_t s, const void* dsrc, void* out, size_t bytes) {
+    return read_words(dsrc, out, bytes) && whole(s, "read");
   }
 
   // readDerived's rho column and readNbrN's counts (src/engine.js:4290-4291)
@@ -1647,7 +1692,7 @@ struct World {
                                                  tmpV);
     if (rho) cudaMemcpyAsync(rho, tmpK, (size_t)h.n * 4, cudaMemcpyDeviceToHost, st);
     if (nbr) cudaMemcpyAsync(nbr, tmpV, (size_t)h.n * 4, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "readFields");
+    return synced(s, "readFields");
   }
 
   bool impulse_now(uint32_t s, int32_t cx, int32_t cy, int32_t r, int32_t ix, int32_t iy, uint32_t limit,
@@ -1657,7 +1702,7 @@ struct World {
     k_impulse_now<<<1, 256, 0, st>>>(b, s, ev, hits);
     uint32_t h = 0;
     cudaMemcpyAsync(&h, hits, 4, cudaMemcpyDeviceToHost, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "impulse")) return false;
+    if (!synced(s, "impulse")) return false;
     if (hitsOut) *hitsOut = h;
     return true;
   }
@@ -1797,8 +1842,9 @@ struct World {
       return fail("a transition produced a seal-class row (containment is not built); results past it are not "
                   "the reference's");
     if (e[0] & ERR_BOND_PARTNER) return fail("a bond partner slot exceeds the 17-bit bond word");
-    if (e[0] & ERR_BARRIER)
-      return fail("a grid barrier timed out; results past it are not valid");
+    bool lost = (e[0] & ERR_BARRIER) || gave_up();
+    for (const SceneHost& h : sh) lost = lost || (h.loaded && h.lost);
+    if (lost) return fail("%s", BARRIER_TEXT);
     if (e[0] & ERR_STAGE_TIMEOUT)
       return fail("a tile's staged copy did not complete within the bounded wait; results past it are not valid");
     return true;
@@ -2352,7 +2398,7 @@ struct World {
   // readBodies: scene s's records in the reference's layout (word 29 zero).
   bool read_bodies(uint32_t s, int32_t* out, size_t words, uint32_t* count) {
     std::vector<int32_t> rec, drv;
-    if (!read_records(rec, drv)) return false;
+    if (!read_records(rec, drv) || !whole(s, "readBodies")) return false;
     const uint32_t nb = scene_bodies(s);
     if (count) *count = nb;
     if (!out) return true;
@@ -2371,7 +2417,7 @@ struct World {
     if (!out || words < (size_t)h.n * 2) return fail("readRestOffsets needs n*2 words");
     return h.n == 0 || (cuda_ok(cudaMemcpyAsync(out, b.rest + h.slotBase, (size_t)h.n * 8, cudaMemcpyDeviceToHost, st),
                                 "rest") &&
-                        cuda_ok(cudaStreamSynchronize(st), "rest"));
+                        synced(s, "readRestOffsets"));
   }
   // restoreAuthoringSnapshot's rigid part (src/engine.js:5838-5880).
   bool restore_bodies(uint32_t s, const int32_t* records, uint32_t nb, const int32_t* rest, size_t restWords) {
@@ -2619,7 +2665,7 @@ struct World {
     if (!h.loaded) return fail("checkpoint of a scene that is not loaded");
     if (pool->device != device) return fail("checkpoint pool is on device %d, the engine on %d", pool->device, device);
     if (layoutDirty && !relayout()) return false;
-    if (!pull_params()) return false;
+    if (!pull_params() || !whole(s, "checkpoint")) return false;
     sn_ckpt_pool::Rec* r = nullptr;
     if (!pool->reserve(ckpt_bytes(s), 2, handle, &r)) return fail("%s", pool->err.c_str());
     char* d = pool->base + r->off;
@@ -2672,6 +2718,7 @@ struct World {
     if (r->n != h.n || r->nFluid != h.nFluid)
       return fail("checkpoint holds n = %u, n_fluid = %u; the scene has n = %u, n_fluid = %u", r->n, r->nFluid, h.n,
                   h.nFluid);
+    if (gave_up() && !recover()) return false;
     if (layoutDirty && !relayout()) return false;
     // the clocks, all that the device changes in the parameters, are the
     // checkpoint's: nothing to fetch, and nothing to wait for
@@ -2704,6 +2751,7 @@ struct World {
     hpar[s].bondDirty = r->dirty;
     hpar[s].substep = (uint32_t)r->substeps;
     eventsDirty = true;
+    h.lost = false;
     return push_scene(s);
   }
 
@@ -2741,7 +2789,11 @@ struct sn_batch {
   World w;
 };
 
-static int rc_of(World& w, bool ok) { return ok ? SN_OK : (w.err.find("cuda") != std::string::npos ? SN_E_CUDA : SN_E_INVALID); }
+static int rc_of(World& w, bool ok) {
+  if (ok) return SN_OK;
+  if (w.err.find(BARRIER_TEXT) != std::string::npos) return SN_E_DEVICE;
+  return w.err.find("cuda") != std::string::npos ? SN_E_CUDA : SN_E_INVALID;
+}
 
 extern "C" {
 
@@ -2788,7 +2840,7 @@ int sn_read_state(sn_engine* e, int32_t* out, size_t words) {
   if (!e || !out) return SN_E_INVALID;
   SceneHost& h = e->w.sh[0];
   if (words < (size_t)h.n * 8) { e->w.err = "output buffer too small"; return SN_E_INVALID; }
-  return rc_of(e->w, e->w.read_words(e->w.b.state + (size_t)h.slotBase * 8, out, (size_t)h.n * 32));
+  return rc_of(e->w, e->w.read_words(0u, e->w.b.state + (size_t)h.slotBase * 8, out, (size_t)h.n * 32));
 }
 int sn_read_initial_positions(sn_engine* e, int32_t* out, size_t words, size_t* words_out) {
   if (!e || !out) return SN_E_INVALID;
@@ -2803,7 +2855,7 @@ int sn_read_scratch(sn_engine* e, int32_t* out, size_t words) {
   if (!e || !out) return SN_E_INVALID;
   SceneHost& h = e->w.sh[0];
   if (words < (size_t)h.n * 2) { e->w.err = "output buffer too small"; return SN_E_INVALID; }
-  return rc_of(e->w, e->w.read_words(e->w.b.stacc + h.slotBase, out, (size_t)h.n * 8));
+  return rc_of(e->w, e->w.read_words(0u, e->w.b.stacc + h.slotBase, out, (size_t)h.n * 8));
 }
 int sn_write_state(sn_engine* e, const int32_t* state, const int32_t* scratch, size_t n) {
   if (!e || !state) return SN_E_INVALID;
@@ -2813,7 +2865,7 @@ int sn_read_bonds(sn_engine* e, uint32_t* out, size_t words) {
   if (!e || !out) return SN_E_INVALID;
   SceneHost& h = e->w.sh[0];
   if (words < (size_t)h.nFluid * BOND_CAP) { e->w.err = "output buffer too small"; return SN_E_INVALID; }
-  return rc_of(e->w, e->w.read_words(e->w.b.bond + (size_t)h.slotBase * BOND_CAP, out, (size_t)h.nFluid * BOND_CAP * 4));
+  return rc_of(e->w, e->w.read_words(0u, e->w.b.bond + (size_t)h.slotBase * BOND_CAP, out, (size_t)h.nFluid * BOND_CAP * 4));
 }
 int sn_read_fields(sn_engine* e, int32_t* rho, uint32_t* nbr_count, size_t n) {
   if (!e) return SN_E_INVALID;
@@ -2831,7 +2883,7 @@ int sn_read_cell_start(sn_engine* e, uint32_t* out, size_t words) {
   const ScenePar& S = w.hpar[0];
   if (words < (size_t)h.cellTotal + 1) { w.err = "output buffer too small"; return SN_E_INVALID; }
   std::vector<uint32_t> dev((size_t)w.hw.K + 1);
-  if (!w.read_words(w.b.cellStart, dev.data(), dev.size() * 4)) return rc_of(w, false);
+  if (!w.read_words(0u, w.b.cellStart, dev.data(), dev.size() * 4)) return rc_of(w, false);
   // the reference's layout: row-major cells, each cell's first position in a
   // sort by cell index (a prefix sum of the cells' occupancies)
   const uint32_t ts = S.tileShift, T = 1u << ts;
@@ -2870,12 +2922,12 @@ int sn_check_errors(sn_engine* e) {
 }
 int sn_sync(sn_engine* e) {
   if (!e) return SN_E_INVALID;
-  return rc_of(e->w, e->w.cuda_ok(cudaStreamSynchronize(e->w.st), "sync"));
+  return rc_of(e->w, e->w.sync());
 }
 int sn_get_info(sn_engine* e, sn_info* out) {
   if (!e || !out) return SN_E_INVALID;
   World& w = e->w;
-  if (!w.pull_params()) return SN_E_CUDA;
+  if (!w.pull_params()) return rc_of(w, false);
   SceneHost& h = w.sh[0];
   out->n = h.n;
   out->n_fluid = h.nFluid;
@@ -2889,7 +2941,7 @@ int sn_get_info(sn_engine* e, sn_info* out) {
 int sn_set_formation_clock(sn_engine* e, uint64_t clock, uint32_t dirty) {
   if (!e) return SN_E_INVALID;
   World& w = e->w;
-  if (!w.pull_params()) return SN_E_CUDA;
+  if (!w.pull_params()) return rc_of(w, false);
   w.hpar[0].formClock = (uint32_t)clock;
   w.hpar[0].bondDirty = dirty ? 1u : 0u;
   return rc_of(w, w.push_scene(0) && w.cuda_ok(cudaStreamSynchronize(w.st), "clock"));
@@ -2983,20 +3035,20 @@ int sn_batch_read_state(sn_batch* b, uint32_t id, int32_t* out, size_t words) {
   if (!b || !out || id >= b->w.maxScenes || !b->w.sh[id].loaded) return SN_E_INVALID;
   SceneHost& h = b->w.sh[id];
   if (words < (size_t)h.n * 8) return SN_E_INVALID;
-  return rc_of(b->w, b->w.read_words(b->w.b.state + (size_t)h.slotBase * 8, out, (size_t)h.n * 32));
+  return rc_of(b->w, b->w.read_words(id, b->w.b.state + (size_t)h.slotBase * 8, out, (size_t)h.n * 32));
 }
 int sn_batch_read_scratch(sn_batch* b, uint32_t id, int32_t* out, size_t words) {
   if (!b || !out || id >= b->w.maxScenes || !b->w.sh[id].loaded) return SN_E_INVALID;
   SceneHost& h = b->w.sh[id];
   if (words < (size_t)h.n * 2) return SN_E_INVALID;
-  return rc_of(b->w, b->w.read_words(b->w.b.stacc + h.slotBase, out, (size_t)h.n * 8));
+  return rc_of(b->w, b->w.read_words(id, b->w.b.stacc + h.slotBase, out, (size_t)h.n * 8));
 }
 int sn_batch_write_state(sn_batch* b, uint32_t id, const int32_t* state, const int32_t* scratch, size_t n,
                          uint64_t substep_count, uint64_t formation_clock, uint32_t dirty) {
   if (!b || !state || id >= b->w.maxScenes || !b->w.sh[id].loaded) return SN_E_INVALID;
   World& w = b->w;
   if (!w.write_state(id, state, scratch, n)) return rc_of(w, false);
-  if (!w.pull_params()) return SN_E_CUDA;
+  if (!w.pull_params()) return rc_of(w, false);
   w.sh[id].substeps = substep_count;
   w.hpar[id].formClock = (uint32_t)formation_clock;
   w.hpar[id].bondDirty = dirty ? 1u : 0u;
@@ -3110,6 +3162,14 @@ int sn_batch_set_persistent(sn_batch* b, uint32_t on) {
   b->w.graphValid = false;
   return SN_OK;
 }
+int sn_set_barrier_wait(sn_engine* e, uint64_t cycles) {
+  if (!e) return SN_E_INVALID;
+  return rc_of(e->w, e->w.set_barrier_wait(cycles));
+}
+int sn_batch_set_barrier_wait(sn_batch* b, uint64_t cycles) {
+  if (!b) return SN_E_INVALID;
+  return rc_of(b->w, b->w.set_barrier_wait(cycles));
+}
 int sn_lanes(sn_engine* e, uint32_t out[5]) {
   if (!e || !out) return SN_E_INVALID;
   const auto& c = e->w.lanesCfg;
@@ -3190,7 +3250,7 @@ int sn_batch_ckpt_load(sn_batch* b, uint32_t id, sn_ckpt_pool* p, uint64_t handl
 int sn_batch_get_info(sn_batch* b, uint32_t id, sn_info* out) {
   if (!b || !out || id >= b->w.maxScenes || !b->w.sh[id].loaded) return SN_E_INVALID;
   World& w = b->w;
-  if (!w.pull_params()) return SN_E_CUDA;
+  if (!w.pull_params()) return rc_of(w, false);
   SceneHost& h = w.sh[id];
   out->n = h.n;
   out->n_fluid = h.nFluid;
@@ -3207,7 +3267,7 @@ int sn_batch_check_errors(sn_batch* b) {
 }
 int sn_batch_sync(sn_batch* b) {
   if (!b) return SN_E_INVALID;
-  return rc_of(b->w, b->w.cuda_ok(cudaStreamSynchronize(b->w.st), "sync"));
+  return rc_of(b->w, b->w.sync());
 }
 int sn_batch_last_timing(sn_batch* b, float* ms, uint64_t* launches) {
   if (!b) return SN_E_INVALID;

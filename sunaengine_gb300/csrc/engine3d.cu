@@ -112,6 +112,7 @@ struct Scene3Host {
   int32_t reach = 0;
   int32_t bondK = 0, bondBrk = 0;  // build-defined bonds (sn3_write_bonds)
   bool bonds = false;              // some slot of the scene has a bond row
+  bool lost = false;               // a substep of it was left half done (Engine3::recover)
 };
 
 struct Engine3 {
@@ -163,7 +164,6 @@ struct Engine3 {
                     b.accLast, b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes, fuWords, fuCount, fuLocal};
     for (void* p : ptrs)
       if (p) cudaFree(p);
-    if (fuErrHost) cudaFreeHost(fuErrHost);
     if (mirror) cudaFreeHost(mirror);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -243,13 +243,12 @@ struct Engine3 {
     fuWords = dalloc3<uint32_t>(4 + F3_MAX_GRID, err);
     fuCount = dalloc3<uint32_t>((size_t)maxCells + 2, err);
     fuLocal = dalloc3<uint32_t>((size_t)maxCells + 2, err);
-    if (cudaHostAlloc((void**)&fuErrHost, 4, cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&fuErrDev, fuErrHost, 0) != cudaSuccess)
-      return fail("cudaHostAlloc failed");
-    *fuErrHost = 0u;
-    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)maxScenes * 64, cudaHostAllocMapped), "mirror") ||
+    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)maxScenes * 64 + 4, cudaHostAllocMapped), "mirror") ||
         !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
       return false;
+    memset(mirror, 0, (size_t)maxScenes * 64 + 4);
+    gaveUp = mirror + (size_t)maxScenes * 16;
+    gaveUpDev = b.mirror + (size_t)maxScenes * 16;
     if (!err.empty()) return false;
     {
       std::vector<int2> wg(LUT_N), pg(PLANE_N);
@@ -444,7 +443,8 @@ struct Engine3 {
   // ---- the fused substep of small worlds (fused3d.cuh) ----
   uint32_t* fuWords = nullptr;  // barrier words (2), error word, pad, slice totals
   uint32_t *fuCount = nullptr, *fuLocal = nullptr;  // [maxCells + 2] each
-  uint32_t *fuErrHost = nullptr, *fuErrDev = nullptr;
+  uint32_t *gaveUp = nullptr, *gaveUpDev = nullptr;  // ERR_BARRIER for the host (mapped)
+  long long waitLimit = sn::BARRIER_WAIT_CYCLES;
   bool graphFused = false;
   static constexpr uint32_t F3_SMEM = 216 * 1024;  // dynamic at most; the static arrays take about 6 KB of the 227
   static constexpr uint32_t F3_FIXED = (LUT_N + PLANE_N) * 8;
@@ -468,9 +468,7 @@ struct Engine3 {
     P.local = fuLocal;
     P.totals = fuWords + 4;
     P.tmp = tmpV;
-    P.bar = fuWords;
-    P.err = fuWords + 2;
-    P.errHost = fuErrDev;
+    P.bar = sn::GridBar{fuWords, fuWords + 2, gaveUpDev, waitLimit};
     const auto fn = k3_substep_fused<L>;
     cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F3_SMEM);
     cudaLaunchConfig_t cfg = {};
@@ -494,11 +492,35 @@ struct Engine3 {
     else launch_fused_as<2>();
     launchesPerSubstep = 1;
   }
-  // The error a fused launch left, after the stream was waited for.
-  bool synced(const char* what) {
-    if (!cuda_ok(cudaStreamSynchronize(st), what)) return false;
-    if (*(volatile uint32_t*)fuErrHost)
-      return fail("%s: a grid barrier timed out; results past it are not valid", what);
+  // A launch whose grid barrier ran out leaves its substep half done in every
+  // scene, and its counts behind; the fused launches after it return at once.
+  // From then on no word of these scenes is given out until they are loaded
+  // again or take a keyframe's words. (gave_up is looked at once the stream has
+  // been waited for.)
+  bool gave_up() const { return *(volatile uint32_t*)gaveUp != 0u; }
+  bool whole(uint32_t s, const char* what) {
+    return !gave_up() && !sh[s].lost ? true : fail("%s: %s", what, sn::BARRIER_TEXT);
+  }
+  bool synced(uint32_t s, const char* what) { return cuda_ok(cudaStreamSynchronize(st), what) && whole(s, what); }
+  bool sync() {
+    return cuda_ok(cudaStreamSynchronize(st), "sync") && (!gave_up() ? true : fail("sync: %s", sn::BARRIER_TEXT));
+  }
+  // The world can be stepped again; the scenes that were in it are lost.
+  bool recover() {
+    if (!cuda_ok(cudaStreamSynchronize(st), "recover")) return false;
+    accFresh = chainFresh = false;
+    for (Scene3Host& h : sh) h.lost = h.lost || (h.used && h.loaded);
+    const bool ok = cuda_ok(cudaMemsetAsync(fuWords, 0, 12, st), "recover") &&
+                    cuda_ok(cudaMemsetAsync(fuCount, 0, ((size_t)maxCells + 2) * 4, st), "recover") &&
+                    cuda_ok(cudaMemsetAsync(b.acc, 0, (size_t)maxScenes * 32, st), "recover") &&
+                    cuda_ok(cudaStreamSynchronize(st), "recover");
+    if (ok) *(volatile uint32_t*)gaveUp = 0u;
+    return ok;
+  }
+  bool set_barrier_wait(uint64_t cycles) {
+    if (cycles > 1ull << 40) return fail("a barrier waits 2^40 cycles at most");
+    waitLimit = (long long)cycles;
+    graphValid = false;
     return true;
   }
   void launch_one(bool fused = false) {
@@ -526,6 +548,7 @@ struct Engine3 {
   bool step(uint32_t count) {
     if (!any_loaded()) return fail("step() called before a scene was loaded");
     if (count == 0) return true;
+    if (gave_up()) return fail("step: %s", sn::BARRIER_TEXT);
     if (layoutDirty && !relayout()) return false;
     if (anyStir && !upload_phase()) return false;
     const bool fused = fused_fits();
@@ -654,12 +677,6 @@ struct Engine3 {
                                            0xa4093822u, 0x299f31d0u, 0x082efa98u, 0xec4e6c89u};
     cudaMemcpyAsync(b.chain + (size_t)s * 8, CHAIN_INIT, 32, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b.acc + (size_t)s * 8, 0, 32, st);
-    if (*(volatile uint32_t*)fuErrHost) {  // a launch that gave up leaves its counts behind
-      cudaMemsetAsync(fuWords, 0, 12, st);
-      cudaMemsetAsync(fuCount, 0, ((size_t)maxCells + 2) * 4, st);
-      if (!cuda_ok(cudaStreamSynchronize(st), "load")) return false;
-      *fuErrHost = 0u;
-    }
     if (!clear_bonds(s)) return false;
     h.n = sc->n;
     h.gx = sc->gx;
@@ -670,7 +687,10 @@ struct Engine3 {
     h.substeps = 0;
     h.loaded = true;
     layoutDirty = true;
-    return cuda_ok(cudaStreamSynchronize(st), "load");
+    bool ok = cuda_ok(cudaStreamSynchronize(st), "load");
+    if (gave_up()) ok = recover() && ok;
+    h.lost = false;
+    return ok;
   }
 
   // A device buffer the scene loads and bond writes upload into before their
@@ -826,7 +846,7 @@ struct Engine3 {
   bool digest(uint32_t s, uint32_t out[8]) {
     if (!check_scene(s)) return false;
     if (accFresh && !layoutDirty) {
-      if (!synced("digest")) return false;
+      if (!synced(s, "digest")) return false;
       memcpy(out, mirror + (size_t)s * 16, 32);
       return true;
     }
@@ -834,7 +854,7 @@ struct Engine3 {
     cudaMemsetAsync(accTmp, 0, sizeof(uint32_t) * 8 * maxScenes, st);
     k3_hash<<<grid_for(hw.slotEnd), 256, 0, st>>>(b, accTmp);
     cudaMemcpyAsync(out, accTmp + s * 8, 32, cudaMemcpyDeviceToHost, st);
-    return synced("digest");
+    return synced(s, "digest");
   }
 
   // chain() (3d/app.js:717-744): stripe words on the device, the 8-lane fold
@@ -844,7 +864,7 @@ struct Engine3 {
     uint32_t words[256];
     k3_fnv<<<1, 256, 0, st>>>(b.state, sh[s].slotBase, sh[s].n, fnvBuf);
     cudaMemcpyAsync(words, fnvBuf, sizeof(words), cudaMemcpyDeviceToHost, st);
-    if (!synced("fnv")) return false;
+    if (!synced(s, "fnv")) return false;
     for (uint32_t L = 0; L < 8; ++L) out[L] = 2166136261u ^ (L * 0x9e3779b9u);
     for (uint32_t k = 0; k < 256; ++k)
       for (uint32_t L = 0; L < 8; ++L) {
@@ -857,12 +877,12 @@ struct Engine3 {
   bool chain(uint32_t s, uint32_t out[8]) {
     if (!check_scene(s)) return false;
     if (chainFresh) {
-      if (!synced("chain")) return false;
+      if (!synced(s, "chain")) return false;
       memcpy(out, mirror + (size_t)s * 16 + 8, 32);
       return true;
     }
     cudaMemcpyAsync(out, b.chain + (size_t)s * 8, 32, cudaMemcpyDeviceToHost, st);
-    return synced("chain");
+    return synced(s, "chain");
   }
 
   bool read_state(uint32_t s, int32_t* out, size_t words) {
@@ -870,7 +890,7 @@ struct Engine3 {
     size_t need = (size_t)sh[s].n * 8;
     if (!out || words < need) return fail("read_state needs %zu words", need);
     cudaMemcpyAsync(out, b.state + (size_t)sh[s].slotBase * 8, need * 4, cudaMemcpyDeviceToHost, st);
-    return synced("read_state");
+    return synced(s, "read_state");
   }
 
   // A keyframe: the state words fully determine every later substep (the
@@ -889,6 +909,8 @@ struct Engine3 {
       cudaMemcpyAsync(b.state + (size_t)h.slotBase * 8, state, (size_t)n * 32, cudaMemcpyHostToDevice, st);
     if (chainIn) cudaMemcpyAsync(b.chain + (size_t)s * 8, chainIn, 32, cudaMemcpyHostToDevice, st);
     if (!cuda_ok(cudaStreamSynchronize(st), "write_state")) return false;
+    if (gave_up() && !recover()) return false;
+    if (chainIn) h.lost = false;  // its words, its clock and its chain are the caller's
     h.n = n;
     h.substeps = substeps;
     layoutDirty = true;
@@ -900,6 +922,7 @@ struct Engine3 {
   bool ckpt_save(uint32_t s, sn_ckpt_pool* pool, uint64_t* handle) {
     if (!check_scene(s)) return false;
     if (pool->device != device) return fail("checkpoint pool is on device %d, the engine on %d", pool->device, device);
+    if (!whole(s, "checkpoint")) return false;
     const Scene3Host& h = sh[s];
     sn_ckpt_pool::Rec* r = nullptr;
     if (!pool->reserve(ckpt_bytes(s), 3, handle, &r)) return fail("%s", pool->err.c_str());
@@ -925,6 +948,7 @@ struct Engine3 {
     if (!r || r->kind != 3) return fail("no 3D checkpoint %llu in the pool", (unsigned long long)handle);
     Scene3Host& h = sh[s];
     if (r->n > h.cap) return fail("checkpoint holds %u particles, above this scene's capacity %u", r->n, h.cap);
+    if (gave_up() && !recover()) return false;
     cudaStreamWaitEvent(st, r->done, 0);
     const char* d = pool->base + r->off;
     bool ok = cuda_ok(cudaMemcpyAsync(b.state + (size_t)h.slotBase * 8, d, (size_t)r->n * 32, cudaMemcpyDeviceToDevice,
@@ -942,6 +966,7 @@ struct Engine3 {
     if (!layoutDirty &&
         !cuda_ok(cudaMemcpyAsync(b.scenes + s, &hpar[s], sizeof(Scene3), cudaMemcpyHostToDevice, st), "load"))
       return false;
+    h.lost = false;
     return true;
   }
 
@@ -960,6 +985,7 @@ struct sn3_engine {
 
 static int rc3(Engine3& w, bool ok) {
   if (ok) return SN_OK;
+  if (w.err.find(sn::BARRIER_TEXT) != std::string::npos) return SN_E_DEVICE;
   return w.err.rfind("cuda", 0) == 0 ? SN_E_CUDA : SN_E_INVALID;
 }
 
@@ -1061,7 +1087,7 @@ int sn3_debug_counters(sn3_engine* e, uint32_t out[16]) {
 }
 int sn3_sync(sn3_engine* e) {
   if (!e) return SN_E_INVALID;
-  return rc3(e->w, e->w.synced("sync"));
+  return rc3(e->w, e->w.sync());
 }
 int sn3_get_info(sn3_engine* e, uint32_t scene, sn3_info* out) {
   if (!e || !out) return SN_E_INVALID;
@@ -1088,6 +1114,10 @@ int sn3_profile_substep(sn3_engine* e, uint32_t reps, float* ms, uint32_t max_ph
   return rc3(e->w, e->w.profile(reps, ms, max_phases, n_phases));
 }
 
+int sn3_set_barrier_wait(sn3_engine* e, uint64_t cycles) {
+  if (!e) return SN_E_INVALID;
+  return rc3(e->w, e->w.set_barrier_wait(cycles));
+}
 int sn3_ckpt_bytes(sn3_engine* e, uint32_t scene, size_t* bytes) {
   if (!e || !bytes) return SN_E_INVALID;
   if (!e->w.check_scene(scene)) return SN_E_INVALID;

@@ -44,7 +44,7 @@ struct FusedPar {
   uint32_t bodies;   // rigid bodies, one CTA each in turn
   uint32_t* count;   // [K] cell counts, zero between launches
   uint32_t* tmp;     // slots by cell in arrival order
-  uint32_t* bar;     // [2] barrier arrivals and finished CTAs, zero between launches
+  GridBar bar;       // count[0] barrier arrivals, count[1] finished CTAs, zero between launches
 };
 
 // Neighbour access of an owned particle: its list row and the kernel tables in
@@ -163,9 +163,9 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   if constexpr (RIG) {
     const bool member = on && (info & INFO_RIGID);
     if (member) b.predSlot[slot] = pred;
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
     for (uint32_t k = cta; k < P.bodies; k += G) rigid_step_body<false, FU_T, false>(b, k, rsum, f);
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
     if (member) pred = b.predSlot[slot];
   }
   if (on) {
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     scol[tid] = make_int2(matw(b, tid, M_eps), matw(b, tid, M_dpMax));
     if (RIG) sfric[tid] = friction_row(b, tid);
   }
-  if (!grid_wait(P.bar, b.err, target)) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- cell ranges (every CTA its own copy), slots to their cells
   for (uint32_t k = tid; k < K; k += FU_T) X[k] = __ldcg(P.count + k);
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   const bool crowded = cta_scan(X, K, ws) > CELL_BIG;
   for (uint32_t k = cta * FU_T + tid; k <= K; k += G * FU_T) b.cellStart[k] = X[k];
   if (on) P.tmp[X[key] + arrival] = slot;
-  if (!grid_wait(P.bar, b.err, target)) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- canonical order inside the cell, working set into sorted space
   for (uint32_t k = cta * FU_T + tid; k < K; k += G * FU_T) P.count[k] = 0u;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     // containStress has work: a held fluid particle
     raise_work(b, 6, !(info & INFO_BOUNDARY) && (info & INFO_PINNED));
   }
-  if (!grid_wait(P.bar, b.err, target)) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- the owned share of each colour class
   // One contiguous share, which has the best of L1, but in worlds with bodies
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       box.w = __reduce_max_sync(0xffffffffu, box.w);
       if (lane == 0) b.CB[k] = box;
     }
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
   }
   __syncthreads();
 
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     }
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
-      if (!grid_wait(P.bar, b.err, target)) return;
+      if (!grid_wait(P.bar, target)) return;
       nb.cut = c == 0 ? lo4[0] : c == 1 ? lo4[1] : c == 2 ? lo4[2] : lo4[3];
       const uint32_t i0 = c == 0 ? own[0] : c == 1 ? own[1] : c == 2 ? own[2] : own[3];
       const uint32_t i1 = c == 0 ? own[1] : c == 1 ? own[2] : c == 2 ? own[3] : own[4];
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       }
     }
     swap_records(b);
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
     if (fric) {
       const NbrOwned nf{b.PL, rows, swg, sca, 0u, 0u};
       // beside bodies few rows rub: their lists over as many lanes as a colour pass
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
         if (!RIG || __any_sync(0xffffffffu, valid))
           friction_particle<false, LF>(b, nf, valid, pOf[r], r, tid & (LF - 1), f);
       }
-      if (!grid_wait(P.bar, b.err, target)) return;
+      if (!grid_wait(P.bar, target)) return;
       for (uint32_t i = tid; i < own[4]; i += FU_T) {
         int4 me = rec[i];
         const uint32_t inf = (uint32_t)me.w, m = inf & INFO_MAT;
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     if constexpr (RIG)
       for (uint32_t k = cta; k < P.bodies; k += G) rigid_solve_body<false, FU_T>(b, k, P.seal != 0u, rsum, f);
     if (RIG || fric) {
-      if (!grid_wait(P.bar, b.err, target)) return;
+      if (!grid_wait(P.bar, target)) return;
     }
     if constexpr (RIG) {
       for (uint32_t i = tid; i < own[4]; i += FU_T) {
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   const NbrOwned nb{b.PL, rows, swg, sca, 0u, 0u};
   if (P.seal && !cutLists) {
     for (uint32_t i = tid; i < own[4]; i += FU_T) contain_particle(b, nb, pOf[i], i, f);
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
   }
   for (uint32_t i = tid / L;; i += FU_T / L) {
     if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
     const uint32_t r = valid ? i : 0u;
     post1_particle<false, L>(b, nb, smat1, valid, pOf[r], r, sub, f);
   }
-  if (!grid_wait(P.bar, b.err, target)) return;
+  if (!grid_wait(P.bar, target)) return;
   for (uint32_t i = tid / L;; i += FU_T / L) {
     if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
     const bool valid = i < own[4];
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   const bool stress = P.seal && *(volatile uint32_t*)(b.work + 6) != 0u;
   const bool forming = P.bonds && *(volatile uint32_t*)(b.work + 5) != 0u;
   if (RIG || stress) {
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
   }
   if (stress) {
     const uint32_t subC = tid & (LC - 1);
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       if (__any_sync(0xffffffffu, held)) contain_stress_slot<false, LC>(b, nb, held, b.sslot[pOf[r]], r, subC, f);
     }
     // a burst takes a member out of its body: the marks below see it
-    if (RIG && !grid_wait(P.bar, b.err, target)) return;
+    if (RIG && !grid_wait(P.bar, target)) return;
   }
   if constexpr (RIG) {
     const uint32_t subC = tid & (LC - 1);
@@ -434,19 +434,19 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       const bool leaves = rigid_leaves<false, LC>(b, nb, member, sl, p, r, subC, tag, f);
       if (member && subC == 0) b.rmark[sl] = leaves ? 1u : 0u;
     }
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
     for (uint32_t k = cta; k < P.bodies; k += G) rigid_member_body<false, FU_T, true>(b, k, rsum, f);
-    if (!forming && !grid_wait(P.bar, b.err, target)) return;
+    if (!forming && !grid_wait(P.bar, target)) return;
   }
   if (forming) {
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
     for (uint32_t i = tid / L;; i += FU_T / L) {
       if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
       const bool valid = i < own[4];
       const uint32_t r = valid ? i : 0u;
       form1_particle<false, L>(b, nb, valid, pOf[r], r, sub, f);
     }
-    if (!grid_wait(P.bar, b.err, target)) return;
+    if (!grid_wait(P.bar, target)) return;
     const bool live = *(volatile uint32_t*)(b.work + 4) != 0u;
     for (uint32_t i = tid / L;; i += FU_T / L) {
       if (__shfl_sync(0xffffffffu, i, 0) >= own[4]) break;
@@ -479,13 +479,13 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   __syncthreads();
   if (tid == 0) {
     __threadfence();
-    lastCta = atomicAdd(P.bar + 1, 1u) == G - 1 ? 1u : 0u;
+    lastCta = atomicAdd(P.bar.count + 1, 1u) == G - 1 ? 1u : 0u;
     __threadfence();
   }
   __syncthreads();
   if (!lastCta) return;
   for (uint32_t s = tid; s < b.world->numScenes; s += FU_T) fold_scene(b, s, P.chain != 0u);
-  if (tid < 2) P.bar[tid] = 0u;
+  if (tid < 2) P.bar.count[tid] = 0u;
 }
 
 }  // namespace d2

@@ -37,9 +37,7 @@ struct Fused3Par {
   uint32_t* local;    // [K] cell starts inside their slice
   uint32_t* totals;   // [grid] particles of each slice
   uint32_t* tmp;      // slots by cell in arrival order
-  uint32_t* bar;      // [2] barrier arrivals and finished CTAs, zero between launches
-  uint32_t* err;      // device error word
-  uint32_t* errHost;  // the same for the host (mapped)
+  GridBar bar;        // count[0] barrier arrivals, count[1] finished CTAs, zero between launches
 };
 
 // Particle s's list by L lanes (a warp calls it together; `valid` false for a lane
@@ -108,12 +106,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   const uint32_t K = b.world->K;
   uint32_t target = 0;
   // an earlier launch gave up: its counts are not zero, and the results are void
-  if (*(volatile uint32_t*)P.err & ERR_BARRIER) return;
-  auto sync = [&]() -> bool {
-    if (grid_wait(P.bar, P.err, target)) return true;
-    if (tid == 0) *(volatile uint32_t*)P.errHost = ERR_BARRIER;
-    return false;
-  };
+  if (*(volatile uint32_t*)P.bar.err & ERR_BARRIER) return;
 
   // ---- predict and cell counts: one slot per thread, warps dealt round the CTAs
   const uint32_t slot = ((tid >> 5) * G + cta) * 32u + lane;
@@ -131,7 +124,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   }
   for (uint32_t k = tid; k < (uint32_t)LUT_N; k += FU_T) swg[k] = __ldg(b.WG + k);
   if (tid < (uint32_t)PLANE_N) spg[tid] = __ldg(b.PG + tid);
-  if (!sync()) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- cell starts inside this CTA's slice of the cells
   const uint32_t c0 = min(cta * P.slice, K), cn = min(P.slice, K - c0);
@@ -140,7 +133,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   cta_scan(X, cn, ws);
   if (tid < cn) P.local[c0 + tid] = X[tid];
   if (tid == 0) P.totals[cta] = X[cn];
-  if (!sync()) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- every slice's base; slots to their cells
   if (tid < G) bases[tid] = __ldcg(P.totals + tid);
@@ -152,7 +145,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   }
   if (cta == 0 && tid == 0) b.cellStart[K] = bases[G];
   if (on) P.tmp[bases[key / P.slice] + __ldcg(P.local + key) + arrival] = slot;
-  if (!sync()) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- canonical order inside the cell, working set into sorted space
   if (on) {
@@ -164,7 +157,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
     b.inv[slot] = p;
     b.sslot[p] = slot;
   }
-  if (!sync()) return;
+  if (!grid_wait(P.bar, target)) return;
 
   // ---- the owned share; neighbour lists
   const uint32_t nAct = bases[G], per = (nAct + G - 1) / G;
@@ -213,7 +206,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
       lamS[r] = lam;
       b.PL[p0 + r] = make_int4(me.x, me.y, me.z, lam);
     }
-    if (!sync()) return;
+    if (!grid_wait(P.bar, target)) return;
     const bool last = it + 1 == P.iters;
     for (uint32_t i = tid / L;; i += FU_T / L) {
       if (__shfl_sync(0xffffffffu, i, 0) >= own) break;
@@ -248,7 +241,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
     int4* t = cur;
     cur = nxt;
     nxt = t;
-    if (!last && !sync()) return;
+    if (!last && !grid_wait(P.bar, target)) return;
   }
 
   // ---- integrate (3d/sim3d.wgsl:542-552), digest and chain
@@ -276,13 +269,13 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   __syncthreads();
   if (tid == 0) {
     __threadfence();
-    lastCta = atomicAdd(P.bar + 1, 1u) == G - 1 ? 1u : 0u;
+    lastCta = atomicAdd(P.bar.count + 1, 1u) == G - 1 ? 1u : 0u;
     __threadfence();
   }
   __syncthreads();
   if (!lastCta) return;
   for (uint32_t s = tid; s < b.world->numScenes; s += FU_T) fold_scene3(b, s, P.chain != 0u);
-  if (tid < 2) P.bar[tid] = 0u;
+  if (tid < 2) P.bar.count[tid] = 0u;
 }
 
 }  // namespace d3

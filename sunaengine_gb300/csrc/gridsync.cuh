@@ -25,23 +25,34 @@ inline cudaError_t refresh_graph(cudaGraph_t fresh, cudaGraph_t& graph, cudaGrap
 constexpr int FU_T = 1024;  // threads of a fused substep's CTA, one CTA to an SM
 constexpr uint32_t ERR_BARRIER = 8u;
 constexpr long long BARRIER_WAIT_CYCLES = 1ll << 31;  // about a second
+constexpr char BARRIER_TEXT[] = "a grid barrier timed out; results past it are not valid";
+
+// The barrier of a cooperative launch: the arrivals' word (zero when the launch
+// begins), where a wait that ran out is reported on the device and to the host
+// (mapped memory), and how long a CTA waits.
+struct GridBar {
+  uint32_t *count, *err, *errHost;
+  long long limit;
+};
 
 // Grid barrier of a cooperative launch: `target` counts the arrivals every CTA
-// waits for (monotonic over the launch). A CTA that waits longer than
-// BARRIER_WAIT_CYCLES raises ERR_BARRIER; false sends the whole CTA out.
-__device__ __forceinline__ bool grid_wait(uint32_t* bar, uint32_t* err, uint32_t& target) {
+// waits for (monotonic over the launch). A CTA that waits longer than the limit
+// raises ERR_BARRIER; false sends the whole CTA out. Nobody passes a barrier that
+// some CTA has not reached, so the others run out at the next one at the latest.
+__device__ __forceinline__ bool grid_wait(const GridBar& bar, uint32_t& target) {
   __syncthreads();
   int bad = 0;
   target += gridDim.x;
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar.count) : "memory");
     const long long t0 = clock64();
     for (;;) {
       uint32_t v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar.count) : "memory");
       if ((int32_t)(v - target) >= 0) break;
-      if (clock64() - t0 > BARRIER_WAIT_CYCLES) {
-        atomicOr(err, ERR_BARRIER);
+      if (clock64() - t0 > bar.limit) {
+        atomicOr(bar.err, ERR_BARRIER);
+        *(volatile uint32_t*)bar.errHost = ERR_BARRIER;
         bad = 1;
         break;
       }

@@ -1744,55 +1744,27 @@ __global__ void __launch_bounds__(256) k_apply_fric(Bufs b) {
 // colour passes and (when some particle has a friction or bond row this
 // substep) friction and applyFric, for worlds with no rigid body (rigidSolve
 // keeps the per-phase launches), the phases separated by grid barriers
-// instead of kernel boundaries. The barrier counts arrivals monotonically in bar[0] (zeroed
-// before each launch) and releases generation g by writing g + 1 to bar[1];
-// a CTA that waits longer than BARRIER_WAIT_CYCLES raises ERR_BARRIER and the
-// kernel returns (its results are then not valid; sn_check_errors reports it).
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t* err, uint32_t& gen) {
-  __shared__ uint32_t okS;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    okS = 1u;
-    __threadfence();
-    const uint32_t target = gridDim.x * (gen + 1u);
-    if (atomicAdd(bar, 1u) + 1u == target) {
-      atomicExch(bar + 1, gen + 1u);
-    } else {
-      const long long t0 = clock64();
-      while (*(volatile uint32_t*)(bar + 1) <= gen) {
-        if (clock64() - t0 > BARRIER_WAIT_CYCLES) {
-          atomicOr(err, ERR_BARRIER);
-          okS = 0u;
-          break;
-        }
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  gen += 1u;
-  return okS != 0u;
-}
+// (grid_wait) instead of kernel boundaries.
 template <bool DBG, int L>
-__global__ void __launch_bounds__(256, 8) k_iters_persistent(Bufs b, uint32_t iters, uint32_t* bar) {
+__global__ void __launch_bounds__(256, 8) k_iters_persistent(Bufs b, uint32_t iters, GridBar bar) {
   Flags<DBG> f{b.dbg};
-  uint32_t gen = 0;
+  uint32_t target = 0;
   for (uint32_t it = 0; it < iters; ++it) {
     solveA_all<DBG, L>(b, it + 1 == iters ? 1 : 0, f);
     for (int c = 0; c < 4; ++c) {
-      if (!grid_barrier(bar, b.err, gen)) return;
+      if (!grid_wait(bar, target)) return;
       colour_all<DBG, L>(b, c, f);
     }
     swap_records(b);
     // friction and applyFric, when some particle has a friction or bond row
     // this substep (the flag is the same for every CTA)
     if (*(volatile uint32_t*)b.work != 0u) {
-      if (!grid_barrier(bar, b.err, gen)) return;
+      if (!grid_wait(bar, target)) return;
       friction_all<DBG, L>(b, f);
-      if (!grid_barrier(bar, b.err, gen)) return;
+      if (!grid_wait(bar, target)) return;
       apply_fric_all<DBG>(b, f);
     }
-    if (it + 1 < iters && !grid_barrier(bar, b.err, gen)) return;
+    if (it + 1 < iters && !grid_wait(bar, target)) return;
   }
 }
 

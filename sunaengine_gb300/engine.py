@@ -599,6 +599,11 @@ class Engine:
         self._check(self._lib.sn_set_persistent(self._h, 1 if on else 0), 'setPersistent')
         return self
 
+    def set_barrier_wait(self, cycles: int):
+        """How long a grid barrier waits, in SM cycles (see sn_set_barrier_wait)."""
+        self._check(self._lib.sn_set_barrier_wait(self._h, int(cycles)), 'setBarrierWait')
+        return self
+
     def profile_substep(self, reps: int = 3) -> np.ndarray:
         """Mean device ms per kernel phase over `reps` real substeps (profileSubstep)."""
         out = np.zeros(64, np.float32)
@@ -880,6 +885,11 @@ class Batch:
     def set_persistent(self, on: bool = True):
         """The solver iterations as one persistent cooperative kernel (sn_batch_set_persistent)."""
         self._check(self._lib.sn_batch_set_persistent(self._h, 1 if on else 0), 'setPersistent')
+        return self
+
+    def set_barrier_wait(self, cycles: int):
+        """How long a grid barrier waits, in SM cycles (see sn_set_barrier_wait)."""
+        self._check(self._lib.sn_batch_set_barrier_wait(self._h, int(cycles)), 'setBarrierWait')
         return self
 
     # device keyframes (sn_batch_ckpt_*): see checkpoints.CheckpointPool

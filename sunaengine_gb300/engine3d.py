@@ -234,6 +234,11 @@ class Engine3D:
         self._check(self._lib.sn3_last_timing(self.h, ctypes.byref(ms), ctypes.byref(launches)), 'last_timing')
         return float(ms.value), int(launches.value)
 
+    def set_barrier_wait(self, cycles: int):
+        """How long a grid barrier waits, in SM cycles (see sn_set_barrier_wait)."""
+        self._check(self._lib.sn3_set_barrier_wait(self.h, int(cycles)), 'set_barrier_wait')
+        return self
+
     def profile_substep(self, reps: int = 10):
         ms = np.zeros(64, np.float32)
         n = ctypes.c_uint32()
