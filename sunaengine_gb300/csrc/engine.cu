@@ -492,7 +492,7 @@ struct World {
     std::memcpy(hauth, hmats, sizeof(hauth));
     matCount = authoredCount = o->mat_count;
     tablesOk = tables_in_range(o->luts);
-    inRange = tablesOk && rows_in_range(hmats, matCount);
+    rowsOk = rows_in_range(hmats, matCount);
     for (uint32_t m = 0; m < matCount; ++m) {
       const int32_t* r = hmats + m * MAT_WORDS;
       if (r[M_eps] < 32768) return fail("mats[%u].eps < 32768", m);
@@ -1097,14 +1097,24 @@ struct World {
     else
       k_nbr<DBG, L, false><<<grid_occ((const void*)k_nbr<DBG, L, false>, (uint64_t)hw.nAct * L), 256, 0, st>>>(b);
   }
+  template <bool DBG, int L, bool WIDE>
+  void launch_post1_as() {
+    k_post1<DBG, L, WIDE><<<grid_occ((const void*)k_post1<DBG, L, WIDE>, (uint64_t)hw.nAct * L), 256, 0, st>>>(b);
+  }
   template <bool DBG, int L>
   void launch_post1() {
-    k_post1<DBG, L><<<grid_occ((const void*)k_post1<DBG, L>, (uint64_t)hw.nAct * L), 256, 0, st>>>(b);
+    if (DBG || rowsOk) launch_post1_as<DBG, L, false>();
+    else launch_post1_as<false, L, true>();
+  }
+  template <bool DBG, bool HASH, int L, bool WIDE>
+  void launch_post2_as(int formFlags) {
+    k_post2<DBG, HASH, L, WIDE><<<grid_occ((const void*)k_post2<DBG, HASH, L, WIDE>, (uint64_t)hw.nAct * L), 256, 0,
+                                  st>>>(b, formFlags);
   }
   template <bool DBG, bool HASH, int L>
   void launch_post2(int formFlags) {
-    k_post2<DBG, HASH, L><<<grid_occ((const void*)k_post2<DBG, HASH, L>, (uint64_t)hw.nAct * L), 256, 0, st>>>(
-        b, formFlags);
+    if (DBG || rowsOk) launch_post2_as<DBG, HASH, L, false>(formFlags);
+    else launch_post2_as<false, HASH, L, true>(formFlags);
   }
 #define SN_LANES(LV, CALL)      \
   switch (LV) {                 \
@@ -1152,9 +1162,9 @@ struct World {
     return true;
   }
   uint32_t* fuCount = nullptr;  // [keyCap] cell counts, zero between launches
-  // the tables and every row lie in the ranges the release kernels are built
-  // for; else the debug kernels, which assume none, run
-  bool inRange = true, tablesOk = true;
+  // the tables, and every row, lie in the ranges the release kernels are built
+  // for; else the debug kernels run, or for rows alone the WIDE post sweeps
+  bool tablesOk = true, rowsOk = true;
   bool graphFused = false;      // what the captured graph launches, and the
   uint32_t graphOwn = 0;        // particles a CTA it was sized for
   // One past the last slot that can hold an active particle.
@@ -1178,7 +1188,7 @@ struct World {
   // slot a thread, the cell ranges, the owned particles' lists).
   bool fused_fits() const {
     const uint64_t G = (uint64_t)numSMs;
-    return !debug && inRange && !staged && !persistent && autoLanes && hw.nAct > 0 &&
+    return !debug && tablesOk && rowsOk && !staged && !persistent && autoLanes && hw.nAct > 0 &&
            slots_used() <= G * FU_T && fused_own() <= fused_own_cap();
   }
   template <int L, int LC, bool RIG>
@@ -1508,7 +1518,7 @@ struct World {
 
   void launch_one(bool fused = false) {
     if (fused) launch_fused();
-    else if (debug || !inRange) launch_substep<true>();
+    else if (debug || !tablesOk) launch_substep<true>();
     else launch_substep<false>();
   }
 
@@ -2505,7 +2515,7 @@ struct World {
   // baked from its ramp, grav scaled by the world gravity. `row` may be the
   // next free row (the table grows) or an existing row past the authored ones.
   bool upload_mats(uint32_t lo, uint32_t hi) {
-    inRange = tablesOk && rows_in_range(hmats, matCount);
+    rowsOk = rows_in_range(hmats, matCount);
     if (hi <= lo) return true;
     graphValid = false;
     accFresh = false;

@@ -107,6 +107,19 @@ __device__ __forceinline__ int32_t mulc(int32_t a, int32_t b, int32_t lo, int32_
   }
 }
 
+// mulf and mulfc where the operands' bounds hold (WIDE false), the forms that need
+// none where they do not.
+template <bool WIDE, int S, bool DBG>
+__device__ __forceinline__ int32_t mulw(int32_t a, int32_t b, const Flags<DBG>& f) {
+  if constexpr (WIDE) return mul<S>(a, b, f);
+  else return mulf<S>(a, b, f);
+}
+template <bool WIDE, int S, bool DBG>
+__device__ __forceinline__ int32_t mulwc(int32_t a, int32_t b, int32_t lo, int32_t hi, const Flags<DBG>& f) {
+  if constexpr (WIDE) return mulc<S>(a, b, lo, hi, f);
+  else return mulfc<S>(a, b, lo, hi, f);
+}
+
 template <bool DBG>
 __device__ __forceinline__ int32_t add_sat(int32_t a, int32_t b, const Flags<DBG>& f) {
   int32_t s = wadd(a, b);

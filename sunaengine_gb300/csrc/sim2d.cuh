@@ -36,11 +36,15 @@
 // gradient term is < 2^19; |lambda| <= 2^22; |vel| <= 2^16; K_ij <= 2^18;
 // |T| <= 2^29; a gradient |G d| >> 26 is below
 // 2^15 and |C d| >> 22, |A d| >> 22 below 2^17 (tables_in_range); a normal sum is
-// below 2^24; |gammaCoh| <= 2^19 and |gammaCur| < 2^11 (rows_in_range). Under
-// these bounds every per-pair product below either fits in i32 after its shift
-// (mulf) or is clamped at once into an i32 range (mulc). The host checks the
-// tables and rows it is given and runs the debug build's kernels, which need
-// none of this, where they lie outside.
+// below 2^24; |gammaCoh| <= 2^19, |gammaCur| < 2^11, |xsph| and |adhesion| <= 2^22,
+// |cond| <= 2^17 and |corrode| <= 2^24 (rows_in_range). Under these bounds every
+// per-pair product below either fits in i32 after its shift (mulf) or is clamped
+// at once into an i32 range (mulc). The host checks what it is given. With a row
+// outside, the two sweeps that read rows' words (post1, post2) run in a form that
+// needs no bound on them (WIDE), in the per-phase launches: us a substep with every
+// row inside / an unused one outside, 262 k particles 441 / 470, 40 k 128 / 209 and
+// 4 k 86 / 149 (one fused launch inside). With tables outside (no shipped ones are)
+// the debug build's kernels run, which need none of this.
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -134,8 +138,13 @@ inline bool tables_in_range(const int32_t* luts) {
 }
 inline bool rows_in_range(const int32_t* mats, uint32_t count) {
   for (uint32_t m = 0; m < count; ++m) {
-    const int32_t coh = mats[m * MAT_WORDS + M_gammaCoh], cur = mats[m * MAT_WORDS + M_gammaCur];
-    if (coh > 1 << 19 || coh < -(1 << 19) || cur > 2047 || cur < -2047) return false;
+    const auto within = [&](int word, int32_t most) {
+      const int32_t v = mats[m * MAT_WORDS + word];
+      return v <= most && v >= -most;
+    };
+    if (!within(M_gammaCoh, 1 << 19) || !within(M_gammaCur, 2047) || !within(M_xsph, 1 << 22) ||
+        !within(M_adhesion, 1 << 22) || !within(M_cond, 1 << 17) || !within(M_corrode, 1 << 24))
+      return false;
   }
   return true;
 }
@@ -1779,7 +1788,7 @@ __device__ __forceinline__ void post1_mats(const Bufs& b, int4* smat) {
 }
 // One particle (a warp calls it together; `valid` false for a lane group with
 // none): p its sorted index, `row` its list in nb.
-template <bool DBG, int L, class NB>
+template <bool DBG, int L, bool WIDE = false, class NB>
 __device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, const int4* smat, bool valid, uint32_t p,
                                                uint32_t row, uint32_t sub, const Flags<DBG>& f) {
   const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
@@ -1838,20 +1847,20 @@ __device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, cons
         vj = make_int2(pq.x - clampi(so.x, pq.x - vmax, pq.x + vmax), pq.y - clampi(so.y, pq.y - vmax, pq.y + vmax));
       }
       const int2 dv = pdelta(vj, vi, f);
-      ax = wadd(ax, mulfc<16>(mulf<12>(dv.x, wk, f), cij, -XS_TERM, XS_TERM, f));
-      ay = wadd(ay, mulfc<16>(mulf<12>(dv.y, wk, f), cij, -XS_TERM, XS_TERM, f));
+      ax = wadd(ax, mulwc<WIDE, 16>(mulf<12>(dv.x, wk, f), cij, -XS_TERM, XS_TERM, f));
+      ay = wadd(ay, mulwc<WIDE, 16>(mulf<12>(dv.y, wk, f), cij, -XS_TERM, XS_TERM, f));
     }
     sx = wadd(sx, mulf<16>(mulf<26>(wg.y, d.x, f), rx.y, f));
     sy = wadd(sy, mulf<16>(mulf<26>(wg.y, d.y, f), rx.y, f));
     {
       int32_t cij = mat_mix(mi.y, mj.y);
-      int32_t wk = mulf<16>(W, cij, f);
+      int32_t wk = mulw<WIDE, 16>(W, cij, f);
       int32_t dT = clampi(sub_sat(rx.z, Ti, f), -DT_CLAMP, DT_CLAMP);
-      hq = wadd(hq, mulfc<12>(dT, wk, -HT_TERM, HT_TERM, f));
+      hq = wadd(hq, mulwc<WIDE, 12>(dT, wk, -HT_TERM, HT_TERM, f));
       if (((uint32_t)o.w & INFO_MAT) != m) {
         int32_t spend = mj.w != CORR_NEVER ? mi.z : 0;
         int32_t str = wadd(mj.z, spend);
-        if (str != 0) hc = wadd(hc, mulfc<12>(W, str, 0, CORR_TERM, f));
+        if (str != 0) hc = wadd(hc, mulwc<WIDE, 12>(W, str, 0, CORR_TERM, f));
       }
     }
   }
@@ -1876,7 +1885,7 @@ __device__ __forceinline__ void post1_particle(const Bufs& b, const NB& nb, cons
   if (doX) vo = make_int2(add_sat(vi.x, shr_rne<8>(ax), f), add_sat(vi.y, shr_rne<8>(ay), f));
   *reinterpret_cast<int4*>(w) = make_int4(pi.x, pi.y, vo.x, vo.y);
 }
-template <bool DBG, int L>
+template <bool DBG, int L, bool WIDE>
 __global__ void __launch_bounds__(256, 4) k_post1(Bufs b) {
   Flags<DBG> f{b.dbg};
   __shared__ int4 smat[MAT_MAX];
@@ -1887,7 +1896,7 @@ __global__ void __launch_bounds__(256, 4) k_post1(Bufs b) {
   const NbrGlobal nb{b.PL, b.NBR, b.nbrStride};
   for (uint32_t p = gtid() / L;; p += G) {
     if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
-    post1_particle<DBG, L>(b, nb, smat, p < nAct, p, p < nAct ? p : 0u, sub, f);
+    post1_particle<DBG, L, WIDE>(b, nb, smat, p < nAct, p, p < nAct ? p : 0u, sub, f);
   }
 }
 
@@ -2164,7 +2173,7 @@ __device__ __forceinline__ void post2_mats(const Bufs& b, int4* smat) {
 }
 // surfaceTension's sums of one particle (a warp calls it together); `act`:
 // it is a fluid particle.
-template <bool DBG, int L, class NB>
+template <bool DBG, int L, bool WIDE = false, class NB>
 __device__ __forceinline__ int2 post2_sums(const Bufs& b, const NB& nb, const int4* smat, bool valid, uint32_t p,
                                            uint32_t row, uint32_t sub, bool& act, const Flags<DBG>& f) {
   const int4 me = valid ? b.PL[p] : make_int4(0, 0, 0, (int32_t)INFO_BOUNDARY);
@@ -2199,25 +2208,25 @@ __device__ __forceinline__ int2 post2_sums(const Bufs& b, const NB& nb, const in
     if (id < 0) continue;
     const int2 ca = nb.ca(b, id);
     if (is_wall(o.w)) {
-      ax = wsub(ax, mulfc<8>(mulf<22>(ca.y, d.x, f), mi.z, -ST_TERM, ST_TERM, f));
-      ay = wsub(ay, mulfc<8>(mulf<22>(ca.y, d.y, f), mi.z, -ST_TERM, ST_TERM, f));
+      ax = wsub(ax, mulwc<WIDE, 8>(mulf<22>(ca.y, d.x, f), mi.z, -ST_TERM, ST_TERM, f));
+      ay = wsub(ay, mulwc<WIDE, 8>(mulf<22>(ca.y, d.y, f), mi.z, -ST_TERM, ST_TERM, f));
       continue;
     }
     const int32_t K = sym_k(rhoi, nq.z, b.rcp, f);
     const int4 mj = smat[(uint32_t)o.w & INFO_MAT];
     const int32_t gCoh = mat_mix(mi.x, mj.x);
     const int32_t gCur = mat_mix(mi.y, mj.y);
-    const int32_t hx = mulf<16>(mulf<22>(ca.x, d.x, f), gCoh, f);
-    const int32_t hy = mulf<16>(mulf<22>(ca.x, d.y, f), gCoh, f);
+    const int32_t hx = mulw<WIDE, 16>(mulf<22>(ca.x, d.x, f), gCoh, f);
+    const int32_t hy = mulw<WIDE, 16>(mulf<22>(ca.x, d.y, f), gCoh, f);
     const int2 dn = pdelta(make_int2(nqi.x, nqi.y), make_int2(nq.x, nq.y), f);
-    const int32_t cx = mulf<16>(dn.x, gCur, f), cy = mulf<16>(dn.y, gCur, f);
-    if constexpr (DBG) {
+    const int32_t cx = mulw<WIDE, 16>(dn.x, gCur, f), cy = mulw<WIDE, 16>(dn.y, gCur, f);
+    if constexpr (DBG || WIDE) {
       const int32_t fx = add_sat(neg_sat(hx, f), neg_sat(cx, f), f), fy = add_sat(neg_sat(hy, f), neg_sat(cy, f), f);
       ax = wadd(ax, mulc<8>(fx, K, -ST_TERM, ST_TERM, f));
       ay = wadd(ay, mulc<8>(fy, K, -ST_TERM, ST_TERM, f));
     } else {
-      // |h| < 2^19.1 and |c| < 2^20 (rows_in_range), K <= 2^18: the product's
-      // shift fits i32
+      // |h| <= 2^20 - 8 and |c| <= 1048064 (rows_in_range), K <= 2^18: the
+      // shifted product is below 2146951168, which fits i32 by 0.02 %
       ax = wadd(ax, mulfc<8>(-hx - cx, K, -ST_TERM, ST_TERM, f));
       ay = wadd(ay, mulfc<8>(-hy - cy, K, -ST_TERM, ST_TERM, f));
     }
@@ -2243,7 +2252,7 @@ __device__ __forceinline__ void post2_finish(const Bufs& b, const ScenePar& S, u
 // Six CTAs an SM (40 registers): us at 262 k / 757 k / 1 M particles with five 84 /
 // 195 / 217, six 78 / 176 / 214, seven 82 / 190 / 245 (spills). The digest's
 // registers make that five.
-template <bool DBG, bool HASH, int L>
+template <bool DBG, bool HASH, int L, bool WIDE>
 __global__ void __launch_bounds__(256, HASH ? 5 : 6) k_post2(Bufs b, int formFlags) {
   Flags<DBG> f{b.dbg};
   __shared__ int4 smat[MAT_MAX];
@@ -2258,7 +2267,7 @@ __global__ void __launch_bounds__(256, HASH ? 5 : 6) k_post2(Bufs b, int formFla
     if (__shfl_sync(0xffffffffu, p, 0) >= nAct) break;  // warp-uniform exit
     const bool valid = p < nAct;
     bool act;
-    const int2 a2 = post2_sums<DBG, L>(b, nb, smat, valid, p, valid ? p : 0u, sub, act, f);
+    const int2 a2 = post2_sums<DBG, L, WIDE>(b, nb, smat, valid, p, valid ? p : 0u, sub, act, f);
     const bool lead = valid && sub == 0;
     uint32_t scene = 0, idx = 0;
     int32_t w8[8];
