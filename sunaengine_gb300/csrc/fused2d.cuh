@@ -16,7 +16,8 @@
 //     ranges the list build needs are in shared memory). Arrival order inside
 //     a cell is whatever the count's atomics gave; each particle then ranks
 //     itself among its cell's slots, which puts the cell into ascending slot
-//     order, the canonical order the radix sort of the large path gives;
+//     order, the canonical order the radix sort of the large path gives (cells
+//     of hundreds are put in order by a whole CTA, see rank_pile);
 //   * the last CTA to finish folds the chain.
 //
 // The sums are those of the per-phase kernels (the same device functions), so
@@ -35,6 +36,7 @@ namespace d2 {
 
 constexpr uint32_t FU_ROW = 52;  // words per list row: 8 lanes of 4 rows, or 4 of 8, fall on different banks
 constexpr uint32_t FU_OWN_BYTES = 16 + 8 + 4 + 4 + 4 * FU_ROW;
+constexpr uint32_t FU_TAIL_WORDS = 2 + FU_ROW;  // of these, what nothing uses before the owned share is known
 
 struct FusedPar {
   uint32_t iters, friction, bonds, seal, chain;
@@ -108,6 +110,31 @@ __device__ __forceinline__ int2 solveB_owned(const Bufs& b, const NbrOwned& nb, 
   return make_int2(gsum<L>(dpx), gsum<L>(dpy));
 }
 
+// The pred box of cell k, [lo, hi) in sorted space, by the whole CTA.
+__device__ __forceinline__ void pile_box(const Bufs& b, uint32_t k, uint32_t lo, uint32_t hi, uint32_t* ws) {
+  int32_t* m = reinterpret_cast<int32_t*>(ws);
+  if (threadIdx.x < 4u) m[threadIdx.x] = threadIdx.x < 2u ? INT32_MAX : INT32_MIN;
+  __syncthreads();
+  int4 box = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
+  for (uint32_t q = lo + threadIdx.x; q < hi; q += FU_T) {
+    const int2 pq = ld_pred(b.PL, q);
+    box = make_int4(min(box.x, pq.x), min(box.y, pq.y), max(box.z, pq.x), max(box.w, pq.y));
+  }
+  box.x = __reduce_min_sync(0xffffffffu, box.x);
+  box.y = __reduce_min_sync(0xffffffffu, box.y);
+  box.z = __reduce_max_sync(0xffffffffu, box.z);
+  box.w = __reduce_max_sync(0xffffffffu, box.w);
+  if ((threadIdx.x & 31u) == 0u) {
+    atomicMin(m, box.x);
+    atomicMin(m + 1, box.y);
+    atomicMax(m + 2, box.z);
+    atomicMax(m + 3, box.w);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0u) b.CB[k] = make_int4(m[0], m[1], m[2], m[3]);
+  __syncthreads();
+}
+
 // L lanes share a particle's list in the sweeps over every owned particle, LC
 // in the colour passes (a quarter of the particles each). RIG: the world has
 // rigid bodies. A body's passes run on one CTA (the bodies dealt round), between
@@ -125,7 +152,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   uint32_t* pOf = X + P.xWords;                                 // [ownCap] sorted index
   uint32_t* word = pOf + P.ownCap;                              // [ownCap] NBRN words
   uint32_t* rows = word + P.ownCap;                             // [ownCap][FU_ROW]
-  __shared__ uint32_t ws[64];
+  __shared__ uint32_t ws[64], mask[FU_T / 32];
   __shared__ int4 smat1[MAT_MAX], smat2[MAT_MAX];
   __shared__ int2 scol[MAT_MAX];  // {eps, dpMax}
   __shared__ bool sfric[MAT_MAX];  // the row rubs or bonds
@@ -186,17 +213,33 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   // ---- cell ranges (every CTA its own copy), slots to their cells
   for (uint32_t k = tid; k < K; k += FU_T) X[k] = __ldcg(P.count + k);
   __syncthreads();
-  const bool crowded = cta_scan(X, K, ws) > CELL_BIG;
+  const uint32_t most = cta_scan(X, K, ws);
+  const bool crowded = most > CELL_BIG, piled = most > CELL_PILE;
+  // this thread's cell of those the CTA looks after (one at most: the cells' words
+  // fit shared memory, so no CTA of 50 or more has over FU_T) is a pile
+  const auto pileHere = [&]() {
+    const uint32_t k = tid * G + cta;
+    return k < K && X[k + 1] - X[k] > CELL_PILE;
+  };
   for (uint32_t k = cta * FU_T + tid; k <= K; k += G * FU_T) b.cellStart[k] = X[k];
   if (on) P.tmp[X[key] + arrival] = slot;
   if (!grid_wait(P.bar, target)) return;
 
   // ---- canonical order inside the cell, working set into sorted space
   for (uint32_t k = cta * FU_T + tid; k < K; k += G * FU_T) P.count[k] = 0u;
+  if (piled) {
+    each_pile(pileHere(), mask, [&](uint32_t t) {
+      const uint32_t k = t * G + cta;
+      rank_pile(P.tmp, X[k], X[k + 1], (P.slots + 31u) / 32u, pOf, P.ownCap * FU_TAIL_WORDS, ws);
+    });
+    if (!grid_wait(P.bar, target)) return;
+  }
   if (on) {
     const uint32_t lo = X[key], hi = X[key + 1];
     uint32_t p = lo;
-    for (uint32_t q = lo; q < hi; ++q) p += P.tmp[q] < slot ? 1u : 0u;
+    if (hi - lo > CELL_PILE) p = P.tmp[lo + arrival] & ~RANKED;
+    else
+      for (uint32_t q = lo; q < hi; ++q) p += P.tmp[q] < slot ? 1u : 0u;
     const int4 r = make_int4(pred.x, pred.y, 0, (int32_t)info);
     b.PL[p] = r;
     if (info & INFO_BOUNDARY) b.PL2[p] = r;
@@ -246,7 +289,7 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
   if (crowded) {
     for (uint32_t k = (tid >> 5) * G + cta; k < K; k += G * (FU_T / 32)) {
       const uint32_t lo = X[k], hi = X[k + 1];
-      if (hi - lo <= CELL_BIG) continue;
+      if (hi - lo <= CELL_BIG || hi - lo > CELL_PILE) continue;
       int4 box = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
       for (uint32_t q = lo + lane; q < hi; q += 32) {
         const int2 pq = ld_pred(b.PL, q);
@@ -258,6 +301,11 @@ __global__ void __launch_bounds__(FU_T, 1) k_substep_fused(Bufs b, FusedPar P) {
       box.w = __reduce_max_sync(0xffffffffu, box.w);
       if (lane == 0) b.CB[k] = box;
     }
+    if (piled)
+      each_pile(pileHere(), mask, [&](uint32_t t) {
+        const uint32_t k = t * G + cta;
+        pile_box(b, k, X[k], X[k + 1], ws);
+      });
     if (!grid_wait(P.bar, target)) return;
   }
   __syncthreads();

@@ -25,6 +25,7 @@ namespace d3 {
 
 constexpr uint32_t F3_ROW = 52;  // words per list row (see FU_ROW)
 constexpr uint32_t F3_OWN_BYTES = 16 + 4 + 4 + 4 * F3_ROW;
+constexpr uint32_t F3_TAIL_WORDS = 2 + F3_ROW;  // of these, what nothing uses before the owned share is known
 constexpr uint32_t F3_MAX_GRID = 256;  // CTAs whose totals a CTA keeps
 constexpr int F3_B = 3;                // neighbours' records in flight
 
@@ -66,7 +67,9 @@ __device__ __forceinline__ uint32_t nbr_rows(const Bufs3& b, bool valid, uint32_
       m[0] = cand_row<4>(b.QC, b.PW, base, lo, hi, s, me);
       if (base + 32u < hi) m[1] = cand_row<4>(b.QC, b.PW, base + 32u, lo, hi, s, me);
       mine = (uint32_t)(__popc(m[0]) + __popc(m[1]));
-      for (uint32_t c = base + 64u; c < hi; c += 32u) mine += (uint32_t)__popc(cand_row<4>(b.QC, b.PW, c, lo, hi, s, me));
+      // (past MAXNBR the count no longer matters)
+      for (uint32_t c = base + 64u; c < hi && mine < MAXNBR; c += 32u)
+        mine += (uint32_t)__popc(cand_row<4>(b.QC, b.PW, c, lo, hi, s, me));
     }
     uint32_t inc = mine;
 #pragma unroll
@@ -99,7 +102,7 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   int32_t* lamS = reinterpret_cast<int32_t*>(spg + PLANE_N);   // [ownCap]
   uint32_t* cntS = reinterpret_cast<uint32_t*>(lamS + P.ownCap);  // [ownCap]
   uint32_t* rows = cntS + P.ownCap;                            // [ownCap][F3_ROW]
-  __shared__ uint32_t ws[64], X[FU_T + 1], bases[F3_MAX_GRID + 1];
+  __shared__ uint32_t ws[64], mask[FU_T / 32], X[FU_T + 1], bases[F3_MAX_GRID + 1];
   __shared__ uint32_t dsacc[8], dsscene, lastCta;
   const Flags<false> f{b.dbg};
   const uint32_t tid = threadIdx.x, lane = tid & 31u, G = gridDim.x, cta = blockIdx.x;
@@ -130,28 +133,39 @@ __global__ void __launch_bounds__(FU_T, 1) k3_substep_fused(Bufs3 b, Fused3Par P
   const uint32_t c0 = min(cta * P.slice, K), cn = min(P.slice, K - c0);
   if (tid < cn) X[tid] = __ldcg(P.count + c0 + tid);
   __syncthreads();
-  cta_scan(X, cn, ws);
+  const uint32_t most = cta_scan(X, cn, ws);
   if (tid < cn) P.local[c0 + tid] = X[tid];
-  if (tid == 0) P.totals[cta] = X[cn];
+  if (tid == 0) P.totals[cta] = X[cn] | (most > CELL_PILE ? RANKED : 0u);
   if (!grid_wait(P.bar, target)) return;
 
   // ---- every slice's base; slots to their cells
-  if (tid < G) bases[tid] = __ldcg(P.totals + tid);
-  __syncthreads();
+  const uint32_t total = tid < G ? __ldcg(P.totals + tid) : 0u;
+  if (tid < G) bases[tid] = total & ~RANKED;
+  const bool piled = __syncthreads_or((int)(total & RANKED)) != 0;  // some slice has a pile
   cta_scan(bases, G, ws);
   if (tid < cn) {
     b.cellStart[c0 + tid] = bases[cta] + X[tid];
     P.count[c0 + tid] = 0u;
   }
   if (cta == 0 && tid == 0) b.cellStart[K] = bases[G];
-  if (on) P.tmp[bases[key / P.slice] + __ldcg(P.local + key) + arrival] = slot;
+  const uint32_t place = on ? bases[key / P.slice] + __ldcg(P.local + key) + arrival : 0u;
+  if (on) P.tmp[place] = slot;
   if (!grid_wait(P.bar, target)) return;
 
   // ---- canonical order inside the cell, working set into sorted space
+  if (piled) {
+    each_pile(tid < cn && X[tid + 1] - X[tid] > CELL_PILE, mask, [&](uint32_t t) {
+      rank_pile(P.tmp, bases[cta] + X[t], bases[cta] + X[t + 1], (P.slots + 31u) / 32u,
+                reinterpret_cast<uint32_t*>(lamS), P.ownCap * F3_TAIL_WORDS, ws);
+    });
+    if (!grid_wait(P.bar, target)) return;
+  }
   if (on) {
     const uint32_t lo = b.cellStart[key], hi = b.cellStart[key + 1];
     uint32_t p = lo;
-    for (uint32_t q = lo; q < hi; ++q) p += P.tmp[q] < slot ? 1u : 0u;
+    if (hi - lo > CELL_PILE) p = P.tmp[place] & ~RANKED;
+    else
+      for (uint32_t q = lo; q < hi; ++q) p += P.tmp[q] < slot ? 1u : 0u;
     b.PW[p] = pr;
     b.QC[p] = cand_code(pr);
     b.inv[slot] = p;
