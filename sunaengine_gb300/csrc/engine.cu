@@ -455,7 +455,7 @@ struct World {
                     b.sslot, b.cellStart, recBuf, b.QC, b.RX, b.NQ, b.POS, b.SCN, b.DP, b.HEAT, b.CORR, b.NBR,
                     b.NBRL, b.NBRN, (void*)b.tiles, b.TR, b.OVF, b.CB,
                     (void*)b.luts, (void*)b.WG, (void*)b.CA, (void*)b.mats, (void*)b.rcp,
-                    b.scenes, b.world, b.acc, b.accLast, b.chain, b.dbg, b.err, b.work, tmpK, tmpV, hist,
+                    b.scenes, b.world, b.acc, b.chain, b.dbg, b.err, b.work, tmpK, tmpV, hist,
                     hits, accTmp, devEv, devEp, boxChunks, upl, uplRes, barBuf, fuBar, fuCount, eraseBuf, initPos};
     for (void* p : ptrs)
       if (p) cudaFree(p);
@@ -545,7 +545,6 @@ struct World {
     b.scenes = dalloc<ScenePar>(scenesCap, err);
     b.world = dalloc<WorldPar>(1, err);
     b.acc = dalloc<uint32_t>((size_t)scenesCap * 8, err);
-    b.accLast = dalloc<uint32_t>((size_t)scenesCap * 8, err);
     b.chain = dalloc<uint32_t>((size_t)scenesCap * 8, err);
     if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)scenesCap * 64 + 4, cudaHostAllocMapped), "mirror") ||
         !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
@@ -965,7 +964,6 @@ struct World {
     if (!reset_chain(s)) return false;
     uint32_t zero8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     cudaMemcpyAsync(b.acc + s * 8, zero8, 32, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(b.accLast + s * 8, zero8, 32, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b.dbg, 0, 64, st);
     cudaMemsetAsync(b.err, 0, 16, st);
     freshScene = s;
@@ -1652,7 +1650,7 @@ struct World {
     return true;
   }
 
-  // accFresh: the last substep's digest (kept by the fold in accLast) is the
+  // accFresh: the last substep's digest (kept by the fold in the mirror) is the
   // digest of the current state, so digest() needs no hashing pass. Any call
   // that changes a scene's state outside a substep clears it.
   bool accFresh = false;

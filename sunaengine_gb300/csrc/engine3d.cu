@@ -161,7 +161,7 @@ struct Engine3 {
     if (graph) cudaGraphDestroy(graph);
     void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.QC, b.NBR,
                     b.NBRN, (void*)b.WG, (void*)b.PG, (void*)b.mats, (void*)b.rcp, b.scenes, b.world, b.acc,
-                    b.accLast, b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes, fuWords, fuCount, fuLocal};
+                    b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes, fuWords, fuCount, fuLocal};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     if (mirror) cudaFreeHost(mirror);
@@ -232,7 +232,6 @@ struct Engine3 {
     b.scenes = dalloc3<Scene3>(maxScenes, err);
     b.world = dalloc3<World3>(1, err);
     b.acc = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
-    b.accLast = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
     b.chain = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
     b.dbg = dalloc3<uint32_t>(16, err);
     tmpK = dalloc3<uint32_t>(C, err);

@@ -190,7 +190,6 @@ struct Bufs {
   ScenePar* scenes;
   WorldPar* world;
   uint32_t* acc;        // [S * 8]
-  uint32_t* accLast;    // [S * 8]
   uint32_t* mirror;     // [S * 16] {digest, chain} of the last substep, in host memory
   uint32_t* chain;      // [S * 8]
   uint32_t* dbg;        // [16]
@@ -2330,7 +2329,6 @@ __device__ __forceinline__ void fold_scene(const Bufs& b, uint32_t s, bool doCha
     for (int j = 0; j < 8; ++j) next[j] = mm_step(b.chain[s * 8 + j], a[j] ^ rotl32(a[(j + 1) & 7], 7));
     for (int j = 0; j < 8; ++j) {
       b.chain[s * 8 + j] = next[j];
-      b.accLast[s * 8 + j] = a[j];
       b.acc[s * 8 + j] = 0;
       b.mirror[s * 16 + j] = a[j];
       b.mirror[s * 16 + 8 + j] = next[j];

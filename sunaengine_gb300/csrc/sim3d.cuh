@@ -126,7 +126,7 @@ struct Bufs3 {
   const uint16_t* rcp;
   Scene3* scenes;
   World3* world;
-  uint32_t *acc, *accLast, *chain, *dbg;
+  uint32_t *acc, *chain, *dbg;
   uint32_t* mirror;   // [S * 16] {digest, chain} of the last substep, in host memory
 };
 
@@ -752,7 +752,6 @@ __device__ __forceinline__ void fold_scene3(const Bufs3& b, uint32_t s, bool doC
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     b.chain[s * 8 + j] = nx[j];
-    b.accLast[s * 8 + j] = a[j];
     b.acc[s * 8 + j] = 0u;
     b.mirror[s * 16 + j] = a[j];
     b.mirror[s * 16 + 8 + j] = nx[j];
