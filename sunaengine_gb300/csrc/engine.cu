@@ -16,6 +16,7 @@
 
 #include "../../include/suna.h"
 #include "ckptpool.h"
+#include "hostwords.cuh"
 #include "radix.cuh"
 #include "fused2d.cuh"
 #include <cmath>
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(256) k_rows_load(const uint2* __restrict__ cop
 }
 
 template <typename T>
-T* dalloc(size_t count, std::string& err) {
+T* dalloc(size_t count, std::string& err, bool wait = true) {
   if (count == 0) count = 1;
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, count * sizeof(T));
@@ -363,9 +364,10 @@ T* dalloc(size_t count, std::string& err) {
     return nullptr;
   }
   // The zeroing runs on the legacy default stream, which does not order with
-  // the engine's non-blocking stream: finish it before anything is queued there.
+  // the engine's non-blocking stream: finish it before anything is queued there
+  // (`wait` false: the caller does).
   cudaMemset(p, 0, count * sizeof(T));
-  cudaDeviceSynchronize();
+  if (wait) cudaDeviceSynchronize();
   return static_cast<T*>(p);
 }
 
@@ -459,7 +461,7 @@ struct World {
                     hits, accTmp, devEv, devEp, boxChunks, upl, uplRes, barBuf, fuBar, fuCount, eraseBuf, initPos};
     for (void* p : ptrs)
       if (p) cudaFree(p);
-    if (mirror) cudaFreeHost(mirror);
+    hostWords.release();
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (evFork) cudaEventDestroy(evFork);
@@ -513,62 +515,63 @@ struct World {
     cudaEventCreateWithFlags(&evFork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&evJoin, cudaEventDisableTiming);
     size_t C = capSlots;
-    b.state = dalloc<int32_t>(C * 8, err);
-    b.stacc = dalloc<int2>(C, err);
-    b.predSlot = dalloc<int2>(C, err);
-    b.sceneOf = dalloc<uint32_t>(C, err);
-    b.keys = dalloc<uint32_t>(C, err);
-    b.inv = dalloc<uint32_t>(C, err);
-    b.bond = dalloc<uint32_t>(C * BOND_CAP, err);
-    b.bondCand = dalloc<uint32_t>(C * BOND_CAP, err);
-    b.skey = dalloc<uint32_t>(C, err);
-    b.sslot = dalloc<uint32_t>(C, err);
-    recBuf = b.PL = dalloc<int4>(2 * C, err);
+    // (the zeroings are waited for once, at the end: a wait for each was a third of a
+    // small engine's creation)
+    b.state = dalloc<int32_t>(C * 8, err, false);
+    b.stacc = dalloc<int2>(C, err, false);
+    b.predSlot = dalloc<int2>(C, err, false);
+    b.sceneOf = dalloc<uint32_t>(C, err, false);
+    b.keys = dalloc<uint32_t>(C, err, false);
+    b.inv = dalloc<uint32_t>(C, err, false);
+    b.bond = dalloc<uint32_t>(C * BOND_CAP, err, false);
+    b.bondCand = dalloc<uint32_t>(C * BOND_CAP, err, false);
+    b.skey = dalloc<uint32_t>(C, err, false);
+    b.sslot = dalloc<uint32_t>(C, err, false);
+    recBuf = b.PL = dalloc<int4>(2 * C, err, false);
     b.PL2 = b.PL + C;
-    b.RX = dalloc<int4>(C, err);
-    b.NQ = dalloc<int4>(C, err);
-    b.QC = dalloc<uint32_t>((C + 7) & ~(size_t)3, err);
-    b.POS = dalloc<int2>(C, err);
-    b.SCN = dalloc<uint32_t>(C, err);
-    b.DP = dalloc<int2>(C, err);
-    b.HEAT = dalloc<int32_t>(C, err);
-    b.CORR = dalloc<int32_t>(C, err);
-    b.NBR = dalloc<uint32_t>(C * MAXNBR, err);
-    b.NBRL = dalloc<uint16_t>(C * MAXNBR, err);
-    b.NBRN = dalloc<uint32_t>(C, err);
+    b.RX = dalloc<int4>(C, err, false);
+    b.NQ = dalloc<int4>(C, err, false);
+    b.QC = dalloc<uint32_t>((C + 7) & ~(size_t)3, err, false);
+    b.POS = dalloc<int2>(C, err, false);
+    b.SCN = dalloc<uint32_t>(C, err, false);
+    b.DP = dalloc<int2>(C, err, false);
+    b.HEAT = dalloc<int32_t>(C, err, false);
+    b.CORR = dalloc<int32_t>(C, err, false);
+    b.NBR = dalloc<uint32_t>(C * MAXNBR, err, false);
+    b.NBRL = dalloc<uint16_t>(C * MAXNBR, err, false);
+    b.NBRN = dalloc<uint32_t>(C, err, false);
     b.nbrStride = (uint32_t)C;
-    uint16_t* drcp = dalloc<uint16_t>(32768, err);
-    int32_t* dl = dalloc<int32_t>(LUT_WORDS, err);
-    int2* dwg = dalloc<int2>(TN, err);
-    int2* dca = dalloc<int2>(TN, err);
-    int32_t* dm = dalloc<int32_t>(MAT_MAX * MAT_WORDS, err);
-    b.scenes = dalloc<ScenePar>(scenesCap, err);
-    b.world = dalloc<WorldPar>(1, err);
-    b.acc = dalloc<uint32_t>((size_t)scenesCap * 8, err);
-    b.chain = dalloc<uint32_t>((size_t)scenesCap * 8, err);
-    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)scenesCap * 64 + 4, cudaHostAllocMapped), "mirror") ||
-        !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
-      return false;
-    std::memset(mirror, 0, (size_t)scenesCap * 64 + 4);
+    uint16_t* drcp = dalloc<uint16_t>(32768, err, false);
+    int32_t* dl = dalloc<int32_t>(LUT_WORDS, err, false);
+    int2* dwg = dalloc<int2>(TN, err, false);
+    int2* dca = dalloc<int2>(TN, err, false);
+    int32_t* dm = dalloc<int32_t>(MAT_MAX * MAT_WORDS, err, false);
+    b.scenes = dalloc<ScenePar>(scenesCap, err, false);
+    b.world = dalloc<WorldPar>(1, err, false);
+    b.acc = dalloc<uint32_t>((size_t)scenesCap * 8, err, false);
+    b.chain = dalloc<uint32_t>((size_t)scenesCap * 8, err, false);
+    if (!cuda_ok(hostWords.alloc((size_t)scenesCap * 16 + 1), "mirror")) return false;
+    mirror = hostWords.host;
+    b.mirror = hostWords.dev;
     gaveUp = mirror + (size_t)scenesCap * 16;
     gaveUpDev = b.mirror + (size_t)scenesCap * 16;
-    b.dbg = dalloc<uint32_t>(16, err);
-    b.err = dalloc<uint32_t>(4, err);
-    b.work = dalloc<uint32_t>(8, err);
-    barBuf = dalloc<uint32_t>(1, err);
-    fuBar = dalloc<uint32_t>(2, err);
-    tmpK = dalloc<uint32_t>(C, err);
-    tmpV = dalloc<uint32_t>(C, err);
-    hist = dalloc<uint32_t>(radix::hist_words((uint32_t)C), err);
-    hits = dalloc<uint32_t>(1, err);
-    accTmp = dalloc<uint32_t>((size_t)scenesCap * 8, err);
-    boxChunks = dalloc<BoxChunk>(C / CELL_CHUNK + C / CELL_BIG + 1, err);
-    devEp = dalloc<EvPar>(scenesCap, err);
-    b.rbody = dalloc<int32_t>((size_t)RG_MAX_BODIES * RG_BODY_WORDS, err);
-    b.rdrv = dalloc<int32_t>((size_t)RG_MAX_BODIES * RG_DRIVER_WORDS, err);
-    b.rest = dalloc<int2>(C, err);
-    b.rmark = dalloc<uint32_t>(C, err);
-    int32_t* dcos = dalloc<int32_t>(RG_COS_N, err);
+    b.dbg = dalloc<uint32_t>(16, err, false);
+    b.err = dalloc<uint32_t>(4, err, false);
+    b.work = dalloc<uint32_t>(8, err, false);
+    barBuf = dalloc<uint32_t>(1, err, false);
+    fuBar = dalloc<uint32_t>(2, err, false);
+    tmpK = dalloc<uint32_t>(C, err, false);
+    tmpV = dalloc<uint32_t>(C, err, false);
+    hist = dalloc<uint32_t>(radix::hist_words((uint32_t)C), err, false);
+    hits = dalloc<uint32_t>(1, err, false);
+    accTmp = dalloc<uint32_t>((size_t)scenesCap * 8, err, false);
+    boxChunks = dalloc<BoxChunk>(C / CELL_CHUNK + C / CELL_BIG + 1, err, false);
+    devEp = dalloc<EvPar>(scenesCap, err, false);
+    b.rbody = dalloc<int32_t>((size_t)RG_MAX_BODIES * RG_BODY_WORDS, err, false);
+    b.rdrv = dalloc<int32_t>((size_t)RG_MAX_BODIES * RG_DRIVER_WORDS, err, false);
+    b.rest = dalloc<int2>(C, err, false);
+    b.rmark = dalloc<uint32_t>(C, err, false);
+    int32_t* dcos = dalloc<int32_t>(RG_COS_N, err, false);
     if (!err.empty()) return false;
     {
       int32_t T[RG_COS_N];
@@ -1673,6 +1676,7 @@ struct World {
   // mirror: the last fold's digests and chains in host memory, where the fold
   // wrote them (a read of 32 bytes from the device costs 12 us). chainFresh: no
   // chain has been written from elsewhere since.
+  HostWords hostWords;
   uint32_t* mirror = nullptr;
   bool chainFresh = false;
   bool read_chain(uint32_t s, uint32_t out[8]) {

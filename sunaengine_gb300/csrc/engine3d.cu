@@ -16,6 +16,7 @@
 
 #include "../../include/suna.h"
 #include "ckptpool.h"
+#include "hostwords.cuh"
 #include "radix.cuh"
 #include "fused3d.cuh"
 
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(256) k3_bond_flags(const uint32_t* __restrict_
 }
 
 template <typename T>
-T* dalloc3(size_t count, std::string& err) {
+T* dalloc3(size_t count, std::string& err, bool wait = true) {
   if (count == 0) count = 1;
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, count * sizeof(T));
@@ -84,9 +85,10 @@ T* dalloc3(size_t count, std::string& err) {
     return nullptr;
   }
   // The zeroing runs on the legacy default stream, which does not order with
-  // the engine's non-blocking stream: finish it before anything is queued there.
+  // the engine's non-blocking stream: finish it before anything is queued there
+  // (`wait` false: the caller does).
   cudaMemset(p, 0, count * sizeof(T));
-  cudaDeviceSynchronize();
+  if (wait) cudaDeviceSynchronize();
   return static_cast<T*>(p);
 }
 
@@ -159,12 +161,12 @@ struct Engine3 {
   ~Engine3() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
-    void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.QC, b.NBR,
+    void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.NBR,
                     b.NBRN, (void*)b.WG, (void*)b.PG, (void*)b.mats, (void*)b.rcp, b.scenes, b.world, b.acc,
-                    b.chain, b.dbg, tmpK, tmpV, hist, accTmp, fnvBuf, ballDev, upl, uplRes, fuWords, fuCount, fuLocal};
+                    b.chain, b.dbg, scratch, ballDev, upl, uplRes};
     for (void* p : ptrs)
       if (p) cudaFree(p);
-    if (mirror) cudaFreeHost(mirror);
+    hostWords.release();
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (evFork) cudaEventDestroy(evFork);
@@ -207,45 +209,51 @@ struct Engine3 {
     cudaEventCreateWithFlags(&evFork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&evJoin, cudaEventDisableTiming);
     size_t C = capSlots;
-    b.state = dalloc3<int32_t>(C * 8, err);
-    b.sceneOf = dalloc3<uint32_t>(C, err);
-    b.bond = dalloc3<uint32_t>(C * BOND3_WORDS, err);
-    b.bflag = dalloc3<uint32_t>(C, err);
-    b.inv = dalloc3<uint32_t>(C, err);
-    b.PRS = dalloc3<int4>(C, err);
-    b.keys = dalloc3<uint32_t>(C, err);
-    b.skey = dalloc3<uint32_t>(C, err);
-    b.sslot = dalloc3<uint32_t>(C, err);
-    b.cellStart = dalloc3<uint32_t>((size_t)maxCells + 2, err);
-    b.PW = dalloc3<int4>(C, err);
-    b.PW2 = dalloc3<int4>(C, err);
-    b.PL = dalloc3<int4>(C, err);
-    b.QC = dalloc3<uint32_t>((C + 7) & ~(size_t)3, err);
-    b.NBR = dalloc3<uint32_t>(C * MAXNBR, err);
-    b.NBRN = dalloc3<uint32_t>(C, err);
+    // (the zeroings are waited for once, at the end)
+    b.state = dalloc3<int32_t>(C * 8, err, false);
+    b.sceneOf = dalloc3<uint32_t>(C, err, false);
+    b.bond = dalloc3<uint32_t>(C * BOND3_WORDS, err, false);
+    b.bflag = dalloc3<uint32_t>(C, err, false);
+    b.inv = dalloc3<uint32_t>(C, err, false);
+    b.PRS = dalloc3<int4>(C, err, false);
+    b.keys = dalloc3<uint32_t>(C, err, false);
+    b.skey = dalloc3<uint32_t>(C, err, false);
+    b.sslot = dalloc3<uint32_t>(C, err, false);
+    b.cellStart = dalloc3<uint32_t>((size_t)maxCells + 2, err, false);
+    b.PW = dalloc3<int4>(C, err, false);
+    b.PW2 = dalloc3<int4>(C, err, false);
+    b.PL = dalloc3<int4>(C, err, false);
+    b.NBR = dalloc3<uint32_t>(C * MAXNBR, err, false);
+    b.NBRN = dalloc3<uint32_t>(C, err, false);
     b.nbrStride = (uint32_t)C;
-    int2* dwg = dalloc3<int2>(LUT_N, err);
-    int2* dpg = dalloc3<int2>(PLANE_N, err);
-    int32_t* dm = dalloc3<int32_t>(4 * matCount, err);
-    uint16_t* drcp = dalloc3<uint16_t>(32768, err);
-    ballDev = dalloc3<int2>((size_t)maxScenes * BALL_N, err);
-    b.scenes = dalloc3<Scene3>(maxScenes, err);
-    b.world = dalloc3<World3>(1, err);
-    b.acc = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
-    b.chain = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
-    b.dbg = dalloc3<uint32_t>(16, err);
-    tmpK = dalloc3<uint32_t>(C, err);
-    tmpV = dalloc3<uint32_t>(C, err);
-    hist = dalloc3<uint32_t>(radix::hist_words((uint32_t)C), err);
-    accTmp = dalloc3<uint32_t>((size_t)maxScenes * 8, err);
-    fnvBuf = dalloc3<uint32_t>(256, err);
-    fuWords = dalloc3<uint32_t>(4 + F3_MAX_GRID, err);
-    fuCount = dalloc3<uint32_t>((size_t)maxCells + 2, err);
-    fuLocal = dalloc3<uint32_t>((size_t)maxCells + 2, err);
-    if (!cuda_ok(cudaHostAlloc((void**)&mirror, (size_t)maxScenes * 64 + 4, cudaHostAllocMapped), "mirror") ||
-        !cuda_ok(cudaHostGetDevicePointer((void**)&b.mirror, mirror, 0), "mirror"))
-      return false;
-    memset(mirror, 0, (size_t)maxScenes * 64 + 4);
+    int2* dwg = dalloc3<int2>(LUT_N, err, false);
+    int2* dpg = dalloc3<int2>(PLANE_N, err, false);
+    int32_t* dm = dalloc3<int32_t>(4 * matCount, err, false);
+    uint16_t* drcp = dalloc3<uint16_t>(32768, err, false);
+    ballDev = dalloc3<int2>((size_t)maxScenes * BALL_N, err, false);
+    b.scenes = dalloc3<Scene3>(maxScenes, err, false);
+    b.world = dalloc3<World3>(1, err, false);
+    b.acc = dalloc3<uint32_t>((size_t)maxScenes * 8, err, false);
+    b.chain = dalloc3<uint32_t>((size_t)maxScenes * 8, err, false);
+    b.dbg = dalloc3<uint32_t>(16, err, false);
+    // the words that live inside one call or substep, as one allocation (each of its
+    // own costs about 60 us to make and give back)
+    {
+      uint32_t** parts[] = {&b.QC, &tmpK, &tmpV, &hist, &accTmp, &fnvBuf, &fuWords, &fuCount, &fuLocal};
+      const size_t words[] = {C + 4, C, C, radix::hist_words((uint32_t)C), (size_t)maxScenes * 8, 256, 4 + F3_MAX_GRID,
+                              (size_t)maxCells + 2, (size_t)maxCells + 2};
+      size_t total = 0;
+      for (size_t w : words) total += (w + 63) & ~(size_t)63;
+      scratch = dalloc3<uint32_t>(total, err, false);
+      uint32_t* at = scratch;
+      for (int k = 0; scratch && k < 9; ++k) {
+        *parts[k] = at;
+        at += (words[k] + 63) & ~(size_t)63;
+      }
+    }
+    if (!cuda_ok(hostWords.alloc((size_t)maxScenes * 16 + 1), "mirror")) return false;
+    mirror = hostWords.host;
+    b.mirror = hostWords.dev;
     gaveUp = mirror + (size_t)maxScenes * 16;
     gaveUpDev = b.mirror + (size_t)maxScenes * 16;
     if (!err.empty()) return false;
@@ -440,6 +448,7 @@ struct Engine3 {
     launchesPerSubstep = (uint64_t)launches;
   }
   // ---- the fused substep of small worlds (fused3d.cuh) ----
+  uint32_t* scratch = nullptr;  // one allocation: QC to fuLocal
   uint32_t* fuWords = nullptr;  // barrier words (2), error word, pad, slice totals
   uint32_t *fuCount = nullptr, *fuLocal = nullptr;  // [maxCells + 2] each
   uint32_t *gaveUp = nullptr, *gaveUpDev = nullptr;  // ERR_BARRIER for the host (mapped)
@@ -840,6 +849,7 @@ struct Engine3 {
   // mirror: the last fold's digests and chains in host memory, where the fold
   // wrote them (a read of 32 bytes from the device costs 12 us). chainFresh: no
   // chain has been written from elsewhere since.
+  sn::HostWords hostWords;
   uint32_t* mirror = nullptr;
   bool chainFresh = false;
   bool digest(uint32_t s, uint32_t out[8]) {
