@@ -217,7 +217,9 @@ int sn_last_timing(sn_engine* e, float* ms, uint64_t* launches);
  * predict, grid sort, cell ranges + gather, neighbour lists, then per solver
  * iteration (solveA, the four colour passes, friction), then
  * finalize/xsph/normals/conduct, surface tension/thermal/formation/digest,
- * chain fold. The substeps are real: the scene advances by `reps`. */
+ * chain fold. The substeps are real: the scene advances by `reps`. They take the
+ * per-phase launches always: a world small enough that sn_step advances it by one
+ * launch a substep spends about half their sum there. */
 int sn_profile_substep(sn_engine* e, uint32_t reps, float* ms, uint32_t max_phases, uint32_t* n_phases);
 int sn_batch_profile_substep(sn_batch* b, uint32_t reps, float* ms, uint32_t max_phases, uint32_t* n_phases);
 
@@ -348,7 +350,9 @@ int sn_lanes(sn_engine* e, uint32_t out[5]);
 int sn_batch_lanes(sn_batch* b, uint32_t out[5]);
 /* Pin {solveA, colours, post1, post2, neighbour lists} lanes (each 1, 2, 4 or
  * 8), e.g. a split tuned on another run of the same workload; afterwards
- * neither the size rule nor sn_autotune changes them. */
+ * neither the size rule nor sn_autotune changes them. The lanes are the per-phase
+ * launches': a world small enough for one launch a substep keeps that (opts.lanes
+ * != 0 keeps it off). */
 int sn_set_lanes(sn_engine* e, const uint32_t lanes[5]);
 int sn_batch_set_lanes(sn_batch* b, const uint32_t lanes[5]);
 /* (no counterpart) The sorted-space layout and gather kernels of solveA and
@@ -506,11 +510,12 @@ int sn3_debug_counters(sn3_engine* e, uint32_t out[16]);
 int sn3_sync(sn3_engine* e);
 int sn3_get_info(sn3_engine* e, uint32_t scene, sn3_info* out);
 int sn3_last_timing(sn3_engine* e, float* ms, uint64_t* launches);
-/* Phases: predict, sort, cellstart+gather, neighbour lists, then density and
- * solve per iteration, integrate(+hash), fold. */
 /* sn_set_barrier_wait for the 3D engine (a keyframe with its chain restores a
  * scene too). */
 int sn3_set_barrier_wait(sn3_engine* e, uint64_t cycles);
+/* Phases: predict, sort, cellstart+gather, neighbour lists, then density and
+ * solve per iteration, integrate(+hash), fold; of the per-phase launches, which
+ * a small world (sn_step's one launch a substep) takes here alone. */
 int sn3_profile_substep(sn3_engine* e, uint32_t reps, float* ms, uint32_t max_phases, uint32_t* n_phases);
 
 /* ---- device checkpoints ------------------------------------------------------

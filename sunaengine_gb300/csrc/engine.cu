@@ -1189,7 +1189,7 @@ struct World {
   // slot a thread, the cell ranges, the owned particles' lists).
   bool fused_fits() const {
     const uint64_t G = (uint64_t)numSMs;
-    return !debug && tablesOk && rowsOk && !staged && !persistent && autoLanes && hw.nAct > 0 &&
+    return !debug && tablesOk && rowsOk && !staged && !persistent && lanesOverride == 0 && hw.nAct > 0 &&
            slots_used() <= G * FU_T && fused_own() <= fused_own_cap();
   }
   template <int L, int LC, bool RIG>
