@@ -17,6 +17,7 @@
 #include "../../include/suna.h"
 #include "ckptpool.h"
 #include "hostwords.cuh"
+#include "inflight.cuh"
 #include "radix.cuh"
 #include "fused2d.cuh"
 #include <cmath>
@@ -426,9 +427,9 @@ struct World {
   bool eventsDirty = false, anyEvents = false;
   bool hasFriction = false, hasBonds = false, hasSeal = false;
   bool layoutDirty = true;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t gexec = nullptr;
-  bool graphValid = false;
+  SubstepGraph graphs[2];  // of the per-phase launches and of the fused one
+  void drop_graphs() { graphs[0].valid = graphs[1].valid = false; }
+  InFlight inFlight;
   bool useGraph = true;
   int lanesOverride = 0;  // 0 = choose from the active particle count
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -449,10 +450,15 @@ struct World {
     if (e == cudaSuccess) return true;
     return fail("%s: %s", what, cudaGetErrorString(e));
   }
+  bool wait(const char* what) {
+    if (!cuda_ok(cudaStreamSynchronize(st), what)) return false;
+    inFlight.idle();
+    return true;
+  }
 
   ~World() {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (graph) cudaGraphDestroy(graph);
+    inFlight.leave();
+    for (SubstepGraph& g : graphs) g.release();
     void* ptrs[] = {b.state, b.stacc, b.predSlot, b.sceneOf, b.keys, b.inv, b.bond, b.bondCand, b.skey,
                     b.sslot, b.cellStart, recBuf, b.QC, b.RX, b.NQ, b.POS, b.SCN, b.DP, b.HEAT, b.CORR, b.NBR,
                     b.NBRL, b.NBRN, (void*)b.tiles, b.TR, b.OVF, b.CB,
@@ -512,6 +518,7 @@ struct World {
     if (!cuda_ok(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking), "stream")) return false;
     cudaEventCreate(&ev0);
     cudaEventCreate(&ev1);
+    inFlight.join(device, ev1);
     cudaEventCreateWithFlags(&evFork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&evJoin, cudaEventDisableTiming);
     size_t C = capSlots;
@@ -639,7 +646,7 @@ struct World {
       if (row(m)[M_bondK] != 0) bo = true;
       if (seal_row(m)) se = true;
     }
-    if (fr != hasFriction || bo != hasBonds || se != hasSeal) graphValid = false;
+    if (fr != hasFriction || bo != hasBonds || se != hasSeal) drop_graphs();
     hasFriction = fr;
     hasBonds = bo;
     hasSeal = se;
@@ -657,7 +664,7 @@ struct World {
     std::vector<ScenePar> dev(maxScenes);
     if (!cuda_ok(cudaMemcpyAsync(dev.data(), b.scenes, sizeof(ScenePar) * maxScenes, cudaMemcpyDeviceToHost, st),
                  "clocks") ||
-        !cuda_ok(cudaStreamSynchronize(st), "clocks"))
+        !wait("clocks"))
       return false;
     for (uint32_t s = 0; s < maxScenes; ++s) {
       if (s == freshScene || !sh[s].used || !sh[s].loaded) continue;
@@ -750,11 +757,11 @@ struct World {
     hw.hasFriction = hasFriction;
     hw.hasBonds = hasBonds;
     layoutDirty = false;
-    graphValid = false;
+    drop_graphs();
     bool ok = cuda_ok(cudaMemcpyAsync(b.world, &hw, sizeof(hw), cudaMemcpyHostToDevice, st), "world") &&
               cuda_ok(cudaMemcpyAsync(b.scenes, hpar.data(), sizeof(ScenePar) * maxScenes,
                                       cudaMemcpyHostToDevice, st), "scenes");
-    return ok && cuda_ok(cudaStreamSynchronize(st), "relayout");
+    return ok && wait("relayout");
   }
 
   // Grow the key- and tile-sized buffers to the layout's needs (cell starts
@@ -801,7 +808,7 @@ struct World {
     if (!cuda_ok(cudaMemcpyAsync(hpar.data(), b.scenes, sizeof(ScenePar) * maxScenes, cudaMemcpyDeviceToHost, st),
                  "pull"))
       return false;
-    if (!cuda_ok(cudaStreamSynchronize(st), "pull")) return false;
+    if (!wait("pull")) return false;
     if (gave_up()) return fail("%s", BARRIER_TEXT);
     paramsStale = false;
     return true;
@@ -866,7 +873,7 @@ struct World {
     if (n) k_load_check<<<grid_for(n), 256, 0, st>>>(upl, sc->n, sc->n_fluid, matCount, present, T, uplRes);
     uint32_t res[4];
     cudaMemcpyAsync(res, uplRes, 16, cudaMemcpyDeviceToHost, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "load check")) return false;
+    if (!wait("load check")) return false;
     if (res[0] != 0xffffffffu) {
       if (!validate_particle(sc, res[0])) return false;
       return fail("particle %u failed the device check but passes the host check", res[0]);
@@ -1140,34 +1147,33 @@ struct World {
     return !gave_up() && !sh[s].lost ? true : fail("%s: %s", what, BARRIER_TEXT);
   }
   bool sync() {
-    return cuda_ok(cudaStreamSynchronize(st), "sync") && (!gave_up() ? true : fail("sync: %s", BARRIER_TEXT));
+    return wait("sync") && (!gave_up() ? true : fail("sync: %s", BARRIER_TEXT));
   }
-  bool synced(uint32_t s, const char* what) { return cuda_ok(cudaStreamSynchronize(st), what) && whole(s, what); }
+  bool synced(uint32_t s, const char* what) { return wait(what) && whole(s, what); }
   // The world can be stepped again; the scenes that were in it are lost.
   bool recover() {
-    if (!cuda_ok(cudaStreamSynchronize(st), "recover")) return false;
+    if (!wait("recover")) return false;
     accFresh = chainFresh = sortedFresh = false;
     for (SceneHost& h : sh) h.lost = h.lost || (h.used && h.loaded);
     const bool ok = cuda_ok(cudaMemsetAsync(b.err, 0, 16, st), "recover") &&
                     cuda_ok(cudaMemsetAsync(fuBar, 0, 8, st), "recover") &&
                     (!fuCount || cuda_ok(cudaMemsetAsync(fuCount, 0, (size_t)keyCap * 4, st), "recover")) &&
                     cuda_ok(cudaMemsetAsync(b.acc, 0, (size_t)maxScenes * 32, st), "recover") &&
-                    cuda_ok(cudaStreamSynchronize(st), "recover");
+                    wait("recover");
     if (ok) *(volatile uint32_t*)gaveUp = 0u;
     return ok;
   }
   bool set_barrier_wait(uint64_t cycles) {
     if (cycles > 1ull << 40) return fail("a barrier waits 2^40 cycles at most");
     waitLimit = (long long)cycles;
-    graphValid = false;
+    drop_graphs();
     return true;
   }
   uint32_t* fuCount = nullptr;  // [keyCap] cell counts, zero between launches
   // the tables, and every row, lie in the ranges the release kernels are built
   // for; else the debug kernels run, or for rows alone the WIDE post sweeps
   bool tablesOk = true, rowsOk = true;
-  bool graphFused = false;      // what the captured graph launches, and the
-  uint32_t graphOwn = 0;        // particles a CTA it was sized for
+  uint32_t graphOwn = 0;        // particles a CTA the captured launch was sized for
   // One past the last slot that can hold an active particle.
   uint32_t slots_used() const {
     uint32_t e = 0;
@@ -1409,7 +1415,7 @@ struct World {
     setLanes = true;
     autoLanes = false;
     lanesTuned = true;
-    graphValid = false;
+    drop_graphs();
     return true;
   }
 
@@ -1480,7 +1486,7 @@ struct World {
         launch_one();
         int used2 = npev;
         pev = nullptr;
-        ok = cuda_ok(cudaStreamSynchronize(st), "tune");
+        ok = wait("tune");
         for (auto& s2 : sh)
           if (s2.used && s2.loaded) s2.substeps += 1;
         paramsStale = true;
@@ -1512,7 +1518,7 @@ struct World {
     lanesCfg = LaneCfg{pick[0], pick[1], pick[2], pick[3], pick[4]};
     lanesTuned = true;
     tunedAtN = hw.nAct;
-    graphValid = false;
+    drop_graphs();
     if (used) *used = n;
     return ok;
   }
@@ -1545,7 +1551,7 @@ struct World {
       ep[s].end = (uint32_t)all.size();
     }
     // the graph holds the impulse kernel only while some event is ahead
-    if (anyEvents != had) graphValid = false;
+    if (anyEvents != had) drop_graphs();
     if (!anyEvents) {
       eventsDirty = false;
       return true;
@@ -1563,7 +1569,7 @@ struct World {
     if (!cuda_ok(cudaMemcpyAsync(devEp, ep.data(), ep.size() * sizeof(EvPar), cudaMemcpyHostToDevice, st), "ep"))
       return false;
     eventsDirty = false;
-    if (devEv != before) graphValid = false;
+    if (devEv != before) drop_graphs();
     return true;
   }
 
@@ -1577,29 +1583,29 @@ struct World {
     if (gave_up()) return fail("step: %s", BARRIER_TEXT);
     if (layoutDirty && !relayout()) return false;
     if (eventsDirty && !upload_events()) return false;
-    const bool fused = fused_fits();
-    if (fused != graphFused || (fused && fused_own() > graphOwn)) graphValid = false;
-    if (useGraph && !graphValid) {
+    const bool fused = fused_fits() && !inFlight.crowded();
+    if (fused && fused_own() > graphOwn) graphs[1].valid = false;
+    SubstepGraph& g = graphs[fused ? 1 : 0];
+    if (useGraph && !g.valid) {
       cudaGraph_t fresh = nullptr;
       if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture")) return false;
       launch_one(fused);
-      graphFused = fused;
       if (!cuda_ok(cudaStreamEndCapture(st, &fresh), "endCapture")) return false;
-      if (!cuda_ok(refresh_graph(fresh, graph, gexec), "instantiate")) return false;
-      graphValid = true;
+      if (!cuda_ok(g.refresh(fresh, launchesPerSubstep), "instantiate")) return false;
     }
+    inFlight.begin();
     cudaEventRecord(ev0, st);
-    for (uint32_t i = 0; i < count; ++i) {
-      if (useGraph) {
-        if (!cuda_ok(cudaGraphLaunch(gexec, st), "graphLaunch")) return false;
-      } else {
-        launch_one(fused);
-      }
+    bool ok = true;
+    for (uint32_t i = 0; ok && i < count; ++i) {
+      if (useGraph) ok = cuda_ok(cudaGraphLaunch(g.exec, st), "graphLaunch");
+      else launch_one(fused);
     }
     cudaEventRecord(ev1, st);
+    inFlight.queued();
+    if (!ok) return false;
     for (auto& s : sh)
       if (s.used && s.loaded) s.substeps += count;
-    lastLaunches = launchesPerSubstep * count;
+    lastLaunches = (useGraph ? g.launches : launchesPerSubstep) * count;
     paramsStale = true;
     accFresh = chainFresh = chainOn;
     sortedFresh = true;
@@ -1628,7 +1634,7 @@ struct World {
       launch_one();
       used = npev;
       pev = nullptr;
-      if (!cuda_ok(cudaStreamSynchronize(st), "profile")) return false;
+      if (!wait("profile")) return false;
       for (int k = 0; k + 1 < used; ++k) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, evs[k], evs[k + 1]);
@@ -1649,6 +1655,7 @@ struct World {
 
   bool timing(float* ms) {
     if (!cuda_ok(cudaEventSynchronize(ev1), "timing")) return false;
+    inFlight.idle();
     cudaEventElapsedTime(ms, ev0, ev1);
     return true;
   }
@@ -1687,7 +1694,7 @@ struct World {
   }
   bool read_words(const void* dsrc, void* out, size_t bytes) {
     cudaMemcpyAsync(out, dsrc, bytes, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "read");
+    return wait("read");
   }
   // words that scene s's substeps write
   bool read_words(uint32_t s, const void* dsrc, void* out, size_t bytes) {
@@ -1786,7 +1793,7 @@ struct World {
     hw.hasBonds = hasBonds;
     ok = push_scene(s) &&
          cuda_ok(cudaMemcpyAsync(b.world, &hw, sizeof(hw), cudaMemcpyHostToDevice, st), "world") &&
-         cuda_ok(cudaStreamSynchronize(st), "spawn");
+         wait("spawn");
     if (nOut) *nOut = newN;
     return ok;
   }
@@ -1827,7 +1834,7 @@ struct World {
     hpar[s].n = h.n;
     bool ok = push_scene(s) &&
               cuda_ok(cudaMemcpyAsync(b.world, &hw, sizeof(hw), cudaMemcpyHostToDevice, st), "world") &&
-              cuda_ok(cudaStreamSynchronize(st), "walls");
+              wait("walls");
     if (onOut) *onOut = h.wallsOn;
     return ok;
   }
@@ -1842,13 +1849,13 @@ struct World {
     bool ok = cuda_ok(cudaMemcpyAsync(b.state + off * 8, state, n * 32, cudaMemcpyHostToDevice, st), "state");
     if (scratch) ok = ok && cuda_ok(cudaMemcpyAsync(b.stacc + off, scratch, n * 8, cudaMemcpyHostToDevice, st), "stacc");
     else ok = ok && cuda_ok(cudaMemsetAsync(b.stacc + off, 0, n * 8, st), "stacc");
-    return ok && cuda_ok(cudaStreamSynchronize(st), "write_state");
+    return ok && wait("write_state");
   }
 
   bool check() {
     uint32_t e[4] = {0, 0, 0, 0};
     cudaMemcpyAsync(e, b.err, 16, cudaMemcpyDeviceToHost, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "checkErrors")) return false;
+    if (!wait("checkErrors")) return false;
     if (!cuda_ok(cudaGetLastError(), "checkErrors")) return false;
     if (e[0] & ERR_UNSUPPORTED_ROW)
       return fail("a transition produced a seal-class row (containment is not built); results past it are not "
@@ -1876,7 +1883,7 @@ struct World {
     cudaMemcpyAsync(b.bond + (size_t)h.slotBase * BOND_CAP, in, (size_t)h.nFluid * BOND_CAP * 4,
                     cudaMemcpyHostToDevice, st);
     mark_bonds_live();
-    return cuda_ok(cudaStreamSynchronize(st), "writeBonds");
+    return wait("writeBonds");
   }
 
   // eraseWhere's compaction (src/engine.js:6460-6650) for scene s: keep[i]
@@ -1911,7 +1918,7 @@ struct World {
     hpar[s].bondDirty = 1;
     layoutDirty = true;
     eventsDirty = true;
-    return push_scene(s) && cuda_ok(cudaStreamSynchronize(st), "erase");
+    return push_scene(s) && wait("erase");
   }
 
   // eraseWhere's compaction on the device (a scene without bodies): survivor
@@ -1956,7 +1963,7 @@ struct World {
     }
     uint32_t kept = 0;
     ok = ok && cuda_ok(cudaMemcpyAsync(&kept, dKept, 4, cudaMemcpyDeviceToHost, st), "erase") &&
-         cuda_ok(cudaStreamSynchronize(st), "erase");
+         wait("erase");
     if (!ok) return false;
     if (kept != newF) return fail("erase: the device kept %u particles, the host %u", kept, newF);
     return true;
@@ -1973,7 +1980,7 @@ struct World {
     cudaMemcpyAsync(scIn.data(), b.stacc + h.slotBase, scIn.size() * 4, cudaMemcpyDeviceToHost, st);
     if (oldF)
       cudaMemcpyAsync(bIn.data(), b.bond + (size_t)h.slotBase * BOND_CAP, bIn.size() * 4, cudaMemcpyDeviceToHost, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "erase read")) return false;
+    if (!wait("erase read")) return false;
     const uint32_t newN = newF + nB;
     std::vector<int32_t> stOut((size_t)newN * 8), scOut((size_t)newN * 2);
     auto mv = [&](uint32_t src, uint32_t dst) {
@@ -2004,7 +2011,7 @@ struct World {
       cudaMemcpyAsync(b.bond + (size_t)h.slotBase * BOND_CAP, bOut.data(), bOut.size() * 4, cudaMemcpyHostToDevice, st);
       mark_bonds_live();
     }
-    return cuda_ok(cudaStreamSynchronize(st), "erase write");
+    return wait("erase write");
   }
 
   // ---- §20 rigid bodies: host side (src/engine.js:2050-2150, 5452-5811) ----------
@@ -2106,15 +2113,15 @@ struct World {
     if (bodies.empty()) return true;
     return cuda_ok(cudaMemcpyAsync(rec.data(), b.rbody, rec.size() * 4, cudaMemcpyDeviceToHost, st), "bodies") &&
            cuda_ok(cudaMemcpyAsync(drv.data(), b.rdrv, drv.size() * 4, cudaMemcpyDeviceToHost, st), "drivers") &&
-           cuda_ok(cudaStreamSynchronize(st), "bodies");
+           wait("bodies");
   }
   bool write_records(const std::vector<int32_t>& rec, const std::vector<int32_t>& drv) {
-    graphValid = false;
+    drop_graphs();
     hw.nBodies = (uint32_t)bodies.size();
     if (bodies.empty()) return true;
     return cuda_ok(cudaMemcpyAsync(b.rbody, rec.data(), rec.size() * 4, cudaMemcpyHostToDevice, st), "bodies") &&
            cuda_ok(cudaMemcpyAsync(b.rdrv, drv.data(), drv.size() * 4, cudaMemcpyHostToDevice, st), "drivers") &&
-           cuda_ok(cudaStreamSynchronize(st), "bodies");
+           wait("bodies");
   }
   // Replace scene s's bodies by (recS, drvS, descS), keeping every other
   // scene's records as they are on the device.
@@ -2147,7 +2154,7 @@ struct World {
     if (h.n == 0) return true;
     return cuda_ok(cudaMemcpyAsync(stw.data(), b.state + (size_t)h.slotBase * 8, stw.size() * 4,
                                    cudaMemcpyDeviceToHost, st), "state") &&
-           cuda_ok(cudaStreamSynchronize(st), "state");
+           wait("state");
   }
   bool write_scene_state(uint32_t s, const std::vector<int32_t>& stw, uint32_t lo, uint32_t hi) {
     const SceneHost& h = sh[s];
@@ -2156,7 +2163,7 @@ struct World {
     sortedFresh = false;
     return cuda_ok(cudaMemcpyAsync(b.state + ((size_t)h.slotBase + lo) * 8, stw.data() + (size_t)lo * 8,
                                    ((size_t)hi - lo + 1) * 32, cudaMemcpyHostToDevice, st), "state") &&
-           cuda_ok(cudaStreamSynchronize(st), "state");
+           wait("state");
   }
   bool mark_bond_dirty(uint32_t s) {
     if (!pull_params()) return false;
@@ -2228,7 +2235,7 @@ struct World {
       for (size_t q = k0; q < k1; ++q) win[q - k0] = make_int2(ox[q], oy[q]);
       if (!cuda_ok(cudaMemcpyAsync(b.rest + base + members[k0], win.data(), win.size() * sizeof(int2),
                                    cudaMemcpyHostToDevice, st), "rest") ||
-          !cuda_ok(cudaStreamSynchronize(st), "rest"))
+          !wait("rest"))
         return false;
       k0 = k1;
     }
@@ -2238,13 +2245,13 @@ struct World {
     bh.axis = axis; bh.user = user;
     bodies.push_back(bh);
     *idx = (int32_t)scene_bodies(s) - 1;
-    graphValid = false;
+    drop_graphs();
     hw.nBodies = (uint32_t)bodies.size();
     return cuda_ok(cudaMemcpyAsync(b.rbody + (size_t)at * RG_BODY_WORDS, rec.data(), RG_BODY_WORDS * 4,
                                    cudaMemcpyHostToDevice, st), "body") &&
            cuda_ok(cudaMemcpyAsync(b.rdrv + (size_t)at * RG_DRIVER_WORDS, drv.data(), RG_DRIVER_WORDS * 4,
                                    cudaMemcpyHostToDevice, st), "driver") &&
-           cuda_ok(cudaStreamSynchronize(st), "body");
+           wait("body");
   }
 
   // makeRigidBody / makeAxisBody (src/engine.js:5722-5780)
@@ -2366,7 +2373,7 @@ struct World {
     const int32_t v = on ? 1 : 0;
     return cuda_ok(cudaMemcpyAsync(b.rbody + (size_t)wi * RG_BODY_WORDS + RB_USER, &v, 4, cudaMemcpyHostToDevice, st),
                    "user") &&
-           cuda_ok(cudaStreamSynchronize(st), "user");
+           wait("user");
   }
   // A body's driver sidecar (the words `_serviceBodyConstraints` uploads,
   // src/engine.js:5370-5412): mask of RD_HAS_* bits and the nine values.
@@ -2378,7 +2385,7 @@ struct World {
     for (int q = 0; q < 9; ++q) d[1 + q] = values ? values[q] : 0;
     return cuda_ok(cudaMemcpyAsync(b.rdrv + (size_t)wi * RG_DRIVER_WORDS, d, sizeof(d), cudaMemcpyHostToDevice, st),
                    "driver") &&
-           cuda_ok(cudaStreamSynchronize(st), "driver");
+           wait("driver");
   }
   bool clear_body_drivers(uint32_t s) {
     const int32_t z[RG_DRIVER_WORDS] = {0};
@@ -2386,7 +2393,7 @@ struct World {
       if (bodies[i].scene == s &&
           !cuda_ok(cudaMemcpyAsync(b.rdrv + i * RG_DRIVER_WORDS, z, sizeof(z), cudaMemcpyHostToDevice, st), "driver"))
         return false;
-    return cuda_ok(cudaStreamSynchronize(st), "driver");
+    return wait("driver");
   }
   // dragGrab's rigid branch (src/engine.js:6111-6140)
   bool drag_body(uint32_t s, uint32_t tag, int32_t tx, int32_t ty, int32_t vx, int32_t vy, bool* moved) {
@@ -2403,7 +2410,7 @@ struct World {
       *moved = true;
       return cuda_ok(cudaMemcpyAsync(b.rbody + i * RG_BODY_WORDS + RB_CX, w4, 16, cudaMemcpyHostToDevice, st), "drag") &&
              cuda_ok(cudaMemcpyAsync(b.rbody + i * RG_BODY_WORDS + RB_RESX, z4, 16, cudaMemcpyHostToDevice, st), "drag") &&
-             cuda_ok(cudaStreamSynchronize(st), "drag");
+             wait("drag");
     }
     return true;
   }
@@ -2439,7 +2446,7 @@ struct World {
     std::vector<int32_t> rec(records, records + (size_t)nb * RG_BODY_WORDS), drv((size_t)nb * RG_DRIVER_WORDS, 0);
     if (rest && restWords &&
         (!cuda_ok(cudaMemcpyAsync(b.rest + sh[s].slotBase, rest, restWords * 4, cudaMemcpyHostToDevice, st), "rest") ||
-         !cuda_ok(cudaStreamSynchronize(st), "rest")))
+         !wait("rest")))
       return false;
     return bodies_from_records(s, rec, drv);
   }
@@ -2468,7 +2475,7 @@ struct World {
     if (h.nFluid &&
         (!cuda_ok(cudaMemcpyAsync(restIn.data(), b.rest + h.slotBase, (size_t)h.nFluid * 8, cudaMemcpyDeviceToHost, st),
                   "rest") ||
-         !cuda_ok(cudaStreamSynchronize(st), "rest")))
+         !wait("rest")))
       return false;
     const uint32_t newF = (uint32_t)surv.size();
     for (uint32_t k = 0; k < (uint32_t)h.cap; ++k) restOut[k] = make_int2(0, 0);
@@ -2507,7 +2514,7 @@ struct World {
     }
     if (!cuda_ok(cudaMemcpyAsync(b.rest + h.slotBase, restOut.data(), (size_t)h.cap * 8, cudaMemcpyHostToDevice, st),
                  "rest") ||
-        !cuda_ok(cudaStreamSynchronize(st), "rest"))
+        !wait("rest"))
       return false;
     return replace_scene_bodies(s, recS, drvS, descS);
   }
@@ -2519,12 +2526,12 @@ struct World {
   bool upload_mats(uint32_t lo, uint32_t hi) {
     rowsOk = rows_in_range(hmats, matCount);
     if (hi <= lo) return true;
-    graphValid = false;
+    drop_graphs();
     accFresh = false;
     return cuda_ok(cudaMemcpyAsync(const_cast<int32_t*>(b.mats) + (size_t)lo * MAT_WORDS, hmats + (size_t)lo * MAT_WORDS,
                                    sizeof(int32_t) * MAT_WORDS * (hi - lo), cudaMemcpyHostToDevice, st),
                    "mats") &&
-           cuda_ok(cudaStreamSynchronize(st), "mats");
+           wait("mats");
   }
   int32_t scaled_grav(int32_t g) const { return (int32_t)idiv_rne64((int64_t)g * gravQ, 65536); }
   bool set_material(uint32_t rowId, const int32_t* w) {
@@ -2592,7 +2599,7 @@ struct World {
   bool put_word(uint32_t s, size_t off, uint32_t v) {
     return cuda_ok(cudaMemcpyAsync(reinterpret_cast<char*>(b.scenes + s) + off, &v, 4, cudaMemcpyHostToDevice, st),
                    "param") &&
-           cuda_ok(cudaStreamSynchronize(st), "param");
+           wait("param");
   }
   bool set_weld_hold(uint32_t s, uint32_t tag) {
     sh[s].weldHold = tag;
@@ -2659,7 +2666,7 @@ struct World {
     for (uint32_t j = 0; j < 8; ++j)
       for (int w = 0; w < 5; ++w) hpar[s].jet[j][w] = j < k ? q[j * 5 + w] : 0;
     if (nOut) *nOut = k;
-    return push_scene(s) && cuda_ok(cudaStreamSynchronize(st), "setJets");
+    return push_scene(s) && wait("setJets");
   }
 
   // Device checkpoint of scene s: [state n*8][stAcc n*2][chain 8][bond rows nFluid*48 when the
@@ -2846,7 +2853,7 @@ int sn_chain(sn_engine* e, uint32_t chain[8]) {
 }
 int sn_reset_chain(sn_engine* e) {
   if (!e) return SN_E_INVALID;
-  return rc_of(e->w, e->w.reset_chain(0) && e->w.cuda_ok(cudaStreamSynchronize(e->w.st), "reset"));
+  return rc_of(e->w, e->w.reset_chain(0) && e->w.wait("reset"));
 }
 int sn_read_state(sn_engine* e, int32_t* out, size_t words) {
   if (!e || !out) return SN_E_INVALID;
@@ -2956,7 +2963,7 @@ int sn_set_formation_clock(sn_engine* e, uint64_t clock, uint32_t dirty) {
   if (!w.pull_params()) return rc_of(w, false);
   w.hpar[0].formClock = (uint32_t)clock;
   w.hpar[0].bondDirty = dirty ? 1u : 0u;
-  return rc_of(w, w.push_scene(0) && w.cuda_ok(cudaStreamSynchronize(w.st), "clock"));
+  return rc_of(w, w.push_scene(0) && w.wait("clock"));
 }
 int sn_profile_substep(sn_engine* e, uint32_t reps, float* ms, uint32_t max_phases, uint32_t* n_phases) {
   if (!e || !ms) return SN_E_INVALID;
@@ -3066,7 +3073,7 @@ int sn_batch_write_state(sn_batch* b, uint32_t id, const int32_t* state, const i
   w.hpar[id].bondDirty = dirty ? 1u : 0u;
   w.hpar[id].substep = (uint32_t)substep_count;
   w.eventsDirty = true;
-  return rc_of(w, w.push_scene(id) && w.cuda_ok(cudaStreamSynchronize(w.st), "write"));
+  return rc_of(w, w.push_scene(id) && w.wait("write"));
 }
 int sn_begin_weld_group(sn_engine* e, uint32_t* tag) {
   if (!e) return SN_E_INVALID;
@@ -3165,13 +3172,13 @@ int sn_batch_set_staged(sn_batch* b, uint32_t on) {
 int sn_set_persistent(sn_engine* e, uint32_t on) {
   if (!e) return SN_E_INVALID;
   e->w.persistent = on != 0;
-  e->w.graphValid = false;
+  e->w.drop_graphs();
   return SN_OK;
 }
 int sn_batch_set_persistent(sn_batch* b, uint32_t on) {
   if (!b) return SN_E_INVALID;
   b->w.persistent = on != 0;
-  b->w.graphValid = false;
+  b->w.drop_graphs();
   return SN_OK;
 }
 int sn_set_barrier_wait(sn_engine* e, uint64_t cycles) {

@@ -17,6 +17,7 @@
 #include "../../include/suna.h"
 #include "ckptpool.h"
 #include "hostwords.cuh"
+#include "inflight.cuh"
 #include "radix.cuh"
 #include "fused3d.cuh"
 
@@ -135,9 +136,10 @@ struct Engine3 {
   World3 hw{};
   uint32_t *tmpK = nullptr, *tmpV = nullptr, *hist = nullptr, *accTmp = nullptr, *fnvBuf = nullptr;
   int2* ballDev = nullptr;
-  bool layoutDirty = true, graphValid = false, useGraph = true, anyStir = false;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t gexec = nullptr;
+  bool layoutDirty = true, useGraph = true, anyStir = false;
+  sn::SubstepGraph graphs[2];  // of the per-phase launches and of the fused one
+  void drop_graphs() { graphs[0].valid = graphs[1].valid = false; }
+  sn::InFlight inFlight;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   uint64_t lastLaunches = 0, launchesPerSubstep = 0;
   bool inRange = true;  // the tables lie in the ranges the release kernels are built for
@@ -157,10 +159,15 @@ struct Engine3 {
     if (e == cudaSuccess) return true;
     return fail("cuda %s: %s", what, cudaGetErrorString(e));
   }
+  bool wait(const char* what) {
+    if (!cuda_ok(cudaStreamSynchronize(st), what)) return false;
+    inFlight.idle();
+    return true;
+  }
 
   ~Engine3() {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (graph) cudaGraphDestroy(graph);
+    inFlight.leave();
+    for (sn::SubstepGraph& g : graphs) g.release();
     void* ptrs[] = {b.state, b.sceneOf, b.bond, b.bflag, b.inv, b.PRS, b.keys, b.skey, b.sslot, b.cellStart, b.PW, b.PW2, b.PL, b.NBR,
                     b.NBRN, (void*)b.WG, (void*)b.PG, (void*)b.mats, (void*)b.rcp, b.scenes, b.world, b.acc,
                     b.chain, b.dbg, scratch, ballDev, upl, uplRes};
@@ -206,6 +213,7 @@ struct Engine3 {
     if (!cuda_ok(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking), "stream")) return false;
     cudaEventCreate(&ev0);
     cudaEventCreate(&ev1);
+    inFlight.join(device, ev1);
     cudaEventCreateWithFlags(&evFork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&evJoin, cudaEventDisableTiming);
     size_t C = capSlots;
@@ -383,9 +391,9 @@ struct Engine3 {
     cudaMemcpyAsync(b.sceneOf, sceneOf.data(), sizeof(uint32_t) * sceneOf.size(), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b.scenes, hpar.data(), sizeof(Scene3) * maxScenes, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b.world, &hw, sizeof(World3), cudaMemcpyHostToDevice, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "relayout")) return false;
+    if (!wait("relayout")) return false;
     layoutDirty = false;
-    graphValid = false;
+    drop_graphs();
     return true;
   }
 
@@ -453,7 +461,6 @@ struct Engine3 {
   uint32_t *fuCount = nullptr, *fuLocal = nullptr;  // [maxCells + 2] each
   uint32_t *gaveUp = nullptr, *gaveUpDev = nullptr;  // ERR_BARRIER for the host (mapped)
   long long waitLimit = sn::BARRIER_WAIT_CYCLES;
-  bool graphFused = false;
   static constexpr uint32_t F3_SMEM = 216 * 1024;  // dynamic at most; the static arrays take about 6 KB of the 227
   static constexpr uint32_t F3_FIXED = (LUT_N + PLANE_N) * 8;
   uint32_t fused_own() const { return (hw.nAct + (uint32_t)numSMs - 1) / (uint32_t)numSMs; }
@@ -509,26 +516,26 @@ struct Engine3 {
   bool whole(uint32_t s, const char* what) {
     return !gave_up() && !sh[s].lost ? true : fail("%s: %s", what, sn::BARRIER_TEXT);
   }
-  bool synced(uint32_t s, const char* what) { return cuda_ok(cudaStreamSynchronize(st), what) && whole(s, what); }
+  bool synced(uint32_t s, const char* what) { return wait(what) && whole(s, what); }
   bool sync() {
-    return cuda_ok(cudaStreamSynchronize(st), "sync") && (!gave_up() ? true : fail("sync: %s", sn::BARRIER_TEXT));
+    return wait("sync") && (!gave_up() ? true : fail("sync: %s", sn::BARRIER_TEXT));
   }
   // The world can be stepped again; the scenes that were in it are lost.
   bool recover() {
-    if (!cuda_ok(cudaStreamSynchronize(st), "recover")) return false;
+    if (!wait("recover")) return false;
     accFresh = chainFresh = false;
     for (Scene3Host& h : sh) h.lost = h.lost || (h.used && h.loaded);
     const bool ok = cuda_ok(cudaMemsetAsync(fuWords, 0, 12, st), "recover") &&
                     cuda_ok(cudaMemsetAsync(fuCount, 0, ((size_t)maxCells + 2) * 4, st), "recover") &&
                     cuda_ok(cudaMemsetAsync(b.acc, 0, (size_t)maxScenes * 32, st), "recover") &&
-                    cuda_ok(cudaStreamSynchronize(st), "recover");
+                    wait("recover");
     if (ok) *(volatile uint32_t*)gaveUp = 0u;
     return ok;
   }
   bool set_barrier_wait(uint64_t cycles) {
     if (cycles > 1ull << 40) return fail("a barrier waits 2^40 cycles at most");
     waitLimit = (long long)cycles;
-    graphValid = false;
+    drop_graphs();
     return true;
   }
   void launch_one(bool fused = false) {
@@ -559,29 +566,28 @@ struct Engine3 {
     if (gave_up()) return fail("step: %s", sn::BARRIER_TEXT);
     if (layoutDirty && !relayout()) return false;
     if (anyStir && !upload_phase()) return false;
-    const bool fused = fused_fits();
-    if (fused != graphFused) graphValid = false;
-    if (useGraph && !graphValid) {
+    const bool fused = fused_fits() && !inFlight.crowded();
+    sn::SubstepGraph& g = graphs[fused ? 1 : 0];
+    if (useGraph && !g.valid) {
       cudaGraph_t fresh = nullptr;
       if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture")) return false;
       launch_one(fused);
-      graphFused = fused;
       if (!cuda_ok(cudaStreamEndCapture(st, &fresh), "endCapture")) return false;
-      if (!cuda_ok(sn::refresh_graph(fresh, graph, gexec), "instantiate")) return false;
-      graphValid = true;
+      if (!cuda_ok(g.refresh(fresh, launchesPerSubstep), "instantiate")) return false;
     }
+    inFlight.begin();
     cudaEventRecord(ev0, st);
-    for (uint32_t i = 0; i < count; ++i) {
-      if (useGraph) {
-        if (!cuda_ok(cudaGraphLaunch(gexec, st), "graphLaunch")) return false;
-      } else {
-        launch_one(fused);
-      }
+    bool ok = true;
+    for (uint32_t i = 0; ok && i < count; ++i) {
+      if (useGraph) ok = cuda_ok(cudaGraphLaunch(g.exec, st), "graphLaunch");
+      else launch_one(fused);
     }
     cudaEventRecord(ev1, st);
+    inFlight.queued();
+    if (!ok) return false;
     for (auto& s : sh)
       if (s.used && s.loaded) s.substeps += count;
-    lastLaunches = launchesPerSubstep * count;
+    lastLaunches = (useGraph ? g.launches : launchesPerSubstep) * count;
     accFresh = chainFresh = chainOn;
     return cuda_ok(cudaGetLastError(), "step");
   }
@@ -603,7 +609,7 @@ struct Engine3 {
       launch_one();
       used = npev;
       pev = nullptr;
-      if (!cuda_ok(cudaStreamSynchronize(st), "profile")) return false;
+      if (!wait("profile")) return false;
       for (int k = 0; k + 1 < used; ++k) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, evs[k], evs[k + 1]);
@@ -676,7 +682,7 @@ struct Engine3 {
       k3_load_check<<<grid_for(sc->n), 256, 0, st>>>(upl, sc->n, matCount, uplRes);
       uint32_t bad = 0;
       cudaMemcpyAsync(&bad, uplRes, 4, cudaMemcpyDeviceToHost, st);
-      if (!cuda_ok(cudaStreamSynchronize(st), "load check")) return false;
+      if (!wait("load check")) return false;
       if (bad != none) return fail("mat[%u] = %u outside the material table", bad, sc->mat[bad]);
       k3_load_pack<<<grid_for(sc->n), 256, 0, st>>>(upl, sc->n, sc->vel ? 1u : 0u, b.state + (size_t)h.slotBase * 8);
       if (!cuda_ok(cudaGetLastError(), "pack")) return false;
@@ -695,7 +701,7 @@ struct Engine3 {
     h.substeps = 0;
     h.loaded = true;
     layoutDirty = true;
-    bool ok = cuda_ok(cudaStreamSynchronize(st), "load");
+    bool ok = wait("load");
     if (gave_up()) ok = recover() && ok;
     h.lost = false;
     return ok;
@@ -743,7 +749,7 @@ struct Engine3 {
     if (h.n) k3_bonds_check<<<grid_for(h.n), 256, 0, st>>>(reinterpret_cast<const uint32_t*>(upl), h.n, uplRes);
     uint32_t res[2];
     cudaMemcpyAsync(res, uplRes, 8, cudaMemcpyDeviceToHost, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "bond check")) return false;
+    if (!wait("bond check")) return false;
     if (res[0] != 0xffffffffu) {
       const uint32_t i = res[0];
       const uint32_t* r = rows + (size_t)i * BOND3_WORDS;
@@ -774,7 +780,7 @@ struct Engine3 {
     h.bondK = k;
     h.bondBrk = brk;
     layoutDirty = true;
-    return cuda_ok(cudaStreamSynchronize(st), "write_bonds");
+    return wait("write_bonds");
   }
 
   bool read_bonds(uint32_t s, uint32_t* out, size_t words) {
@@ -782,12 +788,12 @@ struct Engine3 {
     const size_t need = (size_t)sh[s].n * BOND3_WORDS;
     if (!out || words < need) return fail("read_bonds needs %zu words", need);
     cudaMemcpyAsync(out, b.bond + (size_t)sh[s].slotBase * BOND3_WORDS, need * 4, cudaMemcpyDeviceToHost, st);
-    return cuda_ok(cudaStreamSynchronize(st), "read_bonds");
+    return wait("read_bonds");
   }
 
   bool remove(uint32_t s) {
     if (!check_scene(s, false)) return false;
-    if (!clear_bonds(s) || !cuda_ok(cudaStreamSynchronize(st), "remove")) return false;
+    if (!clear_bonds(s) || !wait("remove")) return false;
     sh[s] = Scene3Host{};
     layoutDirty = true;
     return true;
@@ -815,7 +821,7 @@ struct Engine3 {
       }
       cudaMemcpyAsync(b.state + (size_t)(h.slotBase + h.n) * 8, words.data(), words.size() * 4,
                       cudaMemcpyHostToDevice, st);
-      if (!cuda_ok(cudaStreamSynchronize(st), "spawn")) return false;
+      if (!wait("spawn")) return false;
       h.n += k;
       layoutDirty = true;
     }
@@ -831,7 +837,7 @@ struct Engine3 {
       std::vector<int2> tab;
       ball_tables(R, tab);
       cudaMemcpyAsync(ballDev + (size_t)s * BALL_N, tab.data(), sizeof(int2) * BALL_N, cudaMemcpyHostToDevice, st);
-      if (!cuda_ok(cudaStreamSynchronize(st), "ball")) return false;
+      if (!wait("ball")) return false;
       h.ballR = R;
     }
     h.ballOn = on != 0;
@@ -917,7 +923,7 @@ struct Engine3 {
     if (n > 0)
       cudaMemcpyAsync(b.state + (size_t)h.slotBase * 8, state, (size_t)n * 32, cudaMemcpyHostToDevice, st);
     if (chainIn) cudaMemcpyAsync(b.chain + (size_t)s * 8, chainIn, 32, cudaMemcpyHostToDevice, st);
-    if (!cuda_ok(cudaStreamSynchronize(st), "write_state")) return false;
+    if (!wait("write_state")) return false;
     if (gave_up() && !recover()) return false;
     if (chainIn) h.lost = false;  // its words, its clock and its chain are the caller's
     h.n = n;
@@ -981,6 +987,7 @@ struct Engine3 {
 
   bool timing(float* ms) {
     if (!cuda_ok(cudaEventSynchronize(ev1), "timing")) return false;
+    inFlight.idle();
     cudaEventElapsedTime(ms, ev0, ev1);
     return true;
   }
@@ -1092,7 +1099,7 @@ int sn3_write_state(sn3_engine* e, uint32_t scene, const int32_t* state, uint32_
 int sn3_debug_counters(sn3_engine* e, uint32_t out[16]) {
   if (!e || !out) return SN_E_INVALID;
   cudaMemcpyAsync(out, e->w.b.dbg, 64, cudaMemcpyDeviceToHost, e->w.st);
-  return rc3(e->w, e->w.cuda_ok(cudaStreamSynchronize(e->w.st), "debug_counters"));
+  return rc3(e->w, e->w.wait("debug_counters"));
 }
 int sn3_sync(sn3_engine* e) {
   if (!e) return SN_E_INVALID;

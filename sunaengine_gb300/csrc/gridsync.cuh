@@ -6,21 +6,38 @@
 
 namespace sn {
 
-// The captured substep graph after a change: an update of the executable graph where
-// the topology allows it (a new scene size does), a new one where it does not.
-inline cudaError_t refresh_graph(cudaGraph_t fresh, cudaGraph_t& graph, cudaGraphExec_t& exec) {
-  if (exec) {
-    cudaGraphExecUpdateResultInfo info;
-    if (cudaGraphExecUpdate(exec, fresh, &info) != cudaSuccess) {
-      cudaGetLastError();  // refused: not an error of the stream
-      cudaGraphExecDestroy(exec);
-      exec = nullptr;
-    }
+// One captured substep. After a change the executable graph is updated where the
+// topology allows it (a new scene size does), and made anew where it does not.
+struct SubstepGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  bool valid = false;
+  uint64_t launches = 0;  // of a substep
+  ~SubstepGraph() { release(); }
+  void release() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    exec = nullptr;
+    graph = nullptr;
+    valid = false;
   }
-  if (graph) cudaGraphDestroy(graph);
-  graph = fresh;
-  return exec ? cudaSuccess : cudaGraphInstantiate(&exec, graph, 0);
-}
+  cudaError_t refresh(cudaGraph_t fresh, uint64_t substepLaunches) {
+    if (exec) {
+      cudaGraphExecUpdateResultInfo info;
+      if (cudaGraphExecUpdate(exec, fresh, &info) != cudaSuccess) {
+        cudaGetLastError();  // refused: not an error of the stream
+        cudaGraphExecDestroy(exec);
+        exec = nullptr;
+      }
+    }
+    if (graph) cudaGraphDestroy(graph);
+    graph = fresh;
+    launches = substepLaunches;
+    const cudaError_t e = exec ? cudaSuccess : cudaGraphInstantiate(&exec, graph, 0);
+    valid = e == cudaSuccess;
+    return e;
+  }
+};
 
 constexpr int FU_T = 1024;  // threads of a fused substep's CTA, one CTA to an SM
 constexpr uint32_t ERR_BARRIER = 8u;
