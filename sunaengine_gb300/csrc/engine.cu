@@ -400,9 +400,8 @@ struct SceneHost {
 struct World {
   int device = 0;
   cudaStream_t st = nullptr;
-  // A side stream for work that runs beside the main chain: each colour
-  // pass's copy of the other colours forks onto it and joins before the next
-  // pass (inside the captured graph, a parallel branch).
+  // A side stream for work that runs beside the main chain: the cell ranges
+  // beside the gather (inside the captured graph, a parallel branch).
   cudaStream_t st2 = nullptr;
   cudaEvent_t evFork = nullptr, evJoin = nullptr;
   bool debug = false, chainOn = true;

@@ -23,10 +23,11 @@
 // The sums are those of the per-phase kernels (the same device functions), so
 // the results are equal word by word. Every wait is bounded (grid_wait).
 //
-// Measured (us a substep, per-phase graph -> this): 1.3 k particles 148 -> 96,
-// 4.7 k 167 -> 98, 21 k 192 -> 116, 62 k 267 -> 193, 92 k 326 -> 290. A barrier
-// costs 1.05-1.3 us and a colour pass about 2 us on its slowest CTA (two
-// dependent L2 round trips); the limit is what fits an SM (fused_fits).
+// Measured (us a substep, the per-phase graph it replaced -> this): 1.5 k particles
+// 149 -> 82, 4.1 k 167 -> 84, 13 k 167 -> 92, 42 k 219 -> 129, 61 k 256 -> 145, 93 k
+// 312 -> 208. A barrier costs 1.05-1.3 us and a colour pass about 2 us on its
+// slowest CTA (two dependent L2 round trips); the limit is what fits an SM
+// (fused_fits).
 #pragma once
 #include "gridsync.cuh"
 #include "rigid.cuh"
@@ -70,9 +71,9 @@ struct NbrOwned {
 // The sums of solveA and solveB with FU_B neighbours' records in flight at a
 // time: the list entries are at hand, so a batch costs one L2 round trip (one
 // ahead of the pair in hand, as the per-phase kernels have it, is one for every
-// neighbour but the first when a CTA has a few warps). With 16 lanes to a
-// colour's particle a substep of 4.7 k particles went from 94 to 86 us, of 40 k
-// from 145 to 128.
+// neighbour but the first when a CTA has a few warps). When they came in, with 16
+// lanes to a colour's particle, a substep of 4.7 k particles went from 94 to 86 us, of
+// 40 k from 145 to 128.
 constexpr int FU_B = 3;
 constexpr uint32_t FU_CHUNK = 16;  // particles of a colour dealt to a CTA at a time, in worlds with bodies
 template <int L>

@@ -13,9 +13,9 @@
 // The sums are the per-phase kernels' own device functions: results are equal
 // word by word. Every wait is bounded (grid_wait).
 //
-// Measured at 4 iterations (us a substep, per-phase graph -> this): 4 k particles
-// 94 -> 45, 16 k 100 -> 60, 33 k 121 -> 74, 64 k 144 -> 103, 91 k 186 -> 148, 125 k
-// 215 -> 174; the limit is what fits an SM (fused_fits).
+// Measured at 4 iterations (us a substep, the per-phase graph it replaced -> this):
+// 4 k particles 88 -> 39, 16 k 100 -> 50, 60 k 146 -> 82, 91 k 236 -> 144, 125 k 277 ->
+// 168; the limit is what fits an SM (fused_fits).
 #pragma once
 #include "gridsync.cuh"
 #include "sim3d.cuh"

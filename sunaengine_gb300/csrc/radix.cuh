@@ -204,7 +204,7 @@ inline void sort_pairs(uint32_t* keys0, uint32_t n, int keyBits, uint32_t* outKe
 constexpr int LAUNCHES_PER_PASS = 3;
 
 // Words of `hist` a sort of up to n keys needs (tile counts plus the digit totals);
-// below MAX_ITEMS a smaller sort may have more tiles, but fewer than 2 MIN_TILES.
+// below MAX_ITEMS a smaller sort may have more tiles, but at most 2 MIN_TILES.
 inline size_t hist_words(uint32_t n) {
   const uint32_t tiles = (n + TPB * items_for(n) - 1) / (TPB * items_for(n));
   return (size_t)RADIX * (std::max<uint32_t>(tiles, 2 * MIN_TILES) + 2);

@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(256) k_cellstart(Bufs b) {
 // (about 28 %) is mostly near enough to be a neighbour for sure; only the ring
 // about the kernel's edge (6 %) goes through the exact test. The list pass of
 // the 1 M scene fell from 261 to 165 us (190 with every survivor tested), a
-// 262 k one from 117 to 70, a fused 40 k world's from 30 to 12. What bounds it
-// now is issue (67 %) at 15 active lanes: a warp's cells differ in survivors.
+// 262 k one from 117 to 70. What bounds it now is issue (67 %) at 15 active
+// lanes: a warp's cells differ in survivors.
 //
 // The filter never drops a neighbour. Quantised places are clamped to the
 // scene's cells as cell_coord is, and clamping brings no two points further
@@ -1273,10 +1273,11 @@ __device__ __forceinline__ void solveB_pair(const Bufs& b, const NB& nb, int2 pi
 }
 
 // solveB_at for one particle.
-// The colour passes (NbrSplit) keep two neighbours' records in flight. More do
-// not fit 32 registers, and the pass wants all its warps: us a substep at 265 k /
-// 1 M one ahead 607 / 1337, two 600 / 1322, two or three with 6 CTAs an SM 603 /
-// 1347 and 600 / 1333, three with 5 607 / 1367.
+// The colour passes (NbrSplit) keep two neighbours' records in flight. That is a
+// word or three past 32 registers already (8 to 16 bytes of spill stores), but the
+// pass wants all its warps: us a substep at 265 k / 1 M one ahead 607 / 1337, two
+// 600 / 1322, two or three without spills and with 6 CTAs an SM 603 / 1347 and 600 /
+// 1333, three with 5 607 / 1367.
 // RIG: the warp holds a rigid member, whose own correction skips the members
 // of its body (src/sim.wgsl:1355-1358).
 struct NbrSplit;

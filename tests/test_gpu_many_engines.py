@@ -29,6 +29,7 @@ def _make(kind, i):
 
 @pytest.mark.parametrize('kind', ['2d', '3d'])
 def test_the_third_shares(kind):
+    time.sleep(0.1)
     es = [_make(kind, i) for i in range(4)]
     for e in es:
         e.step(2)
@@ -50,6 +51,7 @@ def test_the_third_shares(kind):
 
 
 def test_an_engine_nobody_waited_for_is_not_counted():
+    time.sleep(0.1)
     es = [_make('2d', i) for i in range(3)]
     for e in es[:2]:
         e.step(2)
